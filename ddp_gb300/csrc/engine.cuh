@@ -40,13 +40,17 @@ constexpr unsigned FULL = 0xffffffffu;
 
 // Control block of one search slot (global memory).  Push counters rotate
 // over 4 phases so that a counter is reset two phases before it is used
-// again, with a single barrier per phase.
+// again, with a single barrier per phase.  One phase's counters are 16
+// bytes, read together after the phase's barrier.
+struct __align__(16) PhaseWords {
+    int nq;            // pushes into near/next (or BFS frontier) this phase
+    int fq;            // pushes into far this phase
+    unsigned int mf;   // min f kept in far during a split phase
+    int err;           // ST_* raised during the phase (read after its barrier)
+};
 struct SearchCtl {
-    int nq[4];            // pushes into near/next (or BFS frontier) this phase
-    int fq[4];            // pushes into far this phase
-    unsigned int mf[4];   // min f kept in far during a split phase
-    int err[4];           // ST_* raised during the phase (read after its barrier)
-    int ck[4];            // chunks of 32 entries claimed so far in the phase
+    PhaseWords ph[4];
+    int ck[4];            // chunks claimed so far in the phase, beyond one per warp
     int touched;          // nodes whose state left the initial value
     int status;           // ST_* bits
     int iters;            // phases run
@@ -61,6 +65,8 @@ struct SearchCtl {
     int cur_ver;          // graph version of the current search (serving)
     unsigned int bar_count, bar_gen;  // grid barrier (single-query form)
     int cold_n;           // entries in the far pile's cold tier (keep mode)
+    // what CTA 0 hands back after running phases alone (run_search)
+    int loc_near, loc_far, loc_waves;
 };
 
 // Buffers of one slot.
@@ -84,6 +90,14 @@ struct CtaGroup {
     __device__ int warp() const { return threadIdx.x >> 5; }
     __device__ int nwarps() const { return blockDim.x >> 5; }
     __device__ void sync() const { __syncthreads(); }
+    template <class F>
+    __device__ void sync_fetch(F fetch) const {  // see grid_sync_fetch
+        __syncthreads();
+        if (threadIdx.x == 0) fetch();
+        __syncthreads();
+    }
+    static constexpr bool multi = false;  // more than one CTA
+    __device__ bool first_cta() const { return true; }
 };
 
 struct GridGroup {
@@ -94,6 +108,10 @@ struct GridGroup {
     __device__ int warp() const { return (blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
     __device__ int nwarps() const { return (gridDim.x * blockDim.x) >> 5; }
     __device__ void sync() const { grid_sync(bar, gridDim.x, status); }
+    template <class F>
+    __device__ void sync_fetch(F fetch) const { grid_sync_fetch(bar, gridDim.x, status, fetch); }
+    static constexpr bool multi = true;
+    __device__ bool first_cta() const { return blockIdx.x == 0; }
 };
 
 // G consecutive CTAs of a cooperative launch working on one query.
@@ -106,6 +124,10 @@ struct SubGridGroup {
     __device__ int warp() const { return rank() >> 5; }
     __device__ int nwarps() const { return size() >> 5; }
     __device__ void sync() const { grid_sync(bar, (unsigned)G, status); }
+    template <class F>
+    __device__ void sync_fetch(F fetch) const { grid_sync_fetch(bar, (unsigned)G, status, fetch); }
+    static constexpr bool multi = true;
+    __device__ bool first_cta() const { return blockIdx.x % G == 0; }
 };
 
 // ---- heuristics (h(v) as uint32, INF_G = "cannot reach the target") -------
@@ -155,11 +177,11 @@ struct HeurManhattan {
 // which is the exact difference when s = 1.  The engines need
 // admissibility only: a node reached again with a smaller g is re-expanded.  A landmark that reaches v but not t, or is
 // reached from t but not from v, proves that v cannot reach t.
-// unroll factor of the landmark row loops (row loads issued ahead of use)
-#ifndef DDP_ALT_UNROLL
-#define DDP_ALT_UNROLL 8
-#endif
-constexpr int ALT_UNROLL = DDP_ALT_UNROLL;
+// unroll factor of the landmark row loops (row loads issued ahead of use).
+// More row loads in flight cost registers that the one-CTA engine spills:
+// 500 queries on 400,000 nodes, 64 landmarks of 8 bits: 8 -> 9.21 ms,
+// 4 -> 8.59, 2 -> 8.37.
+constexpr int ALT_UNROLL = 2;
 struct HeurALT {
     const uint2 *tab;  // DevGraph::lm: rows of 2L entries
     int32_t L;         // landmarks, a multiple of 4 (16-bit) or 8 (8-bit)
@@ -298,18 +320,36 @@ __device__ __forceinline__ int warp_excl_scan(int x, int *total) {
     return v - x;
 }
 
-// Claims the next chunk of a phase for this warp (dynamic balance: warps
-// that finish early take more chunks).  Returns the chunk index.
-__device__ __forceinline__ int64_t claim_chunk(int *counter) {
-    int c = 0;
-    if ((threadIdx.x & 31) == 0) c = atomicAdd(counter, 1);
-    return (int64_t)__shfl_sync(0xffffffffu, c, 0);
-}
+// Chunks of a phase over `cnt` entries: warp w takes chunk w, and only a
+// phase with more chunks than warps claims the rest from a counter (dynamic
+// balance: warps that finish early take more).  A narrow phase then costs no
+// claim atomics (they serialise on one L2 line: two per warp of a full grid
+// took 5-10 us a phase), and its entries are spread over the warps instead
+// of filling the first few.
+struct Chunks {
+    int size;      // entries per chunk, at most 32
+    int64_t first; // this warp's first chunk
+    bool more;     // further chunks are claimed
+    int nw;
+    int *counter;
+    __device__ Chunks(int64_t cnt, int warp, int nwarps, int *ck) : first(warp), nw(nwarps), counter(ck) {
+        const int64_t per = (cnt + nwarps - 1) / nwarps;
+        size = per >= 32 ? 32 : per < 1 ? 1 : (int)per;
+        more = cnt > (int64_t)size * nwarps;
+    }
+    // the chunk after c (a count past the end when there is none)
+    __device__ int64_t next(int64_t cnt) const {
+        if (!more) return cnt;
+        int c = 0;
+        if ((threadIdx.x & 31) == 0) c = atomicAdd(counter, 1);
+        return (int64_t)nw + __shfl_sync(0xffffffffu, c, 0);
+    }
+};
 
 // Records an error for phase `ph` (consistent control flow after the
 // barrier) and in the sticky status word (reporting).
 __device__ __forceinline__ void raise_err(SearchCtl *ctl, int ph, int bit) {
-    atomicOr(&ctl->err[ph], bit);
+    atomicOr(&ctl->ph[ph].err, bit);
     atomicOr(&ctl->status, bit);
 }
 
@@ -366,6 +406,50 @@ __device__ __forceinline__ void stage_flush(T *buf, int &cnt, int *counter, T *d
     cnt = 0;
 }
 
+// What a phase leaves in a warp's staging buffers, for the three pushes a
+// search makes, copied out CTA-wide: one reservation per queue and CTA
+// instead of one per queue and warp.
+struct CtaFlush {
+    int cnt[3][32];   // entries per warp, then the warp's offset
+};
+// near, far and touched entries of this warp; call from every thread.
+template <class TN, class TF>
+__device__ __forceinline__ void cta_flush(CtaFlush *cf, WarpRows &wr, const TN *bn, int c_n, int *k_n, TN *d_n,
+                                          int64_t base_n, int64_t cap_n, const TF *bf, int c_f, int *k_f, TF *d_f,
+                                          int64_t base_f, int64_t cap_f, int c_t, int *k_t, int32_t *d_t,
+                                          int64_t cap_t, SearchCtl *ctl, int ph) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)((blockDim.x + 31) >> 5);
+    if (lane == 0) {
+        cf->cnt[0][warp] = c_n;
+        cf->cnt[1][warp] = c_f;
+        cf->cnt[2][warp] = c_t;
+    }
+    __syncthreads();
+    for (int q = warp; q < 3; q += nw) {
+        const int x = lane < nw ? cf->cnt[q][lane] : 0;
+        int total;
+        const int ex = warp_excl_scan(x, &total);
+        int b = 0;
+        if (lane == 0 && total) b = atomicAdd(q == 0 ? k_n : q == 1 ? k_f : k_t, total);
+        b = __shfl_sync(FULL, b, 0);
+        if (lane < nw) cf->cnt[q][lane] = b + ex;
+    }
+    __syncthreads();
+    const int64_t on = base_n + cf->cnt[0][warp], of = base_f + cf->cnt[1][warp], ot = cf->cnt[2][warp];
+    for (int i = lane; i < c_n; i += 32) {
+        if (on + i < cap_n) d_n[on + i] = bn[i];
+        else raise_err(ctl, ph, ST_OVERFLOW);
+    }
+    for (int i = lane; i < c_f; i += 32) {
+        if (of + i < cap_f) d_f[of + i] = bf[i];
+        else raise_err(ctl, ph, ST_OVERFLOW);
+    }
+    for (int i = lane; i < c_t; i += 32) {
+        if (ot + i < cap_t) d_t[ot + i] = wr.st[i];
+        else raise_err(ctl, ph, ST_OVERFLOW);
+    }
+}
+
 __device__ __forceinline__ int row_owner(const WarpRows &wr, int k) {
     int o = 0;
 #pragma unroll
@@ -411,6 +495,163 @@ struct SearchResult {
     int iters;
 };
 
+// ---- narrow phases on one CTA -------------------------------------------------
+// A phase of a few hundred entries gives a grid little to do and still costs
+// its barrier and four dependent trips to memory.  While the near list holds
+// at most LOCAL_IN entries, CTA 0 runs the search's phases alone: the list
+// lives in shared memory, an entry carries its row bounds (read beside the
+// relaxation that pushed it), eight lanes walk one row, and a phase ends with
+// a block barrier.  It hands the list back when it outgrows LOCAL_OUT entries
+// or after LOCAL_WAVES phases (the other CTAs wait in a bounded barrier).
+// A 511 x 511 maze query (1,926 phases of 20-70 entries) so takes 3.6 ms;
+// with every phase on the grid it took 44 ms (23 us a phase).
+constexpr int LOCAL_IN = 256, LOCAL_OUT = 512;
+constexpr int LOCAL_WAVES = 4096;
+constexpr int LOCAL_LANES = 8;  // lanes per entry
+
+// entries that the warp rows (16 per CTA in every search kernel) hold as two
+// lists of uint4
+constexpr int LOCAL_CAP = (int)(16 * sizeof(WarpRows) / (2 * sizeof(uint4)));
+static_assert(LOCAL_CAP >= LOCAL_IN && LOCAL_CAP >= LOCAL_OUT, "local lists hold a whole phase");
+
+// near: nnear entries in qcur (rewritten on return with the entries left).
+// Results go to ctl->loc_*; far pushes and first touches are appended as a
+// grid phase does.
+template <class Heur>
+__device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H, const SearchParams &P,
+                             WarpRows *wrows, uint2 *qcur, int nnear, uint4 *fcur, int64_t nfar0, uint32_t T,
+                             uint32_t ht, unsigned long long &n_exp, unsigned long long &n_scan,
+                             unsigned long long &n_rel) {
+    SearchCtl *ctl = B.ctl;
+    // {node, g, row begin, row end}
+    uint4 *buf = reinterpret_cast<uint4 *>(wrows);
+    constexpr int cap = LOCAL_CAP;
+    __shared__ int cnt[3];  // entries per wave, rotating
+    __shared__ int c_far, c_touch;
+    __shared__ unsigned int tg;
+    const int sub = threadIdx.x & (LOCAL_LANES - 1);
+    const int team = threadIdx.x / LOCAL_LANES, teams = blockDim.x / LOCAL_LANES;
+    const int touch0 = *(volatile int *)&ctl->touched;
+    if (threadIdx.x == 0) {
+        cnt[0] = nnear;
+        cnt[1] = cnt[2] = 0;
+        c_far = c_touch = 0;
+        tg = P.t >= 0 ? st_g(__ldcg(B.state + P.t)) : 0xFFFFFFFFu;
+    }
+    for (int i = threadIdx.x; i < nnear; i += blockDim.x) {
+        const uint2 en = __ldcg(qcur + i);
+        buf[i] = make_uint4(en.x, en.y, (uint32_t)row_begin(G.off, G.oend, (int)en.x),
+                            (uint32_t)row_end(G.off, G.oend, (int)en.x));
+    }
+    __syncthreads();
+    int m = nnear, wv = 0;
+    uint4 *cur = buf, *nxt = buf + cap;
+    for (;;) {
+        int *push = &cnt[(wv + 1) % 3];
+        if (threadIdx.x == 0) cnt[(wv + 2) % 3] = 0;
+        const uint64_t ft64 = (uint64_t)(*(volatile unsigned int *)&tg) + ht;
+        const uint32_t ft = ft64 >= 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)ft64;
+        auto to_far = [&](uint32_t v, uint32_t g, uint32_t f) {
+            const int64_t p = nfar0 + atomicAdd(&c_far, 1);
+            if (p < B.cap_f) fcur[p] = make_uint4(v, g, f, 0u);
+            else atomicOr(&ctl->status, ST_OVERFLOW);
+        };
+        for (int i = team; i < m; i += teams) {
+            const uint4 en = cur[i];
+            const int u = (int)en.x;
+            const uint32_t gu = en.y;
+            int j = (int)en.z + sub;
+            const int r1 = (int)en.w;
+            // the first arcs load beside the label that decides about them
+            uint2 a = j < r1 ? (G.oend ? __ldcg(G.arc + j) : __ldg(G.arc + j)) : make_uint2(0xFFFFFFFFu, 0u);
+            const uint64_t su = __ldcg(B.state + u);
+            const uint32_t hu = (ft < T || (P.keep && ft != 0xFFFFFFFFu)) ? H(u) : 0u;
+            if (st_g(su) != gu || u == P.t) continue;
+            if ((uint64_t)gu + hu >= ft) {
+                if (P.keep && sub == 0) to_far((uint32_t)u, gu, 0u);  // keep mode: f re-derived
+                continue;
+            }
+            if (sub == 0) {
+                n_exp++;
+                n_scan += (unsigned long long)(r1 - (int)en.z);
+            }
+            for (;;) {
+                const int v = (int)a.x;
+                const uint64_t ng64 = (uint64_t)gu + a.y;
+                if (v >= 0 && ng64 < INF_G) {
+                    const uint32_t ng = (uint32_t)ng64;
+                    const uint64_t nv = st_make(ng, u);
+                    uint64_t c0;
+                    bool inst = false, first = false;
+                    const int rb = row_begin(G.off, G.oend, v), re = row_end(G.off, G.oend, v);
+                    uint32_t hv;
+                    if (!P.keep && a.y != 0) {
+                        // one atomic per arc (the asynchronous engine's latency
+                        // form: over a positive arc a tie may swap the parent
+                        // for an equal-cost one)
+                        hv = H(v);
+                        c0 = atomicMin(B.state + v, nv);
+                        inst = ng < st_g(c0);
+                    } else {
+                        c0 = __ldcg(B.state + v);
+                        hv = H(v);
+                        if (P.keep ? hv < INF_G : (uint64_t)ng + hv < ft) {
+                            while (ng < st_g(c0)) {
+                                const uint64_t got = atomicCAS(B.state + v, c0, nv);
+                                if (got == c0) {
+                                    inst = true;
+                                    break;
+                                }
+                                c0 = got;
+                            }
+                        }
+                    }
+                    if (inst) {
+                        first = !P.no_touch_log && st_g(c0) >= INF_G;
+                        if (v == P.t) atomicMin(&tg, ng);
+                        const uint64_t fv = (uint64_t)ng + hv;
+                        if (fv < T) {
+                            n_rel++;
+                            const int p = atomicAdd(push, 1);
+                            if (p < cap) nxt[p] = make_uint4((uint32_t)v, ng, (uint32_t)rb, (uint32_t)re);
+                            else if (p < B.cap_q) qcur[p] = make_uint2((uint32_t)v, ng);  // past shared memory
+                            else atomicOr(&ctl->status, ST_OVERFLOW);
+                        } else if (P.keep || fv < ft) {
+                            n_rel++;
+                            to_far((uint32_t)v, ng, fv >= 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)fv);
+                        }
+                        if (first) {
+                            const int p = touch0 + atomicAdd(&c_touch, 1);
+                            if (p < G.n) B.touched[p] = v;
+                            else atomicOr(&ctl->status, ST_OVERFLOW);
+                        }
+                    }
+                }
+                j += LOCAL_LANES;
+                if (j >= r1) break;
+                a = G.oend ? __ldcg(G.arc + j) : __ldg(G.arc + j);
+            }
+        }
+        __syncthreads();
+        wv++;
+        m = cnt[wv % 3];
+        uint4 *t = cur;
+        cur = nxt;
+        nxt = t;
+        if (m == 0 || m > LOCAL_OUT || wv >= LOCAL_WAVES || nfar0 + c_far > B.cap_f / 2) break;
+        __syncthreads();  // every thread has read c_far
+    }
+    // the entries left go back to the near list (those past the shared list
+    // are there already)
+    for (int i = threadIdx.x; i < min(m, cap); i += blockDim.x) qcur[i] = make_uint2(cur[i].x, cur[i].y);
+    if (threadIdx.x == 0) {
+        ctl->loc_near = m;
+        ctl->loc_far = (int)(nfar0 + c_far);
+        ctl->loc_waves = wv;
+        ctl->touched = touch0 + c_touch;
+    }
+}
+
 // One A* run on one slot, executed collectively by every thread of `grp`.
 // Precondition: slot state is all-ones (unreached) for every node.
 template <class Grp, class Heur>
@@ -420,13 +661,18 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
     const int lane = lane_id();
     WarpRows &wr = wrows[threadIdx.x >> 5];
     const bool has_diff = G.doff != nullptr;
+    // words every thread needs after a barrier, read by one thread per CTA
+    __shared__ struct {
+        PhaseWords w;
+        int status;
+        uint32_t tg;
+        int loc_near, loc_far, loc_waves;
+    } pc;
+    __shared__ CtaFlush cf;
 
     if (grp.rank() == 0) {
         for (int i = 0; i < 4; i++) {
-            ctl->nq[i] = 0;
-            ctl->fq[i] = 0;
-            ctl->mf[i] = 0xFFFFFFFFu;
-            ctl->err[i] = 0;
+            ctl->ph[i] = PhaseWords{0, 0, 0xFFFFFFFFu, 0};
             ctl->ck[i] = 0;
         }
         ctl->iters = 0;
@@ -442,7 +688,8 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
     }
     const int64_t far_resume = P.resume ? (int64_t)(*(volatile int *)&ctl->far_n) : 0;
     const bool far_in_f1 = P.resume && (*(volatile int *)&ctl->far_sel) != 0;
-    grp.sync();
+    auto read_tg = [&]() -> uint32_t { return P.t >= 0 ? st_g(__ldcg(B.state + P.t)) : 0xFFFFFFFFu; };
+    grp.sync_fetch([&] { pc.tg = read_tg(); });
 
     uint2 *qcur = B.q0, *qnxt = B.q1;
     uint4 *fcur = far_in_f1 ? B.f1 : B.f0, *falt = far_in_f1 ? B.f0 : B.f1;
@@ -461,8 +708,11 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
     int64_t far_after_compact = 0;
     unsigned long long n_exp = 0, n_scan = 0, n_rel = 0;
     int it = 0;
+    int64_t waves = 0;  // phases that CTA 0 ran alone
     int status = 0;
     const int64_t max_phases = 4 * (int64_t)G.n + (1 << 22);
+    const uint32_t ht = P.t >= 0 ? H(P.t) : 0u;
+    uint32_t tg = pc.tg;  // g(t): only decreases, so a stale value only prunes less
     // cold tier (keep mode, resumed): made by the first split
     uint32_t cold_x = (P.keep && P.resume && P.cold) ? P.cold_x : 0xFFFFFFFFu;
     bool cold_pass = cold_x != 0xFFFFFFFFu;
@@ -470,25 +720,53 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
     uint2 *cold_stage = reinterpret_cast<uint2 *>(wr.snr);
 
     for (;;) {
+        if constexpr (Grp::multi) {
+            if (!splitting && head == 0 && nnext == 0 && !has_diff && nnear <= LOCAL_IN &&
+                nfar <= B.cap_f / 2 && (P.K <= 0 || P.K >= LOCAL_OUT)) {
+                if (grp.first_cta()) local_phases(G, B, H, P, wrows, qcur, (int)nnear, fcur, nfar, T, ht, n_exp, n_scan, n_rel);
+                grp.sync_fetch([&] {
+                    pc.loc_near = *(volatile int *)&ctl->loc_near;
+                    pc.loc_far = *(volatile int *)&ctl->loc_far;
+                    pc.loc_waves = *(volatile int *)&ctl->loc_waves;
+                    pc.status = *(volatile int *)&ctl->status;
+                    pc.tg = read_tg();
+                });
+                nnear = pc.loc_near;
+                nfar = pc.loc_far;
+                waves += pc.loc_waves;
+                status = pc.status;
+                tg = pc.tg;
+                if (status & (ST_OVERFLOW | ST_TIMEOUT)) break;
+                if (it + waves > max_phases) {
+                    if (grp.rank() == 0) atomicOr(&ctl->status, ST_TIMEOUT);
+                    break;
+                }
+                if (nnear == 0) {
+                    splitting = true;
+                    Tsplit = sat_add(T, P.delta);
+                } else if (nfar > B.cap_f / 2 && nfar - far_after_compact > B.cap_f / 8) {
+                    compacting = true;
+                    splitting = true;
+                }
+            }
+        }
         const int PH = (it + 1) & 3, RS = (it + 3) & 3;
-        // f(t) snapshot: only decreases, so a stale value only prunes less.
-        const uint64_t st_t = P.t >= 0 ? __ldcg(B.state + P.t) : ~0ull;
-        const uint32_t ht = P.t >= 0 ? H(P.t) : 0u;
-        const uint64_t ft64 = (uint64_t)st_g(st_t) + ht;
+        const uint64_t ft64 = (uint64_t)tg + ht;
         const uint32_t ft = ft64 >= 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)ft64;
         int64_t end = 0;
         if (!splitting) {
             end = (P.K > 0) ? min(nnear, head + (int64_t)P.K) : nnear;
             int c_n = 0, c_f = 0, c_t = 0;  // staged pushes of this warp
-            // chunk claims are prefetched one ahead to hide their round trip
-            int64_t cnext = claim_chunk(&ctl->ck[PH]);
-            for (int64_t base = head + 32 * cnext; base < end; base = head + 32 * cnext) {
-                cnext = claim_chunk(&ctl->ck[PH]);
+            const Chunks ch(end - head, grp.warp(), grp.nwarps(), &ctl->ck[PH]);
+            // claims are made one chunk ahead to hide their round trip
+            int64_t cnext = ch.first;
+            for (int64_t base = head + ch.size * cnext; base < end; base = head + ch.size * cnext) {
+                cnext = ch.next(end);
                 const int64_t idx = base + lane;
                 int u = -1, rb = 0, bdeg = 0, drb = 0, deg = 0;
                 uint32_t gu = 0;
                 bool requeue = false;
-                if (idx < end) {
+                if (lane < ch.size && idx < end) {
                     const uint2 en = __ldcg(qcur + idx);
                     u = (int)en.x;
                     gu = en.y;
@@ -518,7 +796,7 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
                         }
                     }
                 }
-                stage_push(requeue, make_uint4((uint32_t)u, gu, 0u, 0u), wr.sf, c_f, &ctl->fq[PH],  // keep mode: f re-derived
+                stage_push(requeue, make_uint4((uint32_t)u, gu, 0u, 0u), wr.sf, c_f, &ctl->ph[PH].fq,  // keep mode: f re-derived
                            fcur, nfar, B.cap_f, ctl, PH);
                 int total;
                 int ex = warp_excl_scan(deg, &total);
@@ -590,18 +868,17 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
                         }
                         if (to_near || to_far) n_rel++;
                         const uint2 en = make_uint2((uint32_t)v[r], ng[r]);
-                        stage_push(to_near, en, wr.sn, c_n, &ctl->nq[PH], qnxt, nnext, B.cap_q, ctl, PH);
+                        stage_push(to_near, en, wr.sn, c_n, &ctl->ph[PH].nq, qnxt, nnext, B.cap_q, ctl, PH);
                         stage_push(to_far, make_uint4(en.x, en.y, sat_add(ng[r], hv[r]), 0u), wr.sf, c_f,
-                                   &ctl->fq[PH], fcur, nfar, B.cap_f, ctl, PH);
+                                   &ctl->ph[PH].fq, fcur, nfar, B.cap_f, ctl, PH);
                         // at most n first touches: the touched log never overflows
                         stage_push(first, v[r], wr.st, c_t, &ctl->touched, B.touched, 0, (int64_t)G.n, ctl, PH);
                     }
                 }
                 __syncwarp();
             }
-            stage_flush(wr.sn, c_n, &ctl->nq[PH], qnxt, nnext, B.cap_q, ctl, PH);
-            stage_flush(wr.sf, c_f, &ctl->fq[PH], fcur, nfar, B.cap_f, ctl, PH);
-            stage_flush(wr.st, c_t, &ctl->touched, B.touched, 0, (int64_t)G.n, ctl, PH);
+            cta_flush(&cf, wr, wr.sn, c_n, &ctl->ph[PH].nq, qnxt, nnext, B.cap_q, wr.sf, c_f, &ctl->ph[PH].fq, fcur,
+                      nfar, B.cap_f, c_t, &ctl->touched, B.touched, (int64_t)G.n, ctl, PH);
         } else {
             // split the far pile at Tsplit (or compact it at T).  Entries
             // carry f from their push: a split reads no node state, stale
@@ -620,8 +897,8 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
             const int64_t dbase = compacting ? nnext : 0;
             unsigned int local_min = 0xFFFFFFFFu;
             int c_n = 0, c_f = 0, c_c = 0;
-            for (int64_t base = 32 * claim_chunk(&ctl->ck[PH]); base < nscan;
-                 base = 32 * claim_chunk(&ctl->ck[PH])) {
+            // uniform work per entry: a fixed stride, no claims
+            for (int64_t base = 32 * (int64_t)grp.warp(); base < nscan; base += 32 * (int64_t)grp.nwarps()) {
                 const int64_t idx = base + lane;
                 bool to_near = false, keep = false, cold = false;
                 uint4 en = make_uint4(0u, 0u, 0u, 0u);
@@ -653,15 +930,15 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
                         }
                     }
                 }
-                stage_push(to_near, make_uint2(en.x, en.y), wr.sn, c_n, &ctl->nq[PH], dst, dbase, B.cap_q, ctl, PH);
+                stage_push(to_near, make_uint2(en.x, en.y), wr.sn, c_n, &ctl->ph[PH].nq, dst, dbase, B.cap_q, ctl, PH);
                 // compaction never grows the pile
-                stage_push(keep, en, wr.sf, c_f, &ctl->fq[PH], falt, 0, B.cap_f, ctl, PH);
+                stage_push(keep, en, wr.sf, c_f, &ctl->ph[PH].fq, falt, 0, B.cap_f, ctl, PH);
                 if (to_cold)
                     stage_push(cold, make_uint2(en.x, en.y), cold_stage, c_c, &ctl->cold_n, P.cold, 0, P.cold_cap,
                                ctl, PH);
             }
-            stage_flush(wr.sn, c_n, &ctl->nq[PH], dst, dbase, B.cap_q, ctl, PH);
-            stage_flush(wr.sf, c_f, &ctl->fq[PH], falt, 0, B.cap_f, ctl, PH);
+            cta_flush(&cf, wr, wr.sn, c_n, &ctl->ph[PH].nq, dst, dbase, B.cap_q, wr.sf, c_f, &ctl->ph[PH].fq, falt, 0,
+                      B.cap_f, 0, &ctl->touched, B.touched, (int64_t)G.n, ctl, PH);
             if (to_cold) stage_flush(cold_stage, c_c, &ctl->cold_n, P.cold, 0, P.cold_cap, ctl, PH);
             if (merge_cold) {
                 ncold = 0;  // every cold entry was examined: none is left
@@ -669,25 +946,27 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) local_min = min(local_min, __shfl_xor_sync(FULL, local_min, o));
-            if (lane == 0 && local_min != 0xFFFFFFFFu) atomicMin(&ctl->mf[PH], local_min);
+            if (lane == 0 && local_min != 0xFFFFFFFFu) atomicMin(&ctl->ph[PH].mf, local_min);
         }
 
-        grp.sync();
+        grp.sync_fetch([&] {
+            const int4 x = __ldcg(reinterpret_cast<const int4 *>(&ctl->ph[PH]));
+            pc.w = PhaseWords{x.x, x.y, (unsigned int)x.z, x.w};
+            pc.status = *(volatile int *)&ctl->status;
+            pc.tg = read_tg();
+        });
         if (grp.rank() == 0) {
-            ctl->nq[RS] = 0;
-            ctl->fq[RS] = 0;
-            ctl->mf[RS] = 0xFFFFFFFFu;
-            ctl->err[RS] = 0;
+            ctl->ph[RS] = PhaseWords{0, 0, 0xFFFFFFFFu, 0};
             ctl->ck[RS] = 0;
         }
-        const int a = *(volatile int *)&ctl->nq[PH];
-        const int b = *(volatile int *)&ctl->fq[PH];
-        const unsigned int m = *(volatile unsigned int *)&ctl->mf[PH];
-        const int perr = *(volatile int *)&ctl->err[PH];
-        status = *(volatile int *)&ctl->status;
+        const int a = pc.w.nq, b = pc.w.fq;
+        const unsigned int m = pc.w.mf;
+        const int perr = pc.w.err;
+        status = pc.status;
+        tg = pc.tg;
         it++;
         if ((perr & ST_OVERFLOW) || (status & ST_TIMEOUT)) break;
-        if (it > max_phases) {
+        if (it + waves > max_phases) {
             // a search never needs this many phases; stop instead of spinning
             if (grp.rank() == 0) atomicOr(&ctl->status, ST_TIMEOUT);
             break;
@@ -752,13 +1031,14 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
     }
 
     // fold per-thread counters
-    if (lane == 0 && n_scan) atomicAdd(&ctl->scanned, n_scan);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         n_exp += __shfl_xor_sync(FULL, n_exp, o);
         n_rel += __shfl_xor_sync(FULL, n_rel, o);
+        n_scan += __shfl_xor_sync(FULL, n_scan, o);
     }
     if (lane == 0) {
+        if (n_scan) atomicAdd(&ctl->scanned, n_scan);
         if (n_exp) atomicAdd(&ctl->expanded, n_exp);
         if (n_rel) atomicAdd(&ctl->relaxed, n_rel);
     }
@@ -780,8 +1060,8 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
     const uint64_t st_t = P.t >= 0 ? __ldcg(B.state + P.t) : ~0ull;
     const uint64_t c = (uint64_t)st_g(st_t) + (P.t >= 0 ? H(P.t) : 0u);
     r.cost = (st_g(st_t) >= INF_G || c >= INF_G) ? 0xFFFFFFFFu : (uint32_t)c;
-    r.iters = it;
-    if (grp.rank() == 0) ctl->iters = it;
+    r.iters = (int)(it + waves);
+    if (grp.rank() == 0) ctl->iters = r.iters;
     return r;
 }
 
@@ -812,13 +1092,16 @@ __device__ uint32_t run_bfs_hops(const Grp &grp, const DevGraph &G, const SlotBu
     int *fb = reinterpret_cast<int *>(B.q1);
     const int64_t capf = 2 * (spare_q0 ? min(B.cap_q, B.cap_f) : B.cap_q);  // uint2 slots reused as ints
     const uint32_t max_lvl = tag ? 254u : 0xFFFFFFF0u;
+    __shared__ struct {
+        int nf, err, status;
+    } pc;
+    __shared__ CtaFlush cf;
 
     if (!tag)
         for (int64_t i = grp.rank(); i < G.n; i += grp.size()) B.hops[i] = HOPS_INF;
     if (grp.rank() == 0) {
         for (int i = 0; i < 4; i++) {
-            ctl->nq[i] = 0;
-            ctl->err[i] = 0;
+            ctl->ph[i] = PhaseWords{0, 0, 0xFFFFFFFFu, 0};
             ctl->ck[i] = 0;
         }
         ctl->bfs_scanned = 0;
@@ -843,10 +1126,13 @@ __device__ uint32_t run_bfs_hops(const Grp &grp, const DevGraph &G, const SlotBu
         const int PH = (it + 1) & 3, RS = (it + 3) & 3;
         const uint32_t claim_val = tag | (lvl + 1);
         int c_b = 0;
-        for (int64_t base = 32 * claim_chunk(&ctl->ck[PH]); base < nf; base = 32 * claim_chunk(&ctl->ck[PH])) {
+        const Chunks ch(nf, grp.warp(), grp.nwarps(), &ctl->ck[PH]);
+        int64_t cnext = ch.first;
+        for (int64_t base = ch.size * cnext; base < nf; base = ch.size * cnext) {
+            cnext = ch.next(nf);
             const int64_t idx = base + lane;
             int rb = 0, bdeg = 0, drb = 0, deg = 0;
-            if (idx < nf) {
+            if (lane < ch.size && idx < nf) {
                 int u = __ldcg(fa + idx);
                 rb = row_begin(G.roff, G.roend, u);
                 bdeg = row_end(G.roff, G.roend, u) - rb;
@@ -877,21 +1163,24 @@ __device__ uint32_t run_bfs_hops(const Grp &grp, const DevGraph &G, const SlotBu
                         if (!seen) claim = atomicCAS(B.hops + p, x, claim_val) == x;
                     }
                 }
-                stage_push(claim, p, wr.st, c_b, &ctl->nq[PH], fb, 0, capf, ctl, PH);
+                stage_push(claim, p, wr.st, c_b, &ctl->ph[PH].nq, fb, 0, capf, ctl, PH);
             }
             __syncwarp();
         }
-        stage_flush(wr.st, c_b, &ctl->nq[PH], fb, 0, capf, ctl, PH);
-        grp.sync();
+        cta_flush(&cf, wr, wr.st, c_b, &ctl->ph[PH].nq, fb, 0, capf, wr.sf, 0, &ctl->ph[PH].fq, B.f0, 0, B.cap_f, 0,
+                  &ctl->touched, B.touched, (int64_t)G.n, ctl, PH);
+        grp.sync_fetch([&] {
+            pc.nf = *(volatile int *)&ctl->ph[PH].nq;
+            pc.err = *(volatile int *)&ctl->ph[PH].err;
+            pc.status = *(volatile int *)&ctl->status;
+        });
         if (grp.rank() == 0) {
-            ctl->nq[RS] = 0;
-            ctl->err[RS] = 0;
+            ctl->ph[RS] = PhaseWords{0, 0, 0xFFFFFFFFu, 0};
             ctl->ck[RS] = 0;
         }
-        nf = *(volatile int *)&ctl->nq[PH];
+        nf = pc.nf;
         b_reached += (unsigned long long)nf;
-        const int perr = *(volatile int *)&ctl->err[PH];
-        const int status = *(volatile int *)&ctl->status;
+        const int perr = pc.err, status = pc.status;
         it++;
         lvl++;
         int *tmp = fa;

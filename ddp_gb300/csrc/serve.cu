@@ -497,7 +497,7 @@ int ddp_serve_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, int64_t 
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate"));
     // slots: occupancy, then the memory budget (half of free memory)
     s->hk = kernel_hk(hkind, g->d_xy != nullptr, false);
-    const int per_sm = std::max(1, slots_per_sm(s->hk, s->block));
+    const int per_sm = std::max(1, slots_per_sm(s->hk, s->block, (s->o.flags & DDP_OPT_SYNC) != 0));
     int nslots = per_sm * device_sms();
     if (s->o.grid > 0) nslots = std::min(nslots, s->o.grid);
     size_t freeb = 0, totalb = 0;

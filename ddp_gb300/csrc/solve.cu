@@ -161,7 +161,10 @@ __global__ void __launch_bounds__(512) k_bfs_single(DevGraph G, SlotArrays sa, u
 
 // Single-query GA* over the whole grid (cooperative launch).
 template <class Heur>
-__global__ void __launch_bounds__(512, 2)
+// One CTA per SM: two would halve the registers (220-640 bytes of spills per
+// thread) and double the CTAs at every barrier (511 x 511 maze 4.58 -> 3.64
+// ms; 250,000 nodes with a caller's heuristic 0.75 -> 0.68 ms).
+__global__ void __launch_bounds__(512, 1)
     k_solve_single(DevGraph G, SlotArrays sa, Heur H, SearchParams P, int32_t *out, int32_t *path,
                    int32_t path_cap) {
     __shared__ WarpRows wrows[MAX_WARPS];
@@ -180,7 +183,7 @@ __global__ void __launch_bounds__(512, 2)
 
 // Exhaustive search from P.s (P.t < 0) over the whole grid; dist[v] = d(s, v)
 // or LM_UNREACHED.
-__global__ void __launch_bounds__(512, 2)
+__global__ void __launch_bounds__(512, 1)
     k_sssp(DevGraph G, SlotArrays sa, SearchParams P, int32_t *dist, int32_t *out) {
     __shared__ WarpRows wrows[MAX_WARPS];
     SlotBufs B = slot_of(sa, 0);
@@ -221,21 +224,20 @@ __global__ void k_alt_values(DevGraph G, int32_t t, int32_t *out) {
 // finishing short searches take the next query (dynamic load balance over
 // uneven depths).  Fewer, wider groups keep fewer per-query state arrays live
 // at once, which lets them stay resident in L2.
-// One search of the slot: the asynchronous single-CTA engine when the slot is
-// one CTA (and the caller did not ask for the phase-synchronous one), else
-// the phase-synchronous group engine.
-template <class Grp, class Heur>
+// One search of the slot: the asynchronous single-CTA engine for one-CTA
+// slots (ASYNC), else the phase-synchronous group engine.
+template <bool ASYNC, class Grp, class Heur>
 __device__ SearchResult slot_search(const Grp &grp, const DevGraph &G, const SlotBufs &B, const Heur &H,
-                                    const SearchParams &P, WarpRows *wrows, CtaQ *sq, bool async) {
+                                    const SearchParams &P, WarpRows *wrows, CtaQ *sq) {
     // throughput (many slots): load + CAS on improving arcs only, unless
     // the heuristic is cheap enough that one atomic per arc wins
-    if (async) return run_search_cta<Heur, heur_cheap<Heur>::value>(G, B, H, P, wrows, sq);
-    return run_search(grp, G, B, H, P, wrows);
+    if constexpr (ASYNC) return run_search_cta<Heur, heur_cheap<Heur>::value>(G, B, H, P, wrows, sq);
+    else return run_search(grp, G, B, H, P, wrows);
 }
 
-template <int HK, class Grp>
+template <int HK, bool ASYNC, class Grp>
 __device__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B, const BatchArgs &A,
-                           uint32_t *epoch, WarpRows *wrows, CtaQ *sq, BiQ *bq, bool async) {
+                           uint32_t *epoch, WarpRows *wrows, CtaQ *sq, BiQ *bq) {
     SearchCtl *ctl = B.ctl;
     long long t0 = 0;
     int vbuf = -1;  // versioned serving: graph buffer the current search holds
@@ -373,16 +375,16 @@ __device__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B
         SearchResult r;
         if (HK == 1) {
             const uint32_t tag = *(volatile uint32_t *)&ctl->tag;
-            const uint32_t cap = run_bfs_hops(grp, G, B, t, wrows, tag, A.bfs_budget, async);
-            r = slot_search(grp, G, B, HeurHops{B.hops, G.wmin, cap, tag}, P, wrows, sq, async);
+            const uint32_t cap = run_bfs_hops(grp, G, B, t, wrows, tag, A.bfs_budget, ASYNC);
+            r = slot_search<ASYNC>(grp, G, B, HeurHops{B.hops, G.wmin, cap, tag}, P, wrows, sq);
         } else if (HK == 2) {
             int2 tp = reinterpret_cast<const int2 *>(G.xy)[t];
-            r = slot_search(grp, G, B, HeurManhattan{G.xy, tp.x, tp.y, G.wmin}, P, wrows, sq, async);
+            r = slot_search<ASYNC>(grp, G, B, HeurManhattan{G.xy, tp.x, tp.y, G.wmin}, P, wrows, sq);
         } else if (HK == 3) {
             int2 tp = reinterpret_cast<const int2 *>(G.xy)[t];
-            r = slot_search(grp, G, B, HeurEuclid{G.xy, tp.x, tp.y, G.rho_fp}, P, wrows, sq, async);
+            r = slot_search<ASYNC>(grp, G, B, HeurEuclid{G.xy, tp.x, tp.y, G.rho_fp}, P, wrows, sq);
         } else if (HK == 4) {
-            r = slot_search(grp, G, B, HeurALT{G.lm, G.lm_L, G.lm_scale, t, G.lm_bits}, P, wrows, sq, async);
+            r = slot_search<ASYNC>(grp, G, B, HeurALT{G.lm, G.lm_L, G.lm_scale, t, G.lm_bits}, P, wrows, sq);
         } else if (bidir_hk(HK)) {
             // bidirectional: one-CTA slots only (the host never launches
             // these kinds with wider slots)
@@ -407,9 +409,9 @@ __device__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B
                 }
             }
         } else {
-            r = slot_search(grp, G, B, HeurZero{}, P, wrows, sq, async);
+            r = slot_search<ASYNC>(grp, G, B, HeurZero{}, P, wrows, sq);
         }
-        if ((async || bidir_hk(HK)) && (*(volatile int *)&ctl->status & (ST_OVERFLOW | ST_TIMEOUT))) {
+        if (ASYNC && (*(volatile int *)&ctl->status & (ST_OVERFLOW | ST_TIMEOUT))) {
             // an aborted asynchronous search may leave ring slots written:
             // clear the ring so the slot's next search starts clean
             for (int64_t i = grp.rank(); i < B.cap_q; i += grp.size()) B.q0[i].x = RING_EMPTY;
@@ -616,6 +618,10 @@ __device__ void service_loop(const BatchArgs &A) {
 #ifndef DDP_BIDIR_MIN_BLOCKS
 #define DDP_BIDIR_MIN_BLOCKS 2
 #endif
+// One-CTA slots.  The group form below is a kernel of its own: both engines
+// in one kernel share a register budget, and the one that a launch does not
+// use makes the other spill (landmark instance: 736 bytes of spill stores
+// with both engines, 1,706 once the group engine also ran narrow phases).
 template <int HK>
 __global__ void __launch_bounds__(512, (bidir_hk(HK) ? DDP_BIDIR_MIN_BLOCKS : 2)) k_batch(DevGraph G, SlotArrays sa, BatchArgs A) {
     __shared__ WarpRows wrows[MAX_WARPS];
@@ -625,16 +631,24 @@ __global__ void __launch_bounds__(512, (bidir_hk(HK) ? DDP_BIDIR_MIN_BLOCKS : 2)
         service_loop(A);
         return;
     }
-    if (A.group <= 1) {
-        SlotBufs B = slot_of(sa, blockIdx.x);
-        CtaGroup grp{&B.ctl->status};
-        batch_loop<HK>(grp, G, B, A, sa.epoch + blockIdx.x, wrows, &sq, &bq, !A.sync_engine);
-    } else {
-        const int slot = blockIdx.x / A.group;
-        SlotBufs B = slot_of(sa, slot);
-        SubGridGroup grp{{&B.ctl->bar_count, &B.ctl->bar_gen}, &B.ctl->status, A.group};
-        batch_loop<HK>(grp, G, B, A, sa.epoch + slot, wrows, &sq, &bq, false);
+    SlotBufs B = slot_of(sa, blockIdx.x);
+    CtaGroup grp{&B.ctl->status};
+    batch_loop<HK, true>(grp, G, B, A, sa.epoch + blockIdx.x, wrows, &sq, &bq);
+}
+
+// Slots of A.group CTAs each (cooperative launch), and one-CTA slots on the
+// phase-synchronous engine (DDP_OPT_SYNC).
+template <int HK>
+__global__ void __launch_bounds__(512, 2) k_batch_group(DevGraph G, SlotArrays sa, BatchArgs A) {
+    __shared__ WarpRows wrows[MAX_WARPS];
+    if (A.svc && (int)blockIdx.x == A.serve_slots) {
+        service_loop(A);
+        return;
     }
+    const int slot = blockIdx.x / A.group;
+    SlotBufs B = slot_of(sa, slot);
+    SubGridGroup grp{{&B.ctl->bar_count, &B.ctl->bar_gen}, &B.ctl->status, A.group};
+    batch_loop<HK, false>(grp, G, B, A, sa.epoch + slot, wrows, nullptr, nullptr);
 }
 
 // Single query on one CTA with the asynchronous engine (narrow searches).
@@ -721,18 +735,20 @@ int hk_slot_kind(int hk) {
     }
 }
 
-static const void *batch_kernel_hk(int hk) {
+// The kernel of an instance; grouped: slots of several CTAs, or one-CTA slots
+// on the phase-synchronous engine (bidirectional kinds have neither).
+static const void *batch_kernel_hk(int hk, bool grouped) {
     switch (hk) {
-    case 1: return (const void *)k_batch<1>;
-    case 2: return (const void *)k_batch<2>;
-    case 3: return (const void *)k_batch<3>;
-    case 4: return (const void *)k_batch<4>;
+    case 1: return grouped ? (const void *)k_batch_group<1> : (const void *)k_batch<1>;
+    case 2: return grouped ? (const void *)k_batch_group<2> : (const void *)k_batch<2>;
+    case 3: return grouped ? (const void *)k_batch_group<3> : (const void *)k_batch<3>;
+    case 4: return grouped ? (const void *)k_batch_group<4> : (const void *)k_batch<4>;
     case 5: return (const void *)k_batch<5>;
     case 6: return (const void *)k_batch<6>;
     case 7: return (const void *)k_batch<7>;
     case 8: return (const void *)k_batch<8>;
     case 9: return (const void *)k_batch<9>;
-    default: return (const void *)k_batch<0>;
+    default: return grouped ? (const void *)k_batch_group<0> : (const void *)k_batch<0>;
     }
 }
 
@@ -755,14 +771,14 @@ cudaError_t svc_run_direct(const SvcSub *subs, int nsub, cudaStream_t st) {
 cudaError_t launch_slots(int hk, int grid, int block, bool coop, DevGraph G, SlotArrays sa, BatchArgs A,
                          cudaStream_t st) {
     void *args[] = {&G, &sa, &A};
-    const void *fn = batch_kernel_hk(hk);
+    const void *fn = batch_kernel_hk(hk, A.group > 1 || A.sync_engine);
     if (coop) return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(block), args, 0, st);
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, st);
 }
 
-int slots_per_sm(int hk, int block) {
+int slots_per_sm(int hk, int block, bool grouped) {
     int per_sm = 0;
-    const void *fn = batch_kernel_hk(hk);
+    const void *fn = batch_kernel_hk(hk, grouped);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, 0);
     return per_sm;
 }
@@ -1377,7 +1393,7 @@ static cudaError_t batch_launch_args(ddp_batch *b, DevGraph G, BatchArgs A) {
     const int grid = b->sa.nslots * b->group;
     SlotArrays sa = b->sa;
     void *args[] = {&G, &sa, &A};
-    const void *fn = batch_kernel_hk(b->hk);
+    const void *fn = batch_kernel_hk(b->hk, A.group > 1 || A.sync_engine);
     if (b->group > 1)
         return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(b->block), args, 0, b->stream);
     return cudaLaunchKernel(fn, dim3(grid), dim3(b->block), args, 0, b->stream);
@@ -1433,8 +1449,9 @@ int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batc
     // slots: occupancy-limited, then memory-limited (half of free memory)
     int per_sm = 0;
     b->hk = kernel_hk(hkind, g->d_xy != nullptr, (b->o.flags & DDP_OPT_HASH) != 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel_hk(b->hk), b->block, 0);
     b->group = is_bidir_kind(hkind) ? 1 : std::max(1, b->o.group);  // bidirectional slots are one CTA
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, batch_kernel_hk(b->hk, b->group > 1 || (b->o.flags & DDP_OPT_SYNC)), b->block, 0);
     const int coresident = std::max(1, per_sm) * sm_count();
     if (b->group > coresident) b->group = coresident;
     int nslots = coresident / b->group;

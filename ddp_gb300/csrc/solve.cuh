@@ -108,7 +108,7 @@ void slots_free(SlotArrays &sa);
 uint32_t *heuristic_hops_ptr(const ddp_heuristic *h);
 cudaError_t launch_slots(int hk, int grid, int block, bool coop, DevGraph G, SlotArrays sa, BatchArgs A,
                          cudaStream_t st);
-int slots_per_sm(int hk, int block);
+int slots_per_sm(int hk, int block, bool grouped);
 int device_sms();
 uint32_t auto_delta(const ddp_graph *g);
 uint32_t auto_delta_bidir(const ddp_graph *g);
