@@ -20,16 +20,30 @@
 //              direction; two nodes share a sector, which pays where node
 //              ids have spatial locality.  Needs a touched log and a reset.
 //   RecHash    an open-addressing table of epoch-tagged records sized to the
-//              touched set instead of n.
-// Entries carry their direction in the top bit of the node id: ring and far
-// entries are {v | dir << 31, key}.  The ring holds one bucket; when it is
-// full, entries stay in the far pile.
+//              settled set instead of n.
 //
-// Work distribution is the asynchronous engine's (engine_async.cuh): the
-// current bucket (keys below the thresholds) is a pool that warps drain
-// concurrently, chasing their own children first and spilling to the ring;
-// a `pending` count in shared memory ends the bucket.  Between buckets the
-// far pile is split at each advancing direction's threshold + delta.
+// Open set: a window of 32 bucket lists per direction (bucket = key / width)
+// in the slot's far memory, written once per push and read once per pop, and
+// a pile for entries past the window or past a list's room, which are put
+// into lists when the window reaches them.  The search runs in waves.  A wave
+// expands the children of the last one that fell into buckets already opened
+// (kept in shared memory) and, while these are fewer than the CTA can expand
+// at once, opens the smallest bucket of the advancing direction(s) as well.
+// A small team of lanes expands one entry, so a wave costs the dependent
+// loads of one entry (row bounds and record together, then arcs) however
+// many it holds; draining each bucket to the end before the next is opened
+// spent most waves on a few last children.
+//
+// Lazy labels (LAZY; graphs without coordinates): a relaxation pushes
+// {node, g, parent} without touching the node's record; the label is
+// installed when the entry is popped and found smaller.  A search of a random
+// digraph pushes eight entries for each one it pops (35k against 4.5k at 4M
+// nodes), so seven eighths of the random record reads and writes are never
+// made.  The meeting test needs only the nodes that the other side settled:
+// a bit filter per direction in shared memory answers "not settled" for most
+// arcs, and only its hits read the record.  On graphs with coordinates nodes
+// are reached from several sides and most relaxations do not improve, so
+// labels are installed at once there (eager).
 //
 // Meeting: relaxing arc (u, v) in direction dir with v's other-side label
 // finite offers mu = g(u) + w + g_other(v), kept with the arc's forward-side
@@ -38,104 +52,80 @@
 // has g_f(x) + w + g_r(y) == mu, and the path is s .. x (forward parents),
 // y .. t (reverse successors).
 //
-// Balance: each direction keeps its own threshold T_d, and a split advances
-// direction d only while its open set is at most twice the other's (plus a
+// Balance: each direction keeps its own position, and a wave opens a bucket
+// of direction d only while its open set is at most twice the other's (plus a
 // little), so the search grows the smaller ball, as bidirectional Dijkstra
 // expands the side with the smaller queue.  A query whose source has only
 // heavy out-arcs then advances the forward side alone instead of letting the
 // reverse ball grow far past the meeting radius.
 //
 // Stop rule (bidirectional Dijkstra; stated here for keys equal to g, and
-// with 2 mu in place of mu for potential keys): after a bucket is drained,
-// every node with a forward distance below the smallest open forward key a
-// is final and expanded, and likewise below b in reverse.  When
+// with 2 mu in place of mu for potential keys): between waves, every node
+// with a forward distance below a (the smallest key of the next wave's
+// children, or the edge of the smallest bucket not opened) is final and
+// expanded, and likewise below b in reverse.  When
 // a + b >= mu, a shorter s-t path P would hold an arc (x, y) with d_s(x) < a and
 // d_t(y) < b; both ends were expanded with final labels, and whichever
-// expansion read the other's word second saw it final (labels are
-// installed by an atomic that completes before the entry is pushed, and
-// the pair is read from L2), so mu <= len(P): no shorter path exists.  An
-// empty direction (a or b infinite) also ends the search.  Relaxations and
-// far entries with g >= mu are dropped: no path through them is shorter.
+// expansion came second saw the other's final label (a label, and its filter
+// bit, are installed by atomics that complete before the node's arcs are
+// walked, and records are read from L2), so mu <= len(P): no shorter path
+// exists.  An empty direction also ends the search.  Within a wave the same
+// bound prunes: an entry with key + (the other side's bound) >= mu is
+// dropped, since a path through it either ends at a node the other side has
+// yet to settle (length >= mu) or meets a settled node, which its arc offered.
 #pragma once
 
 #include "engine_async.cuh"
 
 namespace ddp {
 
-// Longest sleep (ns) of an idle warp's poll for bucket work.  With 64 ns
-// polls, idle warps executed half of all instructions of a batch; backing
-// off to 1 us halves the instruction count and costs no time.
-#ifndef DDP_BIDIR_SPIN_CAP
-#define DDP_BIDIR_SPIN_CAP 1024
-#endif
-
-// Fewest ring entries a warp claims at once (at most 32).  A warp claims
-// ceil(available / warps) entries, clamped to [DDP_BIDIR_CLAIM_MIN, 32]:
-// a bucket of a few hundred entries then keeps every warp busy instead of
-// queueing 32-entry chunks (8 dependent rounds of arcs each) on a few.
-#ifndef DDP_BIDIR_CLAIM_MIN
-#define DDP_BIDIR_CLAIM_MIN 4
-#endif
-
-// Far entries a lane loads at once when a split scans the far pile.
-#ifndef DDP_BIDIR_SPLIT_UNROLL
-#define DDP_BIDIR_SPLIT_UNROLL 4
-#endif
-
 constexpr uint32_t DIR_BIT = 0x80000000u;
 constexpr uint32_t NODE_MASK = 0x7FFFFFFFu;
 
-struct BiQ {
-    int head, tail;     // ring positions of the current bucket
-    int pending;        // entries pushed to the bucket and not yet retired
-    int far_cnt;        // far pushes appended this bucket
-    int alt_cnt;        // split: far entries kept
-    int status;
-    unsigned int minkey[2];  // split: smallest key left open, per direction
-    int open_dir[2];         // far entries per direction (kept by the last split + pushed since)
-    int moved_dir[2];        // split: entries moved to the ring, per direction
-    unsigned long long mu;   // (best s-t length << 32) | forward-side tail of its arc
+constexpr int WAVE_LISTS = 32;     // bucket lists per direction (a power of two, one per lane)
+constexpr int WAVE_NEAR = 1024;    // entries of one wave held in shared memory
+constexpr int WAVE_ROOM = 4096;    // entries per list at most
+// A wave of fewer children also opens a bucket.  4M nodes, 4,096 pairs: 16 ->
+// 22 waves a query, 32 -> 20, 64 -> 18 but 7 % more expansions; 2048 x 2048
+// maze, longest of 16: 16 -> 5,886 waves and 470k expansions, 32 -> 3,285 and
+// 591k, 64 -> 2,530 and 792k (29.4, 20.0, 21.9 ms); buckets drained one by
+// one: 12,949 waves, 524k, 42.6 ms.
+constexpr int WAVE_FILL = 32;
+// How many buckets past its smallest unexpanded key a direction may open.
+// Without a limit a search that starts along a chain of single arcs opens a
+// bucket per wave, and when its ball grows at last all of it counts as
+// opened (4M nodes: 472k expansions and 33 ms for one such query, 15k and
+// 1.3 ms with 2).  Frontiers on graphs with coordinates grow slowly and
+// profit from more overlap (maze, 2 -> 25.9 ms, 8 -> 19.4, 16 -> 19.1).
+constexpr uint32_t WAVE_AHEAD = 2, WAVE_AHEAD_XY = 16;
+constexpr int WAVE_FILTER = 1024;  // words of a direction's settled filter (32,768 bits)
+
+// What a wave expands, decided between two waves by the CTA's first warp.
+struct WavePlan {
+    int m;                // children of the last wave
+    int n[2];             // entries of the buckets opened now
+    uint32_t c[2];        // last bucket opened, per direction
+    uint32_t lo[2];       // first bucket of the lists' window
+    uint32_t lim[2];      // keys below belong to opened buckets
+    uint32_t lb[2];       // keys below are settled and expanded
+    int act;              // 0: expand, 1: done, 2: the pile's turn
 };
 
-// Reserves k ring slots (lane 0 only); returns the first position or -1 when
-// the ring would overflow (the caller then sends the entries to far).
-__device__ __forceinline__ int bi_ring_reserve(BiQ *sq, int k, int cap) {
-    for (;;) {
-        const int t = *(volatile int *)&sq->tail;
-        if (t + k > cap) return -1;
-        if (atomicCAS(&sq->tail, t, t + k) == t) return t;
-    }
-}
-
-// Flushes a warp's staged split entries to the ring; entries past the
-// ring's capacity go to the far pile `falt` instead, where they stay open
-// (the stop rule reads its keys) and move at the next split.
-__device__ __forceinline__ void flush_ring_or_far(uint2 *buf, int &cnt, BiQ *sq, uint2 *ring, int cap, uint2 *falt,
-                                                  int64_t cap_f, SearchCtl *ctl) {
-    if (cnt == 0) return;  // warp-uniform
-    __syncwarp();
-    const int lane = threadIdx.x & 31;
-    int b = 0;
-    if (lane == 0) b = atomicAdd(&sq->tail, cnt);
-    b = __shfl_sync(FULL, b, 0);
-    const int over = min(cnt, max(0, b + cnt - cap));
-    int fb = 0;
-    if (over > 0 && lane == 0) fb = atomicAdd(&sq->alt_cnt, over);
-    fb = __shfl_sync(FULL, fb, 0);
-    const int first_over = max(b, cap);
-    for (int i = lane; i < cnt; i += 32) {
-        const int pos = b + i;
-        if (pos < cap) {
-            ring[pos] = buf[i];
-        } else {
-            const int64_t p2 = (int64_t)fb + (pos - first_over);
-            if (p2 < cap_f) falt[p2] = buf[i];
-            else raise_err(ctl, 0, ST_OVERFLOW);
-        }
-    }
-    __syncwarp();
-    cnt = 0;
-}
+// Shared memory of one search.
+struct WaveQ {
+    unsigned long long mu;           // (best s-t length << 32) | forward-side tail of its arc
+    WavePlan plan;
+    int lcnt[2][WAVE_LISTS];         // entries pushed per bucket list (those past its room went to the pile)
+    int near[3];                     // children per wave, rotating
+    unsigned int near_min[3][2];     // their smallest key per direction
+    int pile_n, pile_alt;            // entries in the pile; kept by the pass over it
+    int pile_dir[2];                 // pile entries per direction
+    unsigned int pile_min[2];        // their smallest key
+    int status;
+    int touched;
+    uint32_t settled[2][WAVE_FILTER];  // lazy labels: filter over settled nodes
+    uint4 list[2][WAVE_NEAR];
+};
 
 // Unit of node v in direction dir of a paired slot's records.
 __device__ __forceinline__ uint4 *unit_ptr(unsigned long long *st, int v, uint32_t dir) {
@@ -182,6 +172,10 @@ struct UnitOps16 {
     using U = uint4;
     static constexpr bool logs = false;  // no touched log: epochs retire the records
     __device__ static U ld(const U *p) { return __ldcg(p); }
+    __device__ static void ld2(const U *p, U &f, U &r) {
+        f = __ldcg(p);
+        r = __ldcg(p + 1);
+    }
     __device__ static uint32_t g(const U &u, uint32_t ep) { return unit_g(u, ep); }
     __device__ static int32_t link(const U &u) { return (int32_t)u.z; }
     __device__ static U make(uint32_t ep, uint32_t g, uint32_t parent, uint32_t keyw) {
@@ -215,6 +209,11 @@ struct RecPair16 {
     __device__ U *claim(int v, uint32_t) const { return st + 2 * (size_t)v; }
     __device__ uint32_t keyw(int) const { return 0u; }
     __device__ static U ld(const U *p) { return __ldcg(p); }
+    __device__ static void ld2(const U *p, U &f, U &r) {
+        const ulonglong2 x = __ldcg(reinterpret_cast<const ulonglong2 *>(p));
+        f = x.x;
+        r = x.y;
+    }
     __device__ static uint32_t g(const U &u, uint32_t) { return min(st_g(u), INF_G); }
     __device__ static int32_t link(const U &u) { return st_parent(u); }
     __device__ static U make(uint32_t, uint32_t g, uint32_t parent, uint32_t) {
@@ -266,13 +265,21 @@ struct RecHash : UnitOps16 {
 };
 
 // Path s..t from the meeting word; returns its length (0 when no path).
+// Called by the CTA's first warp.  buf: two arrays of PATH_BUF node ids in
+// shared memory.  The lanes test the arcs of the meeting row together, then
+// lane 0 walks to s and lane 1 to t at the same time, once: a walk is a chain
+// of dependent loads (three walks by one thread took 10-17 us a query on
+// random digraphs, a tenth of its service time).
+constexpr int PATH_BUF = 4096;
 template <class Rec>
 __device__ inline int32_t write_path_bidir(const DevGraph &G, const Rec &R, uint32_t ep, int32_t s, int32_t t,
-                                           unsigned long long mu, int32_t *path, int32_t cap, int *status) {
+                                           unsigned long long mu, int32_t *path, int32_t cap, int *status,
+                                           int32_t *buf) {
     const uint32_t cost = uint32_t(mu >> 32);
+    const int lane = lane_id();
     if (cost >= INF_G) return 0;
     if (s == t) {
-        if (cap > 0) path[0] = s;
+        if (cap > 0 && lane == 0) path[0] = s;
         return 1;
     }
     // label of node v in direction dir (unit absent: unreached) and its
@@ -292,45 +299,51 @@ __device__ inline int32_t write_path_bidir(const DevGraph &G, const Rec &R, uint
     const uint32_t gx = lab(x, 0, &lk);
     int32_t y = -1;
     const int r1 = row_end(G.off, G.oend, x);
-    for (int k = row_begin(G.off, G.oend, x); k < r1 && y < 0; k++) {
-        const uint2 a = G.oend ? __ldcg(G.arc + k) : __ldg(G.arc + k);
-        if ((int)a.x < 0) continue;
-        const uint32_t gr = lab((int)a.x, 1, &lk);
-        if (gr < INF_G && (uint64_t)gx + a.y + gr == cost) y = (int32_t)a.x;
+    for (int k0 = row_begin(G.off, G.oend, x); k0 < r1 && y < 0; k0 += 32) {
+        const int k = k0 + lane;
+        const uint2 a = k < r1 ? (G.oend ? __ldcg(G.arc + k) : __ldg(G.arc + k)) : make_uint2(0xFFFFFFFFu, 0u);
+        bool hit = false;
+        if ((int)a.x >= 0) {
+            const uint32_t gr = lab((int)a.x, 1, &lk);
+            hit = gr < INF_G && (uint64_t)gx + a.y + gr == cost;
+        }
+        const unsigned m = __ballot_sync(FULL, hit);
+        if (m) y = __shfl_sync(FULL, (int)a.x, __ffs(m) - 1);
     }
     if (y < 0) {
-        atomicOr(status, ST_TIMEOUT);  // no meeting arc: report the query failed
+        if (lane == 0) atomicOr(status, ST_TIMEOUT);  // no meeting arc: report the query failed
         return 0;
     }
-    // lengths of s..x (forward parents) and y..t (reverse successors)
-    int32_t lf = 0, lr = 0;
-    for (int32_t c = x; c >= 0 && lf <= G.n;) {
-        lf++;
-        if (c == s) break;
-        lab(c, 0, &lk);
-        c = lk;
+    // x..s by forward parents (lane 0) and y..t by reverse successors (lane 1)
+    int32_t len = 0;
+    if (lane < 2) {
+        const int32_t end = lane ? t : s;
+        for (int32_t c = lane ? y : x; c >= 0 && len <= G.n;) {
+            if (len < PATH_BUF) buf[lane * PATH_BUF + len] = c;
+            len++;
+            if (c == end) break;
+            lab(c, (uint32_t)lane, &lk);
+            c = lk;
+        }
     }
-    for (int32_t c = y; c >= 0 && lr <= G.n;) {
-        lr++;
-        if (c == t) break;
-        lab(c, 1, &lk);
-        c = lk;
+    __syncwarp();
+    const int32_t lf = __shfl_sync(FULL, len, 0), lr = __shfl_sync(FULL, len, 1);
+    if (lf + lr > cap && lane == 0) atomicOr(status, ST_PATH_TRUNC);
+    if (lf <= PATH_BUF && lr <= PATH_BUF) {
+        for (int32_t i = lane; i < lf; i += 32)
+            if (lf - 1 - i < cap) path[lf - 1 - i] = buf[i];
+        for (int32_t i = lane; i < lr; i += 32)
+            if (lf + i < cap) path[lf + i] = buf[PATH_BUF + i];
+    } else if (lane < 2) {
+        // longer than the buffer: a second walk writes it
+        int32_t i = lane ? lf : lf - 1;
+        for (int32_t c = lane ? y : x; c >= 0 && i >= 0 && i < lf + lr; i += lane ? 1 : -1) {
+            if (i < cap) path[i] = c;
+            lab(c, (uint32_t)lane, &lk);
+            c = lk;
+        }
     }
-    const int32_t len = lf + lr;
-    if (len > cap) atomicOr(status, ST_PATH_TRUNC);
-    int32_t i = lf - 1;
-    for (int32_t c = x; c >= 0 && i >= 0; i--) {
-        if (i < cap) path[i] = c;
-        lab(c, 0, &lk);
-        c = lk;
-    }
-    i = lf;
-    for (int32_t c = y; c >= 0 && i < len; i++) {
-        if (i < cap) path[i] = c;
-        lab(c, 1, &lk);
-        c = lk;
-    }
-    return len;
+    return lf + lr;
 }
 
 // ---- potentials (bidirectional A*) ------------------------------------------
@@ -402,51 +415,105 @@ __device__ __forceinline__ uint64_t bi_key_bound(uint32_t mu) {
     return Pot::on ? 2 * (uint64_t)mu : (uint64_t)mu;
 }
 
+// What an open entry holds: {node | dir << 31, key} and, with lazy labels, the
+// parent, with potentials, the label g that the key was made from.
+template <bool WIDE>
+struct WaveEntry {
+    using T = uint4;
+    __device__ static T make(uint32_t vd, uint32_t key, uint32_t x) { return make_uint4(vd, key, x, 0u); }
+    __device__ static uint32_t extra(const T &e) { return e.z; }
+};
+template <>
+struct WaveEntry<false> {
+    using T = uint2;
+    __device__ static T make(uint32_t vd, uint32_t key, uint32_t) { return make_uint2(vd, key); }
+    __device__ static uint32_t extra(const T &e) { return e.y; }  // no potentials: the key is g
+};
+
 // ep: the slot's epoch for this query (never 0; units of other epochs read
 // as unreached).
-template <class Pot, class Rec>
+template <bool LAZY, class Pot, class Rec>
 __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, const SearchParams &P, uint32_t ep,
-                                      WarpRows *wrows, BiQ *sq, const Pot &pot, const Rec &R) {
+                                      WaveQ *q, const Pot &pot, const Rec &R) {
+    static_assert(!(LAZY && Pot::on), "lazy labels are keyed by g");
+    using WE = WaveEntry<LAZY || Pot::on>;
+    using E = typename WE::T;
     SearchCtl *ctl = B.ctl;
     const int lane = lane_id();
-    const int warp = threadIdx.x >> 5;
-    const int nw = (int)(blockDim.x >> 5);
-    WarpRows &wr = wrows[warp];
-    uint2 *ring = B.q0;
-    const int cap = (int)min(B.cap_q, (int64_t)0x3FFFFFFF);
+    // arcs per lane whose loads are in flight together
+    constexpr int AU = Pot::on ? 1 : LAZY ? 4 : 2;
+    constexpr uint32_t ahead = LAZY ? WAVE_AHEAD : WAVE_AHEAD_XY;
+    // the slot's far memory: 2 x 32 lists (a quarter), two halves of a pile,
+    // two spill areas for waves that outgrow shared memory (an eighth each)
+    const int64_t total = 2 * B.cap_f * (int64_t)sizeof(uint2) / (int64_t)sizeof(E);
+    const int room = (int)min(total / (8 * WAVE_LISTS), (int64_t)WAVE_ROOM);  // entries per list
+    const int scap = (int)min(total / 8, (int64_t)0x0FFFFFFF);
+    const int pcap = (int)min((total - (int64_t)2 * WAVE_LISTS * room - 2 * (int64_t)scap) / 2, (int64_t)0x3FFFFFFF);
+    E *lists = reinterpret_cast<E *>(B.f0);
+    E *pile0 = lists + (int64_t)2 * WAVE_LISTS * room;
+    E *spill0 = pile0 + 2 * (int64_t)pcap;
+    E *near0 = reinterpret_cast<E *>(q->list[0]);
+    constexpr int NEAR_STRIDE = (int)(sizeof(q->list[0]) / sizeof(E));
+    // keys are doubled with potentials: so is the bucket width
+    const uint32_t dk = Pot::on ? 2 * P.delta : P.delta;
+    constexpr uint32_t NONE = 0xFFFFFFFFu;
+    // bucket of a key: one multiplication by 2^32 / width (buckets then are a
+    // little wider than the width: what counts is that they grow with the
+    // key and that edge(b) is the smallest key of bucket b)
+    const uint32_t rec_dk = dk <= 1 ? NONE : (uint32_t)(0x100000000ull / dk);
+    auto bucket = [&](uint32_t key) -> uint32_t { return __umulhi(key, rec_dk); };
+    auto edge = [&](uint32_t b) -> uint32_t {
+        const uint64_t k = (((uint64_t)b << 32) + rec_dk - 1) / rec_dk;
+        return k >= NONE ? NONE : (uint32_t)k;
+    };
 
+    for (int i = threadIdx.x; i < 2 * WAVE_LISTS; i += blockDim.x) q->lcnt[0][i] = 0;
+    if constexpr (LAZY)
+        for (int i = threadIdx.x; i < 2 * WAVE_FILTER; i += blockDim.x) q->settled[0][i] = 0u;
+    __syncthreads();
     if (threadIdx.x == 0) {
         ctl->iters = 0;
         ctl->expanded = ctl->scanned = ctl->relaxed = 0;
         ctl->far_scanned = 0;
-        sq->head = 0;
-        sq->tail = 0;
-        sq->pending = 0;
-        sq->far_cnt = 0;
-        sq->alt_cnt = 0;
-        sq->status = 0;
-        sq->minkey[0] = sq->minkey[1] = 0xFFFFFFFFu;
-        sq->open_dir[0] = sq->open_dir[1] = 0;
-        sq->moved_dir[0] = sq->moved_dir[1] = 0;
+        ctl->touched = 0;
+        for (int i = 0; i < 3; i++) {
+            q->near[i] = 0;
+            q->near_min[i][0] = q->near_min[i][1] = NONE;
+        }
+        q->pile_n = 0;
+        q->pile_dir[0] = q->pile_dir[1] = 0;
+        q->pile_min[0] = q->pile_min[1] = NONE;
+        q->status = room < 1 ? ST_OVERFLOW : 0;
+        q->touched = 0;
         if (P.s == P.t) {
-            sq->mu = (unsigned long long)(uint32_t)P.s;  // length 0
-            ctl->touched = 0;
+            q->mu = (unsigned long long)(uint32_t)P.s;  // length 0
         } else {
-            sq->mu = ~0ull;
-            // the endpoints' records (a fresh slot's table has room for two)
-            typename Rec::U *rs = R.claim(P.s, ep);
-            typename Rec::U *rt = R.claim(P.t, ep);
-            rs[0] = Rec::make(ep, 0u, 0xFFFFFFFFu, R.keyw(P.s));
-            rt[1] = Rec::make(ep, 0u, 0xFFFFFFFFu, 0u);
-            if constexpr (Rec::logs) {
-                B.touched[0] = P.s;
-                B.touched[1] = P.t;
+            q->mu = ~0ull;
+            if constexpr (!LAZY) {
+                typename Rec::U *rs = R.claim(P.s, ep);
+                typename Rec::U *rt = R.claim(P.t, ep);
+                rs[0] = Rec::make(ep, 0u, NONE, R.keyw(P.s));
+                rt[1] = Rec::make(ep, 0u, NONE, 0u);
+                if constexpr (Rec::logs) {
+                    B.touched[0] = P.s;
+                    B.touched[1] = P.t;
+                }
+                q->touched = 2;
             }
-            ctl->touched = 2;
-            ring[0] = make_uint2((uint32_t)P.s, bi_key<Pot>(0u, 0u, pot.at(P.s)));
-            ring[1] = make_uint2((uint32_t)P.t | DIR_BIT, bi_key<Pot>(0u, 1u, pot.at(P.t)));
-            sq->tail = 2;
-            sq->pending = 2;
+            const uint32_t ks = bi_key<Pot>(0u, 0u, pot.at(P.s)), kt = bi_key<Pot>(0u, 1u, pot.at(P.t));
+            q->plan.lo[0] = bucket(ks);
+            q->plan.lo[1] = bucket(kt);
+            q->plan.c[0] = q->plan.lo[0] - 1;  // nothing opened yet
+            q->plan.c[1] = q->plan.lo[1] - 1;
+            if (room >= 1) {
+                // lazy: no parent; else the label
+                const uint32_t x = LAZY ? NONE : 0u;
+                const int l0 = (int)(q->plan.lo[0] % WAVE_LISTS), l1 = (int)(q->plan.lo[1] % WAVE_LISTS);
+                lists[(int64_t)l0 * room] = WE::make((uint32_t)P.s, ks, x);
+                lists[(int64_t)(WAVE_LISTS + l1) * room] = WE::make((uint32_t)P.t | DIR_BIT, kt, x);
+                q->lcnt[0][l0] = 1;
+                q->lcnt[1][l1] = 1;
+            }
         }
     }
     __syncthreads();
@@ -457,434 +524,387 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
         return r0;
     }
 
-    // ring and far entries hold {v | dir << 31, key}
-    uint2 *fcur = reinterpret_cast<uint2 *>(B.f0), *falt = reinterpret_cast<uint2 *>(B.f1);
-    uint2 *sf2 = reinterpret_cast<uint2 *>(wr.sf);  // staged far pushes
-    int64_t nfar = 0;
-    // the current bucket holds keys < T0 (forward) and < T1 (reverse); lo_d
-    // is a lower bound of direction d's open keys when its last advance
-    // moved nothing (the next advance jumps there)
-    // keys are doubled with potentials: so is the bucket width
-    const uint32_t dk = Pot::on ? 2 * P.delta : P.delta;
-    uint32_t T0 = sat_add(bi_key<Pot>(0u, 0u, pot.at(P.s)), dk), T1 = sat_add(bi_key<Pot>(0u, 1u, pot.at(P.t)), dk);
-    uint32_t lo0 = 0, lo1 = 0;
-    bool do_expand = true;
-    unsigned long long n_exp = 0, n_scan = 0, n_rel = 0, n_first = 0;
-    int phases = 0;
-    const int64_t max_phases = 4 * (int64_t)G.n + (1 << 22);
+    bool flip = false;  // which half the pile is in
+    unsigned long long n_exp = 0, n_scan = 0, n_rel = 0, n_far = 0;
+    unsigned int n_first = 0;
+    int wv = 0;
+    const int64_t max_waves = 4 * (int64_t)G.n + (1 << 22);
+    uint32_t lb0 = 0, lb1 = 0;
+
+    // the length in mu (its high word: one 32-bit read)
+    auto mu_now = [&]() -> uint32_t { return reinterpret_cast<volatile uint32_t *>(&q->mu)[1]; };
+    // the bound that a key must stay below, given the other side's lb
+    auto key_limit = [&](uint32_t mu, uint32_t lbo) -> uint32_t {
+        const uint64_t kb = bi_key_bound<Pot>(mu);
+        return kb <= lbo ? 0u : (uint32_t)min(kb - lbo, (uint64_t)NONE);
+    };
+    uint32_t lim0 = 0, lim1 = 0, lo0 = 0, lo1 = 0;  // the wave's plan
+    auto to_pile = [&](const E e, uint32_t key, uint32_t dir, int *count, E *pile) {
+        const int p = atomicAdd(count, 1);
+        if (p < pcap) pile[p] = e;
+        else atomicOr(&q->status, ST_OVERFLOW);
+        atomicAdd(&q->pile_dir[dir], 1);
+        atomicMin(&q->pile_min[dir], key);
+    };
+    // appends e to bucket b's list, or (past the window, past its room) to the pile
+    auto to_lists = [&](const E e, uint32_t key, uint32_t dir, uint32_t b, int *count, E *pile) {
+        if (b - (dir ? lo1 : lo0) < (uint32_t)WAVE_LISTS) {
+            const int l = (int)(dir * WAVE_LISTS + (b & (WAVE_LISTS - 1)));
+            const int p = atomicAdd(&q->lcnt[0][l], 1);
+            if (p < room) {
+                lists[(int64_t)l * room + p] = e;
+                return;
+            }
+        }
+        to_pile(e, key, dir, count, pile);
+    };
+    // an entry of an opened bucket: wave w expands it
+    auto to_near = [&](const E e, uint32_t key, uint32_t dir, int w) -> bool {
+        const int p = atomicAdd(&q->near[w % 3], 1);
+        if (p >= WAVE_NEAR + scap) return false;
+        atomicMin(&q->near_min[w % 3][dir], key);
+        if (p < WAVE_NEAR) near0[(w & 1) * NEAR_STRIDE + p] = e;
+        else spill0[(int64_t)(w & 1) * scap + (p - WAVE_NEAR)] = e;
+        return true;
+    };
+    auto push = [&](uint32_t vd, uint32_t key, uint32_t x) {
+        const uint32_t dir = vd >> 31;
+        const E e = WE::make(vd, key, x);
+        if (key >= (dir ? lim1 : lim0)) to_lists(e, key, dir, bucket(key), &q->pile_n, pile0 + (flip ? pcap : 0));
+        else if (!to_near(e, key, dir, wv + 1)) atomicOr(&q->status, ST_OVERFLOW);
+    };
+    // expands one entry with a team of 2^tsh lanes
+    auto expand = [&](const E en, const int tsh) {
+        const int tw = 1 << tsh, sub = lane & (tw - 1);
+        const uint32_t vd = en.x, key = en.y;
+        const uint32_t dir = vd >> 31;
+        const int u = (int)(vd & NODE_MASK);
+        const uint32_t lbo = dir ? lb0 : lb1;
+        // row bounds load beside the record
+        const int r0 = dir ? row_begin(G.roff, G.roend, u) : row_begin(G.off, G.oend, u);
+        const int r1 = dir ? row_end(G.roff, G.roend, u) : row_end(G.off, G.oend, u);
+        const uint2 *arcs = dir ? G.rarc : G.arc;
+        uint2 a[AU];
+        auto load_arcs = [&](int j) {
+#pragma unroll
+            for (int k = 0; k < AU; k++)
+                a[k] = j + k * tw < r1 ? (G.oend ? __ldcg(arcs + j + k * tw) : __ldg(arcs + j + k * tw))
+                                       : make_uint2(NONE, 0u);
+        };
+        uint32_t gu;
+        bool ok = false;
+        if constexpr (LAZY) {
+            gu = key;
+            typename Rec::U *w = nullptr;
+            typename Rec::U c{};
+            if (sub == 0 && key < key_limit(mu_now(), lbo)) {
+                typename Rec::U *rv = R.claim(u, ep);
+                if (rv) {
+                    w = rv + dir;
+                    c = Rec::ld(w);
+                } else {
+                    atomicOr(&q->status, ST_OVERFLOW);  // the slot's table is full
+                }
+            }
+            load_arcs(r0 + sub);  // beside the label's compare-and-swap
+            if (w) {
+                const typename Rec::U nv = Rec::make(ep, gu, WE::extra(en), dir ? 0u : R.keyw(u));
+                while (gu < Rec::g(c, ep)) {
+                    const typename Rec::U got = Rec::cas(w, c, nv);
+                    if (Rec::eq(got, c)) {
+                        ok = true;
+                        if (Rec::g(c, ep) >= INF_G) {
+                            n_first++;
+                            const uint32_t h = ((uint32_t)u * 0x9E3779B1u) >> 17;
+                            atomicOr(&q->settled[dir][h >> 5], 1u << (h & 31));
+                        }
+                        break;
+                    }
+                    c = got;
+                }
+                // label, then filter bit, then the walk over the arcs
+                __threadfence_block();
+            }
+            ok = __shfl_sync(((1u << tw) - 1u) << (lane & ~(tw - 1)), (int)ok, lane & ~(tw - 1)) != 0;
+        } else {
+            gu = WE::extra(en);
+            const typename Rec::U *ru = R.find(u, ep);
+            const uint32_t gl = Rec::g(Rec::ld(ru + dir), ep);
+            load_arcs(r0 + sub);
+            // current, and a path through it may still be shorter
+            ok = gl == gu && key < key_limit(mu_now(), lbo);
+        }
+        if (!ok) return;
+        if (sub == 0) {
+            n_exp++;
+            n_scan += (unsigned long long)(r1 - r0);
+        }
+        for (int j = r0 + sub;;) {
+            const uint32_t mu = mu_now();
+            // weights below room keep g below min(mu, unreached)
+            const uint32_t top = min(mu, INF_G), room_w = top > gu ? top - gu : 0u;
+            if constexpr (LAZY) {
+#pragma unroll
+                for (int k = 0; k < AU; k++) {
+                    const int v = (int)a[k].x;
+                    if (v < 0 || a[k].y >= room_w) continue;
+                    const uint32_t ng = gu + a[k].y;
+                    const uint32_t h = ((uint32_t)v * 0x9E3779B1u) >> 17;
+                    const uint32_t f0 = *(volatile uint32_t *)&q->settled[0][h >> 5];
+                    const uint32_t f1 = *(volatile uint32_t *)&q->settled[1][h >> 5];
+                    if (((f0 | f1) >> (h & 31)) & 1u) {
+                        // v may be settled: by this side (no need to come
+                        // again) or by the other (the searches meet here)
+                        const typename Rec::U *rv = R.find(v, ep);
+                        if (rv) {
+                            typename Rec::U uf, ur;
+                            Rec::ld2(rv, uf, ur);
+                            const uint64_t c = (uint64_t)ng + Rec::g(dir ? uf : ur, ep);
+                            if (c < mu) atomicMin(&q->mu, (c << 32) | (dir ? (uint32_t)v : (uint32_t)u));
+                            if (Rec::g(dir ? ur : uf, ep) <= ng) continue;
+                        }
+                    }
+                    if (ng >= key_limit(mu_now(), lbo)) continue;
+                    n_rel++;
+                    push((uint32_t)v | (dir << 31), ng, (uint32_t)u);
+                }
+            } else {
+                typename Rec::U uf[AU], ur[AU];
+                uint2 pv[AU];  // {pt(v), ps(v)}
+                bool live[AU];
+                // every load of the step before any is used
+#pragma unroll
+                for (int k = 0; k < AU; k++) {
+                    live[k] = (int)a[k].x >= 0 && a[k].y < room_w;
+                    pv[k] = make_uint2(0u, 0u);
+                    uf[k] = typename Rec::U{};
+                    ur[k] = typename Rec::U{};
+                    if (live[k]) {
+                        Rec::ld2(R.find((int)a[k].x, ep), uf[k], ur[k]);
+                        if constexpr (Pot::on) pv[k] = pot.at((int)a[k].x);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < AU; k++) {
+                    const int v = (int)a[k].x;
+                    const uint32_t ng = gu + a[k].y;
+                    // a path through v is at least g + the bound of the other side
+                    if (!live[k] || (Pot::on && (uint64_t)ng + (dir ? pv[k].y : pv[k].x) >= (uint64_t)mu)) continue;
+                    const uint64_t mc = (uint64_t)ng + Rec::g(dir ? uf[k] : ur[k], ep);
+                    if (mc < mu) atomicMin(&q->mu, (mc << 32) | (dir ? (uint32_t)v : (uint32_t)u));
+                    const uint32_t nk = bi_key<Pot>(ng, dir, pv[k]);
+                    typename Rec::U c = dir ? ur[k] : uf[k];
+                    if (ng >= Rec::g(c, ep) || nk >= key_limit(mu_now(), lbo)) continue;
+                    const typename Rec::U nv = Rec::make(ep, ng, (uint32_t)u, dir ? 0u : R.keyw(v));
+                    typename Rec::U *rv = R.claim(v, ep);
+                    bool inst = false;
+                    do {
+                        const typename Rec::U got = Rec::cas(rv + dir, c, nv);
+                        if (Rec::eq(got, c)) {
+                            inst = true;
+                            break;
+                        }
+                        c = got;
+                    } while (ng < Rec::g(c, ep));
+                    if (!inst) continue;
+                    n_rel++;
+                    if (Rec::g(c, ep) >= INF_G) {
+                        if constexpr (Rec::logs) {
+                            // first touches of either direction (a node may be
+                            // logged twice; the reset takes it twice)
+                            const int p = atomicAdd(&q->touched, 1);
+                            if ((int64_t)p < 2 * (int64_t)G.n) B.touched[p] = v;
+                        } else {
+                            n_first++;
+                        }
+                    }
+                    push((uint32_t)v | (dir << 31), nk, ng);
+                }
+            }
+            j += AU * tw;
+            if (j >= r1) break;
+            load_arcs(j);
+        }
+    };
 
     for (;;) {
-        if (do_expand) {
-            int c_f = 0, c_loc = 0, c_t = 0;  // staged far pushes, own children, touches
-            int nf0 = 0, nf1 = 0;             // far pushes per direction (this lane)
+        __syncthreads();  // the last wave's pushes are in place
+        if (threadIdx.x < 32) {
+            // ---- plan the next wave ------------------------------------------
+            WavePlan p;
+            const int cur = wv % 3;
+            p.m = min(q->near[cur], WAVE_NEAR + scap);
+            p.c[0] = q->plan.c[0];
+            p.c[1] = q->plan.c[1];
+            // the buckets opened are no longer in the window
+            p.lo[0] = p.c[0] + 1;
+            p.lo[1] = p.c[1] + 1;
+            p.n[0] = p.n[1] = 0;
+            p.act = 0;
+            const int x0 = min(q->lcnt[0][(p.lo[0] + lane) & (WAVE_LISTS - 1)], room);
+            const int x1 = min(q->lcnt[1][(p.lo[1] + lane) & (WAVE_LISTS - 1)], room);
+            const unsigned m0 = __ballot_sync(FULL, x0 > 0), m1 = __ballot_sync(FULL, x1 > 0);
+            const int pd0 = q->pile_dir[0], pd1 = q->pile_dir[1];
+            const uint32_t nb0 = m0 ? p.lo[0] + (uint32_t)__ffs(m0) - 1u : NONE;
+            const uint32_t nb1 = m1 ? p.lo[1] + (uint32_t)__ffs(m1) - 1u : NONE;
+            const uint32_t pm0 = pd0 ? q->pile_min[0] : NONE, pm1 = pd1 ? q->pile_min[1] : NONE;
+            const uint32_t k0 = q->near_min[cur][0], k1 = q->near_min[cur][1];
+            const uint32_t e0 = nb0 == NONE ? NONE : edge(nb0), e1 = nb1 == NONE ? NONE : edge(nb1);
+            p.lb[0] = min(min(k0, pm0), e0);
+            p.lb[1] = min(min(k1, pm1), e1);
+            // an empty direction, or nothing open that could be shorter: mu is the distance
+            if (p.lb[0] == NONE || p.lb[1] == NONE ||
+                (uint64_t)p.lb[0] + p.lb[1] >= bi_key_bound<Pot>(mu_now()) || q->status) {
+                p.act = 1;
+            } else if (p.m >= WAVE_FILL) {
+                // enough to do
+            } else if (pm0 < e0 || pm1 < e1) {
+                // the pile holds a direction's smallest bucket (a bucket whose
+                // list was full leaves the rest there)
+                p.act = 2;
+                if (nb0 == NONE && pd0 && pm0 >= edge(p.lo[0])) p.lo[0] = bucket(pm0);  // nothing listed below
+                if (nb1 == NONE && pd1 && pm1 >= edge(p.lo[1])) p.lo[1] = bucket(pm1);
+                p.c[0] = p.lo[0] - 1;
+                p.c[1] = p.lo[1] - 1;
+            } else {
+                // open the next bucket of the direction(s) whose open set is
+                // not much larger than the other's
+                int o0 = x0, o1 = x1;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    o0 += __shfl_xor_sync(FULL, o0, o);
+                    o1 += __shfl_xor_sync(FULL, o1, o);
+                }
+                o0 += pd0;
+                o1 += pd1;
+                if (nb0 != NONE && ((int64_t)o0 <= 2 * (int64_t)o1 + 64 || nb1 == NONE) &&
+                    (k0 == NONE || nb0 - bucket(k0) <= ahead)) {
+                    p.c[0] = nb0;
+                    p.n[0] = __shfl_sync(FULL, x0, __ffs(m0) - 1);
+                    p.lo[0] = nb0;
+                }
+                if (nb1 != NONE && ((int64_t)o1 <= 2 * (int64_t)o0 + 64 || nb0 == NONE) &&
+                    (k1 == NONE || nb1 - bucket(k1) <= ahead)) {
+                    p.c[1] = nb1;
+                    p.n[1] = __shfl_sync(FULL, x1, __ffs(m1) - 1);
+                    p.lo[1] = nb1;
+                }
+            }
+            p.lim[0] = edge(p.c[0] + 1);
+            p.lim[1] = edge(p.c[1] + 1);
+            __syncwarp();
+            if (lane == 0) {
+                // a bucket opened gives its list back after this wave: lo
+                // keeps the bucket that would reuse it out of the window
+                if (p.n[0]) q->lcnt[0][p.c[0] & (WAVE_LISTS - 1)] = 0;
+                if (p.n[1]) q->lcnt[1][p.c[1] & (WAVE_LISTS - 1)] = 0;
+                const int nn = (wv + 2) % 3;  // the counters of the wave after the next
+                q->near[nn] = 0;
+                q->near_min[nn][0] = q->near_min[nn][1] = NONE;
+                q->plan = p;
+            }
+        }
+        __syncthreads();
+        const int act = q->plan.act;
+        lb0 = q->plan.lb[0];
+        lb1 = q->plan.lb[1];
+        lim0 = q->plan.lim[0];
+        lim1 = q->plan.lim[1];
+        lo0 = q->plan.lo[0];
+        lo1 = q->plan.lo[1];
+        if (act == 1) break;
+        if (act == 2) {
+            // put what the window covers of the pile into the lists, and
+            // what belongs to buckets already opened into this wave
+            const int n = min(q->pile_n, pcap);
+            const uint32_t mu = mu_now();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                q->pile_alt = 0;
+                q->pile_dir[0] = q->pile_dir[1] = 0;
+                q->pile_min[0] = q->pile_min[1] = NONE;
+                n_far += (unsigned long long)n;
+            }
+            __syncthreads();
+            const E *src = pile0 + (flip ? pcap : 0);
+            E *dst = pile0 + (flip ? 0 : pcap);
+            for (int i = threadIdx.x; i < n; i += blockDim.x) {
+                const E e = __ldcg(src + i);
+                const uint32_t dir = e.x >> 31;
+                if (e.y >= key_limit(mu, dir ? lb0 : lb1)) continue;
+                if (e.y >= (dir ? lim1 : lim0)) to_lists(e, e.y, dir, bucket(e.y), &q->pile_alt, dst);
+                else if (!to_near(e, e.y, dir, wv)) to_pile(e, e.y, dir, &q->pile_alt, dst);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) q->pile_n = q->pile_alt;
+            flip = !flip;
+            continue;  // plan again
+        }
+        if (wv >= max_waves) {
+            if (threadIdx.x == 0) atomicOr(&ctl->status, ST_TIMEOUT);
+            break;
+        }
+        // ---- the wave ---------------------------------------------------------
+        const int m = q->plan.m, n0 = q->plan.n[0], n1 = q->plan.n[1];
+        const E *l0 = lists + (int64_t)(q->plan.c[0] & (WAVE_LISTS - 1)) * room;
+        const E *l1 = lists + (int64_t)(WAVE_LISTS + (q->plan.c[1] & (WAVE_LISTS - 1))) * room;
+        const E *cur = near0 + (wv & 1) * NEAR_STRIDE;
+        if (threadIdx.x == 0) n_far += (unsigned long long)(n0 + n1);
+        const int W = m + n0 + n1;
+        auto entry = [&](int i) -> E {
+            if (i < m) return i < WAVE_NEAR ? cur[i] : __ldcg(spill0 + (int64_t)(wv & 1) * scap + (i - WAVE_NEAR));
+            return i - m < n0 ? __ldcg(l0 + (i - m)) : __ldcg(l1 + (i - m - n0));
+        };
+        // lanes per entry: the wave's entries spread over the CTA, at least
+        // two lanes each with lazy labels (a lane filters four arcs at once),
+        // four otherwise (each arc is a record read and maybe a
+        // compare-and-swap).  4M nodes, 4,096 pairs: 2 lanes 3.74 ms, 4 lanes
+        // 4.36 ms, 1 lane 3.75 ms; 1M points, 200 pairs: 4 lanes 42.9 ms, 2
+        // lanes 53.5 ms
+        const int nt = (int)blockDim.x;
+        const int tsh = W * 16 <= nt ? 4 : W * 8 <= nt ? 3 : (!LAZY || W * 4 <= nt) ? 2 : 1;
+        const int teams = nt >> tsh;
+        int i = (int)threadIdx.x >> tsh;
+        if (i < W) {
+            E e = entry(i);
             for (;;) {
-                const uint32_t mu = uint32_t(*(volatile unsigned long long *)&sq->mu >> 32);
-                // 1. take work: own children first, else claim from the ring
-                int n = 0;
-                uint2 en = make_uint2(RING_EMPTY, 0u);
-                if (c_loc > 0) {
-                    n = min(32, c_loc);
-                    if (lane < n) en = wr.sn[c_loc - n + lane];
-                    c_loc -= n;
-                    __syncwarp();
-                } else {
-                    int h0 = 0;
-                    if (lane == 0) {
-                        n = -1;
-                        // an idle warp backs off exponentially (up to
-                        // DDP_BIDIR_SPIN_CAP ns): its polls would otherwise
-                        // take issue slots from the warps that have work
-                        unsigned int ns = 32;
-                        for (uint32_t spins = 0;; spins++) {
-                            const int h = *(volatile int *)&sq->head, t = *(volatile int *)&sq->tail;
-                            if (h < t) {
-                                // a small bucket is spread over the CTA's
-                                // warps instead of going to the first few
-                                const int k = min(t - h, min(32, max(DDP_BIDIR_CLAIM_MIN, (t - h + nw - 1) / nw)));
-                                if (atomicCAS(&sq->head, h, h + k) == h) {
-                                    n = k;
-                                    h0 = h;
-                                    break;
-                                }
-                                continue;
-                            }
-                            if (*(volatile int *)&sq->pending == 0) break;  // bucket done
-                            if (spins > SPIN_LIMIT) {
-                                atomicOr(&sq->status, ST_TIMEOUT);
-                                break;
-                            }
-                            __nanosleep(ns);
-                            if (ns < DDP_BIDIR_SPIN_CAP) ns <<= 1;
-                        }
-                    }
-                    n = __shfl_sync(FULL, n, 0);
-                    h0 = __shfl_sync(FULL, h0, 0);
-                    if (n < 0) break;
-                    if (lane < n) {
-                        volatile uint2 *slot = reinterpret_cast<volatile uint2 *>(ring + h0 + lane);
-                        uint2 x = make_uint2(slot->x, slot->y);
-                        for (uint32_t spins = 0; x.x == RING_EMPTY; spins++) {
-                            // reserved by a producer that has not written yet
-                            if (spins > SPIN_LIMIT) {
-                                atomicOr(&sq->status, ST_TIMEOUT);
-                                break;
-                            }
-                            __nanosleep(32);
-                            x = make_uint2(slot->x, slot->y);
-                        }
-                        en = x;
-                        slot->x = RING_EMPTY;  // clean for the next bucket
-                    }
-                }
-                // 2. entry stage: live entries below mu expand
-                int rb = 0, deg = 0;
-                uint32_t gu = 0, ud = 0;
-                if (lane < n && en.x != RING_EMPTY) {
-                    ud = en.x;
-                    gu = en.y;  // the entry's key
-                    const int u = (int)(ud & NODE_MASK);
-                    const uint32_t dir = ud >> 31;
-                    // the row bounds load beside the record (used only when
-                    // the entry turns out current): one round trip less
-                    const int r0 = dir ? row_begin(G.roff, G.roend, u) : row_begin(G.off, G.oend, u);
-                    const int r1 = dir ? row_end(G.roff, G.roend, u) : row_end(G.off, G.oend, u);
-                    const typename Rec::U *ru = R.find(u, ep);
-                    const uint32_t gl = ru ? Rec::g(Rec::ld(ru + dir), ep) : INF_G;
-                    bool cur = false;
-                    if constexpr (Pot::on) {
-                        // the entry is current when its key is the label's key
-                        cur = gl < INF_G && bi_key<Pot>(gl, dir, pot.at(u)) == gu &&
-                              (uint64_t)gu < bi_key_bound<Pot>(mu);
-                        gu = gl;
-                    } else {
-                        cur = gl == gu && gu < mu;
-                    }
-                    if (cur) {
-                        rb = r0;
-                        deg = r1 - r0;
-                        n_exp++;
-                    }
-                }
-                int total;
-                const int ex = warp_excl_scan(deg, &total);
-                wr.excl[lane] = ex;
-                wr.rb[lane] = rb;
-                wr.bdeg[lane] = deg;
-                wr.drb[lane] = 0;
-                wr.g[lane] = gu;
-                wr.u[lane] = (int)ud;
-                __syncwarp();
-                n_scan += (lane == 0) ? (unsigned long long)total : 0ull;
-                for (int kb = 0; kb < total; kb += 32) {
-                    const int k = kb + lane;
-                    bool live = false, first = false;
-                    uint2 pv = make_uint2(0u, 0u);  // {pt(v), ps(v)}
-                    typename Rec::U *rv = nullptr;  // v's record
-                    int v = 0;
-                    uint32_t ng = 0, dir = 0;
-                    uint32_t uo = 0;
-                    typename Rec::U uf{}, ur{};
-                    if (k < total) {
-                        const int o = row_owner(wr, k);
-                        uo = (uint32_t)wr.u[o];
-                        dir = uo >> 31;
-                        const uint2 a = row_arc(G, wr, o, k, dir == 0);
-                        v = (int)a.x;
-                        const uint64_t ng64 = (uint64_t)wr.g[o] + a.y;
-                        live = v >= 0 && ng64 < (uint64_t)min(mu, INF_G);
-                        ng = (uint32_t)ng64;
-                        // a layout whose records need no claim (dense,
-                        // 16-byte pairs) loads v's record beside v's
-                        // potentials, before the pruning test needs them: one
-                        // dependent round trip less per generation of a long
-                        // chain (a record loaded for a pruned v is not used)
-                        constexpr bool early = Pot::on && !Rec::hashed;
-                        if constexpr (early) {
-                            if (live) {
-                                rv = R.claim(v, ep);
-                                uf = Rec::ld(rv);
-                                ur = Rec::ld(rv + 1);
-                            }
-                        }
-                        if constexpr (Pot::on) {
-                            if (live) {
-                                // a path through v is at least g + the
-                                // bound of the other side
-                                pv = pot.at(v);
-                                live = ng64 + (dir ? pv.y : pv.x) < (uint64_t)mu;
-                            }
-                        }
-                        if (live && !early) {
-                            // the node's record: both units, one sector
-                            rv = R.claim(v, ep);
-                            if (rv) {
-                                uf = Rec::ld(rv);
-                                ur = Rec::ld(rv + 1);
-                            } else {
-                                atomicOr(&sq->status, ST_OVERFLOW);  // the slot's table is full
-                                live = false;
-                            }
-                        }
-                    }
-                    if (live) {
-                        const typename Rec::U mine = dir ? ur : uf;
-                        const uint32_t go = Rec::g(dir ? uf : ur, ep);
-                        if (go < INF_G) {
-                            // the two searches meet over this arc
-                            const uint64_t c = (uint64_t)ng + go;
-                            if (c < mu) {
-                                const uint32_t x = dir ? (uint32_t)v : (uo & NODE_MASK);
-                                atomicMin(&sq->mu, (c << 32) | x);
-                            }
-                        }
-                        live = ng < Rec::g(mine, ep);
-                        if (live) {
-                            const typename Rec::U nv = Rec::make(ep, ng, uo & NODE_MASK, dir ? 0u : R.keyw(v));
-                            typename Rec::U *w = rv + dir;
-                            typename Rec::U c0 = mine;
-                            live = false;
-                            // bounded: contention on one unit comes from at
-                            // most the CTA's own threads
-                            for (int tries = 0;; tries++) {
-                                if (tries == 4096) {
-                                    atomicOr(&sq->status, ST_TIMEOUT);
-                                    break;
-                                }
-                                const typename Rec::U got = Rec::cas(w, c0, nv);
-                                if (Rec::eq(got, c0)) {
-                                    live = true;
-                                    first = Rec::g(c0, ep) >= INF_G;
-                                    break;
-                                }
-                                c0 = got;
-                                if (ng >= Rec::g(c0, ep)) break;
-                            }
-                        }
-                    }
-                    const uint32_t nk = bi_key<Pot>(ng, dir, pv);
-                    bool to_near = live && nk < (dir ? T1 : T0);
-                    bool to_far = live && !to_near;
-                    if (live) n_rel++;
-                    const uint32_t vd = (uint32_t)v | (dir << 31);
-                    // near pushes: counted in `pending` first, then kept as
-                    // this warp's own work, or spilled to the ring when full
-                    const unsigned mn = __ballot_sync(FULL, to_near);
-                    if (mn) {
-                        const int kn = __popc(mn);
-                        const int rank_in = __popc(mn & ((1u << lane) - 1u));
-                        if (lane == 0) atomicAdd(&sq->pending, kn);
-                        __syncwarp();
-                        if (c_loc + kn <= 64) {
-                            if (to_near) wr.sn[c_loc + rank_in] = make_uint2(vd, nk);
-                            c_loc += kn;
-                        } else {
-                            int p0 = 0;
-                            if (lane == 0) p0 = bi_ring_reserve(sq, kn, cap);
-                            p0 = __shfl_sync(FULL, p0, 0);
-                            if (p0 >= 0) {
-                                if (to_near) {
-                                    volatile unsigned long long *slot =
-                                        reinterpret_cast<volatile unsigned long long *>(ring + p0 + rank_in);
-                                    *slot = ((unsigned long long)nk << 32) | vd;
-                                }
-                            } else {
-                                if (lane == 0) atomicSub(&sq->pending, kn);
-                                to_far = to_far || to_near;
-                            }
-                        }
-                        __syncwarp();
-                    }
-                    if (to_far) {
-                        if (dir) nf1++;
-                        else nf0++;
-                    }
-                    stage_push(to_far, make_uint2(vd, nk), sf2, c_f, &sq->far_cnt, fcur, nfar, B.cap_f,
-                               ctl, 0);
-                    if constexpr (Rec::logs) {
-                        // first touches of either direction (a node may be
-                        // logged twice; the reset takes it twice)
-                        stage_push(first, v, wr.st, c_t, &ctl->touched, B.touched, 0, 2 * (int64_t)G.n, ctl, 0);
-                    } else if (first) {
-                        n_first++;
-                    }
-                }
-                __syncwarp();
-                // 3. retire the chunk (its children are already counted)
-                if (lane == 0 && n > 0) atomicSub(&sq->pending, n);
-                if (*(volatile int *)&sq->status & ST_TIMEOUT) break;
+                const int ni = i + teams;
+                E en = e;
+                if (ni < W) en = entry(ni);  // loads while this one expands
+                expand(e, tsh);
+                if (ni >= W) break;
+                i = ni;
+                e = en;
             }
-            stage_flush(sf2, c_f, &sq->far_cnt, fcur, nfar, B.cap_f, ctl, 0);
-            if constexpr (Rec::logs) stage_flush(wr.st, c_t, &ctl->touched, B.touched, 0, 2 * (int64_t)G.n, ctl, 0);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                nf0 += __shfl_xor_sync(FULL, nf0, o);
-                nf1 += __shfl_xor_sync(FULL, nf1, o);
-            }
-            if (lane == 0) {
-                if (nf0) atomicAdd(&sq->open_dir[0], nf0);
-                if (nf1) atomicAdd(&sq->open_dir[1], nf1);
-            }
-            __syncthreads();
-            phases++;
-            nfar += *(volatile int *)&sq->far_cnt;
-            const int st = *(volatile int *)&sq->status | *(volatile int *)&ctl->status;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                sq->far_cnt = 0;
-                sq->head = 0;
-                sq->tail = 0;
-                sq->pending = 0;
-            }
-            if (st & (ST_OVERFLOW | ST_TIMEOUT)) {
-                if (threadIdx.x == 0) atomicOr(&ctl->status, st & (ST_OVERFLOW | ST_TIMEOUT));
-                break;
-            }
-            if (nfar > B.cap_f) {
-                if (threadIdx.x == 0) atomicOr(&ctl->status, ST_OVERFLOW);
-                break;
-            }
-            __syncthreads();
         }
-        // ---- split the far pile, and the stop test -------------------------
-        {
-            const uint32_t mu = uint32_t(*(volatile unsigned long long *)&sq->mu >> 32);
-            // advance the direction(s) whose open set is not much larger
-            const int o0 = *(volatile int *)&sq->open_dir[0], o1 = *(volatile int *)&sq->open_dir[1];
-            const bool adv0 = (int64_t)o0 <= 2 * (int64_t)o1 + 64;
-            const bool adv1 = (int64_t)o1 <= 2 * (int64_t)o0 + 64;
-            const uint32_t Ts0 = adv0 ? sat_add(max(T0, lo0), dk) : T0;
-            const uint32_t Ts1 = adv1 ? sat_add(max(T1, lo1), dk) : T1;
-            const uint64_t kb = bi_key_bound<Pot>(mu);
-            unsigned int kmin0 = 0xFFFFFFFFu, kmin1 = 0xFFFFFFFFu;
-            int kp0 = 0, kp1 = 0, mv0 = 0, mv1 = 0;  // kept / moved per direction (this lane)
-            int c_n = 0, c_f = 0;
-            if (threadIdx.x == 0) ctl->far_scanned += (unsigned long long)nfar;
-            // DDP_BIDIR_SPLIT_UNROLL entries per lane per step: their loads
-            // are issued together, then consumed one by one
-            constexpr int SU = DDP_BIDIR_SPLIT_UNROLL;
-            for (int64_t base0 = (int64_t)warp * 32 * SU; base0 < nfar; base0 += (int64_t)nw * 32 * SU) {
-                uint2 ens[SU];
-#pragma unroll
-                for (int k = 0; k < SU; k++) {
-                    const int64_t idx = base0 + 32 * k + lane;
-                    ens[k] = idx < nfar ? __ldcg(fcur + idx) : make_uint2(0u, 0u);
-                }
-#pragma unroll
-                for (int k = 0; k < SU; k++) {
-                    const int64_t idx = base0 + 32 * k + lane;
-                    bool to_near = false, keep = false;
-                    uint2 en = make_uint2(0u, 0u);
-                    if (idx < nfar) {
-                        en = ens[k];
-                        if ((uint64_t)en.y < kb) {
-                            const bool rev = (en.x >> 31) != 0;
-                            if (en.y < (rev ? Ts1 : Ts0)) to_near = true;
-                            else keep = true;
-                            if (rev) {
-                                kmin1 = min(kmin1, en.y);
-                                if (to_near) mv1++;
-                                else kp1++;
-                            } else {
-                                kmin0 = min(kmin0, en.y);
-                                if (to_near) mv0++;
-                                else kp0++;
-                            }
-                        }
-                    }
-                    {
-                        const unsigned m = __ballot_sync(FULL, to_near);
-                        if (to_near) wr.sn[c_n + __popc(m & ((1u << lane) - 1u))] = en;
-                        c_n += __popc(m);
-                        if (c_n >= 32) flush_ring_or_far(wr.sn, c_n, sq, ring, cap, falt, B.cap_f, ctl);
-                    }
-                    stage_push(keep, en, sf2, c_f, &sq->alt_cnt, falt, 0, B.cap_f, ctl, 0);
-                }
-            }
-            flush_ring_or_far(wr.sn, c_n, sq, ring, cap, falt, B.cap_f, ctl);
-            stage_flush(sf2, c_f, &sq->alt_cnt, falt, 0, B.cap_f, ctl, 0);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                kmin0 = min(kmin0, __shfl_xor_sync(FULL, kmin0, o));
-                kmin1 = min(kmin1, __shfl_xor_sync(FULL, kmin1, o));
-                kp0 += __shfl_xor_sync(FULL, kp0, o);
-                kp1 += __shfl_xor_sync(FULL, kp1, o);
-                mv0 += __shfl_xor_sync(FULL, mv0, o);
-                mv1 += __shfl_xor_sync(FULL, mv1, o);
-            }
-            __syncthreads();  // every thread has read open_dir
-            if (threadIdx.x == 0) sq->open_dir[0] = sq->open_dir[1] = 0;
-            __syncthreads();
-            if (lane == 0) {
-                if (kmin0 != 0xFFFFFFFFu) atomicMin(&sq->minkey[0], kmin0);
-                if (kmin1 != 0xFFFFFFFFu) atomicMin(&sq->minkey[1], kmin1);
-                if (kp0) atomicAdd(&sq->open_dir[0], kp0);
-                if (kp1) atomicAdd(&sq->open_dir[1], kp1);
-                if (mv0) atomicAdd(&sq->moved_dir[0], mv0);
-                if (mv1) atomicAdd(&sq->moved_dir[1], mv1);
-            }
-            __syncthreads();
-            const int m = min(*(volatile int *)&sq->tail, cap);
-            const int kept = *(volatile int *)&sq->alt_cnt;
-            const unsigned int a = *(volatile unsigned int *)&sq->minkey[0];
-            const unsigned int b = *(volatile unsigned int *)&sq->minkey[1];
-            const int moved0 = *(volatile int *)&sq->moved_dir[0], moved1 = *(volatile int *)&sq->moved_dir[1];
-            const uint32_t mu2 = uint32_t(*(volatile unsigned long long *)&sq->mu >> 32);
-            const int st = *(volatile int *)&ctl->status;
-            phases++;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                sq->alt_cnt = 0;
-                sq->minkey[0] = sq->minkey[1] = 0xFFFFFFFFu;
-                sq->moved_dir[0] = sq->moved_dir[1] = 0;
-                sq->head = 0;
-                sq->tail = m;  // entries past the ring's capacity stayed in far
-                sq->pending = m;
-            }
-            uint2 *t2 = fcur;
-            fcur = falt;
-            falt = t2;
-            nfar = kept;
-            if (st & (ST_OVERFLOW | ST_TIMEOUT)) break;
-            if (phases > max_phases) {
-                if (threadIdx.x == 0) atomicOr(&ctl->status, ST_TIMEOUT);
-                break;
-            }
-            // an empty direction, or a + b >= mu: mu is the distance.  The
-            // ring entries just moved hold the direction minima too.
-            if (a == 0xFFFFFFFFu || b == 0xFFFFFFFFu || (uint64_t)a + b >= bi_key_bound<Pot>(mu2)) {
-                // the ring may hold moved entries nobody will pop: clear it
-                for (int i = threadIdx.x; i < m; i += blockDim.x) ring[i].x = RING_EMPTY;
-                break;
-            }
-            // a direction that advanced without moving anything jumps to its
-            // smallest open key next time
-            lo0 = (adv0 && moved0 == 0) ? a : 0u;
-            lo1 = (adv1 && moved1 == 0) ? b : 0u;
-            T0 = Ts0;
-            T1 = Ts1;
-            do_expand = m > 0;
-            __syncthreads();
-        }
+        wv++;
     }
+    if (threadIdx.x == 0 && q->status) atomicOr(&ctl->status, q->status);
 
-    if (lane == 0 && n_scan) atomicAdd(&ctl->scanned, n_scan);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         n_exp += __shfl_xor_sync(FULL, n_exp, o);
+        n_scan += __shfl_xor_sync(FULL, n_scan, o);
         n_rel += __shfl_xor_sync(FULL, n_rel, o);
         n_first += __shfl_xor_sync(FULL, n_first, o);
     }
     if (lane == 0) {
         if (n_exp) atomicAdd(&ctl->expanded, n_exp);
+        if (n_scan) atomicAdd(&ctl->scanned, n_scan);
         if (n_rel) atomicAdd(&ctl->relaxed, n_rel);
         if (n_first) atomicAdd(&ctl->touched, (int)n_first);
     }
-    if (threadIdx.x == 0) ctl->iters = phases;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ctl->iters = wv;
+        ctl->far_scanned = n_far;
+        if constexpr (Rec::logs) ctl->touched = (int)min((int64_t)q->touched, 2 * (int64_t)G.n);
+    }
     __syncthreads();
     SearchResult r;
-    const unsigned long long mw = *(volatile unsigned long long *)&sq->mu;
+    const unsigned long long mw = *(volatile unsigned long long *)&q->mu;
     r.cost = uint32_t(mw >> 32) >= INF_G ? 0xFFFFFFFFu : uint32_t(mw >> 32);
-    r.iters = phases;
+    r.iters = wv;
     return r;
 }
 

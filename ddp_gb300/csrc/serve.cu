@@ -487,7 +487,7 @@ int ddp_serve_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, int64_t 
     graph_ref(g);
     s->hkind = hkind;
     if (opts) s->o = *opts;
-    s->block = s->o.block > 0 ? std::min(s->o.block, 512) : 512;  // wider slots: lower latency, more per-query parallelism
+    s->block = s->o.block > 0 ? std::min((s->o.block + 31) & ~31, 512) : 512;  // wider slots: lower latency, more per-query parallelism
     s->cap = max_requests;
     auto bail = [&](int rc) {
         ddp_serve_free(s);
@@ -515,6 +515,7 @@ int ddp_serve_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, int64_t 
         const int64_t fit = share > fixed ? (int64_t)((share - fixed) / per_entry) : 0;
         capq = std::min<int64_t>((int64_t)g->n + 4096, std::max<int64_t>(1 << 16, fit));
         capf = std::min<int64_t>(2 * (int64_t)g->n + 4096, 2 * capq);
+        if (is_bidir_kind(hkind)) capf = std::max<int64_t>(capf, (1 << 18) + 4096);  // bucket lists
     }
     const size_t per = slot_bytes(g->n, capq, capf, hops);
     if ((size_t)nslots * per > freeb / 2) nslots = (int)std::max<size_t>(1, (freeb / 2) / per);

@@ -24,9 +24,10 @@ constexpr int MAX_WARPS = 16;  // blocks of at most 512 threads
 
 // ---- slot arrays -------------------------------------------------------------
 // Paired (bidirectional) slots hold a 32-byte record per node (two
-// epoch-tagged units), no touched log, one ring and 8-byte far entries;
-// the others one 8-byte state word per node, a touched log, two queues and
-// 16-byte far entries.
+// epoch-tagged units), no touched log, no queues, and 2 x cap_f x 8 bytes of
+// far memory (bucket lists and a pile, engine_bidir.cuh); the others one
+// 8-byte state word per node, a touched log, two queues and 16-byte far
+// entries.
 // Hashed records per slot: a quarter of the nodes, between 2^16 and 2^20
 // (a C4 query touches about 35k nodes; the table stays under 15 % full).
 int hash_bits(int32_t n) {
@@ -48,7 +49,7 @@ size_t slot_bytes(int32_t n, int64_t cap_q, int64_t cap_f, int kind, int hbits) 
         if (!pair) b += sizeof(int32_t) * (size_t)n;              // touched
     }
     if (kind & SLOT_HOPS) b += sizeof(uint32_t) * (size_t)n;
-    b += (pair ? 1 : 2) * sizeof(uint2) * (size_t)cap_q;
+    b += (pair ? 0 : 2) * sizeof(uint2) * (size_t)cap_q;
     b += 2 * (pair ? sizeof(uint2) : sizeof(uint4)) * (size_t)cap_f;
     b += sizeof(SearchCtl);
     return b;
@@ -75,9 +76,9 @@ int slots_alloc(SlotArrays &sa, int32_t n, int nslots, int64_t cap_q, int64_t ca
     DDP_CUDA(cudaMalloc(&sa.state, sizeof(unsigned long long) * (size_t)sa.sstride * S));
     if (!pair || p16) DDP_CUDA(cudaMalloc(&sa.touched, sizeof(int32_t) * (size_t)n * (p16 ? 2 : 1) * S));
     if (hops) DDP_CUDA(cudaMalloc(&sa.hops, sizeof(uint32_t) * (size_t)n * S));
-    const size_t qn = pair ? 1 : 2;                             // rings per slot
+    const size_t qn = pair ? 0 : 2;                             // queues per slot
     const size_t fb = pair ? sizeof(uint2) : sizeof(uint4);     // bytes per far entry
-    DDP_CUDA(cudaMalloc(&sa.q, sizeof(uint2) * (size_t)cap_q * qn * S));
+    if (qn) DDP_CUDA(cudaMalloc(&sa.q, sizeof(uint2) * (size_t)cap_q * qn * S));
     DDP_CUDA(cudaMalloc(&sa.f, fb * (size_t)cap_f * 2 * S));
     DDP_CUDA(cudaMalloc(&sa.ctl, sizeof(SearchCtl) * S));
     DDP_CUDA(cudaMalloc(&sa.epoch, sizeof(uint32_t) * S));
@@ -88,7 +89,7 @@ int slots_alloc(SlotArrays &sa, int32_t n, int nslots, int64_t cap_q, int64_t ca
                              sizeof(unsigned long long) * (size_t)sa.sstride * S, st));
     if (hops) DDP_CUDA(cudaMemsetAsync(sa.hops, 0, sizeof(uint32_t) * (size_t)n * S, st));
     // queue slots start as "empty" (the asynchronous engine's ring marker)
-    DDP_CUDA(cudaMemsetAsync(sa.q, 0xFF, sizeof(uint2) * (size_t)cap_q * qn * S, st));
+    if (qn) DDP_CUDA(cudaMemsetAsync(sa.q, 0xFF, sizeof(uint2) * (size_t)cap_q * qn * S, st));
     DDP_CUDA(cudaMemsetAsync(sa.ctl, 0, sizeof(SearchCtl) * S, st));
     return DDP_OK;
 }
@@ -111,10 +112,8 @@ __device__ __forceinline__ SlotBufs slot_of(const SlotArrays &sa, int i) {
     b.touched = sa.touched ? sa.touched + n * (sa.words == 2 ? 2 : 1) * i : nullptr;
     b.hops = sa.hops ? sa.hops + n * i : nullptr;
     if (sa.pair) {
-        // paired slots: one ring; far piles of 8-byte entries (the uint4
-        // pointers only carry the address)
-        b.q0 = sa.q + (size_t)sa.cap_q * i;
-        b.q1 = b.q0;
+        // paired slots: no queues; the uint4 pointers only carry addresses
+        b.q0 = b.q1 = nullptr;
         uint2 *fb = reinterpret_cast<uint2 *>(sa.f) + (size_t)sa.cap_f * 2 * i;
         b.f0 = reinterpret_cast<uint4 *>(fb);
         b.f1 = reinterpret_cast<uint4 *>(fb + sa.cap_f);
@@ -235,9 +234,16 @@ __device__ SearchResult slot_search(const Grp &grp, const DevGraph &G, const Slo
     else return run_search(grp, G, B, H, P, wrows);
 }
 
+// The plain bidirectional search with labels installed at once (not inlined:
+// the lazy form's registers are not shared with it).
+__device__ __noinline__ SearchResult run_bidir_eager(const DevGraph &G, const SlotBufs &B, const SearchParams &P,
+                                                     uint32_t ep, WaveQ *q) {
+    return run_bidir_cta<false>(G, B, P, ep, q, PotNone{}, RecDense{{}, B.state});
+}
+
 template <int HK, bool ASYNC, class Grp>
 __device__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B, const BatchArgs &A,
-                           uint32_t *epoch, WarpRows *wrows, CtaQ *sq, BiQ *bq) {
+                           uint32_t *epoch, WarpRows *wrows, CtaQ *sq, WaveQ *bq) {
     SearchCtl *ctl = B.ctl;
     long long t0 = 0;
     int vbuf = -1;  // versioned serving: graph buffer the current search holds
@@ -391,51 +397,77 @@ __device__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B
             if constexpr (std::is_same<Grp, CtaGroup>::value) {
                 const uint32_t ep = *(volatile uint32_t *)&ctl->tag;
                 if constexpr (HK == 5) {
-                    r = run_bidir_cta(G, B, P, ep, wrows, bq, PotNone{}, RecDense{{}, B.state});
+                    r = run_bidir_cta<true>(G, B, P, ep, bq, PotNone{}, RecDense{{}, B.state});
+                    if (*(volatile int *)&ctl->status & ST_OVERFLOW) {
+                        // lazy labels keep up to one open entry per arc: a
+                        // search that floods the graph (the target lies in
+                        // another component, say) starts again with labels
+                        // installed at once, which keeps about one per node
+                        grp.sync();
+                        if (grp.rank() == 0) {
+                            const uint32_t e2 = *epoch + 1;
+                            if (e2 != 0) {  // else leave the overflow standing
+                                *epoch = e2;
+                                ctl->tag = e2;
+                                ctl->status = 0;
+                            }
+                        }
+                        grp.sync();
+                        if (*(volatile int *)&ctl->status == 0)
+                            r = run_bidir_eager(G, B, P, *(volatile uint32_t *)&ctl->tag, bq);
+                    }
                 } else if constexpr (HK == 8) {
                     const RecHash R{{}, B.state, (1u << B.hbits) - 1u, 32 - B.hbits};
-                    r = run_bidir_cta(G, B, P, ep, wrows, bq, PotNone{}, R);
+                    r = run_bidir_cta<true>(G, B, P, ep, bq, PotNone{}, R);
                 } else if constexpr (HK == 9) {
-                    r = run_bidir_cta(G, B, P, ep, wrows, bq, PotNone{}, RecPair16{B.state});
+                    r = run_bidir_cta<false>(G, B, P, ep, bq, PotNone{}, RecPair16{B.state});
                 } else {
                     const int2 sp = reinterpret_cast<const int2 *>(G.xy)[s];
                     const int2 tp = reinterpret_cast<const int2 *>(G.xy)[t];
                     if constexpr (HK == 6)
-                        r = run_bidir_cta(G, B, P, ep, wrows, bq, PotEuclid{G.xy, sp, tp, G.rho_fp / 65536.0},
-                                          RecDense{{}, B.state});
+                        r = run_bidir_cta<false>(G, B, P, ep, bq, PotEuclid{G.xy, sp, tp, G.rho_fp / 65536.0},
+                                                 RecDense{{}, B.state});
                     else
-                        r = run_bidir_cta(G, B, P, ep, wrows, bq, PotManhattan{G.xy, sp, tp, G.wmin},
-                                          RecDense{{}, B.state});
+                        r = run_bidir_cta<false>(G, B, P, ep, bq, PotManhattan{G.xy, sp, tp, G.wmin},
+                                                 RecDense{{}, B.state});
                 }
             }
         } else {
             r = slot_search<ASYNC>(grp, G, B, HeurZero{}, P, wrows, sq);
         }
-        if (ASYNC && (*(volatile int *)&ctl->status & (ST_OVERFLOW | ST_TIMEOUT))) {
+        if (ASYNC && !bidir_hk(HK) && (*(volatile int *)&ctl->status & (ST_OVERFLOW | ST_TIMEOUT))) {
             // an aborted asynchronous search may leave ring slots written:
             // clear the ring so the slot's next search starts clean
             for (int64_t i = grp.rank(); i < B.cap_q; i += grp.size()) B.q0[i].x = RING_EMPTY;
             grp.sync();
         }
-        if (grp.rank() == 0) {
-            const int st = ctl->status;
-            int32_t len = 0;
-            if (!(st & (ST_OVERFLOW | ST_TIMEOUT)) && A.paths) {
-                if (HK == 8)
-                    len = write_path_bidir(G, RecHash{{}, B.state, (1u << B.hbits) - 1u, 32 - B.hbits}, ctl->tag, s,
-                                           t, bq->mu, A.paths + (size_t)q * A.path_cap, A.path_cap, &ctl->status);
-                else if (pair16_hk(HK))
-                    len = write_path_bidir(G, RecPair16{B.state}, ctl->tag, s, t, bq->mu,
-                                           A.paths + (size_t)q * A.path_cap, A.path_cap, &ctl->status);
-                else if (bidir_hk(HK))
-                    len = write_path_bidir(G, RecDense{{}, B.state}, ctl->tag, s, t, bq->mu,
-                                           A.paths + (size_t)q * A.path_cap, A.path_cap, &ctl->status);
+        int32_t blen = 0;  // path length (bidirectional kinds; the first warp)
+        if constexpr (bidir_hk(HK)) {
+            if (grp.rank() < 32 && A.paths && !(*(volatile int *)&ctl->status & (ST_OVERFLOW | ST_TIMEOUT))) {
+                int32_t *path = A.paths + (size_t)q * A.path_cap;
+                int32_t *buf = reinterpret_cast<int32_t *>(bq->list);  // the wave lists are free now
+                static_assert(sizeof(bq->list) >= 2 * PATH_BUF * sizeof(int32_t), "two path halves");
+                const uint32_t ep = *(volatile uint32_t *)&ctl->tag;
+                const unsigned long long mu = *(volatile unsigned long long *)&bq->mu;
+                if constexpr (HK == 8)
+                    blen = write_path_bidir(G, RecHash{{}, B.state, (1u << B.hbits) - 1u, 32 - B.hbits}, ep, s, t, mu,
+                                            path, A.path_cap, &ctl->status, buf);
+                else if constexpr (pair16_hk(HK))
+                    blen = write_path_bidir(G, RecPair16{B.state}, ep, s, t, mu, path, A.path_cap, &ctl->status, buf);
                 else
-                    len = write_path(B, s, t, A.paths + (size_t)q * A.path_cap, A.path_cap, G.n,
-                                     &ctl->status);
+                    blen = write_path_bidir(G, RecDense{{}, B.state}, ep, s, t, mu, path, A.path_cap, &ctl->status,
+                                            buf);
+            }
+        }
+        if (grp.rank() == 0) {
+            const int st = *(volatile int *)&ctl->status;
+            int32_t len = blen;
+            if constexpr (!bidir_hk(HK)) {
+                if (!(st & (ST_OVERFLOW | ST_TIMEOUT)) && A.paths)
+                    len = write_path(B, s, t, A.paths + (size_t)q * A.path_cap, A.path_cap, G.n, &ctl->status);
             }
             // a bidirectional search that found no meeting arc failed
-            const int stf = ctl->status;
+            const int stf = *(volatile int *)&ctl->status;
             A.cost[q] = ((st | stf) & (ST_OVERFLOW | ST_TIMEOUT)) ? -1
                         : (r.cost >= INF_G)                ? DDP_INF
                                                            : (int32_t)r.cost;
@@ -609,31 +641,29 @@ __device__ void service_loop(const BatchArgs &A) {
     }
 }
 
-// CTAs per SM the bidirectional instance is compiled for (its register
-// budget per thread: 2 -> 64, 3 -> 40, 4 -> 32; the engine spills 220,
-// 472 and 772 bytes per thread at those budgets, and three or four CTAs'
-// spills outgrow the L1 left beside their shared memory).  Measured on the
-// 4M-node batch of 4,096 pairs with ring claims spread over the warps:
-// 2 -> 379k queries/s (304 slots), 3 -> 363k (456), 4 -> 228k (608).
-#ifndef DDP_BIDIR_MIN_BLOCKS
-#define DDP_BIDIR_MIN_BLOCKS 2
-#endif
+// Bidirectional instances are compiled for 64 registers (1,024 threads on an
+// SM in any split): a launch picks 1,024, 512 or 256 threads per query
+// (batch_shape).
 // One-CTA slots.  The group form below is a kernel of its own: both engines
 // in one kernel share a register budget, and the one that a launch does not
 // use makes the other spill (landmark instance: 736 bytes of spill stores
 // with both engines, 1,706 once the group engine also ran narrow phases).
 template <int HK>
-__global__ void __launch_bounds__(512, (bidir_hk(HK) ? DDP_BIDIR_MIN_BLOCKS : 2)) k_batch(DevGraph G, SlotArrays sa, BatchArgs A) {
-    __shared__ WarpRows wrows[MAX_WARPS];
-    __shared__ CtaQ sq;
-    __shared__ BiQ bq;
+__global__ void __launch_bounds__(bidir_hk(HK) ? 1024 : 512, bidir_hk(HK) ? 1 : 2) k_batch(DevGraph G, SlotArrays sa, BatchArgs A) {
     if (A.svc && (int)blockIdx.x == A.serve_slots) {
         service_loop(A);
         return;
     }
     SlotBufs B = slot_of(sa, blockIdx.x);
     CtaGroup grp{&B.ctl->status};
-    batch_loop<HK, true>(grp, G, B, A, sa.epoch + blockIdx.x, wrows, &sq, &bq);
+    if constexpr (bidir_hk(HK)) {
+        __shared__ WaveQ bq;
+        batch_loop<HK, true>(grp, G, B, A, sa.epoch + blockIdx.x, nullptr, nullptr, &bq);
+    } else {
+        __shared__ WarpRows wrows[MAX_WARPS];
+        __shared__ CtaQ sq;
+        batch_loop<HK, true>(grp, G, B, A, sa.epoch + blockIdx.x, wrows, &sq, nullptr);
+    }
 }
 
 // Slots of A.group CTAs each (cooperative launch), and one-CTA slots on the
@@ -1384,19 +1414,31 @@ static bool batch_args(ddp_batch *b, int32_t n, const int32_t *dS, const int32_t
     return !(b->hkind == DDP_H_LANDMARK && !G->lm);
 }
 
+// Threads per bidirectional query of a launch of n queries; returns the CTAs
+// per SM.
+static int batch_shape(int32_t n, int *block) {
+    const int sms = device_sms();
+    *block = n <= sms + sms / 2 ? 1024 : n <= 6 * sms ? 512 : 256;
+    return 1024 / *block;
+}
+
 static cudaError_t batch_launch_args(ddp_batch *b, DevGraph G, BatchArgs A) {
     cudaError_t e = cudaMemsetAsync(b->d_work, 0, sizeof(int) * 2, b->stream);
     if (e != cudaSuccess) return e;
     // fresh control blocks (barrier counters included) for every launch
     e = cudaMemsetAsync(b->sa.ctl, 0, sizeof(SearchCtl) * (size_t)b->sa.nslots, b->stream);
     if (e != cudaSuccess) return e;
-    const int grid = b->sa.nslots * b->group;
+    int block = b->block, grid = b->sa.nslots * b->group;
+    if (is_bidir_kind(b->hkind) && b->o.block <= 0) {
+        const int per_sm = batch_shape(A.nq, &block);
+        grid = std::min({grid, per_sm * device_sms(), std::max(A.nq, 1)});
+    }
     SlotArrays sa = b->sa;
     void *args[] = {&G, &sa, &A};
     const void *fn = batch_kernel_hk(b->hk, A.group > 1 || A.sync_engine);
     if (b->group > 1)
-        return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(b->block), args, 0, b->stream);
-    return cudaLaunchKernel(fn, dim3(grid), dim3(b->block), args, 0, b->stream);
+        return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(block), args, 0, b->stream);
+    return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, b->stream);
 }
 
 // Field-by-field equality of the by-value kernel arguments (padding bytes
@@ -1438,7 +1480,8 @@ int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batc
     graph_ref(g);
     b->hkind = hkind;
     if (opts) b->o = *opts;
-    b->block = b->o.block > 0 ? std::min(b->o.block, 512) : 512;
+    // whole warps; bidirectional launches choose per batch unless told
+    b->block = b->o.block > 0 ? std::min((b->o.block + 31) & ~31, is_bidir_kind(hkind) ? 1024 : 512) : 512;
     b->path_cap = 1024;
     cudaError_t e = b->o.stream ? cudaSuccess : cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (b->o.stream) b->stream = (cudaStream_t)b->o.stream;
@@ -1451,13 +1494,12 @@ int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batc
     b->hk = kernel_hk(hkind, g->d_xy != nullptr, (b->o.flags & DDP_OPT_HASH) != 0);
     b->group = is_bidir_kind(hkind) ? 1 : std::max(1, b->o.group);  // bidirectional slots are one CTA
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, batch_kernel_hk(b->hk, b->group > 1 || (b->o.flags & DDP_OPT_SYNC)), b->block, 0);
+        &per_sm, batch_kernel_hk(b->hk, b->group > 1 || (b->o.flags & DDP_OPT_SYNC)),
+        is_bidir_kind(hkind) && b->o.block <= 0 ? 256 : b->block, 0);
     const int coresident = std::max(1, per_sm) * sm_count();
     if (b->group > coresident) b->group = coresident;
     int nslots = coresident / b->group;
     if (b->o.grid > 0) nslots = std::min(b->o.grid, b->group > 1 ? nslots : b->o.grid);
-    // the bidirectional ring holds one bucket and spills to the far pile
-    // when full, so it needs far less than a node count
     const int64_t cap = b->o.queue_cap > 0      ? b->o.queue_cap
                         : is_bidir_kind(hkind) ? std::min<int64_t>((int64_t)g->n + 4096, 1 << 18)
                                                 : (int64_t)g->n + 4096;
@@ -1465,7 +1507,10 @@ int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batc
     cudaMemGetInfo(&freeb, &totalb);
     // the far pile holds every open node beyond the current bucket: twice the
     // node count leaves room for stale copies between compactions
-    const int64_t cap_f = b->o.queue_cap > 0 ? b->o.queue_cap : 2 * (int64_t)g->n + 4096;
+    // (small graphs with bidirectional slots: room for the bucket lists)
+    const int64_t cap_f = b->o.queue_cap > 0      ? b->o.queue_cap
+                          : is_bidir_kind(hkind) ? std::max<int64_t>(2 * (int64_t)g->n, 1 << 18) + 4096
+                                                  : 2 * (int64_t)g->n + 4096;
     const int skind = hk_slot_kind(b->hk);
     const int hb = (skind & SLOT_HASH) ? hash_bits(g->n) : 0;
     const size_t per = slot_bytes(g->n, cap, cap_f, skind, hb);

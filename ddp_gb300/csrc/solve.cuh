@@ -14,12 +14,12 @@ struct SlotArrays {
     int words = 1;        // 64-bit state words per node: 1, or 4 (paired slots: a 32-byte record)
     int64_t sstride = 0;  // state words per slot
     int hbits = 0;        // hashed paired slots: log2 of the records per slot
-    bool pair = false;    // bidirectional queue layout (one ring, 8-byte far entries)
+    bool pair = false;    // bidirectional layout (no queues, 8-byte units of far memory)
     int64_t cap_q = 0, cap_f = 0;
     unsigned long long *state = nullptr;  // nslots x n x words
     int32_t *touched = nullptr;           // nslots x n (null for paired slots)
     uint32_t *hops = nullptr;             // nslots x n (per-target heuristic) or null
-    uint2 *q = nullptr;                   // nslots x 2 x cap_q
+    uint2 *q = nullptr;                   // nslots x 2 x cap_q (null for paired slots)
     uint4 *f = nullptr;                   // nslots x 2 x cap_f {node, g, f, 0}
     SearchCtl *ctl = nullptr;             // nslots
     uint32_t *epoch = nullptr;            // nslots: per-query tag counter of the hop array
