@@ -443,11 +443,12 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
     // arcs per lane whose loads are in flight together
     constexpr int AU = Pot::on ? 1 : LAZY ? 4 : 2;
     constexpr uint32_t ahead = LAZY ? WAVE_AHEAD : WAVE_AHEAD_XY;
-    // the slot's far memory: 2 x 32 lists (a quarter), two halves of a pile,
-    // two spill areas for waves that outgrow shared memory (an eighth each)
+    // the slot's far memory: 2 x 32 lists (at most a quarter), two halves of a
+    // pile, two spill areas for waves that outgrow shared memory (a sixteenth
+    // each)
     const int64_t total = 2 * B.cap_f * (int64_t)sizeof(uint2) / (int64_t)sizeof(E);
     const int room = (int)min(total / (8 * WAVE_LISTS), (int64_t)WAVE_ROOM);  // entries per list
-    const int scap = (int)min(total / 8, (int64_t)0x0FFFFFFF);
+    const int scap = (int)min(total / 16, (int64_t)0x0FFFFFFF);
     const int pcap = (int)min((total - (int64_t)2 * WAVE_LISTS * room - 2 * (int64_t)scap) / 2, (int64_t)0x3FFFFFFF);
     E *lists = reinterpret_cast<E *>(B.f0);
     E *pile0 = lists + (int64_t)2 * WAVE_LISTS * room;

@@ -416,7 +416,7 @@ int launch(ddp_server *s) {
     A.work = s->d_work;
     A.status = s->d_work + 1;
     A.delta = s->o.delta > 0                ? (uint32_t)s->o.delta
-              : is_bidir_kind(s->hkind) ? auto_delta_bidir(s->g)
+              : bidir_hk(s->hk)         ? auto_delta_bidir(s->g)
                                         : auto_delta(s->g);
     A.K = s->o.K;
     A.bfs_budget = s->hkind == DDP_H_BFS_CAPPED ? bfs_budget(s->g->n) : 0;
@@ -496,7 +496,7 @@ int ddp_serve_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, int64_t 
     cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate"));
     // slots: occupancy, then the memory budget (half of free memory)
-    s->hk = kernel_hk(hkind, g->d_xy != nullptr, false);
+    s->hk = kernel_hk(hkind, g->d_xy != nullptr, false, 1, s->o.flags);
     const int per_sm = std::max(1, slots_per_sm(s->hk, s->block, (s->o.flags & DDP_OPT_SYNC) != 0));
     int nslots = per_sm * device_sms();
     if (s->o.grid > 0) nslots = std::min(nslots, s->o.grid);
@@ -515,8 +515,8 @@ int ddp_serve_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, int64_t 
         const int64_t fit = share > fixed ? (int64_t)((share - fixed) / per_entry) : 0;
         capq = std::min<int64_t>((int64_t)g->n + 4096, std::max<int64_t>(1 << 16, fit));
         capf = std::min<int64_t>(2 * (int64_t)g->n + 4096, 2 * capq);
-        if (is_bidir_kind(hkind)) capf = std::max<int64_t>(capf, (1 << 18) + 4096);  // bucket lists
     }
+    if (bidir_hk(s->hk)) capf = bidir_cap_f(capf);
     const size_t per = slot_bytes(g->n, capq, capf, hops);
     if ((size_t)nslots * per > freeb / 2) nslots = (int)std::max<size_t>(1, (freeb / 2) / per);
     int rc = slots_alloc(s->sa, g->n, nslots, capq, capf, hops, s->stream);

@@ -738,7 +738,11 @@ static int rerun_kind(int hkind) { return is_bidir_kind(hkind) ? DDP_H_ZERO : hk
 // 16-byte pairs (8-9 % more serving capacity on the 8M-point graph); else
 // 32-byte epoch-tagged records (the potential-steered kinds too: on the
 // 2048^2 maze they were faster, 16.4 against 17.8 ms).
-int kernel_hk(int hkind, bool has_xy, bool hash) {
+int kernel_hk(int hkind, bool has_xy, bool hash, int group, int flags) {
+    if (!is_bidir_kind(hkind) && batch_bidir(hkind, group, flags)) {
+        hkind = DDP_H_BIDIR;
+        hash = false;
+    }
     if (is_bfs_kind(hkind)) return 1;
     if (hkind == DDP_H_MANHATTAN) return 2;
     if (hkind == DDP_H_EUCLID) return 3;
@@ -766,10 +770,11 @@ int hk_slot_kind(int hk) {
 }
 
 // The kernel of an instance; grouped: slots of several CTAs, or one-CTA slots
-// on the phase-synchronous engine (bidirectional kinds have neither).
+// on the phase-synchronous engine (bidirectional kinds have neither, and no
+// bound or hop bounds have nothing else: batch_bidir).
 static const void *batch_kernel_hk(int hk, bool grouped) {
     switch (hk) {
-    case 1: return grouped ? (const void *)k_batch_group<1> : (const void *)k_batch<1>;
+    case 1: return (const void *)k_batch_group<1>;
     case 2: return grouped ? (const void *)k_batch_group<2> : (const void *)k_batch<2>;
     case 3: return grouped ? (const void *)k_batch_group<3> : (const void *)k_batch<3>;
     case 4: return grouped ? (const void *)k_batch_group<4> : (const void *)k_batch<4>;
@@ -778,7 +783,7 @@ static const void *batch_kernel_hk(int hk, bool grouped) {
     case 7: return (const void *)k_batch<7>;
     case 8: return (const void *)k_batch<8>;
     case 9: return (const void *)k_batch<9>;
-    default: return grouped ? (const void *)k_batch_group<0> : (const void *)k_batch<0>;
+    default: return (const void *)k_batch_group<0>;
     }
 }
 
@@ -1404,7 +1409,7 @@ static bool batch_args(ddp_batch *b, int32_t n, const int32_t *dS, const int32_t
     A.work = b->d_work;
     A.status = b->d_status;
     A.delta = b->o.delta > 0                ? (uint32_t)b->o.delta
-              : is_bidir_kind(b->hkind) ? auto_delta_bidir(b->g)
+              : bidir_hk(b->hk)         ? auto_delta_bidir(b->g)
                                         : auto_delta(b->g);
     A.bfs_budget = b->hkind == DDP_H_BFS_CAPPED ? bfs_budget(b->g->n) : 0;
     A.K = b->o.K;
@@ -1429,7 +1434,7 @@ static cudaError_t batch_launch_args(ddp_batch *b, DevGraph G, BatchArgs A) {
     e = cudaMemsetAsync(b->sa.ctl, 0, sizeof(SearchCtl) * (size_t)b->sa.nslots, b->stream);
     if (e != cudaSuccess) return e;
     int block = b->block, grid = b->sa.nslots * b->group;
-    if (is_bidir_kind(b->hkind) && b->o.block <= 0) {
+    if (bidir_hk(b->hk) && b->o.block <= 0) {
         const int per_sm = batch_shape(A.nq, &block);
         grid = std::min({grid, per_sm * device_sms(), std::max(A.nq, 1)});
     }
@@ -1481,7 +1486,10 @@ int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batc
     b->hkind = hkind;
     if (opts) b->o = *opts;
     // whole warps; bidirectional launches choose per batch unless told
-    b->block = b->o.block > 0 ? std::min((b->o.block + 31) & ~31, is_bidir_kind(hkind) ? 1024 : 512) : 512;
+    b->hk = kernel_hk(hkind, g->d_xy != nullptr, (b->o.flags & DDP_OPT_HASH) != 0, b->o.group, b->o.flags);
+    const bool bidir = bidir_hk(b->hk);
+    // whole warps; bidirectional launches choose per batch unless told
+    b->block = b->o.block > 0 ? std::min((b->o.block + 31) & ~31, bidir ? 1024 : 512) : 512;
     b->path_cap = 1024;
     cudaError_t e = b->o.stream ? cudaSuccess : cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (b->o.stream) b->stream = (cudaStream_t)b->o.stream;
@@ -1491,26 +1499,23 @@ int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batc
     }
     // slots: occupancy-limited, then memory-limited (half of free memory)
     int per_sm = 0;
-    b->hk = kernel_hk(hkind, g->d_xy != nullptr, (b->o.flags & DDP_OPT_HASH) != 0);
-    b->group = is_bidir_kind(hkind) ? 1 : std::max(1, b->o.group);  // bidirectional slots are one CTA
+    b->group = bidir ? 1 : std::max(1, b->o.group);  // bidirectional slots are one CTA
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, batch_kernel_hk(b->hk, b->group > 1 || (b->o.flags & DDP_OPT_SYNC)),
-        is_bidir_kind(hkind) && b->o.block <= 0 ? 256 : b->block, 0);
+        bidir && b->o.block <= 0 ? 256 : b->block, 0);
     const int coresident = std::max(1, per_sm) * sm_count();
     if (b->group > coresident) b->group = coresident;
     int nslots = coresident / b->group;
     if (b->o.grid > 0) nslots = std::min(b->o.grid, b->group > 1 ? nslots : b->o.grid);
     const int64_t cap = b->o.queue_cap > 0      ? b->o.queue_cap
-                        : is_bidir_kind(hkind) ? std::min<int64_t>((int64_t)g->n + 4096, 1 << 18)
+                        : bidir               ? std::min<int64_t>((int64_t)g->n + 4096, 1 << 18)
                                                 : (int64_t)g->n + 4096;
     size_t freeb = 0, totalb = 0;
     cudaMemGetInfo(&freeb, &totalb);
     // the far pile holds every open node beyond the current bucket: twice the
     // node count leaves room for stale copies between compactions
-    // (small graphs with bidirectional slots: room for the bucket lists)
-    const int64_t cap_f = b->o.queue_cap > 0      ? b->o.queue_cap
-                          : is_bidir_kind(hkind) ? std::max<int64_t>(2 * (int64_t)g->n, 1 << 18) + 4096
-                                                  : 2 * (int64_t)g->n + 4096;
+    int64_t cap_f = b->o.queue_cap > 0 ? b->o.queue_cap : 2 * (int64_t)g->n + 4096;
+    if (bidir) cap_f = bidir_cap_f(cap_f);
     const int skind = hk_slot_kind(b->hk);
     const int hb = (skind & SLOT_HASH) ? hash_bits(g->n) : 0;
     const size_t per = slot_bytes(g->n, cap, cap_f, skind, hb);

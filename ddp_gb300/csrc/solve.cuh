@@ -89,7 +89,22 @@ inline bool is_bidir_kind(int k) {
 // 16-byte pairs (graphs with coordinates)
 constexpr bool bidir_hk(int hk) { return hk >= 5 && hk <= 9; }
 constexpr bool pair16_hk(int hk) { return hk == 9; }
-int kernel_hk(int hkind, bool has_xy, bool hash);
+// Whether slots of `group` CTAs answer a batch kind by the bidirectional
+// search: the bidirectional kinds always; one-CTA slots also for no bound and
+// for hop bounds.  These are admissible on every graph, so the costs are the
+// same, and a one-directional search under so weak a bound expands orders of
+// magnitude more (300 queries, 100,000 nodes, hop bound: a reverse BFS of the
+// whole graph and 45k expansions per query, 9.86 ms; bidirectional: 0.8k
+// expansions, no BFS).  Wider slots and DDP_OPT_SYNC keep the A* engine.
+inline bool batch_bidir(int hkind, int group, int flags) {
+    if (is_bidir_kind(hkind)) return true;
+    return group <= 1 && !(flags & DDP_OPT_SYNC) &&
+           (hkind == DDP_H_ZERO || hkind == DDP_H_BFS_HOPS || hkind == DDP_H_BFS_CAPPED);
+}
+// Far memory (8-byte units per half, slot_bytes) of a bidirectional slot: the
+// bucket lists want 4 MB however small the graph or the caller's capacity.
+inline int64_t bidir_cap_f(int64_t want) { return want > (1 << 18) ? want : (int64_t)(1 << 18) + 4096; }
+int kernel_hk(int hkind, bool has_xy, bool hash, int group, int flags);
 int hk_slot_kind(int hk);
 
 // Slot kinds (bits): a per-target hop array; paired forward/reverse state;

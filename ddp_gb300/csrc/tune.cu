@@ -85,7 +85,7 @@ int ddp_batch_tune(ddp_graph *g, int32_t hkind, int32_t n, const int32_t *source
     }
     // 2. bucket width: half and twice the automatic one, then further steps
     //    of 2/3 (or 3/2) while the winning direction keeps winning
-    const uint32_t d0 = is_bidir_kind(hkind) ? auto_delta_bidir(g) : auto_delta(g);
+    const uint32_t d0 = batch_bidir(hkind, top_o.group, top_o.flags) ? auto_delta_bidir(g) : auto_delta(g);
     const ddp_opts shape = top_o;
     uint32_t best_d = d0;
     for (uint32_t dv : {d0 / 2, d0 * 2}) {

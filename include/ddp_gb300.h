@@ -46,7 +46,11 @@ enum ddp_status {
     DDP_ERR_NO_DEVICE = 7       /* no usable CUDA device                       */
 };
 
-/* Heuristic kinds for ddp_heuristic_build. */
+/* Heuristic kinds for ddp_heuristic_build, batches and serving.  One-CTA
+ * batch and serving slots answer DDP_H_ZERO, DDP_H_BFS_HOPS and
+ * DDP_H_BFS_CAPPED by the bidirectional search (same costs, no per-query BFS:
+ * the BFS fields of their stats are 0); slots of several CTAs (opts.group > 1)
+ * and DDP_OPT_SYNC run A* under these bounds. */
 enum ddp_heuristic_kind {
     DDP_H_ZERO = 0,      /* h = 0 (Dijkstra order)                              */
     DDP_H_BFS_HOPS = 1,  /* reverse-BFS hop count to the target x min arc
@@ -91,7 +95,8 @@ typedef struct ddp_opts {
     int32_t K;         /* nodes expanded per iteration (the reference's K queues);
                           0 = the whole current bucket                          */
     int32_t delta;     /* bucket width on f; 0 = chosen from the arc weights    */
-    int32_t block;     /* threads per CTA                                        */
+    int32_t block;     /* threads per CTA (bidirectional batches: 0 = chosen by
+                          the batch's size)                                       */
     int32_t grid;      /* CTAs (single query) or concurrent slots (batch)        */
     int64_t queue_cap; /* entries per search queue                               */
     void *stream;      /* cudaStream_t; NULL = the handle's own stream           */

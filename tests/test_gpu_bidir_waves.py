@@ -115,3 +115,36 @@ def test_flooding_search_on_the_device_path(gpu, oracle):
         assert np.array_equal(dc.cpu().numpy(), want)
     be.close()
     dg.close()
+
+
+@pytest.mark.parametrize("wmin,wmax", [(0, 3), (1, 1), (1, 1000000)])
+def test_hop_and_zero_bounds_agree_with_their_own_engine(gpu, oracle, wmin, wmax):
+    """One-CTA slots answer these kinds bidirectionally; wider slots and
+    DDP_OPT_SYNC run the A* engine.  Same costs, also on the layout that
+    updates leave behind and for unreachable and equal endpoints."""
+    d = gpu
+    rng = np.random.default_rng(wmax)
+    n, e = 3000, 9000  # no chain: some pairs are disconnected
+    u = np.sort(rng.integers(0, n, e))
+    off = np.concatenate([[0], np.cumsum(np.bincount(u, minlength=n))]).astype(np.int32)
+    g = d.CSR(n, off, rng.integers(0, n, e).astype(np.int32), rng.integers(wmin, wmax + 1, e).astype(np.uint32))
+    dg = d.DeviceGraph.from_csr(g)
+    S, T = rng.integers(0, n, 120).astype(np.int32), rng.integers(0, n, 120).astype(np.int32)
+    T[:3] = S[:3]
+    for rnd in range(2):
+        want = _want(oracle, g, S, T)
+        for kind in (d.H_ZERO, d.H_BFS_HOPS, d.H_BFS_CAPPED):
+            for kw in ({}, {"flags": d.OPT_SYNC}, {"group": 2}, {"delta": 7}, {"queue_cap": 64}):
+                be = d.BatchEngine(dg, kind, grid=12, **kw)
+                _check(oracle, be, g, S, T, want)
+                be.close()
+        if rnd == 0:
+            dj = rng.choice(e, 300, replace=False)
+            dyn = d.DynamicSearch(dg, 0, 1, d.H_ZERO)
+            iu, iv = rng.integers(0, n, 300).astype(np.int32), rng.integers(0, n, 300).astype(np.int32)
+            dyn.update(np.concatenate([np.zeros(300, np.int32), np.ones(300, np.int32)]),
+                       np.concatenate([u[dj], iu]), np.concatenate([g.col[dj], iv]),
+                       np.concatenate([g.w[dj], rng.integers(wmin, wmax + 1, 300).astype(np.uint32)]))
+            dyn.close()
+            g = dg.read_csr()
+    dg.close()
