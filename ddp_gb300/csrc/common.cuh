@@ -43,7 +43,8 @@ __host__ __device__ __forceinline__ uint64_t st_make(uint32_t g, int32_t p) {
 enum : int {
     ST_OVERFLOW = 1,  // a queue outgrew its capacity
     ST_TIMEOUT = 2,   // a bounded barrier wait gave up
-    ST_PATH_TRUNC = 4 // a path did not fit its buffer
+    ST_PATH_TRUNC = 4, // a path did not fit its buffer
+    ST_BUDGET = 8      // a search stopped at its budget of expansions
 };
 
 // Arcs are stored interleaved as {col, weight}: one 8-byte load per arc.

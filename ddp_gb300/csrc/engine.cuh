@@ -66,7 +66,8 @@ struct SearchCtl {
     unsigned int bar_count, bar_gen;  // grid barrier (single-query form)
     int cold_n;           // entries in the far pile's cold tier (keep mode)
     // what CTA 0 hands back after running phases alone (run_search)
-    int loc_near, loc_far, loc_waves;
+    int loc_near, loc_far, loc_waves, loc_flip, loc_done;
+    uint32_t loc_T;
 };
 
 // Buffers of one slot.
@@ -488,6 +489,7 @@ struct SearchParams {
     uint2 *cold = nullptr;
     int64_t cold_cap = 0;
     uint32_t cold_x = 0xFFFFFFFFu;
+    int64_t budget = 0;  // bidirectional search: entries it may expand (0: any number)
 };
 
 struct SearchResult {
@@ -503,11 +505,18 @@ struct SearchResult {
 // relaxation that pushed it), eight lanes walk one row, and a phase ends with
 // a block barrier.  It hands the list back when it outgrows LOCAL_OUT entries
 // or after LOCAL_WAVES phases (the other CTAs wait in a bounded barrier).
-// A 511 x 511 maze query (1,926 phases of 20-70 entries) so takes 3.6 ms;
-// with every phase on the grid it took 44 ms (23 us a phase).
+// While the far pile is small (LOCAL_FAR) it splits it too, and while the
+// list is narrow (LOCAL_FILL) it takes the next bucket in early, so that the
+// floods of successive buckets overlap instead of running one after the other
+// (out of keep mode; at most LOCAL_AHEAD buckets before the list empties).
+// A 511 x 511 maze query took 44 ms with every phase on the grid (1,926
+// phases of 20-70 entries, 23 us each), 3.2 ms with narrow phases here, 1.6
+// ms with overlapping buckets (16, 32 or 64 entries alike; wider buckets
+// instead expand nodes again and again: width 4 -> 6.6 ms).
 constexpr int LOCAL_IN = 256, LOCAL_OUT = 512;
+constexpr int LOCAL_FAR = 4096;
+constexpr int LOCAL_FILL = 32, LOCAL_AHEAD = 16;
 constexpr int LOCAL_WAVES = 4096;
-constexpr int LOCAL_LANES = 8;  // lanes per entry
 
 // entries that the warp rows (16 per CTA in every search kernel) hold as two
 // lists of uint4
@@ -519,23 +528,26 @@ static_assert(LOCAL_CAP >= LOCAL_IN && LOCAL_CAP >= LOCAL_OUT, "local lists hold
 // grid phase does.
 template <class Heur>
 __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H, const SearchParams &P,
-                             WarpRows *wrows, uint2 *qcur, int nnear, uint4 *fcur, int64_t nfar0, uint32_t T,
-                             uint32_t ht, unsigned long long &n_exp, unsigned long long &n_scan,
+                             WarpRows *wrows, uint2 *qcur, int nnear, uint4 *fcur, uint4 *falt, int64_t nfar0,
+                             uint32_t T, uint32_t ht, unsigned long long &n_exp, unsigned long long &n_scan,
                              unsigned long long &n_rel) {
     SearchCtl *ctl = B.ctl;
     // {node, g, row begin, row end}
     uint4 *buf = reinterpret_cast<uint4 *>(wrows);
     constexpr int cap = LOCAL_CAP;
     __shared__ int cnt[3];  // entries per wave, rotating
-    __shared__ int c_far, c_touch;
-    __shared__ unsigned int tg;
-    const int sub = threadIdx.x & (LOCAL_LANES - 1);
-    const int team = threadIdx.x / LOCAL_LANES, teams = blockDim.x / LOCAL_LANES;
+    __shared__ int c_far, c_touch, c_alt;
+    __shared__ unsigned int tg, far_min;  // far_min: no far entry has a smaller f
+    // lanes per entry: four for rows of four arcs or fewer on average
+    const int lanes = G.e <= 4 * (int64_t)G.n ? 4 : 8;
+    const int sub = threadIdx.x & (lanes - 1);
+    const int team = threadIdx.x / lanes, teams = blockDim.x / lanes;
     const int touch0 = *(volatile int *)&ctl->touched;
     if (threadIdx.x == 0) {
         cnt[0] = nnear;
         cnt[1] = cnt[2] = 0;
         c_far = c_touch = 0;
+        far_min = 0;
         tg = P.t >= 0 ? st_g(__ldcg(B.state + P.t)) : 0xFFFFFFFFu;
     }
     for (int i = threadIdx.x; i < nnear; i += blockDim.x) {
@@ -544,15 +556,67 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                             (uint32_t)row_end(G.off, G.oend, (int)en.x));
     }
     __syncthreads();
-    int m = nnear, wv = 0;
+    int m = nnear, wv = 0, ahead = 0, flip = 0, done = 0;
+    unsigned long long n_far = 0;
     uint4 *cur = buf, *nxt = buf + cap;
     for (;;) {
+        if (!P.keep && m < LOCAL_FILL) {
+            // the list is empty or narrow: the far pile's turn
+            const int64_t nf = nfar0 + c_far;
+            const uint64_t ft64 = (uint64_t)tg + ht;
+            const uint32_t ft = ft64 >= 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)ft64;
+            const uint32_t fm = far_min;
+            __syncthreads();  // every thread has read the words the branches below depend on
+            if (m == 0) ahead = 0;
+            if (nf == 0 || fm >= ft) {
+                if (m == 0) {
+                    done = 1;  // no open node with f < f(t)
+                    break;
+                }
+            } else if (nf <= LOCAL_FAR && (m == 0 || ahead < LOCAL_AHEAD)) {
+                T = sat_add(max(fm, T), P.delta);  // above the smallest f: something moves
+                ahead++;
+                n_far += (unsigned long long)nf;
+                if (threadIdx.x == 0) {
+                    c_alt = 0;
+                    far_min = 0xFFFFFFFFu;
+                }
+                __syncthreads();
+                for (int64_t i = threadIdx.x; i < nf; i += blockDim.x) {
+                    const uint4 e = __ldcg(fcur + i);
+                    if (e.z >= ft) continue;
+                    if (e.z < T) {
+                        const int p = atomicAdd(&cnt[wv % 3], 1);
+                        if (p < cap) {
+                            cur[p] = make_uint4(e.x, e.y, (uint32_t)row_begin(G.off, G.oend, (int)e.x),
+                                                (uint32_t)row_end(G.off, G.oend, (int)e.x));
+                            continue;
+                        }
+                    }
+                    falt[atomicAdd(&c_alt, 1)] = e;  // no more than were read
+                    atomicMin(&far_min, e.z);
+                }
+                __syncthreads();
+                nfar0 = c_alt;
+                m = min(cnt[wv % 3], cap);
+                uint4 *t = fcur;
+                fcur = falt;
+                falt = t;
+                flip ^= 1;
+                if (threadIdx.x == 0) c_far = 0;
+                __syncthreads();
+                if (m == 0) continue;  // far_min is known now: the next split moves something
+            } else if (m == 0) {
+                break;  // a large pile: the grid splits it
+            }
+        }
         int *push = &cnt[(wv + 1) % 3];
         if (threadIdx.x == 0) cnt[(wv + 2) % 3] = 0;
         const uint64_t ft64 = (uint64_t)(*(volatile unsigned int *)&tg) + ht;
         const uint32_t ft = ft64 >= 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)ft64;
         auto to_far = [&](uint32_t v, uint32_t g, uint32_t f) {
             const int64_t p = nfar0 + atomicAdd(&c_far, 1);
+            atomicMin(&far_min, f);
             if (p < B.cap_f) fcur[p] = make_uint4(v, g, f, 0u);
             else atomicOr(&ctl->status, ST_OVERFLOW);
         };
@@ -627,7 +691,7 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                         }
                     }
                 }
-                j += LOCAL_LANES;
+                j += lanes;
                 if (j >= r1) break;
                 a = G.oend ? __ldcg(G.arc + j) : __ldg(G.arc + j);
             }
@@ -638,9 +702,10 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
         uint4 *t = cur;
         cur = nxt;
         nxt = t;
-        if (m == 0 || m > LOCAL_OUT || wv >= LOCAL_WAVES || nfar0 + c_far > B.cap_f / 2) break;
-        __syncthreads();  // every thread has read c_far
+        if ((m == 0 && P.keep) || m > LOCAL_OUT || wv >= LOCAL_WAVES || nfar0 + c_far > B.cap_f / 2) break;
+        __syncthreads();  // every thread has read the counters
     }
+    __syncthreads();
     // the entries left go back to the near list (those past the shared list
     // are there already)
     for (int i = threadIdx.x; i < min(m, cap); i += blockDim.x) qcur[i] = make_uint2(cur[i].x, cur[i].y);
@@ -648,6 +713,10 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
         ctl->loc_near = m;
         ctl->loc_far = (int)(nfar0 + c_far);
         ctl->loc_waves = wv;
+        ctl->loc_T = T;
+        ctl->loc_flip = flip;
+        ctl->loc_done = done;
+        ctl->far_scanned += n_far;
         ctl->touched = touch0 + c_touch;
     }
 }
@@ -666,7 +735,8 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
         PhaseWords w;
         int status;
         uint32_t tg;
-        int loc_near, loc_far, loc_waves;
+        int loc_near, loc_far, loc_waves, loc_flip, loc_done;
+        uint32_t loc_T;
     } pc;
     __shared__ CtaFlush cf;
 
@@ -723,20 +793,30 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
         if constexpr (Grp::multi) {
             if (!splitting && head == 0 && nnext == 0 && !has_diff && nnear <= LOCAL_IN &&
                 nfar <= B.cap_f / 2 && (P.K <= 0 || P.K >= LOCAL_OUT)) {
-                if (grp.first_cta()) local_phases(G, B, H, P, wrows, qcur, (int)nnear, fcur, nfar, T, ht, n_exp, n_scan, n_rel);
+                if (grp.first_cta()) local_phases(G, B, H, P, wrows, qcur, (int)nnear, fcur, falt, nfar, T, ht, n_exp, n_scan, n_rel);
                 grp.sync_fetch([&] {
                     pc.loc_near = *(volatile int *)&ctl->loc_near;
                     pc.loc_far = *(volatile int *)&ctl->loc_far;
                     pc.loc_waves = *(volatile int *)&ctl->loc_waves;
+                    pc.loc_flip = *(volatile int *)&ctl->loc_flip;
+                    pc.loc_done = *(volatile int *)&ctl->loc_done;
+                    pc.loc_T = *(volatile uint32_t *)&ctl->loc_T;
                     pc.status = *(volatile int *)&ctl->status;
                     pc.tg = read_tg();
                 });
                 nnear = pc.loc_near;
                 nfar = pc.loc_far;
+                T = pc.loc_T;
+                if (pc.loc_flip) {
+                    uint4 *t2 = fcur;
+                    fcur = falt;
+                    falt = t2;
+                }
                 waves += pc.loc_waves;
                 status = pc.status;
                 tg = pc.tg;
                 if (status & (ST_OVERFLOW | ST_TIMEOUT)) break;
+                if (pc.loc_done) break;  // no open node with f < f(t)
                 if (it + waves > max_phases) {
                     if (grp.rank() == 0) atomicOr(&ctl->status, ST_TIMEOUT);
                     break;
@@ -1192,6 +1272,45 @@ __device__ uint32_t run_bfs_hops(const Grp &grp, const DevGraph &G, const SlotBu
     if (grp.rank() == 0) ctl->bfs_reached = b_reached;
     grp.sync();
     return complete ? HOPS_INF : lvl + 1;
+}
+
+// Parent walk t -> s into path[0..cap) in s..t order; returns the length
+// (0 when unreachable).  One CTA; buf holds bcap ids in shared memory: one
+// thread walks the chain of parents into it, then all copy it out in order
+// (reversing it in place took as long again as the walk).
+__device__ inline int32_t write_path_cta(const SlotBufs &B, int32_t s, int32_t t, int32_t *path, int32_t cap,
+                                         int32_t n, int *status, int32_t *buf, int32_t bcap) {
+    __shared__ int32_t s_len;
+    if (threadIdx.x == 0) {
+        int32_t len = 0;
+        uint64_t st = __ldcg(B.state + t);
+        if (st_g(st) < INF_G) {
+            for (int32_t c = t; c >= 0 && len <= n;) {
+                if (len < bcap) buf[len] = c;
+                len++;
+                if (c == s) break;
+                c = st_parent(st);
+                if (c >= 0) st = __ldcg(B.state + c);
+            }
+            if (len > cap) atomicOr(status, ST_PATH_TRUNC);
+            if (len > bcap) {
+                // longer than the buffer: a second walk writes it
+                int32_t c = t;
+                for (int32_t i = len - 1; i >= 0 && c >= 0; i--) {
+                    if (i < cap) path[i] = c;
+                    c = st_parent(__ldcg(B.state + c));
+                }
+            }
+        }
+        s_len = len;
+    }
+    __syncthreads();
+    const int32_t len = s_len;
+    if (len <= bcap)
+        for (int32_t i = threadIdx.x; i < len; i += blockDim.x)
+            if (len - 1 - i < cap) path[len - 1 - i] = buf[i];
+    __syncthreads();
+    return len;
 }
 
 // Parent walk t -> s into path[0..cap) in s..t order; returns the length

@@ -123,6 +123,7 @@ struct WaveQ {
     unsigned int pile_min[2];        // their smallest key
     int status;
     int touched;
+    long long spent;                 // entries expanded or dropped
     uint32_t settled[2][WAVE_FILTER];  // lazy labels: filter over settled nodes
     uint4 list[2][WAVE_NEAR];
 };
@@ -486,6 +487,7 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
         q->pile_min[0] = q->pile_min[1] = NONE;
         q->status = room < 1 ? ST_OVERFLOW : 0;
         q->touched = 0;
+        q->spent = 0;
         if (P.s == P.t) {
             q->mu = (unsigned long long)(uint32_t)P.s;  // length 0
         } else {
@@ -799,6 +801,13 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
                 // keeps the bucket that would reuse it out of the window
                 if (p.n[0]) q->lcnt[0][p.c[0] & (WAVE_LISTS - 1)] = 0;
                 if (p.n[1]) q->lcnt[1][p.c[1] & (WAVE_LISTS - 1)] = 0;
+                if (p.act == 0) {
+                    q->spent += p.m + p.n[0] + p.n[1];
+                    if (P.budget > 0 && q->spent > P.budget) {
+                        p.act = 1;
+                        q->status = ST_BUDGET;
+                    }
+                }
                 const int nn = (wv + 2) % 3;  // the counters of the wave after the next
                 q->near[nn] = 0;
                 q->near_min[nn][0] = q->near_min[nn][1] = NONE;

@@ -150,6 +150,7 @@ void graph_release(ddp_graph *g) {
     if (!g) return;
     graph_flush_frees(g);
     workspace_release(g);
+    for (uint32_t *p : g->spare) cudaFree(p);
     cudaFree(g->d_off);
     cudaFree(g->d_arc);
     cudaFree(g->d_roff);

@@ -66,6 +66,9 @@ struct ddp_graph {
     int32_t lm_bits = 16;
     int64_t lm_stamp = -1;
     std::vector<int32_t> lm_ids;
+    // arrays of n words that freed heuristics left for the next ones (two at most)
+    std::mutex spare_mu;
+    std::vector<uint32_t *> spare;
     // single-query workspace, allocated on first use
     struct Workspace *ws = nullptr;
 };

@@ -146,35 +146,128 @@ __global__ void k_reset_touched(SlotArrays sa) {
         B.state[B.touched[i]] = ~0ull;
 }
 
-// Single-query reverse BFS (heuristic build) over the whole grid.
+// What a single-query kernel returns, in host memory mapped into the device:
+// the host reads it after one synchronisation, with no copies of its own.
+constexpr int SOLVE_PATH = 4096;  // path ids returned with it
+struct SolveOut {
+    int32_t cost, len, status, iters;
+    long long expanded, scanned, relaxed, far_scanned, touched;
+    uint32_t hcap;  // BFS: hop cap of unreached nodes
+    int32_t path[SOLVE_PATH];
+};
+
+// Single-query reverse BFS (heuristic build) over the whole grid; values,
+// when wanted, receives every node's bound (-1: cannot reach the target).
 __global__ void __launch_bounds__(512) k_bfs_single(DevGraph G, SlotArrays sa, uint32_t *hops,
-                                                    int32_t t, long long budget) {
+                                                    int32_t t, long long budget, int32_t *values, SolveOut *out) {
     __shared__ WarpRows wrows[MAX_WARPS];
     SlotBufs B = slot_of(sa, 0);
     B.hops = hops;
     GridGroup grp{{&B.ctl->bar_count, &B.ctl->bar_gen}, &B.ctl->status};
     // q0 is the ring of the asynchronous engine: keep it clean
     const uint32_t cap = run_bfs_hops(grp, G, B, t, wrows, 0u, (int64_t)budget, true);
-    if (grp.rank() == 0) B.ctl->hcap = cap;
+    if (values)
+        for (int64_t v = grp.rank(); v < G.n; v += grp.size()) {
+            const uint32_t x = __ldcg(hops + v);
+            const uint32_t hv = x == HOPS_INF ? cap : x;
+            const unsigned long long p = (unsigned long long)hv * G.wmin;
+            values[v] = hv == HOPS_INF ? -1 : p >= (unsigned long long)INT32_MAX - 1 ? INT32_MAX - 1 : (int32_t)p;
+        }
+    if (grp.rank() == 0) {
+        out->hcap = cap;
+        out->status = *(volatile int *)&B.ctl->status;
+    }
 }
 
-// Single-query GA* over the whole grid (cooperative launch).
+// The end of a single query, by its first CTA: path (to the device array and,
+// as far as it fits, to the host's), result and counters.  warp: the path is
+// the caller's already (len >= 0), else it is walked here.
+__device__ void solve_report(const DevGraph &G, const SlotBufs &B, const SearchParams &P, const SearchResult &r,
+                             SolveOut *out, int32_t *path, int32_t path_cap, int32_t len, int32_t *buf, int32_t bcap) {
+    const bool ok = !(*(volatile int *)&B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT | ST_BUDGET));
+    if (len < 0) len = ok ? write_path_cta(B, P.s, P.t, path, path_cap, G.n, &B.ctl->status, buf, bcap) : 0;
+    for (int32_t i = threadIdx.x; i < min(len, SOLVE_PATH); i += blockDim.x) out->path[i] = __ldcg(path + i);
+    if (threadIdx.x == 0) {
+        out->cost = r.cost >= INF_G ? DDP_INF : (int32_t)r.cost;
+        out->len = len;
+        out->status = *(volatile int *)&B.ctl->status;
+        out->iters = r.iters;
+        out->expanded = (long long)B.ctl->expanded;
+        out->scanned = (long long)B.ctl->scanned;
+        out->relaxed = (long long)B.ctl->relaxed;
+        out->far_scanned = (long long)B.ctl->far_scanned;
+        out->touched = (long long)B.ctl->touched;
+    }
+}
+
+// Single-query GA* over the whole grid (cooperative launch).  One CTA per SM:
+// two would halve the registers (220-640 bytes of spills per thread) and
+// double the CTAs at every barrier (511 x 511 maze 4.58 -> 3.64 ms; 250,000
+// nodes with a caller's heuristic 0.75 -> 0.68 ms).
 template <class Heur>
-// One CTA per SM: two would halve the registers (220-640 bytes of spills per
-// thread) and double the CTAs at every barrier (511 x 511 maze 4.58 -> 3.64
-// ms; 250,000 nodes with a caller's heuristic 0.75 -> 0.68 ms).
 __global__ void __launch_bounds__(512, 1)
-    k_solve_single(DevGraph G, SlotArrays sa, Heur H, SearchParams P, int32_t *out, int32_t *path,
+    k_solve_single(DevGraph G, SlotArrays sa, Heur H, SearchParams P, SolveOut *out, int32_t *path,
                    int32_t path_cap) {
     __shared__ WarpRows wrows[MAX_WARPS];
     SlotBufs B = slot_of(sa, 0);
     GridGroup grp{{&B.ctl->bar_count, &B.ctl->bar_gen}, &B.ctl->status};
-    SearchResult r = run_search(grp, G, B, H, P, wrows);
-    if (grp.rank() == 0) {
-        out[0] = r.cost >= INF_G ? DDP_INF : (int32_t)r.cost;
-        out[1] = write_path(B, P.s, P.t, path, path_cap, G.n, &B.ctl->status);
-        out[2] = B.ctl->status;
-        out[3] = r.iters;
+    const SearchResult r = run_search(grp, G, B, H, P, wrows);
+    if (grp.first_cta())
+        solve_report(G, B, P, r, out, path, path_cap, -1, reinterpret_cast<int32_t *>(wrows),
+                     (int32_t)(sizeof(wrows) / sizeof(int32_t)));
+    grp.sync();  // the path is read: the labels may go
+    const int cnt = *(volatile int *)&B.ctl->touched;
+    for (int i = grp.rank(); i < cnt; i += grp.size()) B.state[B.touched[i]] = ~0ull;
+}
+
+// Single query on one CTA by the bidirectional search (HK as in k_batch).
+template <int HK>
+__global__ void __launch_bounds__(1024, 1)
+    k_solve_bidir(DevGraph G, SlotArrays sa, SearchParams P, SolveOut *out, int32_t *path, int32_t path_cap) {
+    __shared__ WaveQ q;
+    __shared__ uint32_t s_ep;
+    __shared__ int32_t s_len;
+    SlotBufs B = slot_of(sa, 0);
+    if (threadIdx.x == 0) {
+        s_ep = *sa.epoch + 1;  // 0: the epochs wrapped, clear the records
+        *sa.epoch = s_ep == 0 ? 1u : s_ep;
+        B.ctl->status = 0;
+    }
+    __syncthreads();
+    uint32_t ep = s_ep;
+    if constexpr (!pair16_hk(HK)) {
+        if (ep == 0) {
+            for (size_t i = threadIdx.x; i < (size_t)B.swords; i += blockDim.x) B.state[i] = 0ull;
+            ep = 1;
+            __syncthreads();
+        }
+    }
+    SearchResult r;
+    int32_t *buf = reinterpret_cast<int32_t *>(q.list);
+    auto walk = [&](const auto &R) {
+        if (threadIdx.x < 32 && !(*(volatile int *)&B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT | ST_BUDGET))) {
+            const int32_t l = write_path_bidir(G, R, ep, P.s, P.t, q.mu, path, path_cap, &B.ctl->status, buf);
+            if (threadIdx.x == 0) s_len = l;
+        }
+    };
+    if (threadIdx.x == 0) s_len = 0;
+    if constexpr (pair16_hk(HK)) {
+        const RecPair16 R{B.state};
+        r = run_bidir_cta<false>(G, B, P, ep, &q, PotNone{}, R);
+        walk(R);
+    } else {
+        const RecDense R{{}, B.state};
+        r = run_bidir_cta<true>(G, B, P, ep, &q, PotNone{}, R);
+        walk(R);
+    }
+    __syncthreads();
+    solve_report(G, B, P, r, out, path, path_cap, s_len, buf, 2 * PATH_BUF);
+    if constexpr (pair16_hk(HK)) {
+        ulonglong4_32a ones;
+        ones.x = ones.y = ones.z = ones.w = ~0ull;
+        const int cnt = *(volatile int *)&B.ctl->touched;
+        for (int i = threadIdx.x; i < cnt; i += blockDim.x)
+            reinterpret_cast<ulonglong4_32a *>(B.state)[B.touched[i] >> 1] = ones;
     }
 }
 
@@ -684,21 +777,18 @@ __global__ void __launch_bounds__(512, 2) k_batch_group(DevGraph G, SlotArrays s
 // Single query on one CTA with the asynchronous engine (narrow searches).
 template <class Heur>
 __global__ void __launch_bounds__(512, 2)
-    k_solve_cta(DevGraph G, SlotArrays sa, Heur H, SearchParams P, int32_t *out, int32_t *path, int32_t path_cap) {
+    k_solve_cta(DevGraph G, SlotArrays sa, Heur H, SearchParams P, SolveOut *out, int32_t *path, int32_t path_cap) {
     __shared__ WarpRows wrows[MAX_WARPS];
     __shared__ CtaQ sq;
     SlotBufs B = slot_of(sa, 0);
-    SearchResult r = run_search_cta<Heur, true>(G, B, H, P, wrows, &sq);  // one query: latency first
-    if (threadIdx.x == 0) {
-        out[0] = r.cost >= INF_G ? DDP_INF : (int32_t)r.cost;
-        out[1] = (B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT)) ? 0 : write_path(B, P.s, P.t, path, path_cap, G.n, &B.ctl->status);
-        out[2] = B.ctl->status;
-        out[3] = r.iters;
-    }
-    if (B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT)) {
-        __syncthreads();
+    const SearchResult r = run_search_cta<Heur, true>(G, B, H, P, wrows, &sq);  // one query: latency first
+    solve_report(G, B, P, r, out, path, path_cap, -1, reinterpret_cast<int32_t *>(wrows),
+                 (int32_t)(sizeof(wrows) / sizeof(int32_t)));
+    __syncthreads();
+    if (B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT))
         for (int64_t i = threadIdx.x; i < B.cap_q; i += blockDim.x) B.q0[i].x = RING_EMPTY;
-    }
+    const int cnt = *(volatile int *)&B.ctl->touched;
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x) B.state[B.touched[i]] = ~0ull;
 }
 
 // ---- launch helpers ---------------------------------------------------------
@@ -845,17 +935,24 @@ using namespace ddp;
 // ---- single-query workspace ------------------------------------------------
 struct Workspace {
     SlotArrays sa;
-    int32_t *d_out = nullptr;   // cost, path len, status, iters
-    int32_t *d_path = nullptr;  // n
+    SlotArrays pa;              // a bidirectional slot (first use)
+    int pa_hk = 0;              // its k_batch instance (0: none, -1: no memory for one)
+    int32_t *d_out = nullptr;   // landmark searches: status
+    int32_t *d_path = nullptr;  // n: a path, or the values of a heuristic
+    SolveOut *h_res = nullptr, *d_res = nullptr;  // results (mapped host memory)
     int64_t cap = 0;
+    bool dirty = true;       // the control block may hold a failed run's words
+    bool ring_dirty = false; // grid searches leave entries in q0, the one-CTA ring
 };
 
 namespace ddp {
 void workspace_release(ddp_graph *g) {
     if (!g->ws) return;
     slots_free(g->ws->sa);
+    slots_free(g->ws->pa);
     cudaFree(g->ws->d_out);
     cudaFree(g->ws->d_path);
+    cudaFreeHost(g->ws->h_res);
     delete g->ws;
     g->ws = nullptr;
 }
@@ -866,14 +963,74 @@ static int workspace_ensure(ddp_graph *g, int64_t cap) {
     Workspace *w = new Workspace();
     g->ws = w;
     int rc = slots_alloc(w->sa, g->n, 1, cap, cap, false, g->stream);
-    if (rc) {
+    cudaError_t e = cudaSuccess;
+    if (!rc) e = cudaMalloc(&w->d_out, sizeof(int32_t) * 8);
+    if (!rc && e == cudaSuccess) e = cudaMalloc(&w->d_path, sizeof(int32_t) * (size_t)g->n);
+    if (!rc && e == cudaSuccess) e = cudaHostAlloc(&w->h_res, sizeof(SolveOut), cudaHostAllocMapped);
+    if (!rc && e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&w->d_res, w->h_res, 0);
+    // the slot is filled on the graph's stream; queries may use another
+    if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    if (rc || e != cudaSuccess) {
         workspace_release(g);
-        return rc;
+        return rc ? rc : cuda_fail(e, "single-query workspace");
     }
     w->cap = cap;
-    DDP_CUDA(cudaMalloc(&w->d_out, sizeof(int32_t) * 8));
-    DDP_CUDA(cudaMalloc(&w->d_path, sizeof(int32_t) * (size_t)g->n));
     return DDP_OK;
+}
+
+// The workspace's bidirectional slot for the graph as it is now (coordinates
+// choose the record layout); false when there is no memory for one.
+static bool workspace_bidir(ddp_graph *g) {
+    Workspace *w = g->ws;
+    const int hk = kernel_hk(DDP_H_BIDIR, g->d_xy != nullptr, false, 1, 0);
+    if (w->pa_hk == hk) return true;
+    if (w->pa_hk == -1) return false;
+    slots_free(w->pa);
+    w->pa_hk = -1;
+    if (slots_alloc(w->pa, g->n, 1, 0, bidir_cap_f(2 * (int64_t)g->n + 4096), hk_slot_kind(hk), g->stream) ||
+        cudaStreamSynchronize(g->stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        slots_free(w->pa);
+        return false;
+    }
+    w->pa_hk = hk;
+    return true;
+}
+
+// A clean control block for the next launch on st.
+static cudaError_t workspace_begin(Workspace *w, cudaStream_t st) {
+    if (!w->dirty) return cudaSuccess;
+    return cudaMemsetAsync(w->sa.ctl, 0, sizeof(SearchCtl), st);
+}
+
+// Arrays of n 32-bit words for heuristics: freed ones are kept (two at most)
+// for the next heuristic of the graph.  Every call that uses one has
+// synchronised its stream before it returns.
+static uint32_t *node_words_take(ddp_graph *g, cudaError_t *e) {
+    {
+        std::lock_guard<std::mutex> lk(g->spare_mu);
+        if (!g->spare.empty()) {
+            uint32_t *p = g->spare.back();
+            g->spare.pop_back();
+            *e = cudaSuccess;
+            return p;
+        }
+    }
+    uint32_t *p = nullptr;
+    *e = cudaMalloc(&p, sizeof(uint32_t) * (size_t)g->n);
+    return *e == cudaSuccess ? p : nullptr;
+}
+
+static void node_words_give(ddp_graph *g, uint32_t *p) {
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> lk(g->spare_mu);
+        if (g->spare.size() < 2) {
+            g->spare.push_back(p);
+            return;
+        }
+    }
+    cudaFree(p);
 }
 }  // namespace ddp
 
@@ -882,7 +1039,7 @@ struct ddp_heuristic {
     int kind = DDP_H_ZERO;
     int32_t target = -1;
     uint32_t *d_hops = nullptr;  // BFS kind
-    int32_t *d_h = nullptr;      // USER kind
+    uint32_t *d_h = nullptr;     // USER kind (int32 values)
     int32_t tx = 0, ty = 0;      // MANHATTAN kind
     uint32_t cap = HOPS_INF;     // hop cap of a BFS kind (HOPS_INF = exact)
 };
@@ -894,6 +1051,20 @@ struct ddp_query {
 };
 
 namespace ddp {
+// Entries a single query may expand bidirectionally on one CTA before the
+// whole GPU takes it.
+constexpr int64_t SOLVE_BIDIR_BUDGET = 32768;
+
+// Whether a single query tries the bidirectional search first: no bound, or
+// a hop bound where the weights differ enough that it says little (with unit
+// weights hops are the distance itself and A* walks straight to the target),
+// and no option that asks for the A* engine's launch.
+static bool solve_bidir_first(const ddp_graph *g, int kind, const ddp_opts &o) {
+    if (o.flags || o.grid || o.block || o.delta || o.queue_cap || o.group) return false;
+    if (kind == DDP_H_ZERO) return true;
+    return is_bfs_kind(kind) && g->wmax / 4 >= std::max(g->wmin, 1u);
+}
+
 uint32_t *heuristic_hops_ptr(const ddp_heuristic *h) { return h ? h->d_hops : nullptr; }
 }  // namespace ddp
 
@@ -922,36 +1093,27 @@ int ddp_heuristic_build(ddp_graph *g, int32_t target, int32_t kind, const int32_
     case DDP_H_BFS_CAPPED: {
         int rc = workspace_ensure(g, (int64_t)g->n + 1024);
         if (rc) return bail(rc);
-        cudaError_t e = cudaMalloc(&h->d_hops, sizeof(uint32_t) * (size_t)g->n);
+        cudaError_t e;
+        h->d_hops = node_words_take(g, &e);
         if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(hops)"));
         DevGraph G = graph_view(g);
-        SlotArrays sa = g->ws->sa;
-        DDP_CUDA(cudaMemsetAsync(sa.ctl, 0, sizeof(SearchCtl), g->stream));
-        int grid = coop_grid(k_bfs_single, 512, 0);
+        Workspace *w = g->ws;
+        DDP_CUDA(workspace_begin(w, g->stream));
+        w->dirty = true;
+        static const int grid = coop_grid(k_bfs_single, 512, 0);
         long long budget = kind == DDP_H_BFS_CAPPED ? (long long)bfs_budget(g->n) : 0;
-        void *args[] = {&G, &sa, &h->d_hops, &target, &budget};
+        int32_t *values = out_h ? w->d_path : nullptr;
+        void *args[] = {&G, &w->sa, &h->d_hops, &target, &budget, &values, &w->d_res};
         e = coop_launch(k_bfs_single, grid, 512, args, g->stream);
         if (e != cudaSuccess) return bail(cuda_fail(e, "k_bfs_single launch"));
-        SearchCtl ctl;
-        DDP_CUDA(cudaMemcpyAsync(&ctl, sa.ctl, sizeof(ctl), cudaMemcpyDeviceToHost, g->stream));
+        if (out_h)
+            DDP_CUDA(cudaMemcpyAsync(out_h, values, sizeof(int32_t) * (size_t)g->n, cudaMemcpyDeviceToHost, g->stream));
         DDP_CUDA(cudaStreamSynchronize(g->stream));
-        if (ctl.status & (ST_OVERFLOW | ST_TIMEOUT))
-            return bail(fail(ctl.status & ST_TIMEOUT ? DDP_ERR_TIMEOUT : DDP_ERR_QUEUE_OVERFLOW,
+        if (w->h_res->status & (ST_OVERFLOW | ST_TIMEOUT))
+            return bail(fail(w->h_res->status & ST_TIMEOUT ? DDP_ERR_TIMEOUT : DDP_ERR_QUEUE_OVERFLOW,
                              "heuristic BFS did not complete"));
-        h->cap = ctl.hcap;
-        if (out_h) {
-            std::vector<uint32_t> hops((size_t)g->n);
-            DDP_CUDA(cudaMemcpy(hops.data(), h->d_hops, sizeof(uint32_t) * (size_t)g->n,
-                                cudaMemcpyDeviceToHost));
-            for (int32_t i = 0; i < g->n; i++) {
-                if (hops[(size_t)i] == HOPS_INF) hops[(size_t)i] = h->cap;
-            }
-            for (int32_t i = 0; i < g->n; i++)
-                out_h[i] = hops[(size_t)i] == HOPS_INF ? -1
-                                                        : (int32_t)std::min<uint64_t>(
-                                                              (uint64_t)hops[(size_t)i] * g->wmin,
-                                                              (uint64_t)INT32_MAX - 1);
-        }
+        w->dirty = false;
+        h->cap = w->h_res->hcap;
         break;
     }
     case DDP_H_MANHATTAN: {
@@ -981,7 +1143,8 @@ int ddp_heuristic_build(ddp_graph *g, int32_t target, int32_t kind, const int32_
     }
     case DDP_H_USER: {
         if (!user_h) return bail(fail(DDP_ERR_INVALID, "user_h is null"));
-        cudaError_t e = cudaMalloc(&h->d_h, sizeof(int32_t) * (size_t)g->n);
+        cudaError_t e;
+        h->d_h = node_words_take(g, &e);
         if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(h)"));
         DDP_CUDA(cudaMemcpy(h->d_h, user_h, sizeof(int32_t) * (size_t)g->n,
                             cudaMemcpyHostToDevice));
@@ -1032,6 +1195,7 @@ static int sssp_into(ddp_graph *g, int32_t src, bool reverse, int32_t *dist) {
         if (rc) return rc;
         Workspace *w = g->ws;
         DDP_CUDA(cudaMemsetAsync(w->sa.ctl, 0, sizeof(SearchCtl), g->stream));
+        w->dirty = true;
         const int grid = coop_grid(k_sssp, 512, 0);
         void *args[] = {&G, &w->sa, &P, &dist, &w->d_out};
         cudaError_t e = coop_launch(k_sssp, grid, 512, args, g->stream);
@@ -1176,8 +1340,8 @@ int ddp_landmarks_build_bits(ddp_graph *g, int32_t count, int32_t bits, uint64_t
 
 int ddp_heuristic_free(ddp_heuristic *h) {
     if (!h) return DDP_OK;
-    cudaFree(h->d_hops);
-    cudaFree(h->d_h);
+    node_words_give(h->g, h->d_hops);
+    node_words_give(h->g, h->d_h);
     graph_unref(h->g);
     delete h;
     return DDP_OK;
@@ -1202,20 +1366,68 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
     const uint32_t delta = o.delta > 0 ? (uint32_t)o.delta : auto_delta(g);
     DevGraph G = graph_view(g);
     SearchParams P{source, target, delta, o.K, 0, 0, 0};
+    const int kind = h ? h->kind : DDP_H_ZERO;
+    // reads what a kernel left in w->h_res; path ids past the host's part come from the device
+    auto result = [&](Workspace *w) -> int {
+        const SolveOut &r = *w->h_res;
+        ddp_query *q = new ddp_query();
+        q->cost = r.cost;
+        q->stats[0] = r.expanded;
+        q->stats[1] = r.scanned;
+        q->stats[2] = r.relaxed;
+        q->stats[3] = r.iters;
+        q->stats[6] = r.far_scanned;
+        q->stats[7] = r.touched;
+        if (r.len > 0) {
+            q->path.resize((size_t)r.len);
+            std::memcpy(q->path.data(), r.path, sizeof(int32_t) * (size_t)std::min(r.len, SOLVE_PATH));
+            if (r.len > SOLVE_PATH) {
+                cudaError_t ce = cudaMemcpy(q->path.data(), w->d_path, sizeof(int32_t) * (size_t)r.len,
+                                            cudaMemcpyDeviceToHost);
+                if (ce != cudaSuccess) {
+                    delete q;
+                    return cuda_fail(ce, "path readback");
+                }
+            }
+        }
+        *out = q;
+        return DDP_OK;
+    };
+    if (solve_bidir_first(g, kind, o)) {
+        int rc = workspace_ensure(g, cap);
+        if (rc) return rc;
+        Workspace *w = g->ws;
+        if (workspace_bidir(g)) {
+            SearchParams Pb = P;
+            Pb.delta = auto_delta_bidir(g);
+            Pb.budget = SOLVE_BIDIR_BUDGET;
+            void *args[] = {&G, &w->pa, &Pb, &w->d_res, &w->d_path, &g->n};
+            const void *fn = pair16_hk(w->pa_hk) ? (const void *)k_solve_bidir<9> : (const void *)k_solve_bidir<5>;
+            cudaError_t e = cudaLaunchKernel(fn, dim3(1), dim3(1024), args, 0, st);
+            if (e != cudaSuccess) return cuda_fail(e, "k_solve_bidir launch");
+            DDP_CUDA(cudaStreamSynchronize(st));
+            if (!(w->h_res->status & (ST_OVERFLOW | ST_TIMEOUT | ST_BUDGET))) return result(w);
+            // a long search: the whole GPU takes it
+        }
+    }
     for (int attempt = 0; attempt < 4; attempt++) {
         int rc = workspace_ensure(g, cap);
         if (rc) return rc;
         Workspace *w = g->ws;
-        DDP_CUDA(cudaMemsetAsync(w->sa.ctl, 0, sizeof(SearchCtl), st));
+        DDP_CUDA(workspace_begin(w, st));
+        w->dirty = true;
         cudaError_t e;
-        const int kind = h ? h->kind : DDP_H_ZERO;
         const bool one_cta = (o.flags & DDP_OPT_ONE_CTA) != 0;
+        if (one_cta && w->ring_dirty) {
+            DDP_CUDA(cudaMemsetAsync(w->sa.q, 0xFF, sizeof(uint2) * (size_t)w->sa.cap_q * 2, st));
+            w->ring_dirty = false;
+        }
         if (one_cta) {
             void *hp = nullptr;
             HeurHops Hh{h ? h->d_hops : nullptr, g->wmin, h ? h->cap : HOPS_INF, 0u};
             HeurManhattan Hm{g->d_xy, h ? h->tx : 0, h ? h->ty : 0, g->wmin};
             HeurEuclid He{g->d_xy, h ? h->tx : 0, h ? h->ty : 0, g->rho_fp};
-            HeurArray Ha{h ? h->d_h : nullptr};
+            HeurArray Ha{h ? reinterpret_cast<const int32_t *>(h->d_h) : nullptr};
             HeurALT Hl{G.lm, G.lm_L, G.lm_scale, target, G.lm_bits};
             HeurZero Hz{};
             const void *fn;
@@ -1225,76 +1437,50 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
             else if (kind == DDP_H_USER) { fn = (const void *)k_solve_cta<HeurArray>; hp = &Ha; }
             else if (kind == DDP_H_LANDMARK) { fn = (const void *)k_solve_cta<HeurALT>; hp = &Hl; }
             else { fn = (const void *)k_solve_cta<HeurZero>; hp = &Hz; }
-            void *args[] = {&G, &w->sa, hp, &P, &w->d_out, &w->d_path, &g->n};
+            void *args[] = {&G, &w->sa, hp, &P, &w->d_res, &w->d_path, &g->n};
             e = cudaLaunchKernel(fn, dim3(1), dim3(block), args, 0, st);
         } else if (kind == DDP_H_BFS_HOPS || kind == DDP_H_BFS_CAPPED) {
             HeurHops H{h->d_hops, g->wmin, h->cap, 0u};
             int grid = coop_grid(k_solve_single<HeurHops>, block, o.grid);
-            void *args[] = {&G, &w->sa, &H, &P, &w->d_out, &w->d_path, &g->n};
+            void *args[] = {&G, &w->sa, &H, &P, &w->d_res, &w->d_path, &g->n};
             e = coop_launch(k_solve_single<HeurHops>, grid, block, args, st);
         } else if (kind == DDP_H_MANHATTAN) {
             HeurManhattan H{g->d_xy, h->tx, h->ty, g->wmin};
             int grid = coop_grid(k_solve_single<HeurManhattan>, block, o.grid);
-            void *args[] = {&G, &w->sa, &H, &P, &w->d_out, &w->d_path, &g->n};
+            void *args[] = {&G, &w->sa, &H, &P, &w->d_res, &w->d_path, &g->n};
             e = coop_launch(k_solve_single<HeurManhattan>, grid, block, args, st);
         } else if (kind == DDP_H_EUCLID) {
             HeurEuclid H{g->d_xy, h->tx, h->ty, g->rho_fp};
             int grid = coop_grid(k_solve_single<HeurEuclid>, block, o.grid);
-            void *args[] = {&G, &w->sa, &H, &P, &w->d_out, &w->d_path, &g->n};
+            void *args[] = {&G, &w->sa, &H, &P, &w->d_res, &w->d_path, &g->n};
             e = coop_launch(k_solve_single<HeurEuclid>, grid, block, args, st);
         } else if (kind == DDP_H_USER) {
-            HeurArray H{h->d_h};
+            HeurArray H{reinterpret_cast<const int32_t *>(h->d_h)};
             int grid = coop_grid(k_solve_single<HeurArray>, block, o.grid);
-            void *args[] = {&G, &w->sa, &H, &P, &w->d_out, &w->d_path, &g->n};
+            void *args[] = {&G, &w->sa, &H, &P, &w->d_res, &w->d_path, &g->n};
             e = coop_launch(k_solve_single<HeurArray>, grid, block, args, st);
         } else if (kind == DDP_H_LANDMARK) {
             HeurALT H{G.lm, G.lm_L, G.lm_scale, target, G.lm_bits};
             int grid = coop_grid(k_solve_single<HeurALT>, block, o.grid);
-            void *args[] = {&G, &w->sa, &H, &P, &w->d_out, &w->d_path, &g->n};
+            void *args[] = {&G, &w->sa, &H, &P, &w->d_res, &w->d_path, &g->n};
             e = coop_launch(k_solve_single<HeurALT>, grid, block, args, st);
         } else {
             HeurZero H{};
             int grid = coop_grid(k_solve_single<HeurZero>, block, o.grid);
-            void *args[] = {&G, &w->sa, &H, &P, &w->d_out, &w->d_path, &g->n};
+            void *args[] = {&G, &w->sa, &H, &P, &w->d_res, &w->d_path, &g->n};
             e = coop_launch(k_solve_single<HeurZero>, grid, block, args, st);
         }
         if (e != cudaSuccess) return cuda_fail(e, "k_solve_single launch");
-        if (!one_cta)  // the phase-synchronous engine leaves entries in q0/q1
-            DDP_CUDA(cudaMemsetAsync(w->sa.q, 0xFF, sizeof(uint2) * (size_t)w->sa.cap_q * 2, st));
-        k_reset_touched<<<dim3(256, 1), 256, 0, st>>>(w->sa);
-        DDP_CUDA(cudaGetLastError());
-        int32_t res[4];
-        SearchCtl ctl;
-        DDP_CUDA(cudaMemcpyAsync(res, w->d_out, sizeof(res), cudaMemcpyDeviceToHost, st));
-        DDP_CUDA(cudaMemcpyAsync(&ctl, w->sa.ctl, sizeof(ctl), cudaMemcpyDeviceToHost, st));
+        if (!one_cta) w->ring_dirty = true;  // the phase-synchronous engine leaves entries in q0
         DDP_CUDA(cudaStreamSynchronize(st));
-        if (res[2] & ST_TIMEOUT) return fail(DDP_ERR_TIMEOUT, "search barrier timed out");
-        if (res[2] & ST_OVERFLOW) {
+        if (w->h_res->status & ST_TIMEOUT) return fail(DDP_ERR_TIMEOUT, "search barrier timed out");
+        if (w->h_res->status & ST_OVERFLOW) {
             if (o.queue_cap > 0) return fail(DDP_ERR_QUEUE_OVERFLOW, "search queue overflow");
             cap *= 2;  // automatic capacity: grow and retry
             continue;
         }
-        ddp_query *q = new ddp_query();
-        q->cost = res[0];
-        q->stats[0] = (int64_t)ctl.expanded;
-        q->stats[1] = (int64_t)ctl.scanned;
-        q->stats[2] = (int64_t)ctl.relaxed;
-        q->stats[3] = res[3];
-        q->stats[4] = 0;
-        q->stats[5] = 0;
-        q->stats[6] = (int64_t)ctl.far_scanned;
-        q->stats[7] = (int64_t)ctl.touched;
-        if (res[1] > 0) {
-            q->path.resize((size_t)res[1]);
-            cudaError_t ce = cudaMemcpy(q->path.data(), w->d_path, sizeof(int32_t) * (size_t)res[1],
-                                        cudaMemcpyDeviceToHost);
-            if (ce != cudaSuccess) {
-                delete q;
-                return cuda_fail(ce, "path readback");
-            }
-        }
-        *out = q;
-        return DDP_OK;
+        w->dirty = false;
+        return result(w);
     }
     return fail(DDP_ERR_QUEUE_OVERFLOW, "search queue overflow after retries");
 }
