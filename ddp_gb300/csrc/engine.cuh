@@ -243,7 +243,11 @@ struct HeurALT {
                 terms<B>(bv, bt, m, cm);
             }
         }
-        if (cm) return INF_G;
+        return cm ? INF_G : top<B>(m);
+    }
+    // the bound of the lane-wise maximum m
+    template <int B>
+    __device__ __forceinline__ uint32_t top(uint32_t m) const {
         const uint32_t mx = B == 8 ? max(max(m & 0xFFu, (m >> 8) & 0xFFu), max((m >> 16) & 0xFFu, m >> 24))
                                    : max(m & 0xFFFFu, m >> 16);
         // mx s <= q s <= the largest table distance, below INF_G

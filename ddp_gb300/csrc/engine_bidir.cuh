@@ -356,8 +356,15 @@ __device__ inline int32_t write_path_bidir(const DevGraph &G, const Rec &R, uint
 // the plain engine holds on the keys, with the stop rule a + b >= 2 mu and
 // pruning of a label g at v when g + pt(v) >= mu (forward) or
 // g + ps(v) >= mu (reverse).  PotNone keeps the keys equal to g.
+//
+// slack: by how much a key may exceed the key of some consistent potential
+// pair.  The proofs hold on the consistent keys, so the stop rule and the
+// pruning allow for it on both sides: a + b >= 2 mu + 2 slack.
+// table: the potentials are read from a table row per node, so they are
+// evaluated only for relaxations that improve the label.
 struct PotNone {
-    static constexpr bool on = false;
+    static constexpr bool on = false, table = false;
+    __device__ uint32_t slack() const { return 0u; }
     __device__ uint2 at(int) const { return make_uint2(0u, 0u); }
 };
 
@@ -366,7 +373,8 @@ struct PotNone {
 // and the rounding error (far below 1) cannot push a floor difference past
 // an integer weight.
 struct PotEuclid {
-    static constexpr bool on = true;
+    static constexpr bool on = true, table = false;
+    __device__ uint32_t slack() const { return 0u; }
     const int32_t *xy;
     int2 s, t;
     double rho;  // rho_fp / 65536
@@ -384,7 +392,8 @@ struct PotEuclid {
 // wmin x Manhattan distance: consistent on grids whose arcs join
 // 4-neighbours (length 1) with weights >= wmin.
 struct PotManhattan {
-    static constexpr bool on = true;
+    static constexpr bool on = true, table = false;
+    __device__ uint32_t slack() const { return 0u; }
     const int32_t *xy;
     int2 s, t;
     uint32_t wmin;
@@ -396,6 +405,100 @@ struct PotManhattan {
         const int2 q = __ldg(reinterpret_cast<const int2 *>(xy) + v);
         return make_uint2(d1(q, t), d1(q, s));
     }
+};
+
+// Landmark bounds (HeurALT) to t and from s, from one read of v's row.  With
+// table entries floor(d / sc) each bound lies at most 2 (sc - 1) below the
+// exact landmark bound, which is consistent, and never above it: a key
+// exceeds its consistent one by at most the error of the bound it subtracts.
+// A bound of INF_G says that the pair is not connected.
+//
+// What an evaluation costs is its instructions.  With 8-bit entries the bytes
+// of a row are spread into 16-bit halves and each difference is one
+// add-and-maximum per pair (256 + a - b, floored at 256); the rows of t and s
+// are prepared in shared memory in the form that the sums want (query_row).
+// The unreachable marker 255 needs no test: as the subtracted entry it gives
+// a negative difference, and as the one subtracted from it says that there is
+// no path, for which every bound holds.  The per-byte compare, subtract and
+// maximum intrinsics, which the hardware does not have, took 2,000
+// instructions per evaluation of 64 landmarks instead of 300.
+struct PotALT {
+    static constexpr bool on = true, table = true;
+    HeurALT alt;  // alt.t: the target
+    int32_t s;
+    const uint4 *cf, *cb;  // 8-bit entries: the query's words (query_row)
+    __device__ uint32_t slack() const { return 2u * (uint32_t)(alt.s - 1); }
+    static constexpr uint32_t C256 = 0x01000100u;
+    static __device__ __forceinline__ uint32_t lo16(uint32_t x) { return __byte_perm(x, 0u, 0x4140); }  // bytes 0, 1
+    static __device__ __forceinline__ uint32_t hi16(uint32_t x) { return __byte_perm(x, 0u, 0x4342); }  // bytes 2, 3
+    // Fills words (two per four landmarks: forward, then backward half):
+    // {t, 256 - s} forward, {256 - t, s} backward.  All threads of a CTA.
+    static __device__ void query_row(const HeurALT &alt, int32_t s, uint4 *words) {
+        const int n4 = alt.L / 4;  // 4-byte words per half row
+        const uint32_t *rt = reinterpret_cast<const uint32_t *>(alt.tab) + (size_t)alt.t * (2 * n4);
+        const uint32_t *rs = reinterpret_cast<const uint32_t *>(alt.tab) + (size_t)s * (2 * n4);
+        for (int i = threadIdx.x; i < 2 * n4; i += blockDim.x) {
+            const uint32_t t = __ldg(rt + i), x = __ldg(rs + i);
+            const uint32_t neg = i < n4 ? x : t, pos = i < n4 ? t : x;
+            words[i] = make_uint4(lo16(pos), hi16(pos), C256 - lo16(neg), C256 - hi16(neg));
+        }
+    }
+    // four landmarks: f, b the row's forward and backward bytes
+    __device__ __forceinline__ void word8(uint32_t f, uint32_t b, int i, uint32_t &mt, uint32_t &ms) const {
+        const uint4 kf = cf[i], kb = cb[i];
+        const uint32_t f0 = lo16(f), f1 = hi16(f), b0 = lo16(b), b1 = hi16(b);
+        mt = __viaddmax_s16x2(kf.x, C256 - f0, mt);  // d(L, t) - d(L, v)
+        mt = __viaddmax_s16x2(kf.y, C256 - f1, mt);
+        ms = __viaddmax_s16x2(f0, kf.z, ms);         // d(L, v) - d(L, s)
+        ms = __viaddmax_s16x2(f1, kf.w, ms);
+        mt = __viaddmax_s16x2(b0, kb.z, mt);         // d(v, L) - d(t, L)
+        mt = __viaddmax_s16x2(b1, kb.w, mt);
+        ms = __viaddmax_s16x2(kb.x, C256 - b0, ms);  // d(s, L) - d(v, L)
+        ms = __viaddmax_s16x2(kb.y, C256 - b1, ms);
+    }
+    __device__ __forceinline__ uint32_t bound8(uint32_t m) const {
+        const uint32_t d = max(m & 0xFFFFu, m >> 16) - 256u;
+        return d ? d * (uint32_t)alt.s - (uint32_t)(alt.s - 1) : 0u;
+    }
+    __device__ __forceinline__ uint2 eval8(int32_t v) const {
+        const int n8 = alt.L / 8;  // 8-byte words per half row
+        const uint2 *rv = alt.tab + (size_t)v * (2 * n8);
+        uint32_t mt = C256, ms = C256;
+        if ((n8 & 1) == 0) {
+            const uint4 *qv = reinterpret_cast<const uint4 *>(rv);
+#pragma unroll 2
+            for (int i = 0; i < n8 / 2; i++) {
+                const uint4 f = __ldg(qv + i), b = __ldg(qv + n8 / 2 + i);
+                word8(f.x, b.x, 4 * i, mt, ms);
+                word8(f.y, b.y, 4 * i + 1, mt, ms);
+                word8(f.z, b.z, 4 * i + 2, mt, ms);
+                word8(f.w, b.w, 4 * i + 3, mt, ms);
+            }
+        } else {
+            for (int i = 0; i < n8; i++) {
+                const uint2 f = __ldg(rv + i), b = __ldg(rv + n8 + i);
+                word8(f.x, b.x, 2 * i, mt, ms);
+                word8(f.y, b.y, 2 * i + 1, mt, ms);
+            }
+        }
+        return make_uint2(bound8(mt), bound8(ms));
+    }
+    __device__ __forceinline__ uint2 eval16(int32_t v) const {
+        const int W = alt.L / 4;  // 8-byte words per half row
+        const uint2 *rv = alt.tab + (size_t)v * (2 * W);
+        const uint2 *rt = alt.tab + (size_t)alt.t * (2 * W), *rs = alt.tab + (size_t)s * (2 * W);
+        uint32_t mt = 0, ct = 0, ms = 0, cs = 0;
+#pragma unroll 2
+        for (int i = 0; i < W; i++) {
+            const uint2 f = __ldg(rv + i), b = __ldg(rv + W + i);
+            alt.terms<16>(__ldg(rt + i), f, mt, ct);
+            alt.terms<16>(b, __ldg(rt + W + i), mt, ct);
+            alt.terms<16>(f, __ldg(rs + i), ms, cs);
+            alt.terms<16>(__ldg(rs + W + i), b, ms, cs);
+        }
+        return make_uint2(ct ? INF_G : alt.top<16>(mt), cs ? INF_G : alt.top<16>(ms));
+    }
+    __device__ uint2 at(int v) const { return alt.bits == 8 ? eval8(v) : eval16(v); }
 };
 
 // Bucket key of label g in direction dir, with pot = {pt(v), ps(v)}.
@@ -443,7 +546,8 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
     const int lane = lane_id();
     // arcs per lane whose loads are in flight together
     constexpr int AU = Pot::on ? 1 : LAZY ? 4 : 2;
-    constexpr uint32_t ahead = LAZY ? WAVE_AHEAD : WAVE_AHEAD_XY;
+    // (eager labels without potentials: coordinates, or a flooding search)
+    const uint32_t ahead = G.xy || (!LAZY && !Pot::on) ? WAVE_AHEAD_XY : WAVE_AHEAD;
     // the slot's far memory: 2 x 32 lists (at most a quarter), two halves of a
     // pile, two spill areas for waves that outgrow shared memory (a sixteenth
     // each)
@@ -536,9 +640,10 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
 
     // the length in mu (its high word: one 32-bit read)
     auto mu_now = [&]() -> uint32_t { return reinterpret_cast<volatile uint32_t *>(&q->mu)[1]; };
+    const uint32_t slack2 = 2u * pot.slack();
     // the bound that a key must stay below, given the other side's lb
     auto key_limit = [&](uint32_t mu, uint32_t lbo) -> uint32_t {
-        const uint64_t kb = bi_key_bound<Pot>(mu);
+        const uint64_t kb = bi_key_bound<Pot>(mu) + slack2;
         return kb <= lbo ? 0u : (uint32_t)min(kb - lbo, (uint64_t)NONE);
     };
     uint32_t lim0 = 0, lim1 = 0, lo0 = 0, lo1 = 0;  // the wave's plan
@@ -575,6 +680,32 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
         const E e = WE::make(vd, key, x);
         if (key >= (dir ? lim1 : lim0)) to_lists(e, key, dir, bucket(key), &q->pile_n, pile0 + (flip ? pcap : 0));
         else if (!to_near(e, key, dir, wv + 1)) atomicOr(&q->status, ST_OVERFLOW);
+    };
+    // eager labels: installs label ng of v (seen with unit c) reached from u
+    // and pushes its entry
+    auto install = [&](uint32_t dir, int u, int v, uint32_t ng, uint2 pv, typename Rec::U c, uint32_t lbo) {
+        const uint32_t nk = bi_key<Pot>(ng, dir, pv);
+        if (ng >= Rec::g(c, ep) || nk >= key_limit(mu_now(), lbo)) return;
+        const typename Rec::U nv = Rec::make(ep, ng, (uint32_t)u, dir ? 0u : R.keyw(v));
+        typename Rec::U *rv = R.claim(v, ep);
+        for (;;) {
+            const typename Rec::U got = Rec::cas(rv + dir, c, nv);
+            if (Rec::eq(got, c)) break;
+            c = got;
+            if (ng >= Rec::g(c, ep)) return;
+        }
+        n_rel++;
+        if (Rec::g(c, ep) >= INF_G) {
+            if constexpr (Rec::logs) {
+                // first touches of either direction (a node may be logged
+                // twice; the reset takes it twice)
+                const int p = atomicAdd(&q->touched, 1);
+                if ((int64_t)p < 2 * (int64_t)G.n) B.touched[p] = v;
+            } else {
+                n_first++;
+            }
+        }
+        push((uint32_t)v | (dir << 31), nk, ng);
     };
     // expands one entry with a team of 2^tsh lanes
     auto expand = [&](const E en, const int tsh) {
@@ -684,7 +815,7 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
                     ur[k] = typename Rec::U{};
                     if (live[k]) {
                         Rec::ld2(R.find((int)a[k].x, ep), uf[k], ur[k]);
-                        if constexpr (Pot::on) pv[k] = pot.at((int)a[k].x);
+                        if constexpr (Pot::on && !Pot::table) pv[k] = pot.at((int)a[k].x);
                     }
                 }
 #pragma unroll
@@ -692,36 +823,17 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
                     const int v = (int)a[k].x;
                     const uint32_t ng = gu + a[k].y;
                     // a path through v is at least g + the bound of the other side
-                    if (!live[k] || (Pot::on && (uint64_t)ng + (dir ? pv[k].y : pv[k].x) >= (uint64_t)mu)) continue;
+                    if (!live[k] || (Pot::on && !Pot::table && (uint64_t)ng + (dir ? pv[k].y : pv[k].x) >= (uint64_t)mu))
+                        continue;
                     const uint64_t mc = (uint64_t)ng + Rec::g(dir ? uf[k] : ur[k], ep);
                     if (mc < mu) atomicMin(&q->mu, (mc << 32) | (dir ? (uint32_t)v : (uint32_t)u));
-                    const uint32_t nk = bi_key<Pot>(ng, dir, pv[k]);
-                    typename Rec::U c = dir ? ur[k] : uf[k];
-                    if (ng >= Rec::g(c, ep) || nk >= key_limit(mu_now(), lbo)) continue;
-                    const typename Rec::U nv = Rec::make(ep, ng, (uint32_t)u, dir ? 0u : R.keyw(v));
-                    typename Rec::U *rv = R.claim(v, ep);
-                    bool inst = false;
-                    do {
-                        const typename Rec::U got = Rec::cas(rv + dir, c, nv);
-                        if (Rec::eq(got, c)) {
-                            inst = true;
-                            break;
-                        }
-                        c = got;
-                    } while (ng < Rec::g(c, ep));
-                    if (!inst) continue;
-                    n_rel++;
-                    if (Rec::g(c, ep) >= INF_G) {
-                        if constexpr (Rec::logs) {
-                            // first touches of either direction (a node may be
-                            // logged twice; the reset takes it twice)
-                            const int p = atomicAdd(&q->touched, 1);
-                            if ((int64_t)p < 2 * (int64_t)G.n) B.touched[p] = v;
-                        } else {
-                            n_first++;
-                        }
+                    if constexpr (Pot::table) {
+                        if (ng >= Rec::g(dir ? ur[k] : uf[k], ep)) continue;
+                        pv[k] = pot.at(v);
+                        const uint32_t hb = dir ? pv[k].y : pv[k].x;
+                        if (hb >= INF_G || (uint64_t)ng + hb >= (uint64_t)mu) continue;
                     }
-                    push((uint32_t)v | (dir << 31), nk, ng);
+                    install(dir, u, v, ng, pv[k], dir ? ur[k] : uf[k], lbo);
                 }
             }
             j += AU * tw;
@@ -757,7 +869,7 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
             p.lb[1] = min(min(k1, pm1), e1);
             // an empty direction, or nothing open that could be shorter: mu is the distance
             if (p.lb[0] == NONE || p.lb[1] == NONE ||
-                (uint64_t)p.lb[0] + p.lb[1] >= bi_key_bound<Pot>(mu_now()) || q->status) {
+                (uint64_t)p.lb[0] + p.lb[1] >= bi_key_bound<Pot>(mu_now()) + slack2 || q->status) {
                 p.act = 1;
             } else if (p.m >= WAVE_FILL) {
                 // enough to do

@@ -415,9 +415,8 @@ int launch(ddp_server *s) {
     A.path_cap = s->path_cap;
     A.work = s->d_work;
     A.status = s->d_work + 1;
-    A.delta = s->o.delta > 0                ? (uint32_t)s->o.delta
-              : bidir_hk(s->hk)         ? auto_delta_bidir(s->g)
-                                        : auto_delta(s->g);
+    if (bidir_hk(s->hk)) bidir_args(s->g, s->o.delta, &A);
+    else A.delta = s->o.delta > 0 ? (uint32_t)s->o.delta : auto_delta(s->g);
     A.K = s->o.K;
     A.bfs_budget = s->hkind == DDP_H_BFS_CAPPED ? bfs_budget(s->g->n) : 0;
     A.group = 1;

@@ -5,6 +5,7 @@
 // iteration) with one cooperative kernel per query (single form) or one
 // persistent kernel per batch (batched form).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <string>
@@ -490,28 +491,39 @@ __device__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B
             if constexpr (std::is_same<Grp, CtaGroup>::value) {
                 const uint32_t ep = *(volatile uint32_t *)&ctl->tag;
                 if constexpr (HK == 5) {
+                    P.budget = A.lazy_budget;
                     r = run_bidir_cta<true>(G, B, P, ep, bq, PotNone{}, RecDense{{}, B.state});
-                    if (*(volatile int *)&ctl->status & ST_OVERFLOW) {
-                        // lazy labels keep up to one open entry per arc: a
-                        // search that floods the graph (the target lies in
-                        // another component, say) starts again with labels
-                        // installed at once, which keeps about one per node
+                    if (*(volatile int *)&ctl->status & (ST_OVERFLOW | ST_BUDGET)) {
+                        // a search that floods its graph (bidir_args), or that
+                        // outgrew the lazy form's memory of up to one open
+                        // entry per arc: start again with labels installed at
+                        // once (about one open entry per node)
                         grp.sync();
                         if (grp.rank() == 0) {
                             const uint32_t e2 = *epoch + 1;
-                            if (e2 != 0) {  // else leave the overflow standing
+                            ctl->status = ST_OVERFLOW;
+                            if (e2 != 0) {  // else (the epochs wrapped) the caller runs it elsewhere
                                 *epoch = e2;
                                 ctl->tag = e2;
                                 ctl->status = 0;
                             }
                         }
                         grp.sync();
+                        P.budget = 0;
+                        P.delta = A.eager_delta;
                         if (*(volatile int *)&ctl->status == 0)
                             r = run_bidir_eager(G, B, P, *(volatile uint32_t *)&ctl->tag, bq);
                     }
                 } else if constexpr (HK == 8) {
                     const RecHash R{{}, B.state, (1u << B.hbits) - 1u, 32 - B.hbits};
                     r = run_bidir_cta<true>(G, B, P, ep, bq, PotNone{}, R);
+                } else if constexpr (HK == 10) {
+                    __shared__ uint4 words[2 * 32];  // up to 128 landmarks of 8 bits
+                    const HeurALT alt{G.lm, G.lm_L, G.lm_scale, t, G.lm_bits};
+                    if (alt.bits == 8) PotALT::query_row(alt, s, words);
+                    grp.sync();
+                    r = run_bidir_cta<false>(G, B, P, ep, bq, PotALT{alt, s, words, words + alt.L / 4},
+                                             RecDense{{}, B.state});
                 } else if constexpr (HK == 9) {
                     r = run_bidir_cta<false>(G, B, P, ep, bq, PotNone{}, RecPair16{B.state});
                 } else {
@@ -830,6 +842,7 @@ static int rerun_kind(int hkind) { return is_bidir_kind(hkind) ? DDP_H_ZERO : hk
 // 2048^2 maze they were faster, 16.4 against 17.8 ms).
 int kernel_hk(int hkind, bool has_xy, bool hash, int group, int flags) {
     if (!is_bidir_kind(hkind) && batch_bidir(hkind, group, flags)) {
+        if (hkind == DDP_H_LANDMARK) return 10;
         hkind = DDP_H_BIDIR;
         hash = false;
     }
@@ -852,7 +865,8 @@ int hk_slot_kind(int hk) {
     case 1: return SLOT_HOPS;
     case 5:
     case 6:
-    case 7: return SLOT_PAIR;
+    case 7:
+    case 10: return SLOT_PAIR;
     case 8: return SLOT_PAIR | SLOT_HASH;
     case 9: return SLOT_PAIR16;
     default: return 0;
@@ -861,18 +875,19 @@ int hk_slot_kind(int hk) {
 
 // The kernel of an instance; grouped: slots of several CTAs, or one-CTA slots
 // on the phase-synchronous engine (bidirectional kinds have neither, and no
-// bound or hop bounds have nothing else: batch_bidir).
+// bound, hop bounds and landmarks nothing else: batch_bidir).
 static const void *batch_kernel_hk(int hk, bool grouped) {
     switch (hk) {
     case 1: return (const void *)k_batch_group<1>;
     case 2: return grouped ? (const void *)k_batch_group<2> : (const void *)k_batch<2>;
     case 3: return grouped ? (const void *)k_batch_group<3> : (const void *)k_batch<3>;
-    case 4: return grouped ? (const void *)k_batch_group<4> : (const void *)k_batch<4>;
+    case 4: return (const void *)k_batch_group<4>;
     case 5: return (const void *)k_batch<5>;
     case 6: return (const void *)k_batch<6>;
     case 7: return (const void *)k_batch<7>;
     case 8: return (const void *)k_batch<8>;
     case 9: return (const void *)k_batch<9>;
+    case 10: return (const void *)k_batch<10>;
     default: return (const void *)k_batch_group<0>;
     }
 }
@@ -919,6 +934,19 @@ int device_sms() { return sm_count(); }
 uint32_t auto_delta_bidir(const ddp_graph *g) {
     const uint32_t d = (g->wmin + g->wmax) / (g->d_xy ? 4 : 12);
     return d < 1 ? 1 : d;
+}
+
+void bidir_args(const ddp_graph *g, int32_t delta, BatchArgs *A) {
+    A->delta = delta > 0 ? (uint32_t)delta : auto_delta_bidir(g);
+    // A search without coordinates that takes far more entries than a random
+    // digraph's (about 3 sqrt(n); up to 20 sqrt(n) seen in 100,000 queries of
+    // 4M nodes) runs on a graph of another kind, planar ones for example:
+    // labels installed at once and wide buckets suit it better (100 queries on
+    // 200,000 planar points without coordinates: 14.2 ms lazily, 8.2 ms with
+    // the second start).  Too low a budget starts long random searches again
+    // (8 sqrt(n): 4.7 ms for the 4M-node batch that takes 3.7).
+    A->lazy_budget = 4096 + (int64_t)(24.0 * std::sqrt((double)g->n));
+    A->eager_delta = delta > 0 ? (uint32_t)delta : auto_delta(g);
 }
 
 uint32_t auto_delta(const ddp_graph *g) {
@@ -1594,9 +1622,8 @@ static bool batch_args(ddp_batch *b, int32_t n, const int32_t *dS, const int32_t
     A.tend = b->d_t1;
     A.work = b->d_work;
     A.status = b->d_status;
-    A.delta = b->o.delta > 0                ? (uint32_t)b->o.delta
-              : bidir_hk(b->hk)         ? auto_delta_bidir(b->g)
-                                        : auto_delta(b->g);
+    if (bidir_hk(b->hk)) bidir_args(b->g, b->o.delta, &A);
+    else A.delta = b->o.delta > 0 ? (uint32_t)b->o.delta : auto_delta(b->g);
     A.bfs_budget = b->hkind == DDP_H_BFS_CAPPED ? bfs_budget(b->g->n) : 0;
     A.K = b->o.K;
     A.group = b->group;
@@ -1646,7 +1673,8 @@ static bool same_args(const BatchArgs &x, const BatchArgs &y) {
     return x.S == y.S && x.T == y.T && x.nq == y.nq && x.cost == y.cost && x.plen == y.plen &&
            x.paths == y.paths && x.path_cap == y.path_cap && x.qstatus == y.qstatus && x.stats == y.stats &&
            x.tstart == y.tstart && x.tend == y.tend && x.work == y.work && x.status == y.status &&
-           x.delta == y.delta && x.K == y.K && x.bfs_budget == y.bfs_budget && x.group == y.group &&
+           x.delta == y.delta && x.K == y.K && x.bfs_budget == y.bfs_budget && x.lazy_budget == y.lazy_budget &&
+           x.eager_delta == y.eager_delta && x.group == y.group &&
            x.sync_engine == y.sync_engine;
 }
 

@@ -58,6 +58,8 @@ struct BatchArgs {
     uint32_t delta;
     int32_t K;
     int64_t bfs_budget;  // capped heuristic BFS (0 = run to completion)
+    int64_t lazy_budget;   // entries a search may expand before it starts again with eager labels
+    uint32_t eager_delta;  // bucket width of that second start
     int group;           // CTAs per query slot
     int sync_engine;     // 1: phase-synchronous engine even for one-CTA slots
     // serving mode (continuous batching): requests are published in host
@@ -86,20 +88,21 @@ inline bool is_bidir_kind(int k) {
     return k == DDP_H_BIDIR || k == DDP_H_BIDIR_EUCLID || k == DDP_H_BIDIR_MANHATTAN;
 }
 // 8: DDP_H_BIDIR with hashed records (DDP_OPT_HASH); 9: DDP_H_BIDIR with
-// 16-byte pairs (graphs with coordinates)
-constexpr bool bidir_hk(int hk) { return hk >= 5 && hk <= 9; }
+// 16-byte pairs (graphs with coordinates); 10: landmark potentials
+constexpr bool bidir_hk(int hk) { return hk >= 5 && hk <= 10; }
 constexpr bool pair16_hk(int hk) { return hk == 9; }
 // Whether slots of `group` CTAs answer a batch kind by the bidirectional
-// search: the bidirectional kinds always; one-CTA slots also for no bound and
-// for hop bounds.  These are admissible on every graph, so the costs are the
-// same, and a one-directional search under so weak a bound expands orders of
-// magnitude more (300 queries, 100,000 nodes, hop bound: a reverse BFS of the
-// whole graph and 45k expansions per query, 9.86 ms; bidirectional: 0.8k
-// expansions, no BFS).  Wider slots and DDP_OPT_SYNC keep the A* engine.
+// search: the bidirectional kinds always; one-CTA slots also for no bound,
+// hop bounds (without them: a one-directional search under so weak a bound
+// expands orders of magnitude more; 300 queries, 100,000 nodes: a reverse BFS
+// of the whole graph and 45k expansions per query, 9.86 ms, against 0.8k
+// expansions, 0.20 ms) and landmarks (as average potentials).  These bounds
+// are admissible on every graph, so the costs are the same.  Wider slots and
+// DDP_OPT_SYNC keep the A* engine.
 inline bool batch_bidir(int hkind, int group, int flags) {
     if (is_bidir_kind(hkind)) return true;
     return group <= 1 && !(flags & DDP_OPT_SYNC) &&
-           (hkind == DDP_H_ZERO || hkind == DDP_H_BFS_HOPS || hkind == DDP_H_BFS_CAPPED);
+           (hkind == DDP_H_ZERO || hkind == DDP_H_BFS_HOPS || hkind == DDP_H_BFS_CAPPED || hkind == DDP_H_LANDMARK);
 }
 // Far memory (8-byte units per half, slot_bytes) of a bidirectional slot: the
 // bucket lists want 4 MB however small the graph or the caller's capacity.
@@ -127,6 +130,8 @@ int slots_per_sm(int hk, int block, bool grouped);
 int device_sms();
 uint32_t auto_delta(const ddp_graph *g);
 uint32_t auto_delta_bidir(const ddp_graph *g);
+// Fills the bucket widths and the budget of a bidirectional launch.
+void bidir_args(const ddp_graph *g, int32_t delta, BatchArgs *A);
 int64_t bfs_budget(int32_t n);
 
 }  // namespace ddp

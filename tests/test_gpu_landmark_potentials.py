@@ -1,0 +1,53 @@
+"""Landmark batches search bidirectionally with the landmark bounds as average
+potentials: costs against the oracle and the A* engine, for every row width
+(whole and odd numbers of 16-byte words), scaled and unscaled tables, nodes
+that landmarks do not relate, and endpoints that are not connected."""
+import os
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+INF = 2147483647
+
+
+def _want(O, g, S, T):
+    gs = g.with_sentinel()
+    cost, _, _, done = O.astar_many(gs.n, gs.off[:-1], gs.col, gs.w, S, T, hkind=0, mode=O.HEAP_POSMAP,
+                                    threads=os.cpu_count() or 1, budget_s=1e9)
+    assert done == len(S)
+    return cost
+
+
+@pytest.mark.parametrize("bits,counts", [(8, (8, 16, 24, 64, 128)), (16, (4, 8, 12, 64))])
+@pytest.mark.parametrize("kind", ["unit", "scaled", "split", "geo"])
+def test_costs_for_every_row_width(gpu, oracle, bits, counts, kind):
+    d = gpu
+    rng = np.random.default_rng(bits)
+    if kind == "split":  # no chain: landmarks miss nodes, pairs are disconnected
+        n, e = 2000, 5000
+        u = np.sort(rng.integers(0, n, e))
+        off = np.concatenate([[0], np.cumsum(np.bincount(u, minlength=n))]).astype(np.int32)
+        g = d.CSR(n, off, rng.integers(0, n, e).astype(np.int32), rng.integers(0, 90, e).astype(np.uint32))
+    elif kind == "geo":
+        g = d.gen_geometric(3000, 5, 1 << 16, 1000, 3)
+    else:
+        g = d.gen_random_chain(2500, 4, 1, 3 if kind == "unit" else 60000, 5)
+    dg = d.DeviceGraph.from_csr(g)
+    S, T = rng.integers(0, g.n, 150).astype(np.int32), rng.integers(0, g.n, 150).astype(np.int32)
+    T[:3] = S[:3]
+    want = _want(oracle, g, S, T)
+    for count in counts:
+        dg.build_landmarks(count, seed=count, bits=bits)
+        for kw in ({}, {"block": 64, "grid": 4}, {"group": 2}, {"delta": 1}, {"flags": d.OPT_SYNC}):
+            be = d.BatchEngine(dg, d.H_LANDMARK, **kw)
+            cost, plen = be.solve(S, T)
+            assert np.array_equal(cost, want), (count, kw, np.flatnonzero(cost != want)[:5])
+            for i in range(0, len(S), 7):
+                p = be.path(i)
+                assert len(p) == plen[i]
+                if want[i] != INF:
+                    ok, why = oracle.check_path(g.off, g.col, g.w, p, int(S[i]), int(T[i]), int(cost[i]))
+                    assert ok, why
+            be.close()
+    dg.close()
