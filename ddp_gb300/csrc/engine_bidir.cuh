@@ -537,7 +537,7 @@ struct WaveEntry<false> {
 // ep: the slot's epoch for this query (never 0; units of other epochs read
 // as unreached).
 template <bool LAZY, class Pot, class Rec>
-__device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, const SearchParams &P, uint32_t ep,
+__device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, const SearchParams &P, uint32_t ep,
                                       WaveQ *q, const Pot &pot, const Rec &R) {
     static_assert(!(LAZY && Pot::on), "lazy labels are keyed by g");
     using WE = WaveEntry<LAZY || Pot::on>;
@@ -545,7 +545,8 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
     SearchCtl *ctl = B.ctl;
     const int lane = lane_id();
     // arcs per lane whose loads are in flight together
-    constexpr int AU = Pot::on ? 1 : LAZY ? 4 : 2;
+    // (two 32-byte records per lane would not fit the registers)
+    constexpr int AU = LAZY ? 4 : Pot::on || !Rec::logs ? 1 : 2;
     // (eager labels without potentials: coordinates, or a flooding search)
     const uint32_t ahead = G.xy || (!LAZY && !Pot::on) ? WAVE_AHEAD_XY : WAVE_AHEAD;
     // the slot's far memory: 2 x 32 lists (at most a quarter), two halves of a
@@ -842,6 +843,112 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
         }
     };
 
+    // Eager labels without potentials: the warp's entries together, one per
+    // team (have: this lane's team has one).  Most relaxations fail, so the
+    // teams' walks diverge: apart, 14 of 32 lanes were active and the compiler
+    // could make it a fifth worse (200 pairs on 1M points: 30.8 or 37.4 ms);
+    // stage by stage, with a step's compare-and-swaps in flight together, 26.9
+    // ms.  Lazy labels and potentials lose by it (4M nodes: 3.68 -> 4.09 ms,
+    // maze 18.6 -> 19.9 ms): their stages are short or rare.
+    auto expand_warp = [&](const bool have, const E en, const int tsh) {
+        const int tw = 1 << tsh, sub = lane & (tw - 1);
+        const uint32_t dir = en.x >> 31, gu = WE::extra(en);
+        const int u = (int)(en.x & NODE_MASK);
+        const uint32_t lbo = dir ? lb0 : lb1;
+        const uint2 *arcs = dir ? G.rarc : G.arc;
+        int r0 = 0, r1 = 0;
+        uint32_t gl = 0;
+        if (have) {
+            // row bounds load beside the record
+            r0 = dir ? row_begin(G.roff, G.roend, u) : row_begin(G.off, G.oend, u);
+            r1 = dir ? row_end(G.roff, G.roend, u) : row_end(G.off, G.oend, u);
+            gl = Rec::g(Rec::ld(R.find(u, ep) + dir), ep);
+        }
+        uint2 a[AU];
+        auto load_arcs = [&](int j) {
+#pragma unroll
+            for (int k = 0; k < AU; k++)
+                a[k] = j + k * tw < r1 ? (G.oend ? __ldcg(arcs + j + k * tw) : __ldg(arcs + j + k * tw))
+                                       : make_uint2(NONE, 0u);
+        };
+        load_arcs(r0 + sub);
+        // current, and a path through it may still be shorter
+        const bool ok = have && gl == gu && en.y < key_limit(mu_now(), lbo);
+        if (ok && sub == 0) {
+            n_exp++;
+            n_scan += (unsigned long long)(r1 - r0);
+        }
+        for (int j = r0 + sub;; j += AU * tw) {
+            const uint32_t mu = mu_now();
+            const uint32_t top = min(mu, INF_G), room_w = ok && top > gu ? top - gu : 0u;
+            typename Rec::U uf[AU], ur[AU], got[AU];
+            bool live[AU];
+            // every load of the step before any is used
+#pragma unroll
+            for (int k = 0; k < AU; k++) {
+                live[k] = (int)a[k].x >= 0 && a[k].y < room_w;
+                uf[k] = typename Rec::U{};
+                ur[k] = typename Rec::U{};
+                if (live[k]) Rec::ld2(R.find((int)a[k].x, ep), uf[k], ur[k]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < AU; k++) {
+                const uint32_t ng = gu + a[k].y;
+                const uint64_t mc = (uint64_t)ng + Rec::g(dir ? uf[k] : ur[k], ep);
+                if (live[k] && mc < mu) atomicMin(&q->mu, (mc << 32) | (dir ? a[k].x : (uint32_t)u));
+                live[k] = live[k] && ng < Rec::g(dir ? ur[k] : uf[k], ep) && ng < key_limit(mu_now(), lbo);
+            }
+            // the step's compare-and-swaps fly together
+#pragma unroll
+            for (int k = 0; k < AU; k++) {
+                got[k] = typename Rec::U{};
+                if (live[k])
+                    got[k] = Rec::cas(R.claim((int)a[k].x, ep) + dir, dir ? ur[k] : uf[k],
+                                      Rec::make(ep, gu + a[k].y, (uint32_t)u, 0u));
+            }
+#pragma unroll
+            for (int k = 0; k < AU; k++) {
+                const int v = (int)a[k].x;
+                const uint32_t ng = gu + a[k].y;
+                typename Rec::U c = dir ? ur[k] : uf[k];
+                bool inst = live[k] && Rec::eq(got[k], c);
+                bool again = live[k] && !inst;  // another relaxation came first
+                if (again) {
+                    c = got[k];
+                    again = ng < Rec::g(c, ep);
+                }
+                while (__any_sync(FULL, again)) {
+                    if (again) {
+                        const typename Rec::U g2 =
+                            Rec::cas(R.claim(v, ep) + dir, c, Rec::make(ep, ng, (uint32_t)u, 0u));
+                        inst = Rec::eq(g2, c);
+                        if (!inst) c = g2;
+                        again = !inst && ng < Rec::g(c, ep);
+                    }
+                }
+                if (inst) {
+                    n_rel++;
+                    if (Rec::g(c, ep) >= INF_G) {
+                        if constexpr (Rec::logs) {
+                            // first touches of either direction (a node may be
+                            // logged twice; the reset takes it twice)
+                            const int p = atomicAdd(&q->touched, 1);
+                            if ((int64_t)p < 2 * (int64_t)G.n) B.touched[p] = v;
+                        } else {
+                            n_first++;
+                        }
+                    }
+                    push((uint32_t)v | (dir << 31), ng, ng);
+                }
+                __syncwarp();
+            }
+            const bool more = ok && j - sub + AU * tw < r1;
+            if (!__any_sync(FULL, more)) break;
+            load_arcs(more ? j + AU * tw : r1);
+        }
+    };
+
     for (;;) {
         __syncthreads();  // the last wave's pushes are in place
         if (threadIdx.x < 32) {
@@ -987,15 +1094,26 @@ __device__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, cons
         const int tsh = W * 16 <= nt ? 4 : W * 8 <= nt ? 3 : (!LAZY || W * 4 <= nt) ? 2 : 1;
         const int teams = nt >> tsh;
         int i = (int)threadIdx.x >> tsh;
-        if (i < W) {
-            E e = entry(i);
-            for (;;) {
-                const int ni = i + teams;
-                E en = e;
-                if (ni < W) en = entry(ni);  // loads while this one expands
-                expand(e, tsh);
-                if (ni >= W) break;
-                i = ni;
+        const int lead = (int)(threadIdx.x & ~31u) >> tsh;  // the warp's first entry
+        if constexpr (LAZY || Pot::on) {
+            if (i < W) {
+                E e = entry(i);
+                for (;;) {
+                    E en = e;
+                    if (i + teams < W) en = entry(i + teams);  // loads while this one expands
+                    expand(e, tsh);
+                    i += teams;
+                    if (i >= W) break;
+                    e = en;
+                }
+            }
+        } else if (lead < W) {
+            E e{};
+            if (i < W) e = entry(i);
+            for (int b = lead; b < W; b += teams, i += teams) {
+                E en{};
+                if (i + teams < W) en = entry(i + teams);
+                expand_warp(i < W, e, tsh);
                 e = en;
             }
         }
