@@ -113,7 +113,7 @@ struct ddp_server {
     int nver = 0;
     std::vector<VBuf> vb;
     DevGraph *h_vtab = nullptr, *d_vtab = nullptr;
-    int *h_inflight = nullptr, *d_inflight = nullptr;
+    int *d_inflight = nullptr;  // searches per version buffer (device memory: slots count in and out)
     std::deque<Delta> deltas;
     Delta cur;  // being recorded by the scatter hook
     cudaStream_t cstream = nullptr;  // maintenance launches while no slot kernel runs
@@ -123,8 +123,8 @@ struct ddp_server {
     char *h_stage = nullptr, *d_stage = nullptr;
     size_t stage_cap = 0;
     std::vector<void *> stage_old;  // pinned buffers to free when no kernel runs
-    // update timings (ns): apply to master, wait for the buffer, patch it
-    int64_t t_apply = 0, t_wait = 0, t_patch = 0;
+    // update timings (ns): apply to master, patch the buffer (once it is free)
+    int64_t t_apply = 0, t_patch = 0;
 };
 
 namespace {
@@ -160,25 +160,30 @@ int stage_reserve(ddp_server *s, size_t bytes) {
 
 // Runs maintenance subs: on the service CTA of the running slot kernel, or
 // with ordinary launches when none runs.
-int svc_run(ddp_server *s, const SvcSub *subs, int nsub) {
+int svc_run(ddp_server *s, const SvcSub *subs, int nsub, int wait_buf = -1) {
     if (kernel_running(s) && s->sa.nslots >= 2) {
         SvcJob *j = s->h_svc;
         const int id = ++s->svc_seq;
         j->nsub = nsub;
+        j->wait_buf = wait_buf;
         for (int i = 0; i < nsub; i++) j->sub[i] = subs[i];
         __atomic_store_n(&j->seq, id, __ATOMIC_RELEASE);
         const int64_t t0 = now_ns();
-        for (;;) {
+        for (int polls = 0;; polls++) {
             if (__atomic_load_n(&j->done, __ATOMIC_ACQUIRE) == id) return DDP_OK;
-            if (!kernel_running(s)) {
+            // (asking the driver takes longer than a poll)
+            if ((polls & 63) == 63 && !kernel_running(s)) {
                 // the kernel left: it ran the job before leaving, or never took it
                 if (__atomic_load_n(&j->done, __ATOMIC_ACQUIRE) == id) return DDP_OK;
                 __atomic_store_n(&j->done, id, __ATOMIC_RELEASE);  // retire it; run it here
                 break;
             }
-            if (now_ns() - t0 > 30000000000LL)
+            const int64_t waited = now_ns() - t0;
+            if (waited > 30000000000LL)
                 return fail(DDP_ERR_TIMEOUT, "service CTA did not run the graph maintenance job");
-            std::this_thread::sleep_for(std::chrono::microseconds(2));
+            // a job of an ordinary batch takes some 10 us; the shortest sleep
+            // takes 60
+            if (waited > 200000) std::this_thread::sleep_for(std::chrono::microseconds(2));
         }
     }
     cudaError_t e = svc_run_direct(subs, nsub, s->cstream);
@@ -237,14 +242,6 @@ int svc_scatter(void *ctx, int kind, void *dst0, void *dst1, const void *list, c
 int fill_buffer(ddp_server *s, int k, int v) {
     ddp_graph *g = s->g;
     const int64_t t0 = now_ns();
-    // the release store of the previous version and this read of the count
-    // pair with the slots' count-then-re-read (both sides fenced)
-    __atomic_thread_fence(__ATOMIC_SEQ_CST);
-    while (__atomic_load_n(&s->h_inflight[k], __ATOMIC_ACQUIRE) != 0) {
-        if (now_ns() - t0 > 30000000000LL) return fail(DDP_ERR_TIMEOUT, "graph version buffer stayed busy");
-        std::this_thread::sleep_for(std::chrono::microseconds(20));
-    }
-    const int64_t t1 = now_ns();
     VBuf &b = s->vb[(size_t)k];
     const int32_t n = g->n;
     bool full = b.held < 0 || b.arc_cap < g->e || b.rarc_cap < g->e_rev;
@@ -326,14 +323,17 @@ int fill_buffer(ddp_server *s, int k, int v) {
         subs[ns++] = sub_of(SVC_GATHER_INTS, (long long)rrow.size(), b.roend, g->d_roend, d + o3, nullptr);
         patched = arc.size() + rarc.size() + row.size() + rrow.size();
     }
-    int rc = svc_run(s, subs, ns);
+    // The release store of the previous version and the service CTA's read of
+    // the buffer's count pair with the slots' count-then-re-read (both sides
+    // fenced).  With no kernel running no search holds a buffer.
+    __atomic_thread_fence(__ATOMIC_SEQ_CST);
+    int rc = svc_run(s, subs, ns, k);
     if (rc) return rc;
     b.held = v;
     const int64_t t2 = now_ns();
-    s->t_wait += t1 - t0;
-    s->t_patch += t2 - t1;
-    trace("serve: version %d in buffer %d: %s (%zu entries), wait %.3f ms, patch %.3f ms", v, k,
-          full ? "full copy" : "patch", patched, (t1 - t0) / 1e6, (t2 - t1) / 1e6);
+    s->t_patch += t2 - t0;
+    trace("serve: version %d in buffer %d: %s (%zu entries), %.3f ms", v, k, full ? "full copy" : "patch", patched,
+          (t2 - t0) / 1e6);
     return DDP_OK;
 }
 
@@ -427,6 +427,8 @@ int launch(ddp_server *s) {
     A.idle_limit = 2000;  // ~2 ms of empty polls
     A.idle_votes = s->d_work + 2;
     A.closing = s->d_work + 3;
+    A.seen = s->d_work + 4;
+    A.tokens = s->d_work + 5;
     // with two or more slots the last CTA is the service CTA
     A.serve_slots = s->sa.nslots >= 2 ? s->sa.nslots - 1 : s->sa.nslots;
     A.svc = s->sa.nslots >= 2 ? s->d_svc : nullptr;
@@ -448,7 +450,9 @@ int launch(ddp_server *s) {
     A.cur_ver = s->d_ctl + 2;
     A.inflight = s->d_inflight;
     DDP_CUDA(cudaMemsetAsync(s->sa.ctl, 0, sizeof(SearchCtl) * (size_t)s->sa.nslots, s->stream));
-    DDP_CUDA(cudaMemsetAsync(s->d_work + 2, 0, sizeof(int) * 2, s->stream));
+    DDP_CUDA(cudaMemsetAsync(s->d_work + 2, 0, sizeof(int) * 4, s->stream));
+    // what was claimed is what the slots have seen: the rest becomes tokens again
+    DDP_CUDA(cudaMemcpyAsync(s->d_work + 4, s->d_work, sizeof(int), cudaMemcpyDeviceToDevice, s->stream));
     cudaError_t e = launch_slots(s->hk, s->sa.nslots, s->block, false, graph_view(s->g), s->sa, A, s->stream);
     if (e != cudaSuccess) return cuda_fail(e, "serving kernel launch");
     s->running = true;
@@ -533,6 +537,7 @@ int ddp_serve_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, int64_t 
     std::memset(s->h_done, 0, sizeof(int) * R);
     std::memset(s->h_ctl, 0, sizeof(int) * 4);
     std::memset(s->h_svc, 0, sizeof(SvcJob));
+    s->h_svc->wait_buf = -1;
     e = cudaHostGetDevicePointer((void **)&s->d_S, s->h_S, 0);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&s->d_T, s->h_T, 0);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&s->d_cost, s->h_cost, 0);
@@ -541,10 +546,10 @@ int ddp_serve_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, int64_t 
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&s->d_ctl, s->h_ctl, 0);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&s->d_svc, s->h_svc, 0);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaHostGetDevicePointer"));
-    e = cudaMalloc(&s->d_work, sizeof(int) * 4);  // claim counter, status, idle votes, closing
+    e = cudaMalloc(&s->d_work, sizeof(int) * 6);  // claim counter, status, idle votes, closing, seen, tokens
     if (e == cudaSuccess) e = cudaMalloc(&s->d_plen, sizeof(int32_t) * R);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(serving state)"));
-    DDP_CUDA(cudaMemsetAsync(s->d_work, 0, sizeof(int) * 4, s->stream));
+    DDP_CUDA(cudaMemsetAsync(s->d_work, 0, sizeof(int) * 6, s->stream));
     DDP_CUDA(cudaStreamSynchronize(s->stream));
     s->t_sub.assign(R, 0);
     s->reported.assign(R, 0);
@@ -555,12 +560,11 @@ int ddp_serve_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, int64_t 
     s->nver = versions;
     s->vb.assign((size_t)versions, VBuf());
     e = cudaHostAlloc(&s->h_vtab, sizeof(DevGraph) * (size_t)versions, flags);
-    if (e == cudaSuccess) e = cudaHostAlloc(&s->h_inflight, sizeof(int) * (size_t)versions, flags);
+    if (e == cudaSuccess) e = cudaMalloc(&s->d_inflight, sizeof(int) * (size_t)versions);
+    if (e == cudaSuccess) e = cudaMemset(s->d_inflight, 0, sizeof(int) * (size_t)versions);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&s->d_vtab, s->h_vtab, 0);
-    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&s->d_inflight, s->h_inflight, 0);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaHostAlloc(graph versions)"));
     std::memset((void *)s->h_vtab, 0, sizeof(DevGraph) * (size_t)versions);
-    std::memset(s->h_inflight, 0, sizeof(int) * (size_t)versions);
     {
         std::lock_guard<std::mutex> glk(g->mu);
         if (g->hook.fn) {
@@ -747,7 +751,7 @@ int ddp_serve_free(ddp_server *s) {
         cudaFree(b.rarc);
     }
     cudaFreeHost(s->h_vtab);
-    cudaFreeHost(s->h_inflight);
+    cudaFree(s->d_inflight);
     cudaFreeHost(s->h_stage);
     for (void *p : s->stage_old) cudaFreeHost(p);
     if (s->cstream) cudaStreamDestroy(s->cstream);

@@ -335,16 +335,28 @@ __device__ __noinline__ SearchResult run_bidir_eager(const DevGraph &G, const Sl
     return run_bidir_cta<false>(G, B, P, ep, q, PotNone{}, RecDense{{}, B.state});
 }
 
-template <int HK, bool ASYNC, class Grp>
-__device__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B, const BatchArgs &A,
+// SERVE: requests and graph versions come from host memory (A.serve); without
+// it the graph is the launch's own, whose fields stay in constant memory.
+template <int HK, bool ASYNC, bool SERVE, class Grp>
+__device__ __forceinline__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B, const BatchArgs &A,
                            uint32_t *epoch, WarpRows *wrows, CtaQ *sq, WaveQ *bq) {
     SearchCtl *ctl = B.ctl;
+    // the query as every thread sees it: read once per CTA (a request and its
+    // graph version lie in host memory, where each read costs a microsecond:
+    // with all warps reading them 512 requests took 1.1 ms to drain)
+    constexpr int GW = (int)(sizeof(DevGraph) / 8);
+    static_assert(sizeof(DevGraph) % 8 == 0 && GW <= 32, "DevGraph is copied in 8-byte words by one warp");
+    __shared__ struct {
+        int q, ver;
+        int32_t s, t;
+        unsigned long long g[GW];
+    } sh;
     long long t0 = 0;
     int vbuf = -1;  // versioned serving: graph buffer the current search holds
     for (;;) {
         if (grp.rank() == 0) {
             int q;
-            if (A.serve) {
+            if (SERVE && A.serve) {
                 // claim the next published request.  A slot that finds no
                 // work for idle_limit polls votes to exit and keeps polling
                 // (new work takes its vote back); when every slot has voted,
@@ -356,17 +368,26 @@ __device__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B
                 // periods (slots that never became resident cannot vote)
                 for (int idle = 0, waited = 0;;) {
                     if (*A.pause || *(volatile int *)A.closing) break;
+                    // whoever sees the published count grow adds as many
+                    // tokens; a claim takes a token, then the next index.  (A
+                    // bounded increment by compare-and-swap made a burst's
+                    // claims retry one another, with two reads of host memory
+                    // between tries: 512 requests took 1.1 ms to drain, 0.2 ms
+                    // of it searching.)
                     const int p = *A.pub;
-                    const int c = *(volatile int *)A.work;
-                    if (c < p) {
-                        if (voted) {
-                            atomicSub(A.idle_votes, 1);
-                            voted = false;
-                        }
-                        if (atomicCAS(A.work, c, c + 1) == c) {
-                            q = c;
+                    const int seen = *(volatile int *)A.seen;
+                    if (p > seen) {
+                        __threadfence_system();  // requests were written before pub
+                        const int old = atomicMax(A.seen, p);
+                        if (p > old) atomicAdd(A.tokens, p - old);
+                    }
+                    if (*(volatile int *)A.tokens > 0) {
+                        if (atomicSub(A.tokens, 1) > 0) {
+                            if (voted) atomicSub(A.idle_votes, 1);
+                            q = atomicAdd(A.work, 1);
                             break;
                         }
+                        atomicAdd(A.tokens, 1);
                         continue;
                     }
                     if (idle < A.idle_limit) {
@@ -384,7 +405,7 @@ __device__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B
                 }
                 __threadfence_system();  // requests were written before pub
                 if (q < 0) q = A.nq;     // exit marker
-                if (q < A.nq && A.vtab) {
+                if (SERVE && q < A.nq && A.vtab) {
                     // pin the latest graph version: count this search on its
                     // buffer, then re-read the version.  Buffer v % K is only
                     // rewritten for version v + K, after version v + K - 1 was
@@ -437,28 +458,43 @@ __device__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B
             if (grp.rank() == 0) ctl->tag = 1;
             grp.sync();
         }
-        const int q = *(volatile int *)&ctl->cur_q;
-        if (q >= A.nq) break;
-        const int qver = A.vtab ? *(volatile int *)&ctl->cur_ver : A.version;
-        DevGraph G = G0;
-        if (A.vtab && qver >= 0) {
-            // the table (host memory) is rewritten while the kernel runs
-            static_assert(sizeof(DevGraph) % 8 == 0, "DevGraph is copied in 8-byte words");
-            const volatile unsigned long long *src =
-                reinterpret_cast<const volatile unsigned long long *>(A.vtab + qver % A.nver);
-            unsigned long long *dst = reinterpret_cast<unsigned long long *>(&G);
-            for (int i = 0; i < (int)(sizeof(DevGraph) / 8); i++) dst[i] = src[i];
+        if (threadIdx.x < 32) {
+            const int q = *(volatile int *)&ctl->cur_q;
+            const int lane = threadIdx.x;
+            if (lane == 0) sh.q = q;
+            if (q < A.nq) {
+                const int ver = SERVE && A.vtab ? *(volatile int *)&ctl->cur_ver : A.version;
+                // serving requests and the version table are written while
+                // the kernel runs: read them uncached
+                if (lane == 0) {
+                    sh.ver = ver;
+                    sh.s = SERVE && A.serve ? *(const volatile int32_t *)(A.S + q) : __ldg(A.S + q);
+                }
+                if (lane == 1) sh.t = SERVE && A.serve ? *(const volatile int32_t *)(A.T + q) : __ldg(A.T + q);
+                if (SERVE && A.vtab && ver >= 0 && lane < GW)
+                    sh.g[lane] =
+                        reinterpret_cast<const volatile unsigned long long *>(A.vtab + ver % A.nver)[lane];
+            }
         }
-        // serving requests live in host memory written while the kernel
-        // runs: read them uncached
-        const int32_t s = A.serve ? *(const volatile int32_t *)(A.S + q) : __ldg(A.S + q);
-        const int32_t t = A.serve ? *(const volatile int32_t *)(A.T + q) : __ldg(A.T + q);
+        __syncthreads();
+        const int q = sh.q;
+        if (q >= A.nq) break;
+        const int qver = sh.ver;
+        const int32_t s = sh.s, t = sh.t;
+        std::conditional_t<SERVE, DevGraph, const DevGraph &> G = G0;
+        if constexpr (SERVE) {
+            if (A.vtab && qver >= 0) {
+                unsigned long long *dst = reinterpret_cast<unsigned long long *>(&G);
+#pragma unroll
+                for (int i = 0; i < GW; i++) dst[i] = sh.g[i];
+            }
+        }
         if (qver < 0 || s < 0 || s >= G.n || t < 0 || t >= G.n) {
             if (grp.rank() == 0) {
                 A.cost[q] = qver < 0 ? -1 : DDP_INF;
                 if (A.plen) A.plen[q] = -1;
                 if (A.qstatus) A.qstatus[q] = -1;
-                if (A.serve) {
+                if (SERVE && A.serve) {
                     A.ver[q] = qver;
                     __threadfence_system();
                     A.done[q] = 1;
@@ -578,7 +614,7 @@ __device__ void batch_loop(const Grp &grp, const DevGraph &G0, const SlotBufs &B
                                                            : (int32_t)r.cost;
             if (A.plen) A.plen[q] = len;
             if (A.qstatus) A.qstatus[q] = ctl->status;
-            if (A.serve) {
+            if (SERVE && A.serve) {
                 A.ver[q] = qver;
                 __threadfence_system();
                 A.done[q] = 1;
@@ -727,10 +763,19 @@ __device__ void service_loop(const BatchArgs &A) {
                     job[0] = 1;
                     job[1] = ns;
                     job[2] = seq;
+                    // a version buffer is rewritten once no search runs on it
+                    const int wb = A.svc->wait_buf;
+                    if (wb >= 0) {
+                        __threadfence_system();
+                        uint32_t polls = 0;
+                        while (*(volatile int *)(A.inflight + wb) != 0 && ++polls < (1u << 25)) __nanosleep(500);
+                        if (polls >= (1u << 25)) job[0] = 0;  // leave: the host gives up first
+                        __threadfence_system();
+                    }
                     break;
                 }
                 if (*(volatile int *)A.closing || *A.pause) break;
-                __nanosleep(2000);
+                __nanosleep(300);
             }
         }
         __syncthreads();
@@ -753,21 +798,24 @@ __device__ void service_loop(const BatchArgs &A) {
 // in one kernel share a register budget, and the one that a launch does not
 // use makes the other spill (landmark instance: 736 bytes of spill stores
 // with both engines, 1,706 once the group engine also ran narrow phases).
-template <int HK>
-__global__ void __launch_bounds__(bidir_hk(HK) ? 1024 : 512, bidir_hk(HK) ? 1 : 2) k_batch(DevGraph G, SlotArrays sa, BatchArgs A) {
-    if (A.svc && (int)blockIdx.x == A.serve_slots) {
-        service_loop(A);
-        return;
+template <int HK, bool SERVE>
+__global__ void __launch_bounds__(bidir_hk(HK) ? 1024 : 512, bidir_hk(HK) ? 1 : 2)
+    k_batch(const __grid_constant__ DevGraph G, SlotArrays sa, BatchArgs A) {
+    if constexpr (SERVE) {
+        if (A.svc && (int)blockIdx.x == A.serve_slots) {
+            service_loop(A);
+            return;
+        }
     }
     SlotBufs B = slot_of(sa, blockIdx.x);
     CtaGroup grp{&B.ctl->status};
     if constexpr (bidir_hk(HK)) {
         __shared__ WaveQ bq;
-        batch_loop<HK, true>(grp, G, B, A, sa.epoch + blockIdx.x, nullptr, nullptr, &bq);
+        batch_loop<HK, true, SERVE>(grp, G, B, A, sa.epoch + blockIdx.x, nullptr, nullptr, &bq);
     } else {
         __shared__ WarpRows wrows[MAX_WARPS];
         __shared__ CtaQ sq;
-        batch_loop<HK, true>(grp, G, B, A, sa.epoch + blockIdx.x, wrows, &sq, nullptr);
+        batch_loop<HK, true, SERVE>(grp, G, B, A, sa.epoch + blockIdx.x, wrows, &sq, nullptr);
     }
 }
 
@@ -783,7 +831,7 @@ __global__ void __launch_bounds__(512, 2) k_batch_group(DevGraph G, SlotArrays s
     const int slot = blockIdx.x / A.group;
     SlotBufs B = slot_of(sa, slot);
     SubGridGroup grp{{&B.ctl->bar_count, &B.ctl->bar_gen}, &B.ctl->status, A.group};
-    batch_loop<HK, false>(grp, G, B, A, sa.epoch + slot, wrows, nullptr, nullptr);
+    batch_loop<HK, false, true>(grp, G, B, A, sa.epoch + slot, wrows, nullptr, nullptr);
 }
 
 // Single query on one CTA with the asynchronous engine (narrow searches).
@@ -876,18 +924,31 @@ int hk_slot_kind(int hk) {
 // The kernel of an instance; grouped: slots of several CTAs, or one-CTA slots
 // on the phase-synchronous engine (bidirectional kinds have neither, and no
 // bound, hop bounds and landmarks nothing else: batch_bidir).
-static const void *batch_kernel_hk(int hk, bool grouped) {
+template <bool SERVE>
+static const void *one_cta_kernel(int hk) {
+    switch (hk) {
+    case 2: return (const void *)k_batch<2, SERVE>;
+    case 3: return (const void *)k_batch<3, SERVE>;
+    case 5: return (const void *)k_batch<5, SERVE>;
+    case 6: return (const void *)k_batch<6, SERVE>;
+    case 7: return (const void *)k_batch<7, SERVE>;
+    case 9: return (const void *)k_batch<9, SERVE>;
+    case 10: return (const void *)k_batch<10, SERVE>;
+    default: return nullptr;
+    }
+}
+
+static const void *batch_kernel_hk(int hk, bool grouped, bool serve) {
+    if (hk == 8) return (const void *)k_batch<8, false>;  // batches only
+    if (!grouped || bidir_hk(hk)) {
+        const void *fn = serve ? one_cta_kernel<true>(hk) : one_cta_kernel<false>(hk);
+        if (fn) return fn;
+    }
     switch (hk) {
     case 1: return (const void *)k_batch_group<1>;
-    case 2: return grouped ? (const void *)k_batch_group<2> : (const void *)k_batch<2>;
-    case 3: return grouped ? (const void *)k_batch_group<3> : (const void *)k_batch<3>;
+    case 2: return (const void *)k_batch_group<2>;
+    case 3: return (const void *)k_batch_group<3>;
     case 4: return (const void *)k_batch_group<4>;
-    case 5: return (const void *)k_batch<5>;
-    case 6: return (const void *)k_batch<6>;
-    case 7: return (const void *)k_batch<7>;
-    case 8: return (const void *)k_batch<8>;
-    case 9: return (const void *)k_batch<9>;
-    case 10: return (const void *)k_batch<10>;
     default: return (const void *)k_batch_group<0>;
     }
 }
@@ -911,14 +972,14 @@ cudaError_t svc_run_direct(const SvcSub *subs, int nsub, cudaStream_t st) {
 cudaError_t launch_slots(int hk, int grid, int block, bool coop, DevGraph G, SlotArrays sa, BatchArgs A,
                          cudaStream_t st) {
     void *args[] = {&G, &sa, &A};
-    const void *fn = batch_kernel_hk(hk, A.group > 1 || A.sync_engine);
+    const void *fn = batch_kernel_hk(hk, A.group > 1 || A.sync_engine, true);
     if (coop) return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(block), args, 0, st);
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, st);
 }
 
 int slots_per_sm(int hk, int block, bool grouped) {
     int per_sm = 0;
-    const void *fn = batch_kernel_hk(hk, grouped);
+    const void *fn = batch_kernel_hk(hk, grouped, true);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, 0);
     return per_sm;
 }
@@ -1653,7 +1714,7 @@ static cudaError_t batch_launch_args(ddp_batch *b, DevGraph G, BatchArgs A) {
     }
     SlotArrays sa = b->sa;
     void *args[] = {&G, &sa, &A};
-    const void *fn = batch_kernel_hk(b->hk, A.group > 1 || A.sync_engine);
+    const void *fn = batch_kernel_hk(b->hk, A.group > 1 || A.sync_engine, false);
     if (b->group > 1)
         return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(block), args, 0, b->stream);
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, b->stream);
@@ -1715,7 +1776,7 @@ int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batc
     int per_sm = 0;
     b->group = bidir ? 1 : std::max(1, b->o.group);  // bidirectional slots are one CTA
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, batch_kernel_hk(b->hk, b->group > 1 || (b->o.flags & DDP_OPT_SYNC)),
+        &per_sm, batch_kernel_hk(b->hk, b->group > 1 || (b->o.flags & DDP_OPT_SYNC), false),
         bidir && b->o.block <= 0 ? 256 : b->block, 0);
     const int coresident = std::max(1, per_sm) * sm_count();
     if (b->group > coresident) b->group = coresident;

@@ -40,10 +40,11 @@ struct SvcSub {
     unsigned long long p0, p1, p2, p3;
 };
 constexpr int SVC_MAX_SUB = 8;
-// The host fills nsub and sub[] and publishes seq; the service CTA marks
+// The host fills nsub, sub[] and wait_buf and publishes seq; the service CTA marks
 // taken = seq, runs the subs in order, and marks done = seq.
 struct SvcJob {
     int seq, taken, done, nsub;
+    int wait_buf, pad;  // version buffer that no search may run on first (-1: none)
     SvcSub sub[SVC_MAX_SUB];
 };
 
@@ -68,6 +69,7 @@ struct BatchArgs {
     const volatile int *pub;    // published request count
     const volatile int *pause;  // non-zero: stop claiming, exit
     int idle_limit;             // polls (~1 us each) before a slot votes to exit
+    int *seen, *tokens;         // published count as the slots know it; requests free to claim
     int *idle_votes;            // slots that found no work for idle_limit polls
     int *closing;               // set once every slot voted: all slots exit
     int serve_slots;            // search slots in the launch
@@ -79,7 +81,7 @@ struct BatchArgs {
     const DevGraph *vtab;         // host memory, rewritten while the kernel runs
     int nver;
     const volatile int *cur_ver;  // latest published version (host memory)
-    int *inflight;                // per buffer: searches running on it (host memory)
+    int *inflight;                // per buffer: searches running on it
 };
 
 // The bidirectional batch kinds, and their k_batch instances (5: no
