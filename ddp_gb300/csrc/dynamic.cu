@@ -19,7 +19,7 @@
 //         their row), and only the touched arc slots / row bounds are
 //         scattered to the device.  Rows carry slack and move to the end of
 //         the arc array when full, so there is no per-batch merge.
-//   device, one cooperative kernel:
+//   device, one cooperative kernel (CTA 0 alone while a step is narrow):
 //     A. heuristic repair: an inserted arc can shorten hop distances to the
 //        target; hops are lowered by decrease propagation over the reverse
 //        graph, so h stays admissible and consistent;
@@ -46,12 +46,10 @@
 
 enum { UPD_INS = 1, UPD_TREE = 2, UPD_LIGHTER = 3 };
 
-// Arcs a repair thread loads at once when it walks a row: the loads of a
-// chunk (and then of its heads' words) are in flight together instead of
+// Arcs a re-seeding thread loads at once when it walks a row: the loads of a
+// chunk (and then of its tails' words) are in flight together instead of
 // one dependent pair per arc.
-#ifndef DYN_ROW_UNROLL
-#define DYN_ROW_UNROLL 8
-#endif
+constexpr int DYN_ROW_UNROLL = 8;
 
 // Host mirror of a dynamic graph: rows with explicit [beg, end) and a
 // capacity, forward and reverse.
@@ -445,8 +443,8 @@ struct DynCtl {
     int hops_lowered;
     int relaxed;
     int reseeded;
-    int pad[7];
-    int local_nf, local_odd;  // a walk's hand-back from CTA 0 (dyn_walk)
+    int stage, nf, odd;  // CTA 0's hand-back (RepairAt; odd: its buffers are swapped)
+    int pad[4];
 };
 
 __device__ __forceinline__ SlotBufs slot_of_dyn(const SlotArrays &sa) {
@@ -464,265 +462,323 @@ __device__ __forceinline__ SlotBufs slot_of_dyn(const SlotArrays &sa) {
     return b;
 }
 
-template <class Grp>
-__device__ void dyn_level_end(const Grp &grp, DynCtl *dc, int it, int &nf) {
-    const int PH = (it + 1) & 3, RS = (it + 3) & 3;
-    grp.sync();
-    if (grp.rank() == 0) dc->cnt[RS] = 0;
-    nf = *(volatile int *)&dc->cnt[PH];
-}
-
 __device__ __forceinline__ GridGroup dyn_group(GridGroup *, const SlotBufs &B) {
     return GridGroup{{&B.ctl->bar_count, &B.ctl->bar_gen}, &B.ctl->status};
 }
 __device__ __forceinline__ CtaGroup dyn_group(CtaGroup *, const SlotBufs &B) { return CtaGroup{&B.ctl->status}; }
 
-// Small frontiers in the repair walks (hop lowering, invalidation): a level
-// of at most DYN_LOCAL_MAX nodes gives a few dozen threads work and still
-// costs a grid barrier, so CTA 0 takes the walk's next levels alone (block
-// barriers, a shared counter) while the grid waits once, and hands the walk
-// back when a level outgrows DYN_LOCAL_BAIL.  step(x, out, counter) expands
-// frontier node x, pushing into out at atomicAdd(counter).  On entry the
-// frontier is in fb (nf nodes); returns true when the walk is over, else
-// leaves the remaining frontier in fb with its size in nf for the grid.
-#ifndef DYN_LOCAL_MAX
-#define DYN_LOCAL_MAX 256
-#endif
-#ifndef DYN_LOCAL_BAIL
-#define DYN_LOCAL_BAIL 2048
-#endif
-template <class Grp, class Step>
-__device__ bool dyn_walk_local(const Grp &grp, int &nf, int32_t *&fa, int32_t *&fb, DynCtl *dc, int *lcnt,
-                               Step &step) {
-    if constexpr (!std::is_same<Grp, GridGroup>::value) {
-        return false;  // one CTA: the grid loop already uses block barriers
-    } else {
-        if (nf > DYN_LOCAL_MAX) return false;
-        if (blockIdx.x == 0) {
-            int lnf = nf, odd = 0;
-            int32_t *la = fa, *lb = fb;
-            for (;;) {
-                int32_t *t = la;
-                la = lb;
-                lb = t;
-                odd ^= 1;
-                if (threadIdx.x == 0) *lcnt = 0;
-                __syncthreads();
-                for (int i = threadIdx.x; i < lnf; i += blockDim.x) step(__ldcg(la + i), lb, lcnt);
-                __syncthreads();
-                lnf = *(volatile int *)lcnt;
-                __syncthreads();  // every thread has read the count before the next reset
-                if (lnf == 0 || lnf > DYN_LOCAL_BAIL) break;
-            }
-            if (threadIdx.x == 0) {
-                dc->local_nf = lnf;
-                dc->local_odd = odd;
-            }
-        }
-        grp.sync();  // CTA 0's pushes and hand-back are visible to every CTA
-        nf = *(volatile int *)&dc->local_nf;
-        if (*(volatile int *)&dc->local_odd) {
-            int32_t *t = fa;  // CTA 0 swapped its buffers an odd number of times
-            fa = fb;
-            fb = t;
-        }
-        return nf == 0;
+// ---- repair ------------------------------------------------------------------
+// The steps before the resumed search, in order.  A walk (hop lowering,
+// invalidation) is a breadth-first search of a few levels of a few dozen
+// nodes: on a grid each level costs a barrier on top of its chain of memory
+// trips, so CTA 0 takes the whole repair alone (block barriers, counters in
+// shared memory, the frontier with its row bounds in shared memory too) and
+// the grid waits once.  It hands over what outgrows it: a level of more than
+// DYN_LOCAL_BAIL nodes, or more than DYN_LOCAL_SEED nodes to re-seed.  A
+// team of DYN_TEAM lanes walks one row, two arcs a lane, so that a level is
+// one chain of arc -> node word -> atomic, where a thread walking a row of
+// ten arcs alone ran two such chains and read the row bounds first.
+// 1M nodes, 1000-update batches (median of 100 updates in the call): 334 us
+// with these steps and the resumed search's splits on 76 CTAs (hops 28 us,
+// invalidation 70, re-seeding and relaxing 17, search 100), 154 us here.
+constexpr int DYN_LOCAL_UPD = 2048;   // updates CTA 0 takes alone
+constexpr int DYN_LOCAL_BAIL = 2048;
+constexpr int DYN_LOCAL_SEED = 1024;
+constexpr int DYN_TEAM = 8;
+enum { REP_HOPS, REP_HOPS_WALK, REP_TREE, REP_TREE_WALK, REP_SEED, REP_DONE };
+
+// The next step, and the frontier of a walk: nf nodes in fb.
+struct RepairAt {
+    int stage, nf;
+    int32_t *fa, *fb;
+};
+
+// Runs the repair from `at` on.  SOLO: on one CTA that returns early (at
+// says where) when a step is too wide for it; lists holds two frontiers of
+// LOCAL_CAP entries {node, row begin, row end} and cnt five counters, all in
+// shared memory.
+template <bool SOLO, class Grp>
+__device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B, uint32_t *hops, const DynArgs &A,
+                           DynCtl *dc, int nupd, RepairAt &at, uint4 *lists, int *cnt) {
+    const int rank = grp.rank(), size = grp.size();
+    const int sub = threadIdx.x & (DYN_TEAM - 1), team = rank / DYN_TEAM, teams = size / DYN_TEAM;
+    uint4 *far_buf = (*(volatile int *)&B.ctl->far_sel) ? B.f1 : B.f0;  // f re-derived (keep mode)
+    const int64_t far_base = *(volatile int *)&B.ctl->far_n;
+    int *inv_n = SOLO ? cnt + 3 : &dc->inv_n;
+    int *far_add = SOLO ? cnt + 4 : &dc->far_add;
+    if (SOLO) {
+        if (threadIdx.x < 5) cnt[threadIdx.x] = 0;
+        __syncthreads();
     }
+    int it = 0;
+    // a level pushes into the counter after its own; the one that no thread
+    // reads any more is cleared for the level after
+    int *next = SOLO ? cnt + 1 : dc->cnt + 1;
+    auto level_end = [&] {
+        if (SOLO) {
+            if (threadIdx.x == 0) cnt[(it + 2) % 3] = 0;
+            __syncthreads();
+            it++;
+            at.nf = *(volatile int *)&cnt[it % 3];
+            next = cnt + (it + 1) % 3;
+        } else {
+            grp.sync();
+            if (rank == 0) dc->cnt[(it + 3) & 3] = 0;
+            it++;
+            at.nf = *(volatile int *)&dc->cnt[it & 3];
+            next = dc->cnt + ((it + 1) & 3);
+        }
+    };
+    auto push = [&](int y, int rb, int re) {
+        const int s = atomicAdd(next, 1);
+        if (s < 2 * B.cap_q) at.fb[s] = y;
+        else atomicOr(&B.ctl->status, ST_OVERFLOW);
+        if (SOLO && s < LOCAL_CAP)
+            lists[((it + 1) & 1) * LOCAL_CAP + s] = make_uint4((uint32_t)y, (uint32_t)rb, (uint32_t)re, 0u);
+    };
+    // walks levels until none is left; false: the level is too wide for SOLO
+    auto walk = [&](const int32_t *rbeg, const int32_t *rend, auto expand) -> bool {
+        while (at.nf > 0) {
+            // a push past the buffer raised an overflow: its count is not a frontier
+            if (SOLO ? at.nf > DYN_LOCAL_BAIL
+                     : (*(volatile int *)&B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT)) != 0)
+                return !SOLO;
+            int32_t *t = at.fa;
+            at.fa = at.fb;
+            at.fb = t;
+            for (int i = team; i < at.nf; i += teams) {
+                int x, b, e;
+                if (SOLO && i < LOCAL_CAP) {
+                    const uint4 en = lists[(it & 1) * LOCAL_CAP + i];
+                    x = (int)en.x;
+                    b = (int)en.y;
+                    e = (int)en.z;
+                } else {
+                    x = __ldcg(at.fa + i);
+                    b = row_begin(rbeg, rend, x);
+                    e = row_end(rbeg, rend, x);
+                }
+                expand(x, b, e);
+            }
+            level_end();
+        }
+        return true;
+    };
+
+    // ---- A. heuristic repair: lower hops over inserted arcs ---------------
+    if (at.stage == REP_HOPS) {
+        for (int i = rank; i < nupd; i += size) {
+            const int4 up = A.upd[i];
+            if (up.x != UPD_INS) continue;
+            const uint32_t hv = __ldcg(hops + up.z);
+            const int rb = row_begin(G.roff, G.roend, up.y), re = row_end(G.roff, G.roend, up.y);
+            if (hv == HOPS_INF) continue;
+            if (hv + 1 < atomicMin(hops + up.y, hv + 1)) {
+                push(up.y, rb, re);
+                atomicAdd(&dc->hops_lowered, 1);
+            }
+        }
+        level_end();
+        at.stage = REP_HOPS_WALK;
+    }
+    if (at.stage == REP_HOPS_WALK) {
+        // lowers the hops of u's in-neighbours from u's; each lowering
+        // pushes once
+        auto lower_from = [&](int u, int b, int e) {
+            const uint32_t hu = __ldcg(hops + u);
+            for (int j0 = b + sub; j0 < e; j0 += 2 * DYN_TEAM) {
+                int p[2], rb[2], re[2];
+                uint32_t old[2];
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+                    p[k] = j0 + k * DYN_TEAM < e ? (int)__ldcg(G.rarc + j0 + k * DYN_TEAM).x : -1;
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    rb[k] = re[k] = 0;
+                    old[k] = 0u;
+                    if (p[k] < 0) continue;
+                    if (SOLO) {
+                        // narrow: the atomic at once, row bounds beside it
+                        rb[k] = row_begin(G.roff, G.roend, p[k]);
+                        re[k] = row_end(G.roff, G.roend, p[k]);
+                        old[k] = atomicMin(hops + p[k], hu + 1);
+                    } else {
+                        old[k] = __ldcg(hops + p[k]);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    if (hu + 1 >= old[k]) continue;
+                    if (!SOLO && hu + 1 >= atomicMin(hops + p[k], hu + 1)) continue;
+                    push(p[k], rb[k], re[k]);
+                    atomicAdd(&dc->hops_lowered, 1);
+                }
+            }
+        };
+        if (!walk(G.roff, G.roend, lower_from)) return;
+        at.stage = REP_TREE;
+    }
+    // ---- B. invalidate subtrees hanging off removed / heavier tree arcs ---
+    auto invalidate = [&](int y, uint64_t sy, int rb, int re) {
+        // a parallel arc's second CAS fails: each node is invalidated once
+        if (atomicCAS(B.state + y, sy, ~0ull) != sy) return;
+        push(y, rb, re);
+        A.inv[atomicAdd(inv_n, 1)] = y;
+    };
+    if (at.stage == REP_TREE) {
+        for (int i = rank; i < nupd; i += size) {
+            const int4 up = A.upd[i];
+            if (up.x != UPD_TREE) continue;
+            const uint64_t sv = __ldcg(B.state + up.z);
+            const int rb = row_begin(G.off, G.oend, up.z), re = row_end(G.off, G.oend, up.z);
+            if (st_g(sv) < INF_G && st_parent(sv) == up.y) invalidate(up.z, sv, rb, re);
+        }
+        level_end();
+        at.stage = REP_TREE_WALK;
+    }
+    if (at.stage == REP_TREE_WALK) {
+        // invalidates x's children in the tree (nodes whose parent is x)
+        auto invalidate_from = [&](int x, int b, int e) {
+            for (int j0 = b + sub; j0 < e; j0 += 2 * DYN_TEAM) {
+                int y[2], rb[2], re[2];
+                uint64_t sy[2];
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+                    y[k] = j0 + k * DYN_TEAM < e ? (int)__ldcg(G.arc + j0 + k * DYN_TEAM).x : -1;
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    rb[k] = re[k] = 0;
+                    sy[k] = y[k] >= 0 ? __ldcg(B.state + y[k]) : ~0ull;
+                    if (SOLO && y[k] >= 0) {
+                        rb[k] = row_begin(G.off, G.oend, y[k]);
+                        re[k] = row_end(G.off, G.oend, y[k]);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+                    if (y[k] >= 0 && st_g(sy[k]) < INF_G && st_parent(sy[k]) == x) invalidate(y[k], sy[k], rb[k], re[k]);
+            }
+        };
+        if (!walk(G.off, G.oend, invalidate_from)) return;
+        at.stage = REP_SEED;
+    }
+    // ---- C. re-seed invalidated nodes from valid in-neighbours ------------
+    const int ninv = *(volatile int *)inv_n;
+    if (SOLO && ninv > DYN_LOCAL_SEED) return;
+    uint2 *best = B.q1;  // one {g, parent} per invalidated node
+    for (int i = rank; i < ninv; i += size) {
+        const int x = A.inv[i];
+        uint32_t bg = INF_G;
+        int bp = -1;
+        const int b = row_begin(G.roff, G.roend, x), e = row_end(G.roff, G.roend, x);
+        for (int j0 = b; j0 < e; j0 += DYN_ROW_UNROLL) {
+            uint2 a[DYN_ROW_UNROLL];
+            uint32_t gp[DYN_ROW_UNROLL];
+#pragma unroll
+            for (int k = 0; k < DYN_ROW_UNROLL; k++)
+                a[k] = j0 + k < e ? __ldcg(G.rarc + j0 + k) : make_uint2(0xFFFFFFFFu, 0u);
+#pragma unroll
+            for (int k = 0; k < DYN_ROW_UNROLL; k++)
+                gp[k] = (int)a[k].x >= 0 ? st_g(__ldcg(B.state + (int)a[k].x)) : INF_G;
+#pragma unroll
+            for (int k = 0; k < DYN_ROW_UNROLL; k++) {
+                if (gp[k] >= INF_G) continue;
+                const uint64_t c = (uint64_t)gp[k] + a[k].y;
+                if (c < bg) {
+                    bg = (uint32_t)c;
+                    bp = (int)a[k].x;
+                }
+            }
+        }
+        best[i] = make_uint2(bg, (uint32_t)bp);
+    }
+    grp.sync();
+    for (int i = rank; i < ninv; i += size) {
+        const uint2 bv = best[i];
+        if (bv.x >= INF_G) continue;
+        const int x = A.inv[i];
+        B.state[x] = st_make(bv.x, (int32_t)bv.y);
+        const int s = atomicAdd(far_add, 1);
+        if (far_base + s < B.cap_f) far_buf[far_base + s] = make_uint4((uint32_t)x, bv.x, 0u, 0u);
+        else atomicOr(&B.ctl->status, ST_OVERFLOW);
+        atomicAdd(&dc->reseeded, 1);
+    }
+    grp.sync();
+    // ---- D. relax heads of inserted / lighter arcs ------------------------
+    for (int i = rank; i < nupd; i += size) {
+        const int4 up = A.upd[i];
+        if (up.x != UPD_INS && up.x != UPD_LIGHTER) continue;
+        const uint32_t gu = st_g(__ldcg(B.state + up.y));
+        uint64_t cur = __ldcg(B.state + up.z);
+        if (gu >= INF_G) continue;
+        const uint64_t ng64 = (uint64_t)gu + (uint32_t)up.w;
+        if (ng64 >= INF_G) continue;
+        const uint32_t ng = (uint32_t)ng64;
+        while (ng < st_g(cur)) {
+            const uint64_t got = atomicCAS(B.state + up.z, cur, st_make(ng, up.y));
+            if (got == cur) {
+                const int s = atomicAdd(far_add, 1);
+                if (far_base + s < B.cap_f) far_buf[far_base + s] = make_uint4((uint32_t)up.z, ng, 0u, 0u);
+                else atomicOr(&B.ctl->status, ST_OVERFLOW);
+                atomicAdd(&dc->relaxed, 1);
+                break;
+            }
+            cur = got;
+        }
+    }
+    grp.sync();
+    if (rank == 0) B.ctl->far_n = (int)min((int64_t)B.cap_f, far_base + *(volatile int *)far_add);
+    at.stage = REP_DONE;
 }
 
-// Grp = GridGroup: every CTA of a cooperative launch (the initial search);
-// Grp = CtaGroup: one CTA (update batches: the repair and the resumed
-// search touch little of the graph, and block barriers are far cheaper than
-// grid barriers between the repair steps and the search phases).
+// Grp = GridGroup: every CTA of a cooperative launch (CTA 0 alone where that
+// is enough); Grp = CtaGroup: one CTA (opts.group = 1).  One CTA an SM: the
+// grid is half the SMs, and 64 registers a thread would spill.
 template <class Grp>
-__global__ void __launch_bounds__(512, 2)
+__global__ void __launch_bounds__(512, 1)
     k_dyn(DevGraph G, SlotArrays sa, uint32_t *hops, SearchParams P, DynArgs A, DynCtl *dc) {
     // a batch the device could not apply leaves graph and search untouched
     // (every CTA returns here, before any barrier; the host takes over)
     if (A.apply_res && *(volatile const int *)(A.apply_res + 1) != 0) return;
     const int nupd = A.nupd_dev ? *(volatile const int *)A.nupd_dev : A.nupd;
     __shared__ WarpRows wrows[16];
-    __shared__ int lsh[1];  // level counter of a walk on one CTA
     SlotBufs B = slot_of_dyn(sa);
     const Grp grp = dyn_group(static_cast<Grp *>(nullptr), B);
-    const int rank = grp.rank(), size = grp.size();
+    const int rank = grp.rank();
     const uint32_t scale = G.wmin;
-    int32_t *fa = reinterpret_cast<int32_t *>(B.q0);
-    int32_t *fb = reinterpret_cast<int32_t *>(B.q1);
-    uint4 *far_buf = (*(volatile int *)&B.ctl->far_sel) ? B.f1 : B.f0;  // f re-derived (keep mode)
-    const int64_t far_base = *(volatile int *)&B.ctl->far_n;
 
     if (!A.initial) {
-        int it = 0, nf = 0;
-        // ---- A. heuristic repair: lower hops over inserted arcs ----------
-        if (A.heur == 1) {
-            for (int i = rank; i < nupd; i += size) {
-                const int4 up = A.upd[i];
-                if (up.x != UPD_INS) continue;
-                const uint32_t hv = __ldcg(hops + up.z);
-                if (hv == HOPS_INF) continue;
-                const uint32_t old = atomicMin(hops + up.y, hv + 1);
-                if (hv + 1 < old) {
-                    const int s = atomicAdd(&dc->cnt[(it + 1) & 3], 1);
-                    fb[s] = up.y;  // each lowering pushes once; bounded by 2 cap_q
-                    atomicAdd(&dc->hops_lowered, 1);
-                }
-            }
-            dyn_level_end(grp, dc, it, nf);
-            it++;
-            // lowers the hops of u's in-neighbours from u's; pushes each
-            // lowered node once per lowering (bounded by 2 cap_q)
-            auto lower_from = [&](int u, int32_t *out, int *counter) {
-                const uint32_t hu = __ldcg(hops + u);
-                const int b = row_begin(G.roff, G.roend, u), e = row_end(G.roff, G.roend, u);
-                for (int j0 = b; j0 < e; j0 += DYN_ROW_UNROLL) {
-                    int p[DYN_ROW_UNROLL];
-                    uint32_t hp[DYN_ROW_UNROLL];
-#pragma unroll
-                    for (int k = 0; k < DYN_ROW_UNROLL; k++) p[k] = j0 + k < e ? (int)__ldcg(G.rarc + j0 + k).x : -1;
-#pragma unroll
-                    for (int k = 0; k < DYN_ROW_UNROLL; k++) hp[k] = p[k] >= 0 ? __ldcg(hops + p[k]) : 0u;
-#pragma unroll
-                    for (int k = 0; k < DYN_ROW_UNROLL; k++) {
-                        if (p[k] < 0 || hu + 1 >= hp[k]) continue;
-                        const uint32_t old = atomicMin(hops + p[k], hu + 1);
-                        if (hu + 1 < old) {
-                            const int s = atomicAdd(counter, 1);
-                            if (s < 2 * B.cap_q) out[s] = p[k];
-                            else atomicOr(&B.ctl->status, ST_OVERFLOW);
-                            atomicAdd(&dc->hops_lowered, 1);
-                        }
+        RepairAt at{A.heur == 1 ? REP_HOPS : REP_TREE, 0, reinterpret_cast<int32_t *>(B.q0),
+                    reinterpret_cast<int32_t *>(B.q1)};
+        if constexpr (Grp::multi) {
+            if (nupd <= DYN_LOCAL_UPD) {
+                if (grp.first_cta()) {
+                    __shared__ int cnt[5];
+                    dyn_repair<true>(CtaGroup{&B.ctl->status}, G, B, hops, A, dc, nupd, at,
+                                     reinterpret_cast<uint4 *>(wrows), cnt);
+                    if (threadIdx.x == 0) {
+                        dc->inv_n = cnt[3];
+                        dc->stage = at.stage;
+                        dc->nf = at.nf;
+                        dc->odd = at.fa != reinterpret_cast<int32_t *>(B.q0);
                     }
                 }
-            };
-            while (nf > 0) {
-                if (dyn_walk_local<Grp>(grp, nf, fa, fb, dc, lsh, lower_from)) break;
-                // a push past the buffer raised an overflow: its count is not a frontier
-                if (*(volatile int *)&B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT)) break;
-                int32_t *t = fa;
-                fa = fb;
-                fb = t;
-                const int PH = (it + 1) & 3;
-                for (int i = rank; i < nf; i += size) lower_from(__ldcg(fa + i), fb, &dc->cnt[PH]);
-                dyn_level_end(grp, dc, it, nf);
-                it++;
-                if (*(volatile int *)&B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT)) break;
-            }
-        }
-        // ---- B. invalidate subtrees hanging off removed / heavier tree arcs
-        {
-            const int PH = (it + 1) & 3;
-            for (int i = rank; i < nupd; i += size) {
-                const int4 up = A.upd[i];
-                if (up.x != UPD_TREE) continue;
-                const uint64_t sv = __ldcg(B.state + up.z);
-                if (st_g(sv) < INF_G && st_parent(sv) == up.y &&
-                    atomicCAS(B.state + up.z, sv, ~0ull) == sv) {
-                    fb[atomicAdd(&dc->cnt[PH], 1)] = up.z;
-                    A.inv[atomicAdd(&dc->inv_n, 1)] = up.z;
+                grp.sync();  // CTA 0's changes and hand-back are visible to every CTA
+                at.stage = *(volatile int *)&dc->stage;
+                at.nf = *(volatile int *)&dc->nf;
+                if (*(volatile int *)&dc->odd) {
+                    at.fa = reinterpret_cast<int32_t *>(B.q1);
+                    at.fb = reinterpret_cast<int32_t *>(B.q0);
+                } else {
+                    at.fa = reinterpret_cast<int32_t *>(B.q0);
+                    at.fb = reinterpret_cast<int32_t *>(B.q1);
                 }
             }
-            dyn_level_end(grp, dc, it, nf);
-            it++;
-            // invalidates x's children in the tree (nodes whose parent is x);
-            // a parallel arc's second CAS fails: each node is invalidated once
-            auto invalidate_from = [&](int x, int32_t *out, int *counter) {
-                const int b = row_begin(G.off, G.oend, x), e = row_end(G.off, G.oend, x);
-                for (int j0 = b; j0 < e; j0 += DYN_ROW_UNROLL) {
-                    int y[DYN_ROW_UNROLL];
-                    uint64_t sy[DYN_ROW_UNROLL];
-#pragma unroll
-                    for (int k = 0; k < DYN_ROW_UNROLL; k++) y[k] = j0 + k < e ? (int)__ldcg(G.arc + j0 + k).x : -1;
-#pragma unroll
-                    for (int k = 0; k < DYN_ROW_UNROLL; k++) sy[k] = y[k] >= 0 ? __ldcg(B.state + y[k]) : ~0ull;
-#pragma unroll
-                    for (int k = 0; k < DYN_ROW_UNROLL; k++) {
-                        if (y[k] >= 0 && st_g(sy[k]) < INF_G && st_parent(sy[k]) == x &&
-                            atomicCAS(B.state + y[k], sy[k], ~0ull) == sy[k]) {
-                            out[atomicAdd(counter, 1)] = y[k];
-                            A.inv[atomicAdd(&dc->inv_n, 1)] = y[k];
-                        }
-                    }
-                }
-            };
-            while (nf > 0) {
-                if (dyn_walk_local<Grp>(grp, nf, fa, fb, dc, lsh, invalidate_from)) break;
-                if (*(volatile int *)&B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT)) break;
-                int32_t *t = fa;
-                fa = fb;
-                fb = t;
-                const int PH2 = (it + 1) & 3;
-                for (int i = rank; i < nf; i += size) invalidate_from(__ldcg(fa + i), fb, &dc->cnt[PH2]);
-                dyn_level_end(grp, dc, it, nf);
-                it++;
-            }
         }
-        // ---- C. re-seed invalidated nodes from valid in-neighbours --------
-        const int ninv = *(volatile int *)&dc->inv_n;
-        uint2 *best = B.q1;  // one {g, parent} per invalidated node
-        for (int i = rank; i < ninv; i += size) {
-            const int x = A.inv[i];
-            uint32_t bg = INF_G;
-            int bp = -1;
-            const int b = row_begin(G.roff, G.roend, x), e = row_end(G.roff, G.roend, x);
-            for (int j0 = b; j0 < e; j0 += DYN_ROW_UNROLL) {
-                uint2 a[DYN_ROW_UNROLL];
-                uint32_t gp[DYN_ROW_UNROLL];
-#pragma unroll
-                for (int k = 0; k < DYN_ROW_UNROLL; k++)
-                    a[k] = j0 + k < e ? __ldcg(G.rarc + j0 + k) : make_uint2(0xFFFFFFFFu, 0u);
-#pragma unroll
-                for (int k = 0; k < DYN_ROW_UNROLL; k++)
-                    gp[k] = (int)a[k].x >= 0 ? st_g(__ldcg(B.state + (int)a[k].x)) : INF_G;
-#pragma unroll
-                for (int k = 0; k < DYN_ROW_UNROLL; k++) {
-                    if (gp[k] >= INF_G) continue;
-                    const uint64_t c = (uint64_t)gp[k] + a[k].y;
-                    if (c < bg) {
-                        bg = (uint32_t)c;
-                        bp = (int)a[k].x;
-                    }
-                }
-            }
-            best[i] = make_uint2(bg, (uint32_t)bp);
+        if (at.stage != REP_DONE) {
+            dyn_repair<false>(grp, G, B, hops, A, dc, nupd, at, nullptr, nullptr);
+            grp.sync();
         }
-        grp.sync();
-        for (int i = rank; i < ninv; i += size) {
-            const uint2 bv = best[i];
-            if (bv.x >= INF_G) continue;
-            const int x = A.inv[i];
-            B.state[x] = st_make(bv.x, (int32_t)bv.y);
-            const int s = atomicAdd(&dc->far_add, 1);
-            if (far_base + s < B.cap_f) far_buf[far_base + s] = make_uint4((uint32_t)x, bv.x, 0u, 0u);
-            else atomicOr(&B.ctl->status, ST_OVERFLOW);
-            atomicAdd(&dc->reseeded, 1);
-        }
-        grp.sync();
-        // ---- D. relax heads of inserted / lighter arcs --------------------
-        for (int i = rank; i < nupd; i += size) {
-            const int4 up = A.upd[i];
-            if (up.x != UPD_INS && up.x != UPD_LIGHTER) continue;
-            const uint32_t gu = st_g(__ldcg(B.state + up.y));
-            if (gu >= INF_G) continue;
-            const uint64_t ng64 = (uint64_t)gu + (uint32_t)up.w;
-            if (ng64 >= INF_G) continue;
-            const uint32_t ng = (uint32_t)ng64;
-            uint64_t cur = __ldcg(B.state + up.z);
-            while (ng < st_g(cur)) {
-                const uint64_t got = atomicCAS(B.state + up.z, cur, st_make(ng, up.y));
-                if (got == cur) {
-                    const int s = atomicAdd(&dc->far_add, 1);
-                    if (far_base + s < B.cap_f) far_buf[far_base + s] = make_uint4((uint32_t)up.z, ng, 0u, 0u);
-                    else atomicOr(&B.ctl->status, ST_OVERFLOW);
-                    atomicAdd(&dc->relaxed, 1);
-                    break;
-                }
-                cur = got;
-            }
-        }
-        grp.sync();
-        if (rank == 0) B.ctl->far_n = (int)min((int64_t)B.cap_f, far_base + *(volatile int *)&dc->far_add);
-        grp.sync();
     }
     // ---- E. (resume) the A* search ---------------------------------------
     SearchResult r;
@@ -1023,10 +1079,10 @@ static int dyn_launch(ddp_dyn *d, int initial, int nupd, const int *dres = nullp
                    d->o.K, 1, initial ? 0 : 1, 1};
     // a resumed search leaves entries with g >= the last cost (f >= g)
     // unexamined until it needs them
-    if (!initial && d->cost >= 0 && d->cost != DDP_INF) {
+    if (!initial) {
         P.cold = d->d_cold;
         P.cold_cap = d->cold_cap;
-        P.cold_x = (uint32_t)d->cost;
+        if (d->cost >= 0 && d->cost != DDP_INF) P.cold_x = (uint32_t)d->cost;
     }
     DynArgs A;
     A.upd = d->d_upd;
@@ -1269,10 +1325,9 @@ int ddp_dyn_create(ddp_graph *g, int32_t source, int32_t target, int32_t hkind, 
     d->grid = std::min(coresident, std::max(1, sms / 2));
     if (d->o.grid > 0) d->grid = std::min(coresident, d->o.grid);
     // update batches: the same grid as the initial search unless opts.group
-    // asks otherwise (1 = the one-CTA kernel).  On 1M nodes with 1000-update
-    // batches one CTA took 7.1 ms per batch against 1.23 ms on 76 CTAs: the
-    // resumed search needs the grid's parallelism more than it pays for the
-    // grid barriers.
+    // asks otherwise (1 = the one-CTA kernel).  CTA 0 takes narrow steps
+    // alone either way; the grid is there for the wide ones (the first split
+    // of the open list alone took one CTA 7.1 ms on 1M nodes).
     d->upd_grid = d->o.group > 0 ? std::min(coresident, d->o.group) : d->grid;
     if (hkind == DDP_H_BFS_HOPS) {
         // exact reverse BFS from the target into the dynamic hop array

@@ -64,7 +64,8 @@ struct SearchCtl {
     int far_n, far_sel;   // far pile left by the last run (dynamic resume)
     int cur_ver;          // graph version of the current search (serving)
     unsigned int bar_count, bar_gen;  // grid barrier (single-query form)
-    int cold_n;           // entries in the far pile's cold tier (keep mode)
+    int cold_n;           // entries in the far pile's cold tier (keep mode) ...
+    unsigned int cold_x;  // ... all with g >= cold_x
     // what CTA 0 hands back after running phases alone (run_search)
     int loc_near, loc_far, loc_waves, loc_flip, loc_done;
     uint32_t loc_T;
@@ -484,12 +485,14 @@ struct SearchParams {
     int resume;    // continue from the slot's far pile instead of starting at s
     int no_touch_log;  // do not log first touches (slots that are never reset)
     // t < 0: no target, the search settles everything reachable from s
-    // Keep mode, resumed searches: cold tier of the far pile.  The first
-    // split moves live entries with g >= cold_x (their f is at least g) to
-    // `cold` unexamined; later splits scan the rest until min(f(t),
-    // threshold) passes cold_x, when one split takes the cold entries back.
-    // They rejoin the far pile when the search ends.  cold_x = 0xFFFFFFFF:
-    // no cold tier.
+    // Keep mode, resumed searches: cold tier of the far pile.  A first split
+    // moves live entries with g >= cold_x (their f is at least g) to `cold`
+    // unexamined; they stay there from one resumed search to the next, with
+    // the threshold they went in under, until min(f(t), threshold) of a
+    // split passes it and takes them back.  On 1M nodes the tier held 671,300
+    // of 671,400 open entries: carried through every search (read, set aside,
+    // appended again) they took 25 us of an update's 220.  cold_x =
+    // 0xFFFFFFFF: no new tier.
     uint2 *cold = nullptr;
     int64_t cold_cap = 0;
     uint32_t cold_x = 0xFFFFFFFFu;
@@ -512,7 +515,7 @@ struct SearchResult {
 // While the far pile is small (LOCAL_FAR) it splits it too, and while the
 // list is narrow (LOCAL_FILL) it takes the next bucket in early, so that the
 // floods of successive buckets overlap instead of running one after the other
-// (out of keep mode; at most LOCAL_AHEAD buckets before the list empties).
+// (at most LOCAL_AHEAD buckets before the list empties).
 // A 511 x 511 maze query took 44 ms with every phase on the grid (1,926
 // phases of 20-70 entries, 23 us each), 3.2 ms with narrow phases here, 1.6
 // ms with overlapping buckets (16, 32 or 64 entries alike; wider buckets
@@ -527,14 +530,15 @@ constexpr int LOCAL_WAVES = 4096;
 constexpr int LOCAL_CAP = (int)(16 * sizeof(WarpRows) / (2 * sizeof(uint4)));
 static_assert(LOCAL_CAP >= LOCAL_IN && LOCAL_CAP >= LOCAL_OUT, "local lists hold a whole phase");
 
-// near: nnear entries in qcur (rewritten on return with the entries left).
+// near: nnear entries in qcur (rewritten on return with the entries left);
+// cold_x: no entry of the cold tier has a smaller f (0xFFFFFFFF: no tier).
 // Results go to ctl->loc_*; far pushes and first touches are appended as a
 // grid phase does.
 template <class Heur>
 __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H, const SearchParams &P,
                              WarpRows *wrows, uint2 *qcur, int nnear, uint4 *fcur, uint4 *falt, int64_t nfar0,
-                             uint32_t T, uint32_t ht, unsigned long long &n_exp, unsigned long long &n_scan,
-                             unsigned long long &n_rel) {
+                             uint32_t T, uint32_t ht, uint32_t cold_x, unsigned long long &n_exp,
+                             unsigned long long &n_scan, unsigned long long &n_rel) {
     SearchCtl *ctl = B.ctl;
     // {node, g, row begin, row end}
     uint4 *buf = reinterpret_cast<uint4 *>(wrows);
@@ -564,7 +568,7 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
     unsigned long long n_far = 0;
     uint4 *cur = buf, *nxt = buf + cap;
     for (;;) {
-        if (!P.keep && m < LOCAL_FILL) {
+        if (m < LOCAL_FILL) {
             // the list is empty or narrow: the far pile's turn
             const int64_t nf = nfar0 + c_far;
             const uint64_t ft64 = (uint64_t)tg + ht;
@@ -572,12 +576,13 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
             const uint32_t fm = far_min;
             __syncthreads();  // every thread has read the words the branches below depend on
             if (m == 0) ahead = 0;
-            if (nf == 0 || fm >= ft) {
+            if ((nf == 0 ? cold_x : min(fm, cold_x)) >= ft) {
                 if (m == 0) {
                     done = 1;  // no open node with f < f(t)
                     break;
                 }
-            } else if (nf <= LOCAL_FAR && (m == 0 || ahead < LOCAL_AHEAD)) {
+            } else if (nf > 0 && nf <= LOCAL_FAR && (m == 0 || ahead < LOCAL_AHEAD) &&
+                       min(ft, sat_add(max(fm, T), P.delta)) <= cold_x) {
                 T = sat_add(max(fm, T), P.delta);  // above the smallest f: something moves
                 ahead++;
                 n_far += (unsigned long long)nf;
@@ -587,9 +592,16 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                 }
                 __syncthreads();
                 for (int64_t i = threadIdx.x; i < nf; i += blockDim.x) {
-                    const uint4 e = __ldcg(fcur + i);
-                    if (e.z >= ft) continue;
-                    if (e.z < T) {
+                    uint4 e = __ldcg(fcur + i);
+                    if (P.keep) {
+                        // h may have changed since the push: f re-derived
+                        const uint64_t se = __ldcg(B.state + e.x);
+                        e.z = sat_add(e.y, H((int)e.x));
+                        if (st_g(se) != e.y) continue;
+                    } else if (e.z >= ft) {
+                        continue;
+                    }
+                    if (e.z < T && e.z < ft) {
                         const int p = atomicAdd(&cnt[wv % 3], 1);
                         if (p < cap) {
                             cur[p] = make_uint4(e.x, e.y, (uint32_t)row_begin(G.off, G.oend, (int)e.x),
@@ -611,7 +623,7 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                 __syncthreads();
                 if (m == 0) continue;  // far_min is known now: the next split moves something
             } else if (m == 0) {
-                break;  // a large pile: the grid splits it
+                break;  // a large pile, or the cold tier's turn: the grid splits it
             }
         }
         int *push = &cnt[(wv + 1) % 3];
@@ -636,7 +648,8 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
             const uint32_t hu = (ft < T || (P.keep && ft != 0xFFFFFFFFu)) ? H(u) : 0u;
             if (st_g(su) != gu || u == P.t) continue;
             if ((uint64_t)gu + hu >= ft) {
-                if (P.keep && sub == 0) to_far((uint32_t)u, gu, 0u);  // keep mode: f re-derived
+                // keep mode: stays open beyond f(t)
+                if (P.keep && sub == 0) to_far((uint32_t)u, gu, sat_add(gu, hu));
                 continue;
             }
             if (sub == 0) {
@@ -706,7 +719,7 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
         uint4 *t = cur;
         cur = nxt;
         nxt = t;
-        if ((m == 0 && P.keep) || m > LOCAL_OUT || wv >= LOCAL_WAVES || nfar0 + c_far > B.cap_f / 2) break;
+        if (m > LOCAL_OUT || wv >= LOCAL_WAVES || nfar0 + c_far > B.cap_f / 2) break;
         __syncthreads();  // every thread has read the counters
     }
     __syncthreads();
@@ -752,8 +765,8 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
         ctl->iters = 0;
         ctl->expanded = ctl->scanned = ctl->relaxed = 0;
         ctl->far_scanned = 0;
-        ctl->cold_n = 0;
         if (!P.resume) {
+            ctl->cold_n = 0;
             ctl->touched = 1;
             B.state[P.s] = st_make(0, -1);
             B.touched[0] = P.s;
@@ -762,6 +775,9 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
     }
     const int64_t far_resume = P.resume ? (int64_t)(*(volatile int *)&ctl->far_n) : 0;
     const bool far_in_f1 = P.resume && (*(volatile int *)&ctl->far_sel) != 0;
+    // cold tier (keep mode, resumed), as the last search left it
+    int64_t ncold = P.resume && P.cold ? min((int64_t)*(volatile int *)&ctl->cold_n, P.cold_cap) : 0;
+    uint32_t cold_x = ncold > 0 ? *(volatile unsigned int *)&ctl->cold_x : 0xFFFFFFFFu;
     auto read_tg = [&]() -> uint32_t { return P.t >= 0 ? st_g(__ldcg(B.state + P.t)) : 0xFFFFFFFFu; };
     grp.sync_fetch([&] { pc.tg = read_tg(); });
 
@@ -787,17 +803,29 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
     const int64_t max_phases = 4 * (int64_t)G.n + (1 << 22);
     const uint32_t ht = P.t >= 0 ? H(P.t) : 0u;
     uint32_t tg = pc.tg;  // g(t): only decreases, so a stale value only prunes less
-    // cold tier (keep mode, resumed): made by the first split
-    uint32_t cold_x = (P.keep && P.resume && P.cold) ? P.cold_x : 0xFFFFFFFFu;
-    bool cold_pass = cold_x != 0xFFFFFFFFu;
-    int64_t ncold = 0;
+    // phases that CTA 0 may run alone
+    const bool local_ok = Grp::multi && !has_diff && (P.K <= 0 || P.K >= LOCAL_OUT);
+    // the first split of a resumed search: it takes the tier back when the two
+    // piles hold half of what one can (their stale entries are dropped), moves
+    // entries to the tier when the pile is more than CTA 0 can split, and is
+    // CTA 0's otherwise
+    bool cold_take = false, cold_pass = false;
+    if (P.resume && P.keep && P.cold) {
+        cold_take = ncold > 0 && ncold + nfar > B.cap_f / 2;
+        if (!cold_take && nfar > LOCAL_FAR) {
+            if (ncold == 0) cold_x = P.cold_x;
+            cold_pass = cold_x != 0xFFFFFFFFu;
+        }
+    }
+    if (P.resume && !cold_take && !cold_pass && local_ok && nfar <= LOCAL_FAR) splitting = false;
     uint2 *cold_stage = reinterpret_cast<uint2 *>(wr.snr);
 
     for (;;) {
         if constexpr (Grp::multi) {
-            if (!splitting && head == 0 && nnext == 0 && !has_diff && nnear <= LOCAL_IN &&
-                nfar <= B.cap_f / 2 && (P.K <= 0 || P.K >= LOCAL_OUT)) {
-                if (grp.first_cta()) local_phases(G, B, H, P, wrows, qcur, (int)nnear, fcur, falt, nfar, T, ht, n_exp, n_scan, n_rel);
+            if (!splitting && head == 0 && nnext == 0 && local_ok && nnear <= LOCAL_IN && nfar <= B.cap_f / 2) {
+                if (grp.first_cta())
+                    local_phases(G, B, H, P, wrows, qcur, (int)nnear, fcur, falt, nfar, T, ht,
+                                 ncold > 0 ? cold_x : 0xFFFFFFFFu, n_exp, n_scan, n_rel);
                 grp.sync_fetch([&] {
                     pc.loc_near = *(volatile int *)&ctl->loc_near;
                     pc.loc_far = *(volatile int *)&ctl->loc_far;
@@ -971,10 +999,10 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
             // stale entries) re-check the state and h.
             const uint32_t thr = compacting ? T : Tsplit;
             const bool recheck = P.keep || compacting;
-            // cold tier: made here (first split of a resumed search), or
+            // cold tier: added to here (first split of a resumed search), or
             // scanned with the pile once min(f(t), threshold) passes cold_x
             const bool to_cold = cold_pass && !compacting;
-            const bool merge_cold = !compacting && ncold > 0 && min(ft, thr) > cold_x;
+            const bool merge_cold = !compacting && ncold > 0 && (cold_take || (!to_cold && min(ft, thr) > cold_x));
             const int64_t nscan = nfar + (merge_cold ? ncold : 0);
             if (grp.rank() == 0) ctl->far_scanned += (unsigned long long)nscan;
             uint2 *dst = compacting ? qnxt : qcur;
@@ -1027,6 +1055,7 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
             if (merge_cold) {
                 ncold = 0;  // every cold entry was examined: none is left
                 cold_x = 0xFFFFFFFFu;
+                cold_take = false;
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) local_min = min(local_min, __shfl_xor_sync(FULL, local_min, o));
@@ -1126,18 +1155,11 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
         if (n_exp) atomicAdd(&ctl->expanded, n_exp);
         if (n_rel) atomicAdd(&ctl->relaxed, n_rel);
     }
-    if (ncold > 0) {
-        // the cold tier rejoins the far pile (f re-derived by the next split)
-        for (int64_t i = grp.rank(); i < ncold; i += grp.size()) {
-            const uint2 c = __ldcg(P.cold + i);
-            if (nfar + i < B.cap_f) fcur[nfar + i] = make_uint4(c.x, c.y, 0u, 0u);
-            else atomicOr(&ctl->status, ST_OVERFLOW);
-        }
-        nfar = min(nfar + ncold, B.cap_f);
-    }
     if (grp.rank() == 0) {
         ctl->far_n = (int)nfar;
         ctl->far_sel = fcur == B.f1 ? 1 : 0;
+        ctl->cold_n = (int)ncold;
+        ctl->cold_x = cold_x;
     }
     grp.sync();
     SearchResult r;
