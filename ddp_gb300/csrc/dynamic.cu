@@ -73,7 +73,7 @@ struct DynMirror {
     bool dev_meta = false;
     int32_t *d_cap = nullptr, *d_rcap = nullptr;  // row capacities, n each
     long long *d_tails = nullptr;                 // first unused slot: forward, reverse
-    int4 *h_ops = nullptr, *d_ops = nullptr;      // one batch {flag, u, v, w}
+    int4 *h_ops = nullptr, *d_ops = nullptr;      // one batch {flag, u, v, w} (mapped host memory, two views)
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};  // DDP_TRACE: around k_apply and k_dyn
     // staging of a batch's scatter lists: pinned host memory (the copy is
     // asynchronous; the buffer is reused once the graph's stream has been
@@ -88,7 +88,6 @@ struct DynMirror {
         cudaFree(d_rcap);
         cudaFree(d_tails);
         cudaFreeHost(h_ops);
-        cudaFree(d_ops);
         for (cudaEvent_t e : ev)
             if (e) cudaEventDestroy(e);
     }
@@ -209,10 +208,11 @@ __global__ void k_scatter_all(ScatterAll j) {
 constexpr int APPLY_MAX = 4096;
 constexpr int DYN_OUT_APPLY = 12;  // words of the dyn output block k_apply writes (of 16)
 constexpr int APPLY_THREADS = 1024;
+constexpr int APPLY_SMEM = 48;  // bytes of shared memory an update takes
 enum { APPLY_NO_ROOM = 1 };
 
 struct ApplyArgs {
-    const int4 *ops;  // {flag, u, v, w}, batch order
+    const int4 *ops;  // {flag, u, v, w}, batch order (host memory)
     int nops;
     int32_t n;
     uint2 *arc, *rarc;
@@ -240,29 +240,55 @@ __device__ __forceinline__ long long grown_cap(int32_t used, int32_t cap, int32_
     return c;
 }
 
-// Sorts a and b (P = power of two entries each) ascending, bitonic.
-__device__ void apply_sort2(unsigned long long *a, unsigned long long *b, int P) {
-    for (int k = 2; k <= P; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < P; i += blockDim.x) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const bool up = (i & k) == 0;
-                    unsigned long long x = a[i], y = a[l];
-                    if ((x > y) == up) {
-                        a[i] = y;
-                        a[l] = x;
-                    }
-                    x = b[i];
-                    y = b[l];
-                    if ((x > y) == up) {
-                        b[i] = y;
-                        b[l] = x;
-                    }
-                }
+// Sorts a and b (P = power of two entries each, at least 32) ascending with
+// ta and tb as second buffers; returns with a and b at the sorted ones.
+// Runs of 32 keys are sorted in a warp (bitonic, shuffles), then merged in
+// pairs: a key's place is its own plus its rank in the sibling run, a binary
+// search in shared memory.  1,024 keys: 2 x 10 us as one bitonic network over
+// the block (55 barriers; half of that with shuffles for the short
+// distances, which then bound it), a third of that as runs and merges.
+__device__ void apply_sort2(unsigned long long *&a, unsigned long long *&b, unsigned long long *ta,
+                            unsigned long long *tb, int P) {
+    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+        unsigned long long x = a[i], y = b[i];
+        for (int k = 2; k <= 32; k <<= 1)
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                // the last stage ascends in every warp
+                const bool low = (k == 32 || (i & k) == 0) == ((i & j) == 0);
+                const unsigned long long x2 = __shfl_xor_sync(FULL, x, j), y2 = __shfl_xor_sync(FULL, y, j);
+                x = low ? min(x, x2) : max(x, x2);
+                y = low ? min(y, y2) : max(y, y2);
             }
-            __syncthreads();
+        a[i] = x;
+        b[i] = y;
+    }
+    __syncthreads();
+    for (int run = 32; run < P; run <<= 1) {
+        for (int i = threadIdx.x; i < P; i += blockDim.x) {
+            const int sib = (i & ~(run - 1)) ^ run;  // the sibling run's first key
+            const bool right = (i & run) != 0;       // equal keys: the left run's first
+            const unsigned long long x = a[i], y = b[i];
+            int ra = 0, rb = 0;  // keys of the sibling run before x, y
+            for (int h = run >> 1; h > 0; h >>= 1) {
+                const unsigned long long ca = a[sib + ra + h - 1], cb = b[sib + rb + h - 1];
+                if (right ? ca <= x : ca < x) ra += h;
+                if (right ? cb <= y : cb < y) rb += h;
+            }
+            const unsigned long long ca = a[sib + ra], cb = b[sib + rb];
+            if (right ? ca <= x : ca < x) ra++;
+            if (right ? cb <= y : cb < y) rb++;
+            const int at = (i & (run - 1)) + (i & ~(2 * run - 1));
+            ta[at + ra] = x;
+            tb[at + rb] = y;
         }
+        __syncthreads();
+        unsigned long long *t = a;
+        a = ta;
+        ta = t;
+        t = b;
+        b = tb;
+        tb = t;
+    }
 }
 
 // First slot in [b, e) whose arc has head x (and weight wt when `weighted`),
@@ -295,15 +321,15 @@ __device__ void apply_grow_row(uint2 *arc, int32_t *beg, int32_t *end, int32_t *
 }
 
 __global__ void __launch_bounds__(APPLY_THREADS) k_apply(ApplyArgs A) {
-    extern __shared__ unsigned long long apply_smem[];
+    extern __shared__ int4 apply_smem[];
     __shared__ unsigned long long need[2];
     __shared__ int nrec;
     int P = 32;
     while (P < A.nops) P <<= 1;
-    unsigned long long *ka = apply_smem;        // (u << 32 | i), every valid op
+    int4 *ops = apply_smem;                     // the batch: host memory is read once
+    unsigned long long *ka = reinterpret_cast<unsigned long long *>(ops + P);  // (u << 32 | i), every valid op
     unsigned long long *kb = ka + P;            // (v << 32 | i), valid inserts
-    int *hit = reinterpret_cast<int *>(kb + P);  // forward slot op i hit (-1: none)
-    uint32_t *w0 = reinterpret_cast<uint32_t *>(hit + P);  // that slot's weight before op i
+    unsigned long long *ta = kb + P, *tb = ta + P;  // second buffers of the sort
     const unsigned long long NONE = ~0ull;
     for (int z = 0; z < 3; z++)
         for (int i = threadIdx.x; i < A.zero_n[z]; i += blockDim.x) A.zero[z][i] = 0u;
@@ -311,7 +337,7 @@ __global__ void __launch_bounds__(APPLY_THREADS) k_apply(ApplyArgs A) {
         ka[i] = kb[i] = NONE;
         if (i < A.nops) {
             const int4 o = A.ops[i];
-            hit[i] = -1;
+            ops[i] = o;
             if (apply_valid(o, A.n)) {
                 ka[i] = ((unsigned long long)(uint32_t)o.y << 32) | (uint32_t)i;
                 if (o.x == 1) kb[i] = ((unsigned long long)(uint32_t)o.z << 32) | (uint32_t)i;
@@ -323,7 +349,13 @@ __global__ void __launch_bounds__(APPLY_THREADS) k_apply(ApplyArgs A) {
         nrec = 0;
     }
     __syncthreads();
-    apply_sort2(ka, kb, P);
+    apply_sort2(ka, kb, ta, tb, P);
+    // in the buffers that the sort left free
+    const bool odd = ka == ta;
+    // forward slot op i hit (-1: none)
+    int *hit = reinterpret_cast<int *>(odd ? reinterpret_cast<unsigned long long *>(ops + P) : ta);
+    uint32_t *w0 = reinterpret_cast<uint32_t *>(hit + P);  // that slot's weight before op i
+    for (int i = threadIdx.x; i < A.nops; i += blockDim.x) hit[i] = -1;
     // room: every row that outgrows its capacity moves to the tail
     for (int p = threadIdx.x; p < P; p += blockDim.x) {
         for (int side = 0; side < 2; side++) {
@@ -332,7 +364,7 @@ __global__ void __launch_bounds__(APPLY_THREADS) k_apply(ApplyArgs A) {
             const int r = (int)(k[p] >> 32);
             int32_t add = 0;
             for (int q = p; q < P && k[q] != NONE && (k[q] >> 32) == (unsigned long long)r; q++)
-                add += A.ops[(uint32_t)k[q]].x == 1;
+                add += ops[(uint32_t)k[q]].x == 1;
             const int32_t *beg = side ? A.roff : A.off, *end = side ? A.roend : A.oend,
                           *cap = side ? A.rcap : A.cap;
             const long long c = grown_cap(end[r] - beg[r], cap[r], add);
@@ -359,15 +391,16 @@ __global__ void __launch_bounds__(APPLY_THREADS) k_apply(ApplyArgs A) {
         while (q1 < P && ka[q1] != NONE && (int)(ka[q1] >> 32) == a) q1++;
         for (int q = p; q < q1; q++) {
             const int i = (int)(uint32_t)ka[q];
-            const int4 o = A.ops[i];
+            const int4 o = ops[i];
             if (o.x == 1) continue;
             const int b = o.z;
+            const int rb = A.roff[b], re = A.roend[b];  // beside the forward row's chain
             const int jf = apply_find(A.arc, A.off[a], A.oend[a], (uint32_t)b, 0u, false);
             if (jf < 0) continue;  // no such arc: nothing to do
             const uint32_t wold = A.arc[jf].y;
             hit[i] = jf;
             w0[i] = wold;
-            const int jr = apply_find(A.rarc, A.roff[b], A.roend[b], (uint32_t)a, wold, true);
+            const int jr = apply_find(A.rarc, rb, re, (uint32_t)a, wold, true);
             if (o.x == 0) {
                 A.arc[jf].x = 0xFFFFFFFFu;
                 if (jr >= 0) A.rarc[jr].x = 0xFFFFFFFFu;
@@ -384,8 +417,8 @@ __global__ void __launch_bounds__(APPLY_THREADS) k_apply(ApplyArgs A) {
             if (!first) continue;
             const uint2 fin = A.arc[hit[i]];
             int4 rec;
-            if ((int32_t)fin.x < 0 || fin.y > w0[i]) rec = make_int4(UPD_TREE, a, A.ops[i].z, 0);
-            else if (fin.y < w0[i]) rec = make_int4(UPD_LIGHTER, a, A.ops[i].z, (int)fin.y);
+            if ((int32_t)fin.x < 0 || fin.y > w0[i]) rec = make_int4(UPD_TREE, a, ops[i].z, 0);
+            else if (fin.y < w0[i]) rec = make_int4(UPD_LIGHTER, a, ops[i].z, (int)fin.y);
             else continue;
             A.ups[atomicAdd(&nrec, 1)] = rec;
         }
@@ -399,14 +432,14 @@ __global__ void __launch_bounds__(APPLY_THREADS) k_apply(ApplyArgs A) {
             const int r = (int)(k[p] >> 32);
             int q1 = p;
             int32_t add = 0;
-            for (; q1 < P && k[q1] != NONE && (int)(k[q1] >> 32) == r; q1++) add += A.ops[(uint32_t)k[q1]].x == 1;
+            for (; q1 < P && k[q1] != NONE && (int)(k[q1] >> 32) == r; q1++) add += ops[(uint32_t)k[q1]].x == 1;
             if (!add) continue;
             uint2 *arc = side ? A.rarc : A.arc;
             int32_t *beg = side ? A.roff : A.off, *end = side ? A.roend : A.oend, *cap = side ? A.rcap : A.cap;
             apply_grow_row(arc, beg, end, cap, A.tails + side, r, grown_cap(end[r] - beg[r], cap[r], add));
             int32_t e = end[r];
             for (int q = p; q < q1; q++) {
-                const int4 o = A.ops[(uint32_t)k[q]];
+                const int4 o = ops[(uint32_t)k[q]];
                 if (o.x != 1) continue;
                 arc[e++] = make_uint2((uint32_t)(side ? o.y : o.z), (uint32_t)o.w);
                 if (!side) A.ups[atomicAdd(&nrec, 1)] = make_int4(UPD_INS, o.y, o.z, o.w);
@@ -421,6 +454,10 @@ __global__ void __launch_bounds__(APPLY_THREADS) k_apply(ApplyArgs A) {
     }
 }
 
+// Results go straight to mapped host memory: cost, counters and paths of up
+// to this many nodes need no copy after the kernel.
+constexpr int DYN_HOST_PATH = 4096;
+
 struct DynArgs {
     const int4 *upd;  // {kind, u, v, w}
     int nupd;
@@ -430,6 +467,7 @@ struct DynArgs {
     int32_t *out;     // cost, path len, status, phases, invalidated, reseeded, relaxed, hops lowered
     int32_t *path;
     int32_t path_cap;
+    int32_t *path_h;  // the same in host memory, when it is at most DYN_HOST_PATH long
     int heur;         // 0: h = 0, 1: hops
     int initial;      // 1: first search from the source (no repair steps)
 };
@@ -739,7 +777,11 @@ __global__ void __launch_bounds__(512, 1)
     k_dyn(DevGraph G, SlotArrays sa, uint32_t *hops, SearchParams P, DynArgs A, DynCtl *dc) {
     // a batch the device could not apply leaves graph and search untouched
     // (every CTA returns here, before any barrier; the host takes over)
-    if (A.apply_res && *(volatile const int *)(A.apply_res + 1) != 0) return;
+    if (A.apply_res) {
+        const int rc = *(volatile const int *)(A.apply_res + 1);
+        if (blockIdx.x == 0 && threadIdx.x == 0) A.out[DYN_OUT_APPLY + 1] = rc;
+        if (rc != 0) return;
+    }
     const int nupd = A.nupd_dev ? *(volatile const int *)A.nupd_dev : A.nupd;
     __shared__ WarpRows wrows[16];
     SlotBufs B = slot_of_dyn(sa);
@@ -782,12 +824,15 @@ __global__ void __launch_bounds__(512, 1)
     }
     // ---- E. (resume) the A* search ---------------------------------------
     SearchResult r;
-    if (A.heur == 1) r = run_search(grp, G, B, HeurHops{hops, scale, HOPS_INF, 0u}, P, wrows);
-    else r = run_search(grp, G, B, HeurZero{}, P, wrows);
+    if (A.heur == 1) r = run_search<true>(grp, G, B, HeurHops{hops, scale, HOPS_INF, 0u}, P, wrows);
+    else r = run_search<true>(grp, G, B, HeurZero{}, P, wrows);
+    if (!grp.first_cta()) return;
+    __shared__ int plen;
     if (rank == 0) {
         const int st = B.ctl->status;
         A.out[0] = (st & (ST_OVERFLOW | ST_TIMEOUT)) ? -1 : (r.cost >= INF_G ? DDP_INF : (int32_t)r.cost);
-        A.out[1] = (st & (ST_OVERFLOW | ST_TIMEOUT)) ? 0 : write_path(B, P.s, P.t, A.path, A.path_cap, G.n, &B.ctl->status);
+        plen = (st & (ST_OVERFLOW | ST_TIMEOUT)) ? 0 : write_path(B, P.s, P.t, A.path, A.path_cap, G.n, &B.ctl->status);
+        A.out[1] = plen;
         A.out[2] = B.ctl->status;
         A.out[3] = r.iters;
         A.out[4] = *(volatile int *)&dc->inv_n;
@@ -797,6 +842,9 @@ __global__ void __launch_bounds__(512, 1)
         A.out[8] = (int32_t)min((unsigned long long)INT32_MAX, (unsigned long long)B.ctl->expanded);
         A.out[9] = (int32_t)min((unsigned long long)INT32_MAX, (unsigned long long)B.ctl->scanned);
     }
+    __syncthreads();
+    if (plen <= DYN_HOST_PATH)
+        for (int i = threadIdx.x; i < plen; i += blockDim.x) A.path_h[i] = A.path[i];
 }
 
 }  // namespace
@@ -812,14 +860,15 @@ struct ddp_dyn {
     SlotArrays sa;
     uint32_t *d_hops = nullptr;
     int32_t *d_inv = nullptr;
-    int32_t *d_out = nullptr;
+    int32_t *d_out = nullptr;  // k_apply's record count and status (DYN_OUT_APPLY)
     int32_t *d_path = nullptr;
     DynCtl *d_dc = nullptr;
     int4 *d_upd = nullptr;
     int32_t upd_cap = 0;
     uint2 *d_cold = nullptr;  // cold tier of the retained far pile
     int64_t cold_cap = 0;
-    int32_t *h_out = nullptr;  // pinned copy of d_out (16 words)
+    int32_t *h_out = nullptr;  // results: 16 words, then a path of up to DYN_HOST_PATH nodes ...
+    int32_t *d_hout = nullptr;  // ... the device's view of them (mapped host memory)
     double t_wait_us = 0;      // DDP_TRACE: host wait of the last launch
     int32_t cost = DDP_INF;
     int32_t path_len = 0;
@@ -1004,10 +1053,16 @@ int dyn_apply_device(ddp_dyn *d, int32_t nupd, const int32_t *flag, const int32_
     if (nupd > APPLY_MAX || g->hook.fn) return 1;
     const int32_t n = g->n;
     if (!m->h_ops) {
-        DDP_CUDA(cudaHostAlloc(&m->h_ops, sizeof(int4) * APPLY_MAX, cudaHostAllocDefault));
-        DDP_CUDA(cudaMalloc(&m->d_ops, sizeof(int4) * APPLY_MAX));
         DDP_CUDA(cudaFuncSetAttribute(k_apply, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      24 * APPLY_MAX));
+                                      APPLY_SMEM * APPLY_MAX));
+        int4 *h = nullptr;
+        DDP_CUDA(cudaHostAlloc(&h, sizeof(int4) * APPLY_MAX, cudaHostAllocMapped));
+        const cudaError_t e = cudaHostGetDevicePointer((void **)&m->d_ops, h, 0);
+        if (e != cudaSuccess) {
+            cudaFreeHost(h);
+            return cuda_fail(e, "cudaHostGetDevicePointer(update batch)");
+        }
+        m->h_ops = h;
     }
     if (!m->dev_meta) {
         // the host copy is current here (only device batches make it stale,
@@ -1030,7 +1085,6 @@ int dyn_apply_device(ddp_dyn *d, int32_t nupd, const int32_t *flag, const int32_
             if (w[i] > g->wmax) g->wmax = w[i];
         }
     }
-    if (nupd) DDP_CUDA(cudaMemcpyAsync(m->d_ops, m->h_ops, sizeof(int4) * nupd, cudaMemcpyHostToDevice, g->stream));
     ApplyArgs A;
     A.ops = m->d_ops;
     A.nops = nupd;
@@ -1060,7 +1114,7 @@ int dyn_apply_device(ddp_dyn *d, int32_t nupd, const int32_t *flag, const int32_
     if (timed && !m->ev[0])
         for (cudaEvent_t &e : m->ev) DDP_CUDA(cudaEventCreate(&e));
     if (timed) DDP_CUDA(cudaEventRecord(m->ev[0], g->stream));
-    k_apply<<<1, APPLY_THREADS, 24 * (size_t)P, g->stream>>>(A);
+    k_apply<<<1, APPLY_THREADS, APPLY_SMEM * (size_t)P, g->stream>>>(A);
     DDP_CUDA(cudaGetLastError());
     if (timed) DDP_CUDA(cudaEventRecord(m->ev[1], g->stream));
     g->update_count++;  // landmark distances no longer hold
@@ -1076,7 +1130,7 @@ static int dyn_launch(ddp_dyn *d, int initial, int nupd, const int *dres = nullp
     ddp_graph *g = d->g;
     DevGraph G = graph_view(g);
     SearchParams P{d->s, d->t, d->o.delta > 0 ? (uint32_t)d->o.delta : std::max(1u, (g->wmin + g->wmax) / 4),
-                   d->o.K, 1, initial ? 0 : 1, 1};
+                   d->o.K, initial ? 0 : 1, 1};
     // a resumed search leaves entries with g >= the last cost (f >= g)
     // unexamined until it needs them
     if (!initial) {
@@ -1090,8 +1144,9 @@ static int dyn_launch(ddp_dyn *d, int initial, int nupd, const int *dres = nullp
     A.nupd_dev = dres;
     A.apply_res = dres;
     A.inv = d->d_inv;
-    A.out = d->d_out;
+    A.out = d->d_hout;
     A.path = d->d_path;
+    A.path_h = d->d_hout + 16;
     A.path_cap = g->n;
     A.heur = d->hkind == DDP_H_BFS_HOPS ? 1 : 0;
     A.initial = initial;
@@ -1109,10 +1164,8 @@ static int dyn_launch(ddp_dyn *d, int initial, int nupd, const int *dres = nullp
         DDP_CUDA(cudaLaunchCooperativeKernel((const void *)k_dyn<GridGroup>, dim3(initial ? d->grid : d->upd_grid),
                                              dim3(512), args, 0, g->stream));
     if (dres && trace_on() && g->dyn->ev[2]) DDP_CUDA(cudaEventRecord(g->dyn->ev[2], g->stream));
-    // out[0..9] from k_dyn; out[DYN_OUT_APPLY..+1] from k_apply (device path)
+    // out[0..9] and, on the device path, k_apply's status (DYN_OUT_APPLY + 1)
     int32_t *out = d->h_out;
-    DDP_CUDA(cudaMemcpyAsync(out, d->d_out, sizeof(int32_t) * (dres ? DYN_OUT_APPLY + 2 : 10),
-                             cudaMemcpyDeviceToHost, g->stream));
     const auto tw = std::chrono::steady_clock::now();
     DDP_CUDA(cudaStreamSynchronize(g->stream));
     d->t_wait_us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - tw).count();
@@ -1306,7 +1359,9 @@ int ddp_dyn_create(ddp_graph *g, int32_t source, int32_t target, int32_t hkind, 
     if (rc) return bail(rc);
     e1 = cudaMalloc(&d->d_inv, sizeof(int32_t) * n);
     if (e1 == cudaSuccess) e1 = cudaMalloc(&d->d_out, sizeof(int32_t) * 16);
-    if (e1 == cudaSuccess) e1 = cudaHostAlloc(&d->h_out, sizeof(int32_t) * 16, cudaHostAllocDefault);
+    if (e1 == cudaSuccess)
+        e1 = cudaHostAlloc(&d->h_out, sizeof(int32_t) * (16 + DYN_HOST_PATH), cudaHostAllocMapped);
+    if (e1 == cudaSuccess) e1 = cudaHostGetDevicePointer((void **)&d->d_hout, d->h_out, 0);
     if (e1 == cudaSuccess) e1 = cudaMalloc(&d->d_path, sizeof(int32_t) * n);
     if (e1 == cudaSuccess) e1 = cudaMalloc(&d->d_dc, sizeof(DynCtl));
     if (e1 == cudaSuccess) e1 = cudaMalloc(&d->d_hops, sizeof(uint32_t) * n);
@@ -1419,7 +1474,10 @@ int ddp_dyn_cost(const ddp_dyn *d, int32_t *cost) {
 int ddp_dyn_path(ddp_dyn *d, int32_t *buf, int32_t cap, int32_t *len) {
     if (!d || !len) return fail(DDP_ERR_INVALID, "null argument");
     *len = d->path_len;
-    if (buf && cap > 0 && d->path_len > 0)
+    if (!buf || cap <= 0 || d->path_len <= 0) return DDP_OK;
+    if (d->path_len <= DYN_HOST_PATH)
+        std::memcpy(buf, d->h_out + 16, sizeof(int32_t) * std::min(cap, d->path_len));
+    else
         DDP_CUDA(cudaMemcpy(buf, d->d_path, sizeof(int32_t) * std::min(cap, d->path_len), cudaMemcpyDeviceToHost));
     return DDP_OK;
 }

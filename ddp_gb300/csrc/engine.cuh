@@ -480,9 +480,7 @@ struct SearchParams {
     int32_t s, t;
     uint32_t delta;
     int32_t K;     // 0 = whole near bucket per iteration
-    int keep;      // keep every generated node open (no f(t) pruning): the
-                   // state stays resumable after graph updates
-    int resume;    // continue from the slot's far pile instead of starting at s
+    int resume;    // keep mode: continue from the slot's far pile instead of starting at s
     int no_touch_log;  // do not log first touches (slots that are never reset)
     // t < 0: no target, the search settles everything reachable from s
     // Keep mode, resumed searches: cold tier of the far pile.  A first split
@@ -534,7 +532,7 @@ static_assert(LOCAL_CAP >= LOCAL_IN && LOCAL_CAP >= LOCAL_OUT, "local lists hold
 // cold_x: no entry of the cold tier has a smaller f (0xFFFFFFFF: no tier).
 // Results go to ctl->loc_*; far pushes and first touches are appended as a
 // grid phase does.
-template <class Heur>
+template <bool KEEP, class Heur>
 __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H, const SearchParams &P,
                              WarpRows *wrows, uint2 *qcur, int nnear, uint4 *fcur, uint4 *falt, int64_t nfar0,
                              uint32_t T, uint32_t ht, uint32_t cold_x, unsigned long long &n_exp,
@@ -565,6 +563,8 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
     }
     __syncthreads();
     int m = nnear, wv = 0, ahead = 0, flip = 0, done = 0;
+    bool recheck = KEEP;
+    if (!KEEP) cold_x = 0xFFFFFFFFu;
     unsigned long long n_far = 0;
     uint4 *cur = buf, *nxt = buf + cap;
     for (;;) {
@@ -591,26 +591,50 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                     far_min = 0xFFFFFFFFu;
                 }
                 __syncthreads();
-                for (int64_t i = threadIdx.x; i < nf; i += blockDim.x) {
-                    uint4 e = __ldcg(fcur + i);
-                    if (P.keep) {
-                        // h may have changed since the push: f re-derived
-                        const uint64_t se = __ldcg(B.state + e.x);
-                        e.z = sat_add(e.y, H((int)e.x));
-                        if (st_g(se) != e.y) continue;
-                    } else if (e.z >= ft) {
-                        continue;
-                    }
-                    if (e.z < T && e.z < ft) {
+                auto split = [&](const uint4 &e) {
+                    if (e.z < T && (!KEEP || e.z < ft)) {
                         const int p = atomicAdd(&cnt[wv % 3], 1);
                         if (p < cap) {
                             cur[p] = make_uint4(e.x, e.y, (uint32_t)row_begin(G.off, G.oend, (int)e.x),
                                                 (uint32_t)row_end(G.off, G.oend, (int)e.x));
-                            continue;
+                            return;
                         }
                     }
                     falt[atomicAdd(&c_alt, 1)] = e;  // no more than were read
                     atomicMin(&far_min, e.z);
+                };
+                if (KEEP && recheck) {
+                    // keep mode, once: h may have changed since the push, f is
+                    // re-derived (entries that go stale later are dropped when
+                    // they are popped); a pile of a few thousand entries, four
+                    // of them in flight a lane
+                    constexpr int U = 4;
+                    for (int64_t base = threadIdx.x; base < nf; base += (int64_t)U * blockDim.x) {
+                        uint4 e[U];
+                        uint64_t se[U];
+                        uint32_t h[U];
+#pragma unroll
+                        for (int k = 0; k < U; k++) {
+                            const int64_t i = base + k * (int)blockDim.x;
+                            e[k] = __ldcg(fcur + (i < nf ? i : base));
+                        }
+#pragma unroll
+                        for (int k = 0; k < U; k++) {
+                            se[k] = __ldcg(B.state + e[k].x);
+                            h[k] = H((int)e[k].x);
+                        }
+#pragma unroll
+                        for (int k = 0; k < U; k++) {
+                            e[k].z = sat_add(e[k].y, h[k]);
+                            if (base + k * (int)blockDim.x < nf && st_g(se[k]) == e[k].y) split(e[k]);
+                        }
+                    }
+                    recheck = false;
+                } else {
+                    for (int64_t i = threadIdx.x; i < nf; i += blockDim.x) {
+                        const uint4 e = __ldcg(fcur + i);
+                        if (KEEP || e.z < ft) split(e);
+                    }
                 }
                 __syncthreads();
                 nfar0 = c_alt;
@@ -645,11 +669,11 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
             // the first arcs load beside the label that decides about them
             uint2 a = j < r1 ? (G.oend ? __ldcg(G.arc + j) : __ldg(G.arc + j)) : make_uint2(0xFFFFFFFFu, 0u);
             const uint64_t su = __ldcg(B.state + u);
-            const uint32_t hu = (ft < T || (P.keep && ft != 0xFFFFFFFFu)) ? H(u) : 0u;
+            const uint32_t hu = (ft < T || (KEEP && ft != 0xFFFFFFFFu)) ? H(u) : 0u;
             if (st_g(su) != gu || u == P.t) continue;
             if ((uint64_t)gu + hu >= ft) {
                 // keep mode: stays open beyond f(t)
-                if (P.keep && sub == 0) to_far((uint32_t)u, gu, sat_add(gu, hu));
+                if (KEEP && sub == 0) to_far((uint32_t)u, gu, sat_add(gu, hu));
                 continue;
             }
             if (sub == 0) {
@@ -666,7 +690,7 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                     bool inst = false, first = false;
                     const int rb = row_begin(G.off, G.oend, v), re = row_end(G.off, G.oend, v);
                     uint32_t hv;
-                    if (!P.keep && a.y != 0) {
+                    if (!KEEP && a.y != 0) {
                         // one atomic per arc (the asynchronous engine's latency
                         // form: over a positive arc a tie may swap the parent
                         // for an equal-cost one)
@@ -676,7 +700,7 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                     } else {
                         c0 = __ldcg(B.state + v);
                         hv = H(v);
-                        if (P.keep ? hv < INF_G : (uint64_t)ng + hv < ft) {
+                        if (KEEP ? hv < INF_G : (uint64_t)ng + hv < ft) {
                             while (ng < st_g(c0)) {
                                 const uint64_t got = atomicCAS(B.state + v, c0, nv);
                                 if (got == c0) {
@@ -697,7 +721,7 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                             if (p < cap) nxt[p] = make_uint4((uint32_t)v, ng, (uint32_t)rb, (uint32_t)re);
                             else if (p < B.cap_q) qcur[p] = make_uint2((uint32_t)v, ng);  // past shared memory
                             else atomicOr(&ctl->status, ST_OVERFLOW);
-                        } else if (P.keep || fv < ft) {
+                        } else if (KEEP || fv < ft) {
                             n_rel++;
                             to_far((uint32_t)v, ng, fv >= 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)fv);
                         }
@@ -739,12 +763,17 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
 }
 
 // One A* run on one slot, executed collectively by every thread of `grp`.
+// KEEP: keep mode, every generated node stays open (no f(t) pruning), so that
+// the state can be resumed after graph updates.  It is a template argument:
+// as a word of P its code beside the plain mode's cost a maze query 4%
+// (1.73 -> 1.80 ms).
 // Precondition: slot state is all-ones (unreached) for every node.
-template <class Grp, class Heur>
+template <bool KEEP = false, class Grp, class Heur>
 __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const SlotBufs &B,
                                    const Heur &H, const SearchParams &P, WarpRows *wrows) {
     SearchCtl *ctl = B.ctl;
     const int lane = lane_id();
+    const bool resume = KEEP && P.resume;
     WarpRows &wr = wrows[threadIdx.x >> 5];
     const bool has_diff = G.doff != nullptr;
     // words every thread needs after a barrier, read by one thread per CTA
@@ -765,7 +794,7 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
         ctl->iters = 0;
         ctl->expanded = ctl->scanned = ctl->relaxed = 0;
         ctl->far_scanned = 0;
-        if (!P.resume) {
+        if (!resume) {
             ctl->cold_n = 0;
             ctl->touched = 1;
             B.state[P.s] = st_make(0, -1);
@@ -773,22 +802,22 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
             B.q0[0] = make_uint2((uint32_t)P.s, 0u);
         }
     }
-    const int64_t far_resume = P.resume ? (int64_t)(*(volatile int *)&ctl->far_n) : 0;
-    const bool far_in_f1 = P.resume && (*(volatile int *)&ctl->far_sel) != 0;
+    const int64_t far_resume = resume ? (int64_t)(*(volatile int *)&ctl->far_n) : 0;
+    const bool far_in_f1 = resume && (*(volatile int *)&ctl->far_sel) != 0;
     // cold tier (keep mode, resumed), as the last search left it
-    int64_t ncold = P.resume && P.cold ? min((int64_t)*(volatile int *)&ctl->cold_n, P.cold_cap) : 0;
+    int64_t ncold = resume && P.cold ? min((int64_t)*(volatile int *)&ctl->cold_n, P.cold_cap) : 0;
     uint32_t cold_x = ncold > 0 ? *(volatile unsigned int *)&ctl->cold_x : 0xFFFFFFFFu;
     auto read_tg = [&]() -> uint32_t { return P.t >= 0 ? st_g(__ldcg(B.state + P.t)) : 0xFFFFFFFFu; };
     grp.sync_fetch([&] { pc.tg = read_tg(); });
 
     uint2 *qcur = B.q0, *qnxt = B.q1;
     uint4 *fcur = far_in_f1 ? B.f1 : B.f0, *falt = far_in_f1 ? B.f0 : B.f1;
-    int64_t nnear = P.resume ? 0 : 1, head = 0, nnext = 0, nfar = far_resume;
+    int64_t nnear = resume ? 0 : 1, head = 0, nnext = 0, nfar = far_resume;
     const uint32_t hs = H(P.s);
     uint32_t T = sat_add(hs, P.delta);
     uint32_t Tsplit = T;
-    bool splitting = P.resume != 0;
-    if (P.resume) {
+    bool splitting = resume;
+    if (resume) {
         T = 0;
         Tsplit = 0;  // the first split only measures the far pile's minimum f
     }
@@ -810,21 +839,21 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
     // entries to the tier when the pile is more than CTA 0 can split, and is
     // CTA 0's otherwise
     bool cold_take = false, cold_pass = false;
-    if (P.resume && P.keep && P.cold) {
+    if (resume && P.cold) {
         cold_take = ncold > 0 && ncold + nfar > B.cap_f / 2;
         if (!cold_take && nfar > LOCAL_FAR) {
             if (ncold == 0) cold_x = P.cold_x;
             cold_pass = cold_x != 0xFFFFFFFFu;
         }
     }
-    if (P.resume && !cold_take && !cold_pass && local_ok && nfar <= LOCAL_FAR) splitting = false;
+    if (resume && !cold_take && !cold_pass && local_ok && nfar <= LOCAL_FAR) splitting = false;
     uint2 *cold_stage = reinterpret_cast<uint2 *>(wr.snr);
 
     for (;;) {
         if constexpr (Grp::multi) {
             if (!splitting && head == 0 && nnext == 0 && local_ok && nnear <= LOCAL_IN && nfar <= B.cap_f / 2) {
                 if (grp.first_cta())
-                    local_phases(G, B, H, P, wrows, qcur, (int)nnear, fcur, falt, nfar, T, ht,
+                    local_phases<KEEP>(G, B, H, P, wrows, qcur, (int)nnear, fcur, falt, nfar, T, ht,
                                  ncold > 0 ? cold_x : 0xFFFFFFFFu, n_exp, n_scan, n_rel);
                 grp.sync_fetch([&] {
                     pc.loc_near = *(volatile int *)&ctl->loc_near;
@@ -889,7 +918,7 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
                     // (relaxations, split and compaction moves alike; T only
                     // grows), so while f(t) >= T the pop test f < f(t)
                     // passes without reading h again; keep mode re-derives it
-                    const uint32_t hu = (ft < T || (P.keep && ft != 0xFFFFFFFFu)) ? H(u) : 0u;
+                    const uint32_t hu = (ft < T || (KEEP && ft != 0xFFFFFFFFu)) ? H(u) : 0u;
                     const int r0 = row_begin(G.off, G.oend, u), r1 = row_end(G.off, G.oend, u);
                     int d0 = 0, d1 = 0;
                     if (has_diff) {
@@ -903,7 +932,7 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
                             drb = d0;
                             deg = bdeg + (d1 - d0);
                             n_exp++;
-                        } else if (P.keep) {
+                        } else if (KEEP) {
                             requeue = true;  // stays open beyond f(t)
                         }
                     }
@@ -956,7 +985,7 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
                     }
 #pragma unroll
                     for (int r = 0; r < ARCS; r++) {
-                        go[r] = live[r] && (P.keep ? hv[r] < INF_G : (uint64_t)ng[r] + hv[r] < ft);
+                        go[r] = live[r] && (KEEP ? hv[r] < INF_G : (uint64_t)ng[r] + hv[r] < ft);
                         prev[r] = go[r] ? atomicCAS(B.state + v[r], sv[r], st_make(ng[r], wr.u[o[r]])) : sv[r];
                     }
 #pragma unroll
@@ -998,7 +1027,7 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
             // have changed since the push) and compaction (which must drop
             // stale entries) re-check the state and h.
             const uint32_t thr = compacting ? T : Tsplit;
-            const bool recheck = P.keep || compacting;
+            const bool recheck = KEEP || compacting;
             // cold tier: added to here (first split of a resumed search), or
             // scanned with the pile once min(f(t), threshold) passes cold_x
             const bool to_cold = cold_pass && !compacting;
@@ -1036,7 +1065,7 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
                     if (live) {
                         if (f < ft && f < thr) {
                             to_near = true;
-                        } else if (f < ft || (P.keep && f < INF_G)) {
+                        } else if (f < ft || (KEEP && f < INF_G)) {
                             keep = true;
                             local_min = min(local_min, (uint32_t)f);
                         }

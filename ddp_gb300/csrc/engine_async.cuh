@@ -18,8 +18,7 @@
 //     clears it after reading, so the ring is clean for the next bucket.
 // Between buckets the CTA synchronises once and splits the far pile at the
 // next threshold exactly as run_search does.  Stale entries (g changed since
-// the push) and entries with f >= f(t) are dropped; keep mode retains them in
-// the far pile, as in run_search.
+// the push) and entries with f >= f(t) are dropped.
 #pragma once
 
 #include "engine.cuh"
@@ -81,27 +80,22 @@ __device__ SearchResult run_search_cta(const DevGraph &G, const SlotBufs &B, con
         sq->alt_cnt = 0;
         sq->minf = 0xFFFFFFFFu;
         sq->status = 0;
-        if (!P.resume) {
-            ctl->touched = 1;
-            B.state[P.s] = st_make(0, -1);
-            B.touched[0] = P.s;
-            ring[0] = make_uint2((uint32_t)P.s, 0u);
-            sq->tail = 1;
-            sq->pending = 1;
-        }
+        ctl->touched = 1;
+        B.state[P.s] = st_make(0, -1);
+        B.touched[0] = P.s;
+        ring[0] = make_uint2((uint32_t)P.s, 0u);
+        sq->tail = 1;
+        sq->pending = 1;
         sq->tg = P.t >= 0 ? (unsigned int)st_g(__ldcg(B.state + P.t)) : 0xFFFFFFFFu;
     }
-    const int64_t far_resume = P.resume ? (int64_t)(*(volatile int *)&ctl->far_n) : 0;
-    const bool far_in_f1 = P.resume && (*(volatile int *)&ctl->far_sel) != 0;
     __syncthreads();
 
-    uint4 *fcur = far_in_f1 ? B.f1 : B.f0, *falt = far_in_f1 ? B.f0 : B.f1;
-    int64_t nfar = far_resume;
+    uint4 *fcur = B.f0, *falt = B.f1;
+    int64_t nfar = 0;
     const uint32_t ht = P.t >= 0 ? H(P.t) : 0u;
     uint32_t T = sat_add(H(P.s), P.delta);
     uint32_t Tsplit = T;
-    bool do_expand = !P.resume;
-    if (P.resume) T = Tsplit = 0;
+    bool do_expand = true;
     unsigned long long n_exp = 0, n_scan = 0, n_rel = 0;
     int phases = 0;
     const int64_t max_phases = 4 * (int64_t)G.n + (1 << 22);
@@ -171,7 +165,6 @@ __device__ SearchResult run_search_cta(const DevGraph &G, const SlotBufs &B, con
                 // 2. entry stage (as run_search)
                 int u = -1, rb = 0, deg = 0;
                 uint32_t gu = 0;
-                bool requeue = false;
                 if (lane < n && en.x != RING_EMPTY) {
                     u = (int)en.x;
                     gu = en.y;
@@ -185,9 +178,8 @@ __device__ SearchResult run_search_cta(const DevGraph &G, const SlotBufs &B, con
                     // every entry of the current bucket was pushed with
                     // f = g + h(u) < T (near pushes, split moves and the
                     // source alike; T only grows), so while f(t) >= T the pop
-                    // test f < f(t) passes without reading h again; keep mode
-                    // re-derives it
-                    const uint32_t hu = (ft < T || (P.keep && ft != 0xFFFFFFFFu)) ? H(u) : 0u;
+                    // test f < f(t) passes without reading h again
+                    const uint32_t hu = ft < T ? H(u) : 0u;
                     const int r0 = have ? pre.x : row_begin(G.off, G.oend, u);
                     const int r1 = have ? pre.y : row_end(G.off, G.oend, u);
                     if (st_g(su) == gu && u != P.t) {
@@ -195,13 +187,9 @@ __device__ SearchResult run_search_cta(const DevGraph &G, const SlotBufs &B, con
                             rb = r0;
                             deg = r1 - r0;
                             n_exp++;
-                        } else if (P.keep) {
-                            requeue = true;
                         }
                     }
                 }
-                stage_push(requeue, make_uint4((uint32_t)u, gu, 0u, 0u), wr.sf, c_f, &sq->far_cnt,  // keep mode: f re-derived
-                           fcur, nfar, B.cap_f, ctl, 0);
                 int total;
                 const int ex = warp_excl_scan(deg, &total);
                 wr.excl[lane] = ex;
@@ -249,7 +237,7 @@ __device__ SearchResult run_search_cta(const DevGraph &G, const SlotBufs &B, con
                     }
                     int2 rows[AA];
                     bool fresh[AA];  // latency mode: the atomic found v unreached
-                    if (!P.keep && latency) {
+                    if (latency) {
                         // one atomic per arc: over a positive-weight arc,
                         // atomicMin on (g << 32 | parent) installs a smaller g
                         // (or, at equal g, a smaller parent id: an equal-cost
@@ -307,7 +295,7 @@ __device__ SearchResult run_search_cta(const DevGraph &G, const SlotBufs &B, con
                         bool to_near = false, to_far = false, first = false;
                         const uint64_t fv = (uint64_t)ng[r] + hv[r];
                         const uint32_t fpush = fv >= 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)fv;
-                        if (!P.keep && latency) {
+                        if (latency) {
                             // the atomic already installed g: log a first touch even
                             // when f >= f(t) prunes the push
                             if (live[r]) {
@@ -318,7 +306,7 @@ __device__ SearchResult run_search_cta(const DevGraph &G, const SlotBufs &B, con
                                     else to_far = true;
                                 }
                             }
-                        } else if (live[r] && (P.keep ? hv[r] < INF_G : fv < ft)) {
+                        } else if (live[r] && fv < ft) {
                             const uint64_t nv = st_make(ng[r], wr.u[o[r]]);
                             uint64_t c0 = cur[r];
                             for (;;) {
@@ -418,23 +406,13 @@ __device__ SearchResult run_search_cta(const DevGraph &G, const SlotBufs &B, con
                 uint4 en = make_uint4(0u, 0u, 0u, 0u);
                 if (idx < nfar) {
                     // entries carry f from their push (no node state read:
-                    // stale entries are dropped when popped); keep mode
-                    // re-checks, since h may have changed since the push
+                    // stale entries are dropped when popped)
                     en = __ldcg(fcur + idx);
-                    bool live = true;
-                    uint64_t f = en.z;
-                    if (P.keep) {
-                        live = st_g(__ldcg(B.state + en.x)) == en.y;
-                        f = (uint64_t)en.y + H((int)en.x);
-                        en.z = f >= 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)f;
-                    }
-                    if (live) {
-                        if (f < ft && f < Tsplit) {
-                            to_near = true;
-                        } else if (f < ft || (P.keep && f < INF_G)) {
-                            keep = true;
-                            local_min = min(local_min, (uint32_t)f);
-                        }
+                    if (en.z < ft && en.z < Tsplit) {
+                        to_near = true;
+                    } else if (en.z < ft) {
+                        keep = true;
+                        local_min = min(local_min, en.z);
                     }
                 }
                 // split output goes to ring positions [0, m): the ring is
@@ -492,11 +470,7 @@ __device__ SearchResult run_search_cta(const DevGraph &G, const SlotBufs &B, con
         if (n_exp) atomicAdd(&ctl->expanded, n_exp);
         if (n_rel) atomicAdd(&ctl->relaxed, n_rel);
     }
-    if (threadIdx.x == 0) {
-        ctl->far_n = (int)nfar;
-        ctl->far_sel = fcur == B.f1 ? 1 : 0;
-        ctl->iters = phases;
-    }
+    if (threadIdx.x == 0) ctl->iters = phases;
     __syncthreads();
     SearchResult r;
     const uint64_t st_t = P.t >= 0 ? __ldcg(B.state + P.t) : ~0ull;

@@ -507,7 +507,7 @@ __device__ __forceinline__ void batch_loop(const Grp &grp, const DevGraph &G0, c
             grp.sync();
             continue;
         }
-        SearchParams P{s, t, A.delta, A.K, 0, 0, 0};
+        SearchParams P{s, t, A.delta, A.K, 0, 0};
         SearchResult r;
         if (HK == 1) {
             const uint32_t tag = *(volatile uint32_t *)&ctl->tag;
@@ -1277,7 +1277,7 @@ static int sssp_into(ddp_graph *g, int32_t src, bool reverse, int32_t *dist) {
         std::swap(G.doff, G.droff);
         std::swap(G.darc, G.drarc);
     }
-    SearchParams P{src, -1, auto_delta(g), 0, 0, 0, 0};
+    SearchParams P{src, -1, auto_delta(g), 0, 0, 0};
     int64_t cap = (int64_t)g->n + 1024;
     for (int attempt = 0; attempt < 4; attempt++) {
         int rc = workspace_ensure(g, cap);
@@ -1454,7 +1454,7 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
     int64_t cap = o.queue_cap > 0 ? o.queue_cap : (int64_t)g->n + 1024;
     const uint32_t delta = o.delta > 0 ? (uint32_t)o.delta : auto_delta(g);
     DevGraph G = graph_view(g);
-    SearchParams P{source, target, delta, o.K, 0, 0, 0};
+    SearchParams P{source, target, delta, o.K, 0, 0};
     const int kind = h ? h->kind : DDP_H_ZERO;
     // reads what a kernel left in w->h_res; path ids past the host's part come from the device
     auto result = [&](Workspace *w) -> int {

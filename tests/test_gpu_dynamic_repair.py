@@ -83,3 +83,19 @@ def test_repair_hands_over_and_cold_tier(gpu, oracle, heur, group):
     for _ in range(3):
         apply([(1, int(rng.integers(n)), int(rng.integers(n)), int(rng.integers(1, 1001)))])
     dyn.close()
+
+
+@pytest.mark.parametrize("length", [1, 2, 4096, 4097, 6000])
+def test_dynamic_paths_around_the_host_buffer(gpu, length):
+    """A chain: the path has exactly `length` nodes, before and after a batch
+    that changes the weight of its first arc (or of one beside it)."""
+    d = gpu
+    n = 6001
+    e = np.arange(n - 1, dtype=np.int32)
+    g = d.CSR(n, np.concatenate([e, [n - 1, n - 1]]).astype(np.int32), e + 1, np.full(n - 1, 2, np.uint32))
+    dg = d.DeviceGraph.from_csr(g)
+    dyn = d.DynamicSearch(dg, 0, length - 1, d.H_ZERO)
+    assert np.array_equal(dyn.path(), np.arange(length)) and dyn.cost == 2 * (length - 1)
+    assert dyn.update(*_batch([(2, 0, 1, 7)])) == (2 * (length - 1) + 5 if length > 1 else 0)
+    assert np.array_equal(dyn.path(), np.arange(length))
+    dyn.close()
