@@ -429,6 +429,7 @@ __device__ __forceinline__ void batch_loop(const Grp &grp, const DevGraph &G0, c
                 }
             } else {
                 q = atomicAdd(A.work, 1);
+                if (A.order && q < A.nq) q = __ldcg(A.order + q);
             }
             ctl->cur_q = q;
             ctl->status = 0;
@@ -793,7 +794,7 @@ __device__ void service_loop(const BatchArgs &A) {
 
 // Bidirectional instances are compiled for 64 registers (1,024 threads on an
 // SM in any split): a launch picks 1,024, 512 or 256 threads per query
-// (batch_shape).
+// (batch_grid).
 // One-CTA slots.  The group form below is a kernel of its own: both engines
 // in one kernel share a register budget, and the one that a launch does not
 // use makes the other spill (landmark instance: 736 bytes of spill stores
@@ -817,6 +818,41 @@ __global__ void __launch_bounds__(bidir_hk(HK) ? 1024 : 512, bidir_hk(HK) ? 1 : 
         __shared__ CtaQ sq;
         batch_loop<HK, true, SERVE>(grp, G, B, A, sa.epoch + blockIdx.x, wrows, &sq, nullptr);
     }
+}
+
+// The claim order of a batch on a graph with coordinates: longest first, by
+// the distance between a query's end points.  What a search opens grows with
+// its square, and a long one claimed last runs on alone: pairs on 1M points,
+// 200 take 26.0 -> 23.1 ms, 700 69.6 -> 49.8, 1,500 129 -> 94.6; 1,000 on 5k
+// points 0.82 -> 0.62 ms, the smallest gain 4,096 on 5k: 2.17 -> 1.96.  The
+// landmarks' bound says too little of a search's work to rank by: 2,000
+// queries on 400k nodes 3.27 -> 3.56 ms.
+// A thread ranks one query among all (ties by index), a tile of distances at
+// a time; ends outside the graph count as 0 (the search refuses them).
+constexpr int ORDER_MAX = 8192;  // past it the last round is a small part
+__global__ void __launch_bounds__(256) k_order(const int32_t *S, const int32_t *T, const int32_t *xy, int32_t n,
+                                               int nq, int32_t *order) {
+    __shared__ float tile[256];
+    auto dist = [&](int q) -> float {
+        const int s = q < nq ? __ldg(S + q) : -1, t = q < nq ? __ldg(T + q) : -1;
+        if (s < 0 || s >= n || t < 0 || t >= n) return 0.f;
+        const int2 a = __ldg(reinterpret_cast<const int2 *>(xy) + s), b = __ldg(reinterpret_cast<const int2 *>(xy) + t);
+        const float dx = (float)a.x - (float)b.x, dy = (float)a.y - (float)b.y;
+        return dx * dx + dy * dy;
+    };
+    const int me = blockIdx.x * 256 + threadIdx.x;
+    const float d = dist(me);
+    int rank = 0;
+    for (int t0 = 0; t0 < nq; t0 += 256) {
+        __syncthreads();
+        tile[threadIdx.x] = dist(t0 + threadIdx.x);
+        __syncthreads();
+        for (int j = 0; j < min(256, nq - t0); j++) {
+            const float e = tile[j];
+            rank += e > d || (e == d && t0 + j < me);
+        }
+    }
+    if (me < nq) order[rank] = me;
 }
 
 // Slots of A.group CTAs each (cooperative launch), and one-CTA slots on the
@@ -1615,6 +1651,7 @@ struct ddp_batch {
     int32_t *d_qstatus = nullptr;
     long long *d_stats = nullptr, *d_t0 = nullptr, *d_t1 = nullptr;
     int *d_work = nullptr, *d_status = nullptr;
+    int32_t *d_order = nullptr;
     int32_t path_cap = 0;
     int32_t last_n = 0;
     int32_t launches = 0;
@@ -1650,6 +1687,7 @@ static int batch_grow(ddp_batch *b, int32_t n) {
     cudaFree(b->d_stats);
     cudaFree(b->d_t0);
     cudaFree(b->d_t1);
+    cudaFree(b->d_order);
     const size_t N = (size_t)n;
     DDP_CUDA(cudaMalloc(&b->d_S, sizeof(int32_t) * N));
     DDP_CUDA(cudaMalloc(&b->d_T, sizeof(int32_t) * N));
@@ -1660,8 +1698,28 @@ static int batch_grow(ddp_batch *b, int32_t n) {
     DDP_CUDA(cudaMalloc(&b->d_stats, sizeof(long long) * DDP_STATS * N));
     DDP_CUDA(cudaMalloc(&b->d_t0, sizeof(long long) * N));
     DDP_CUDA(cudaMalloc(&b->d_t1, sizeof(long long) * N));
+    DDP_CUDA(cudaMalloc(&b->d_order, sizeof(int32_t) * N));
     b->cap_q_n = n;
     return DDP_OK;
+}
+
+// Whether k_order ranks a batch of n queries (if there are more than slots).
+static bool batch_ranked(const ddp_batch *b, const DevGraph &G, int32_t n) {
+    return bidir_hk(b->hk) && G.xy && n <= ORDER_MAX;
+}
+
+// CTAs of a launch of n queries and the threads of one.  A ranked batch holds
+// on to wide CTAs longer, since its second round is its short queries: 300
+// pairs on 1M points take 23.5 ms on 1,024 threads, 38.9 ms on 512 (50k
+// points: 1.92, 2.59), 600 pairs on 50k points 3.63 and 2.65 ms.
+static int batch_grid(const ddp_batch *b, const DevGraph &G, int32_t n, int *block) {
+    *block = b->block;
+    const int grid = b->sa.nslots * b->group;
+    if (!bidir_hk(b->hk) || b->o.block > 0) return grid;
+    const int sms = device_sms();
+    const int wide = batch_ranked(b, G, n) ? 5 * sms / 2 : sms + sms / 2;
+    *block = n <= wide ? 1024 : n <= 6 * sms ? 512 : 256;
+    return std::min({grid, 1024 / *block * sms, std::max(n, 1)});
 }
 
 // Kernel arguments of one batch launch.  Returns false when the landmark
@@ -1690,15 +1748,10 @@ static bool batch_args(ddp_batch *b, int32_t n, const int32_t *dS, const int32_t
     A.group = b->group;
     A.sync_engine = (b->o.flags & DDP_OPT_SYNC) != 0;
     *G = graph_view(b->g);
+    // with more queries than slots the order counts
+    int block = 0;
+    if (batch_ranked(b, *G, n) && n > batch_grid(b, *G, n, &block)) A.order = b->d_order;
     return !(b->hkind == DDP_H_LANDMARK && !G->lm);
-}
-
-// Threads per bidirectional query of a launch of n queries; returns the CTAs
-// per SM.
-static int batch_shape(int32_t n, int *block) {
-    const int sms = device_sms();
-    *block = n <= sms + sms / 2 ? 1024 : n <= 6 * sms ? 512 : 256;
-    return 1024 / *block;
 }
 
 static cudaError_t batch_launch_args(ddp_batch *b, DevGraph G, BatchArgs A) {
@@ -1707,10 +1760,12 @@ static cudaError_t batch_launch_args(ddp_batch *b, DevGraph G, BatchArgs A) {
     // fresh control blocks (barrier counters included) for every launch
     e = cudaMemsetAsync(b->sa.ctl, 0, sizeof(SearchCtl) * (size_t)b->sa.nslots, b->stream);
     if (e != cudaSuccess) return e;
-    int block = b->block, grid = b->sa.nslots * b->group;
-    if (bidir_hk(b->hk) && b->o.block <= 0) {
-        const int per_sm = batch_shape(A.nq, &block);
-        grid = std::min({grid, per_sm * device_sms(), std::max(A.nq, 1)});
+    int block = 0;
+    const int grid = batch_grid(b, G, A.nq, &block);
+    if (A.order) {
+        k_order<<<(A.nq + 255) / 256, 256, 0, b->stream>>>(A.S, A.T, G.xy, G.n, A.nq, A.order);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
     }
     SlotArrays sa = b->sa;
     void *args[] = {&G, &sa, &A};
@@ -1733,7 +1788,7 @@ static bool same_view(const DevGraph &x, const DevGraph &y) {
 static bool same_args(const BatchArgs &x, const BatchArgs &y) {
     return x.S == y.S && x.T == y.T && x.nq == y.nq && x.cost == y.cost && x.plen == y.plen &&
            x.paths == y.paths && x.path_cap == y.path_cap && x.qstatus == y.qstatus && x.stats == y.stats &&
-           x.tstart == y.tstart && x.tend == y.tend && x.work == y.work && x.status == y.status &&
+           x.tstart == y.tstart && x.tend == y.tend && x.work == y.work && x.status == y.status && x.order == y.order &&
            x.delta == y.delta && x.K == y.K && x.bfs_budget == y.bfs_budget && x.lazy_budget == y.lazy_budget &&
            x.eager_delta == y.eager_delta && x.group == y.group &&
            x.sync_engine == y.sync_engine;
@@ -2023,6 +2078,7 @@ int ddp_batch_free(ddp_batch *b) {
     cudaFree(b->d_t0);
     cudaFree(b->d_t1);
     cudaFree(b->d_work);
+    cudaFree(b->d_order);
     if (b->stream && !b->o.stream) cudaStreamDestroy(b->stream);
     graph_unref(b->g);
     delete b;

@@ -56,6 +56,7 @@ struct BatchArgs {
     int32_t *qstatus;
     long long *stats, *tstart, *tend;
     int *work, *status;
+    int32_t *order;  // non-null: the queries in the order they are claimed (k_order)
     uint32_t delta;
     int32_t K;
     int64_t bfs_budget;  // capped heuristic BFS (0 = run to completion)
