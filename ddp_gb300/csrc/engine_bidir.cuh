@@ -124,6 +124,7 @@ struct WaveQ {
     int status;
     int touched;
     long long spent;                 // entries expanded or dropped
+    unsigned long long edge_mul;     // 2^64 / (2^32 / bucket width)
     uint32_t settled[2][WAVE_FILTER];  // lazy labels: filter over settled nodes
     uint4 list[2][WAVE_NEAR];
 };
@@ -569,8 +570,16 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
     // key and that edge(b) is the smallest key of bucket b)
     const uint32_t rec_dk = dk <= 1 ? NONE : (uint32_t)(0x100000000ull / dk);
     auto bucket = [&](uint32_t key) -> uint32_t { return __umulhi(key, rec_dk); };
+    // ceil(b 2^32 / rec_dk): two multiplications by 2^64 / rec_dk come out at
+    // most a few below it.  With a 64-bit division here, four in each plan,
+    // the CTA waited about a microsecond longer for every wave: 16 maze pairs
+    // 26.2 -> 22.3 ms, 200 pairs on 1M points 23.2 -> 22.0, 4,096 on 4M nodes
+    // 3.69 -> 3.59, 500 landmark queries 1.47 -> 1.37.
+    if (threadIdx.x == 0) q->edge_mul = ~0ull / rec_dk;
     auto edge = [&](uint32_t b) -> uint32_t {
-        const uint64_t k = (((uint64_t)b << 32) + rec_dk - 1) / rec_dk;
+        const unsigned long long M = q->edge_mul;
+        uint64_t k = (uint64_t)b * (uint32_t)(M >> 32) + (((uint64_t)b * (uint32_t)M) >> 32);
+        while (k < NONE && bucket((uint32_t)k) < b) k++;
         return k >= NONE ? NONE : (uint32_t)k;
     };
 
@@ -991,14 +1000,8 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
             } else {
                 // open the next bucket of the direction(s) whose open set is
                 // not much larger than the other's
-                int o0 = x0, o1 = x1;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    o0 += __shfl_xor_sync(FULL, o0, o);
-                    o1 += __shfl_xor_sync(FULL, o1, o);
-                }
-                o0 += pd0;
-                o1 += pd1;
+                const int o0 = (int)__reduce_add_sync(FULL, (unsigned)x0) + pd0;
+                const int o1 = (int)__reduce_add_sync(FULL, (unsigned)x1) + pd1;
                 if (nb0 != NONE && ((int64_t)o0 <= 2 * (int64_t)o1 + 64 || nb1 == NONE) &&
                     (k0 == NONE || nb0 - bucket(k0) <= ahead)) {
                     p.c[0] = nb0;
