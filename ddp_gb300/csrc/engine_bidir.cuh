@@ -962,78 +962,75 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
         __syncthreads();  // the last wave's pushes are in place
         if (threadIdx.x < 32) {
             // ---- plan the next wave ------------------------------------------
-            WavePlan p;
+            // even lanes decide for the forward direction, odd lanes for the
+            // backward one: the CTA waits, and an instruction that comes by
+            // once a wave costs several cycles to fetch
+            const uint32_t dir = lane & 1;
             const int cur = wv % 3;
-            p.m = min(q->near[cur], WAVE_NEAR + scap);
-            p.c[0] = q->plan.c[0];
-            p.c[1] = q->plan.c[1];
+            const int m = min(q->near[cur], WAVE_NEAR + scap);
             // the buckets opened are no longer in the window
-            p.lo[0] = p.c[0] + 1;
-            p.lo[1] = p.c[1] + 1;
-            p.n[0] = p.n[1] = 0;
-            p.act = 0;
-            const int x0 = min(q->lcnt[0][(p.lo[0] + lane) & (WAVE_LISTS - 1)], room);
-            const int x1 = min(q->lcnt[1][(p.lo[1] + lane) & (WAVE_LISTS - 1)], room);
+            const uint32_t b0 = q->plan.c[0] + 1, b1 = q->plan.c[1] + 1;
+            uint32_t lo = dir ? b1 : b0, c = lo - 1;
+            int n = 0, act = 0;
+            const int x0 = min(q->lcnt[0][(b0 + lane) & (WAVE_LISTS - 1)], room);
+            const int x1 = min(q->lcnt[1][(b1 + lane) & (WAVE_LISTS - 1)], room);
             const unsigned m0 = __ballot_sync(FULL, x0 > 0), m1 = __ballot_sync(FULL, x1 > 0);
-            const int pd0 = q->pile_dir[0], pd1 = q->pile_dir[1];
-            const uint32_t nb0 = m0 ? p.lo[0] + (uint32_t)__ffs(m0) - 1u : NONE;
-            const uint32_t nb1 = m1 ? p.lo[1] + (uint32_t)__ffs(m1) - 1u : NONE;
-            const uint32_t pm0 = pd0 ? q->pile_min[0] : NONE, pm1 = pd1 ? q->pile_min[1] : NONE;
-            const uint32_t k0 = q->near_min[cur][0], k1 = q->near_min[cur][1];
-            const uint32_t e0 = nb0 == NONE ? NONE : edge(nb0), e1 = nb1 == NONE ? NONE : edge(nb1);
-            p.lb[0] = min(min(k0, pm0), e0);
-            p.lb[1] = min(min(k1, pm1), e1);
+            const int first = __ffs(dir ? m1 : m0) - 1;
+            const int pd = q->pile_dir[dir];
+            const uint32_t nb = first >= 0 ? lo + (uint32_t)first : NONE;
+            const uint32_t pm = pd ? q->pile_min[dir] : NONE;
+            const uint32_t k = q->near_min[cur][dir];
+            const uint32_t e = nb == NONE ? NONE : edge(nb);
+            const uint32_t lb = min(min(k, pm), e), lbo = __shfl_xor_sync(FULL, lb, 1);
+            const bool piled = __any_sync(FULL, pm < e);
             // an empty direction, or nothing open that could be shorter: mu is the distance
-            if (p.lb[0] == NONE || p.lb[1] == NONE ||
-                (uint64_t)p.lb[0] + p.lb[1] >= bi_key_bound<Pot>(mu_now()) + slack2 || q->status) {
-                p.act = 1;
-            } else if (p.m >= WAVE_FILL) {
+            if (lb == NONE || lbo == NONE || (uint64_t)lb + lbo >= bi_key_bound<Pot>(mu_now()) + slack2 || q->status) {
+                act = 1;
+            } else if (m >= WAVE_FILL) {
                 // enough to do
-            } else if (pm0 < e0 || pm1 < e1) {
+            } else if (piled) {
                 // the pile holds a direction's smallest bucket (a bucket whose
                 // list was full leaves the rest there)
-                p.act = 2;
-                if (nb0 == NONE && pd0 && pm0 >= edge(p.lo[0])) p.lo[0] = bucket(pm0);  // nothing listed below
-                if (nb1 == NONE && pd1 && pm1 >= edge(p.lo[1])) p.lo[1] = bucket(pm1);
-                p.c[0] = p.lo[0] - 1;
-                p.c[1] = p.lo[1] - 1;
+                act = 2;
+                if (nb == NONE && pd && pm >= edge(lo)) lo = bucket(pm);  // nothing listed below
+                c = lo - 1;
             } else {
                 // open the next bucket of the direction(s) whose open set is
                 // not much larger than the other's
-                const int o0 = (int)__reduce_add_sync(FULL, (unsigned)x0) + pd0;
-                const int o1 = (int)__reduce_add_sync(FULL, (unsigned)x1) + pd1;
-                if (nb0 != NONE && ((int64_t)o0 <= 2 * (int64_t)o1 + 64 || nb1 == NONE) &&
-                    (k0 == NONE || nb0 - bucket(k0) <= ahead)) {
-                    p.c[0] = nb0;
-                    p.n[0] = __shfl_sync(FULL, x0, __ffs(m0) - 1);
-                    p.lo[0] = nb0;
-                }
-                if (nb1 != NONE && ((int64_t)o1 <= 2 * (int64_t)o0 + 64 || nb0 == NONE) &&
-                    (k1 == NONE || nb1 - bucket(k1) <= ahead)) {
-                    p.c[1] = nb1;
-                    p.n[1] = __shfl_sync(FULL, x1, __ffs(m1) - 1);
-                    p.lo[1] = nb1;
+                const int o0 = (int)__reduce_add_sync(FULL, (unsigned)x0), o1 = (int)__reduce_add_sync(FULL, (unsigned)x1);
+                const int o = (dir ? o1 : o0) + pd, oo = __shfl_xor_sync(FULL, o, 1);
+                const uint32_t nbo = __shfl_xor_sync(FULL, nb, 1);
+                const int y0 = __shfl_sync(FULL, x0, first & 31), y1 = __shfl_sync(FULL, x1, first & 31);
+                if (nb != NONE && ((int64_t)o <= 2 * (int64_t)oo + 64 || nbo == NONE) &&
+                    (k == NONE || nb - bucket(k) <= ahead)) {
+                    c = lo = nb;
+                    n = dir ? y1 : y0;
                 }
             }
-            p.lim[0] = edge(p.c[0] + 1);
-            p.lim[1] = edge(p.c[1] + 1);
-            __syncwarp();
-            if (lane == 0) {
+            const int nn = (wv + 2) % 3;  // the counters of the wave after the next
+            if (lane < 2) {
+                q->plan.c[dir] = c;
+                q->plan.lo[dir] = lo;
+                q->plan.lb[dir] = lb;
+                q->plan.lim[dir] = edge(c + 1);
+                q->plan.n[dir] = n;
                 // a bucket opened gives its list back after this wave: lo
                 // keeps the bucket that would reuse it out of the window
-                if (p.n[0]) q->lcnt[0][p.c[0] & (WAVE_LISTS - 1)] = 0;
-                if (p.n[1]) q->lcnt[1][p.c[1] & (WAVE_LISTS - 1)] = 0;
-                if (p.act == 0) {
-                    q->spent += p.m + p.n[0] + p.n[1];
+                if (n) q->lcnt[dir][c & (WAVE_LISTS - 1)] = 0;
+                q->near_min[nn][dir] = NONE;
+            }
+            const int n_both = n + __shfl_xor_sync(FULL, n, 1);
+            if (lane == 0) {
+                if (act == 0) {
+                    q->spent += m + n_both;
                     if (P.budget > 0 && q->spent > P.budget) {
-                        p.act = 1;
+                        act = 1;
                         q->status = ST_BUDGET;
                     }
                 }
-                const int nn = (wv + 2) % 3;  // the counters of the wave after the next
                 q->near[nn] = 0;
-                q->near_min[nn][0] = q->near_min[nn][1] = NONE;
-                q->plan = p;
+                q->plan.m = m;
+                q->plan.act = act;
             }
         }
         __syncthreads();
