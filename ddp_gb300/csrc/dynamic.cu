@@ -1131,6 +1131,7 @@ static int dyn_launch(ddp_dyn *d, int initial, int nupd, const int *dres = nullp
     DevGraph G = graph_view(g);
     SearchParams P{d->s, d->t, d->o.delta > 0 ? (uint32_t)d->o.delta : std::max(1u, (g->wmin + g->wmax) / 4),
                    d->o.K, initial ? 0 : 1, 1};
+    if (d->o.delta <= 0) P.delta_loose = loose_delta(g);
     // a resumed search leaves entries with g >= the last cost (f >= g)
     // unexamined until it needs them
     if (!initial) {

@@ -1053,6 +1053,8 @@ uint32_t auto_delta(const ddp_graph *g) {
     return d < 1 ? 1 : d;
 }
 
+uint32_t loose_delta(const ddp_graph *g) { return std::max(auto_delta(g), g->wmin / 2 + g->wmax / 2); }
+
 }  // namespace ddp
 
 using namespace ddp;
@@ -1491,6 +1493,7 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
     const uint32_t delta = o.delta > 0 ? (uint32_t)o.delta : auto_delta(g);
     DevGraph G = graph_view(g);
     SearchParams P{source, target, delta, o.K, 0, 0};
+    if (o.delta <= 0) P.delta_loose = loose_delta(g);
     const int kind = h ? h->kind : DDP_H_ZERO;
     // reads what a kernel left in w->h_res; path ids past the host's part come from the device
     auto result = [&](Workspace *w) -> int {

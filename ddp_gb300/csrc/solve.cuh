@@ -132,6 +132,7 @@ cudaError_t launch_slots(int hk, int grid, int block, bool coop, DevGraph G, Slo
 int slots_per_sm(int hk, int block, bool grouped);
 int device_sms();
 uint32_t auto_delta(const ddp_graph *g);
+uint32_t loose_delta(const ddp_graph *g);  // SearchParams::delta_loose
 uint32_t auto_delta_bidir(const ddp_graph *g);
 // Fills the bucket widths and the budget of a bidirectional launch.
 void bidir_args(const ddp_graph *g, int32_t delta, BatchArgs *A);
