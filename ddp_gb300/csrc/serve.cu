@@ -2,7 +2,7 @@
 // edge-update batches interleaved.
 //
 // No reference counterpart (the reference answers one (s,t) per process).
-// Requests are written to a ring in pinned host memory that the device reads
+// Requests are written to pinned host memory that the device reads
 // directly (cudaHostAllocMapped); publishing a request is a store of the
 // published count.  The persistent slot kernel (k_batch in serving mode) keeps
 // one search per CTA: a slot that finishes claims the next published request
@@ -14,9 +14,9 @@
 // requests keep coming.  Submit and poll relaunch the kernel when requests
 // are pending and it is not running.
 //
-// Admission by memory: every slot owns a fixed footprint (state n x 8 B,
-// touched-log n x 4 B, four queues); the number of slots is what fits in the
-// memory budget, and a request waits in the ring until a slot is free.  A
+// Admission by memory: every slot owns a fixed footprint (its records and its
+// queues or bucket lists); the number of slots is what fits in the memory
+// budget, and a request waits until a slot is free.  A
 // request whose search outgrows its slot is re-run on the single-query engine
 // (which grows its queues) when it is polled.
 //

@@ -181,8 +181,8 @@ __global__ void __launch_bounds__(512) k_bfs_single(DevGraph G, SlotArrays sa, u
 }
 
 // The end of a single query, by its first CTA: path (to the device array and,
-// as far as it fits, to the host's), result and counters.  warp: the path is
-// the caller's already (len >= 0), else it is walked here.
+// as far as it fits, to the host's), result and counters.  len >= 0: the
+// caller has written the path; else it is walked here.
 __device__ void solve_report(const DevGraph &G, const SlotBufs &B, const SearchParams &P, const SearchResult &r,
                              SolveOut *out, int32_t *path, int32_t path_cap, int32_t len, int32_t *buf, int32_t bcap) {
     const bool ok = !(*(volatile int *)&B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT | ST_BUDGET));
@@ -922,8 +922,8 @@ static int rerun_kind(int hkind) { return is_bidir_kind(hkind) ? DDP_H_ZERO : hk
 // kind); for the plain kind on graphs with coordinates, whose numbering
 // (Morton order of points) puts a search's neighbours in shared sectors,
 // 16-byte pairs (8-9 % more serving capacity on the 8M-point graph); else
-// 32-byte epoch-tagged records (the potential-steered kinds too: on the
-// 2048^2 maze they were faster, 16.4 against 17.8 ms).
+// 32-byte epoch-tagged records (pairs for all: 4,096 pairs on 4M nodes 3.41 ->
+// 3.71 ms, 16 maze pairs under potentials 17.1 -> 17.7, landmarks 1.49 -> 1.48).
 int kernel_hk(int hkind, bool has_xy, bool hash, int group, int flags) {
     if (!is_bidir_kind(hkind) && batch_bidir(hkind, group, flags)) {
         if (hkind == DDP_H_LANDMARK) return 10;
