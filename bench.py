@@ -187,11 +187,11 @@ def peak_hbm():
 # smaller case of the same kernel (the 400k-node graph of the family, 1,024
 # pairs, one slot per SM), whose state still exceeds L2; a full launch's
 # traffic is this ratio times its own algorithmic bytes.  Capture:
-#   ncu --set full --clock-control none -k regex:k_batch -s 2 -c 1 -o prof \
-#       python bench.py --config c4-small --slots 152 --no-tune --delta 8 \
-#       --steps 1 --warmup 1 --plain-sample 0 --serve-rates= --no-cpu-baseline --other-configs=
+#   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:k_batch -s 2 -c 1 \
+#       python bench.py --config c4-small --slots 152 --no-tune --delta 4 --steps 1 --warmup 1 \
+#       --plain-sample 0 --serve-rates= --no-cpu-baseline --other-configs=
 TRAFFIC_PER_ALG_BYTE = {
-    ("c4", "bidir"): (1.607848e9 + 0.625154e9) / 372759272,
+    ("c4", "bidir"): (273967360 + 73768448) / 254808776,
 }
 
 

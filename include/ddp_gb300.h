@@ -187,10 +187,11 @@ int ddp_query_free(ddp_query *q);
  * inside the batch kernel), DDP_H_MANHATTAN, DDP_H_EUCLID (coordinates),
  * DDP_H_LANDMARK (ddp_landmarks_build first) or DDP_H_BIDIR,
  * DDP_H_BIDIR_EUCLID, DDP_H_BIDIR_MANHATTAN (one-CTA slots, 32 bytes per
- * node of slot state).  opts: group = CTAs per slot
- * (1 = the asynchronous one-CTA engine), block, K, delta, grid = slot cap;
- * ddp_batch_tune picks them.  A query whose search outgrew
- * its slot's queues reports cost -1 from ddp_batch_solve_device;
+ * node of slot state).  opts: group = CTAs per slot (1: the bidirectional
+ * search, for MANHATTAN and EUCLID the asynchronous A*), block, K, delta,
+ * grid = slot cap; ddp_batch_tune picks them.  On a graph with coordinates a
+ * bidirectional batch starts its longest queries first.  A query whose
+ * search outgrew its slot's queues reports cost -1 from ddp_batch_solve_device;
  * ddp_batch_solve re-runs such queries on the single-query engine. */
 int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batch **out);
 /* Solves n queries from host arrays; out_cost[n]; out_path_len[n] optional. */
