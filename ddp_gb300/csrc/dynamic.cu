@@ -513,16 +513,20 @@ __device__ __forceinline__ CtaGroup dyn_group(CtaGroup *, const SlotBufs &B) { r
 // shared memory, the frontier with its row bounds in shared memory too) and
 // the grid waits once.  It hands over what outgrows it: a level of more than
 // DYN_LOCAL_BAIL nodes, or more than DYN_LOCAL_SEED nodes to re-seed.  A
-// team of DYN_TEAM lanes walks one row, two arcs a lane, so that a level is
+// team of up to DYN_TEAM lanes (as many as spread the level over the
+// threads) walks one row, DYN_ARCS arcs a lane, so that a level is
 // one chain of arc -> node word -> atomic, where a thread walking a row of
 // ten arcs alone ran two such chains and read the row bounds first.
 // 1M nodes, 1000-update batches (median of 100 updates in the call): 334 us
 // with these steps and the resumed search's splits on 76 CTAs (hops 28 us,
-// invalidation 70, re-seeding and relaxing 17, search 100), 154 us here.
-constexpr int DYN_LOCAL_UPD = 2048;   // updates CTA 0 takes alone
+// invalidation 70, re-seeding and relaxing 17, search 100), 154 us here.  1024 x
+// 1024 maze, batches of 2,238 changes with 17k nodes invalidated over hundreds
+// of levels: 5.0 -> 3.1 ms (6.9 with every level on the grid).
+constexpr int DYN_LOCAL_UPD = 4096;   // updates CTA 0 takes alone
 constexpr int DYN_LOCAL_BAIL = 2048;
 constexpr int DYN_LOCAL_SEED = 1024;
 constexpr int DYN_TEAM = 8;
+constexpr int DYN_ARCS = 2;
 enum { REP_HOPS, REP_HOPS_WALK, REP_TREE, REP_TREE_WALK, REP_SEED, REP_DONE };
 
 // The next step, and the frontier of a walk: nf nodes in fb.
@@ -539,7 +543,7 @@ template <bool SOLO, class Grp>
 __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B, uint32_t *hops, const DynArgs &A,
                            DynCtl *dc, int nupd, RepairAt &at, uint4 *lists, int *cnt) {
     const int rank = grp.rank(), size = grp.size();
-    const int sub = threadIdx.x & (DYN_TEAM - 1), team = rank / DYN_TEAM, teams = size / DYN_TEAM;
+    int tw = DYN_TEAM, sub = 0;  // lanes of this level's teams, this one's place
     uint4 *far_buf = (*(volatile int *)&B.ctl->far_sel) ? B.f1 : B.f0;  // f re-derived (keep mode)
     const int64_t far_base = *(volatile int *)&B.ctl->far_n;
     int *inv_n = SOLO ? cnt + 3 : &dc->inv_n;
@@ -584,7 +588,10 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
             int32_t *t = at.fa;
             at.fa = at.fb;
             at.fb = t;
-            for (int i = team; i < at.nf; i += teams) {
+            tw = DYN_TEAM;
+            while (tw > 1 && (int64_t)at.nf * tw > size) tw >>= 1;
+            sub = rank & (tw - 1);
+            for (int i = rank / tw; i < at.nf; i += size / tw) {
                 int x, b, e;
                 if (SOLO && i < LOCAL_CAP) {
                     const uint4 en = lists[(it & 1) * LOCAL_CAP + i];
@@ -624,14 +631,14 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
         // pushes once
         auto lower_from = [&](int u, int b, int e) {
             const uint32_t hu = __ldcg(hops + u);
-            for (int j0 = b + sub; j0 < e; j0 += 2 * DYN_TEAM) {
-                int p[2], rb[2], re[2];
-                uint32_t old[2];
+            for (int j0 = b + sub; j0 < e; j0 += DYN_ARCS * tw) {
+                int p[DYN_ARCS], rb[DYN_ARCS], re[DYN_ARCS];
+                uint32_t old[DYN_ARCS];
 #pragma unroll
-                for (int k = 0; k < 2; k++)
-                    p[k] = j0 + k * DYN_TEAM < e ? (int)__ldcg(G.rarc + j0 + k * DYN_TEAM).x : -1;
+                for (int k = 0; k < DYN_ARCS; k++)
+                    p[k] = j0 + k * tw < e ? (int)__ldcg(G.rarc + j0 + k * tw).x : -1;
 #pragma unroll
-                for (int k = 0; k < 2; k++) {
+                for (int k = 0; k < DYN_ARCS; k++) {
                     rb[k] = re[k] = 0;
                     old[k] = 0u;
                     if (p[k] < 0) continue;
@@ -645,7 +652,7 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
                     }
                 }
 #pragma unroll
-                for (int k = 0; k < 2; k++) {
+                for (int k = 0; k < DYN_ARCS; k++) {
                     if (hu + 1 >= old[k]) continue;
                     if (!SOLO && hu + 1 >= atomicMin(hops + p[k], hu + 1)) continue;
                     push(p[k], rb[k], re[k]);
@@ -677,14 +684,14 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
     if (at.stage == REP_TREE_WALK) {
         // invalidates x's children in the tree (nodes whose parent is x)
         auto invalidate_from = [&](int x, int b, int e) {
-            for (int j0 = b + sub; j0 < e; j0 += 2 * DYN_TEAM) {
-                int y[2], rb[2], re[2];
-                uint64_t sy[2];
+            for (int j0 = b + sub; j0 < e; j0 += DYN_ARCS * tw) {
+                int y[DYN_ARCS], rb[DYN_ARCS], re[DYN_ARCS];
+                uint64_t sy[DYN_ARCS];
 #pragma unroll
-                for (int k = 0; k < 2; k++)
-                    y[k] = j0 + k * DYN_TEAM < e ? (int)__ldcg(G.arc + j0 + k * DYN_TEAM).x : -1;
+                for (int k = 0; k < DYN_ARCS; k++)
+                    y[k] = j0 + k * tw < e ? (int)__ldcg(G.arc + j0 + k * tw).x : -1;
 #pragma unroll
-                for (int k = 0; k < 2; k++) {
+                for (int k = 0; k < DYN_ARCS; k++) {
                     rb[k] = re[k] = 0;
                     sy[k] = y[k] >= 0 ? __ldcg(B.state + y[k]) : ~0ull;
                     if (SOLO && y[k] >= 0) {
@@ -693,7 +700,7 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
                     }
                 }
 #pragma unroll
-                for (int k = 0; k < 2; k++)
+                for (int k = 0; k < DYN_ARCS; k++)
                     if (y[k] >= 0 && st_g(sy[k]) < INF_G && st_parent(sy[k]) == x) invalidate(y[k], sy[k], rb[k], re[k]);
             }
         };

@@ -521,7 +521,8 @@ struct SearchResult {
 // While the far pile is small (LOCAL_FAR) it splits it too, and while the
 // list is narrow (LOCAL_FILL) it takes the next bucket in early, so that the
 // floods of successive buckets overlap instead of running one after the other
-// (at most LOCAL_AHEAD buckets before the list empties).
+// (at most LOCAL_AHEAD buckets before the list empties; not in keep mode,
+// where it tripled the expansions of a maze's update batches and cost 20 %).
 // A 511 x 511 maze query took 44 ms with every phase on the grid (1,926
 // phases of 20-70 entries, 23 us each), 3.2 ms with narrow phases here, 1.6
 // ms with overlapping buckets (16, 32 or 64 entries alike; wider buckets
@@ -576,7 +577,7 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
     unsigned long long n_far = 0;
     uint4 *cur = buf, *nxt = buf + cap;
     for (;;) {
-        if (m < LOCAL_FILL) {
+        if (m < (KEEP ? 1 : LOCAL_FILL)) {
             // the list is empty or narrow: the far pile's turn
             const int64_t nf = nfar0 + c_far;
             const uint64_t ft64 = (uint64_t)tg + ht;

@@ -69,7 +69,7 @@ def test_repair_hands_over_and_cold_tier(gpu, oracle, heur, group):
     assert low == 5
     assert apply([(0, s, t, 0)]) > low
     # batches of unrelated changes on both sides of one CTA's limit
-    for m in (1, 2047, 2048, 2049, 4096):
+    for m in (1, 2047, 2048, 2049, 4095, 4096, 4097):
         k = m // 2
         ins = [(1, int(a), int(b), int(x)) for a, b, x in zip(rng.integers(0, n, m - k), rng.integers(0, n, m - k),
                                                               rng.integers(1, 1001, m - k))]
