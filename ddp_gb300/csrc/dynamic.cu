@@ -513,7 +513,7 @@ __device__ __forceinline__ CtaGroup dyn_group(CtaGroup *, const SlotBufs &B) { r
 // shared memory, the frontier with its row bounds in shared memory too) and
 // the grid waits once.  It hands over what outgrows it: a level of more than
 // DYN_LOCAL_BAIL nodes, or more than DYN_LOCAL_SEED nodes to re-seed.  A
-// team of up to DYN_TEAM lanes (as many as spread the level over the
+// team of up to eight lanes (as many as spread the level over the
 // threads) walks one row, DYN_ARCS arcs a lane, so that a level is
 // one chain of arc -> node word -> atomic, where a thread walking a row of
 // ten arcs alone ran two such chains and read the row bounds first.
@@ -525,7 +525,7 @@ __device__ __forceinline__ CtaGroup dyn_group(CtaGroup *, const SlotBufs &B) { r
 constexpr int DYN_LOCAL_UPD = 4096;   // updates CTA 0 takes alone
 constexpr int DYN_LOCAL_BAIL = 2048;
 constexpr int DYN_LOCAL_SEED = 1024;
-constexpr int DYN_TEAM = 8;
+constexpr int DYN_TEAM_SHIFT = 3;
 constexpr int DYN_ARCS = 2;
 enum { REP_HOPS, REP_HOPS_WALK, REP_TREE, REP_TREE_WALK, REP_SEED, REP_DONE };
 
@@ -543,7 +543,7 @@ template <bool SOLO, class Grp>
 __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B, uint32_t *hops, const DynArgs &A,
                            DynCtl *dc, int nupd, RepairAt &at, uint4 *lists, int *cnt) {
     const int rank = grp.rank(), size = grp.size();
-    int tw = DYN_TEAM, sub = 0;  // lanes of this level's teams, this one's place
+    int tw = 1, sub = 0;  // lanes of this level's teams, this one's place
     uint4 *far_buf = (*(volatile int *)&B.ctl->far_sel) ? B.f1 : B.f0;  // f re-derived (keep mode)
     const int64_t far_base = *(volatile int *)&B.ctl->far_n;
     int *inv_n = SOLO ? cnt + 3 : &dc->inv_n;
@@ -588,10 +588,11 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
             int32_t *t = at.fa;
             at.fa = at.fb;
             at.fb = t;
-            tw = DYN_TEAM;
-            while (tw > 1 && (int64_t)at.nf * tw > size) tw >>= 1;
+            int ts = DYN_TEAM_SHIFT;
+            while (ts > 0 && (int64_t)at.nf << ts > size) ts--;
+            tw = 1 << ts;
             sub = rank & (tw - 1);
-            for (int i = rank / tw; i < at.nf; i += size / tw) {
+            for (int i = rank >> ts; i < at.nf; i += size >> ts) {
                 int x, b, e;
                 if (SOLO && i < LOCAL_CAP) {
                     const uint4 en = lists[(it & 1) * LOCAL_CAP + i];
