@@ -33,6 +33,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "rules.h"
 
 namespace ddp {
 
@@ -758,8 +759,10 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
     __syncthreads();
     // the entries left go back to the near list (those past the shared list
     // are there already)
-    for (int i = threadIdx.x; i < min(m, cap); i += blockDim.x) qcur[i] = make_uint2(cur[i].x, cur[i].y);
+    const int back = local_handback(m, cap, B.cap_q);
+    for (int i = threadIdx.x; i < back; i += blockDim.x) qcur[i] = make_uint2(cur[i].x, cur[i].y);
     if (threadIdx.x == 0) {
+        if (m > B.cap_q) atomicOr(&ctl->status, ST_OVERFLOW);
         ctl->loc_near = m;
         ctl->loc_far = (int)(nfar0 + c_far);
         ctl->loc_waves = wv;

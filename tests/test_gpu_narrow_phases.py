@@ -72,3 +72,22 @@ def test_update_batches_over_layers(gpu, oracle, width):
         assert got == (want if f else d.INF)
     dyn.close()
     dg.close()
+
+
+@pytest.mark.parametrize("queue_cap", [1, 16, 300, 520, 1400, 1600])
+@pytest.mark.parametrize("width", [200, 600, 1450, 4000])
+def test_short_queues_overflow_or_answer(gpu, oracle, queue_cap, width):
+    """A near queue shorter than the lists that one CTA keeps: the call
+    answers exactly or reports the overflow, and the handle stays usable."""
+    d = gpu
+    g, s, t = _layers(d, width, 3, 1, 50, width + queue_cap)
+    dg = d.DeviceGraph.from_csr(g)
+    gs = g.with_sentinel()
+    f, want, _, _, _ = oracle.astar(gs.n, gs.off[:-1], gs.col, gs.w, np.zeros(gs.n, np.int32), s, t)
+    for _ in range(2):
+        try:
+            assert dg.solve(s, t, queue_cap=queue_cap).cost == want
+        except d.DdpError as e:
+            assert e.code == 5
+    assert dg.solve(s, t).cost == want
+    dg.close()

@@ -1,0 +1,35 @@
+"""The kernels' size rules (ddp_gb300/csrc/rules.h), compiled for the host:
+the same functions that the device code calls, over the values at which they
+change."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "ddp_gb300", "csrc")
+SHIM = """
+#include "rules.h"
+extern "C" {
+int local_handback(int m, int list_cap, int64_t cap_q) { return ddp::local_handback(m, list_cap, cap_q); }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    d = tmp_path_factory.mktemp("rules")
+    src, so = d / "rules.cpp", d / "rules.so"
+    src.write_text(SHIM)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-shared", "-fPIC", "-I" + CSRC, "-o", str(so), str(src)],
+                   check=True)
+    return C.CDLL(str(so))
+
+
+@pytest.mark.parametrize("cap_q", [1, 16, 300, 1535, 1536, 1537, 1 << 33])
+def test_local_lists_hand_back_what_the_queue_holds(rules, cap_q):
+    """A list that one CTA kept in shared memory never goes back past the
+    end of a near queue shorter than it."""
+    f = lambda m: rules.local_handback(m, 1536, C.c_int64(cap_q))  # noqa: E731
+    for m in (0, 1, 15, 16, 17, 299, 301, 512, 513, 1535, 1536, 1537, 100000):
+        assert f(m) == min(m, 1536, cap_q)
