@@ -22,4 +22,10 @@ DDP_RULE int local_handback(int m, int list_cap, int64_t cap_q) {
     return k < cap_q ? k : (int)cap_q;
 }
 
+// Threads of a CTA for opts.block = want (> 0): whole warps, at most top (a
+// multiple of 32).  The engines deal work out by warps: with part of a warp
+// over, warps of the grid would not be warps of the hardware, and with fewer
+// than 32 threads there would be none.
+DDP_RULE int block_threads(int want, int top) { return want >= top ? top : (want + 31) & ~31; }
+
 }  // namespace ddp

@@ -1488,7 +1488,7 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
     ddp_opts o = opts ? *opts : ddp_opts{};
     std::lock_guard<std::mutex> lk(g->mu);
     cudaStream_t st = o.stream ? (cudaStream_t)o.stream : g->stream;
-    const int block = o.block > 0 ? std::min(o.block, 512) : 512;
+    const int block = o.block > 0 ? block_threads(o.block, 512) : 512;
     int64_t cap = o.queue_cap > 0 ? o.queue_cap : (int64_t)g->n + 1024;
     const uint32_t delta = o.delta > 0 ? (uint32_t)o.delta : auto_delta(g);
     DevGraph G = graph_view(g);
@@ -1818,11 +1818,10 @@ int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batc
     graph_ref(g);
     b->hkind = hkind;
     if (opts) b->o = *opts;
-    // whole warps; bidirectional launches choose per batch unless told
     b->hk = kernel_hk(hkind, g->d_xy != nullptr, (b->o.flags & DDP_OPT_HASH) != 0, b->o.group, b->o.flags);
     const bool bidir = bidir_hk(b->hk);
     // whole warps; bidirectional launches choose per batch unless told
-    b->block = b->o.block > 0 ? std::min((b->o.block + 31) & ~31, bidir ? 1024 : 512) : 512;
+    b->block = b->o.block > 0 ? block_threads(b->o.block, bidir ? 1024 : 512) : 512;
     b->path_cap = 1024;
     cudaError_t e = b->o.stream ? cudaSuccess : cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (b->o.stream) b->stream = (cudaStream_t)b->o.stream;

@@ -96,3 +96,19 @@ def test_heuristic_arrays_are_reused(gpu, oracle):
         for h in hs + [user]:
             h.close()
     dg.close()
+
+
+@pytest.mark.parametrize("block", [1, 16, 31, 33, 48, 100, 511, 2000])
+def test_blocks_of_any_size(gpu, oracle, block):
+    """opts.block is taken up to whole warps by every engine."""
+    d = gpu
+    g = d.gen_random_chain(6000, 6, 1, 30, 11)
+    dg = d.DeviceGraph.from_csr(g)
+    s, t = 17, 4321
+    want = _cost(oracle, g, s, t)
+    h = dg.heuristic(t, d.H_BFS_HOPS)
+    for kw in ({}, {"grid": 3}, {"K": 64}, {"flags": d.OPT_ONE_CTA}):
+        for hh in (None, h):
+            _check(oracle, g, dg.solve(s, t, hh, block=block, **kw), s, t, want)
+    h.close()
+    dg.close()

@@ -12,6 +12,7 @@ SHIM = """
 #include "rules.h"
 extern "C" {
 int local_handback(int m, int list_cap, int64_t cap_q) { return ddp::local_handback(m, list_cap, cap_q); }
+int block_threads(int want, int top) { return ddp::block_threads(want, top); }
 }
 """
 
@@ -33,3 +34,10 @@ def test_local_lists_hand_back_what_the_queue_holds(rules, cap_q):
     f = lambda m: rules.local_handback(m, 1536, C.c_int64(cap_q))  # noqa: E731
     for m in (0, 1, 15, 16, 17, 299, 301, 512, 513, 1535, 1536, 1537, 100000):
         assert f(m) == min(m, 1536, cap_q)
+
+
+@pytest.mark.parametrize("top", [512, 1024])
+def test_blocks_are_whole_warps(rules, top):
+    for want in (1, 16, 31, 32, 33, 48, 100, 511, 512, 513, 1023, 1025, (1 << 31) - 1):
+        got = rules.block_threads(want, top)
+        assert got % 32 == 0 and got >= min(want, top) and got <= min(want + 31, top)
