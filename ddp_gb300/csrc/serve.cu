@@ -113,7 +113,10 @@ struct ddp_server {
     int nver = 0;
     std::vector<VBuf> vb;
     DevGraph *h_vtab = nullptr, *d_vtab = nullptr;
-    int *d_inflight = nullptr;  // searches per version buffer (device memory: slots count in and out)
+    // searches per version buffer: slots count in and out.  Device memory, which
+    // the service CTA reads; a one-slot server has no service CTA, there the
+    // host waits on the counts (h_inflight, mapped)
+    int *h_inflight = nullptr, *d_inflight = nullptr;
     std::deque<Delta> deltas;
     Delta cur;  // being recorded by the scatter hook
     cudaStream_t cstream = nullptr;  // maintenance launches while no slot kernel runs
@@ -158,8 +161,10 @@ int stage_reserve(ddp_server *s, size_t bytes) {
     return DDP_OK;
 }
 
-// Runs maintenance subs: on the service CTA of the running slot kernel, or
-// with ordinary launches when none runs.
+// Runs maintenance subs, once no search runs on version buffer wait_buf (-1:
+// none to wait for): on the service CTA of the running slot kernel, which
+// waits itself, or with ordinary launches when no kernel or no service CTA
+// runs.
 int svc_run(ddp_server *s, const SvcSub *subs, int nsub, int wait_buf = -1) {
     if (kernel_running(s) && s->sa.nslots >= 2) {
         SvcJob *j = s->h_svc;
@@ -184,6 +189,13 @@ int svc_run(ddp_server *s, const SvcSub *subs, int nsub, int wait_buf = -1) {
             // a job of an ordinary batch takes some 10 us; the shortest sleep
             // takes 60
             if (waited > 200000) std::this_thread::sleep_for(std::chrono::microseconds(2));
+        }
+    } else if (wait_buf >= 0 && s->h_inflight) {
+        // one slot, no service CTA: its search may be on the buffer
+        const int64_t t0 = now_ns();
+        while (__atomic_load_n(&s->h_inflight[wait_buf], __ATOMIC_ACQUIRE) != 0 && kernel_running(s)) {
+            if (now_ns() - t0 > 30000000000LL) return fail(DDP_ERR_TIMEOUT, "graph version buffer stayed busy");
+            std::this_thread::sleep_for(std::chrono::microseconds(20));
         }
     }
     cudaError_t e = svc_run_direct(subs, nsub, s->cstream);
@@ -323,9 +335,10 @@ int fill_buffer(ddp_server *s, int k, int v) {
         subs[ns++] = sub_of(SVC_GATHER_INTS, (long long)rrow.size(), b.roend, g->d_roend, d + o3, nullptr);
         patched = arc.size() + rarc.size() + row.size() + rrow.size();
     }
-    // The release store of the previous version and the service CTA's read of
-    // the buffer's count pair with the slots' count-then-re-read (both sides
-    // fenced).  With no kernel running no search holds a buffer.
+    // The release store of the previous version and svc_run's read of the
+    // buffer's count (by the service CTA, or here with one slot) pair with the
+    // slots' count-then-re-read (both sides fenced).  With no kernel running no
+    // search holds a buffer.
     __atomic_thread_fence(__ATOMIC_SEQ_CST);
     int rc = svc_run(s, subs, ns, k);
     if (rc) return rc;
@@ -560,8 +573,14 @@ int ddp_serve_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, int64_t 
     s->nver = versions;
     s->vb.assign((size_t)versions, VBuf());
     e = cudaHostAlloc(&s->h_vtab, sizeof(DevGraph) * (size_t)versions, flags);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_inflight, sizeof(int) * (size_t)versions);
-    if (e == cudaSuccess) e = cudaMemset(s->d_inflight, 0, sizeof(int) * (size_t)versions);
+    if (e == cudaSuccess && nslots < 2) {
+        e = cudaHostAlloc(&s->h_inflight, sizeof(int) * (size_t)versions, flags);
+        if (e == cudaSuccess) std::memset(s->h_inflight, 0, sizeof(int) * (size_t)versions);
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&s->d_inflight, s->h_inflight, 0);
+    } else if (e == cudaSuccess) {
+        e = cudaMalloc(&s->d_inflight, sizeof(int) * (size_t)versions);
+        if (e == cudaSuccess) e = cudaMemsetAsync(s->d_inflight, 0, sizeof(int) * (size_t)versions, s->stream);
+    }
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&s->d_vtab, s->h_vtab, 0);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaHostAlloc(graph versions)"));
     std::memset((void *)s->h_vtab, 0, sizeof(DevGraph) * (size_t)versions);
@@ -751,7 +770,8 @@ int ddp_serve_free(ddp_server *s) {
         cudaFree(b.rarc);
     }
     cudaFreeHost(s->h_vtab);
-    cudaFree(s->d_inflight);
+    if (s->h_inflight) cudaFreeHost(s->h_inflight);
+    else cudaFree(s->d_inflight);
     cudaFreeHost(s->h_stage);
     for (void *p : s->stage_old) cudaFreeHost(p);
     if (s->cstream) cudaStreamDestroy(s->cstream);

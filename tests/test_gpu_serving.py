@@ -218,3 +218,36 @@ def test_serving_paths(gpu, oracle):
     with pytest.raises(d.DdpError):
         srv.path(max(fin)[1])  # the costliest random pair: far more than two nodes
     srv.close()
+
+
+@pytest.mark.parametrize("kind", ["H_BIDIR", "H_EUCLID"])
+@pytest.mark.parametrize("nver", [2, 3])
+def test_one_slot_and_updates_during_its_searches(gpu, oracle, kind, nver):
+    """A server of one slot has no service CTA: a version buffer that its
+    search is on is left alone until the search ends.  Updates that change
+    the weights over the whole graph follow one another while requests run
+    and wait; each answer is exact for the version it reports."""
+    d = gpu
+    g, dg = _geo(d, 60_000, 61)
+    srv = d.Server(dg, getattr(d, kind), max_requests=1024, versions=nver, grid=1)
+    rng = np.random.default_rng(nver)
+    S = rng.integers(0, g.n, 24).astype(np.int32)
+    T = rng.integers(0, g.n, 24).astype(np.int32)
+    assert srv.stats()["slots"] == 1
+    src = np.repeat(np.arange(g.n, dtype=np.int32), np.diff(g.off))
+    w, versions = g.w.copy(), [g.w.copy()]
+    first = srv.submit(S, T)
+    for _ in range(6):
+        # heavier arcs only: the Euclidean scale stays a lower bound
+        j = rng.choice(g.e, 3000, replace=False)
+        w[j] = w[j] + rng.integers(1, 2000, len(j)).astype(np.uint32)
+        srv.update(np.full(len(j), 2, np.int32), src[j], g.col[j], w[j])
+        versions.append(w.copy())
+    ids, costs, _, ver = srv.drain()
+    assert sorted(ids.tolist()) == list(range(first, first + 24))
+    for k in range(24):
+        i = int(ids[k]) - first
+        gv = d.CSR(g.n, g.off, g.col, versions[int(ver[k])], xy=g.xy)
+        assert costs[k] == _oracle(oracle, gv, int(S[i]), int(T[i]), 0), (i, int(ver[k]))
+    assert srv.stats()["version"] == 6
+    srv.close()
