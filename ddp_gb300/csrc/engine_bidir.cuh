@@ -68,11 +68,12 @@
 // d_t(y) < b; both ends were expanded with final labels, and whichever
 // expansion came second saw the other's final label (a label, and its filter
 // bit, are installed by atomics that complete before the node's arcs are
-// walked, and records are read from L2), so mu <= len(P): no shorter path
-// exists.  An empty direction also ends the search.  Within a wave the same
-// bound prunes: an entry with key + (the other side's bound) >= mu is
-// dropped, since a path through it either ends at a node the other side has
-// yet to settle (length >= mu) or meets a settled node, which its arc offered.
+// walked, each install setting the bit itself, and records are read from L2),
+// so mu <= len(P): no shorter path exists.  An empty direction also ends the
+// search.  Within a wave the same bound prunes: an entry with key + (the other
+// side's bound) >= mu is dropped, since a path through it either ends at a node
+// the other side has yet to settle (length >= mu) or meets a settled node,
+// which its arc offered.
 #pragma once
 
 #include "engine_async.cuh"
@@ -758,11 +759,13 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
                     const typename Rec::U got = Rec::cas(w, c, nv);
                     if (Rec::eq(got, c)) {
                         ok = true;
-                        if (Rec::g(c, ep) >= INF_G) {
-                            n_first++;
-                            const uint32_t h = ((uint32_t)u * 0x9E3779B1u) >> 17;
-                            atomicOr(&q->settled[dir][h >> 5], 1u << (h & 31));
-                        }
+                        n_first += Rec::g(c, ep) >= INF_G;
+                        // every install sets the bit, not the first alone:
+                        // the thread of the first may not have come to it
+                        // when a second, smaller label is installed and
+                        // walked, and the other side would miss that one
+                        const uint32_t h = ((uint32_t)u * 0x9E3779B1u) >> 17;
+                        atomicOr(&q->settled[dir][h >> 5], 1u << (h & 31));
                         break;
                     }
                     c = got;
