@@ -96,8 +96,12 @@ __device__ __forceinline__ int row_begin(const int32_t *off, const int32_t *oend
 // ---- bounded-wait barriers -------------------------------------------------
 // Spin limit for every device-side wait: ~2^22 polls with backoff (seconds),
 // after which the waiter records ST_TIMEOUT and proceeds; callers check the
-// status word after each barrier and leave their loops.
-constexpr uint32_t SPIN_LIMIT = 1u << 22;
+// status word after each barrier and leave their loops.  (A build with a
+// small limit lets a test see waits run out.)
+#ifndef DDP_SPIN_LIMIT
+#define DDP_SPIN_LIMIT (1u << 22)
+#endif
+constexpr uint32_t SPIN_LIMIT = DDP_SPIN_LIMIT;
 
 struct GridBarrier {
     unsigned int *count;  // arrivals in the current generation

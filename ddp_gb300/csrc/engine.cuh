@@ -64,6 +64,7 @@ struct SearchCtl {
     int cur_q;            // query the slot is working on (batch)
     int far_n, far_sel;   // far pile left by the last run (dynamic resume)
     int cur_ver;          // graph version of the current search (serving)
+    int path_len;         // single query: the path as walked before the labels go (walk_path)
     unsigned int bar_count, bar_gen;  // grid barrier (single-query form)
     int cold_n;           // entries in the far pile's cold tier (keep mode) ...
     unsigned int cold_x;  // ... all with g >= cold_x
@@ -1343,41 +1344,47 @@ __device__ uint32_t run_bfs_hops(const Grp &grp, const DevGraph &G, const SlotBu
     return complete ? HOPS_INF : lvl + 1;
 }
 
-// Parent walk t -> s into path[0..cap) in s..t order; returns the length
-// (0 when unreachable).  One CTA; buf holds bcap ids in shared memory: one
-// thread walks the chain of parents into it, then all copy it out in order
-// (reversing it in place took as long again as the walk).
-__device__ inline int32_t write_path_cta(const SlotBufs &B, int32_t s, int32_t t, int32_t *path, int32_t cap,
-                                         int32_t n, int *status, int32_t *buf, int32_t bcap) {
-    __shared__ int32_t s_len;
-    if (threadIdx.x == 0) {
-        int32_t len = 0;
-        uint64_t st = __ldcg(B.state + t);
-        if (st_g(st) < INF_G) {
-            for (int32_t c = t; c >= 0 && len <= n;) {
-                if (len < bcap) buf[len] = c;
-                len++;
-                if (c == s) break;
-                c = st_parent(st);
-                if (c >= 0) st = __ldcg(B.state + c);
-            }
-            if (len > cap) atomicOr(status, ST_PATH_TRUNC);
-            if (len > bcap) {
-                // longer than the buffer: a second walk writes it
-                int32_t c = t;
-                for (int32_t i = len - 1; i >= 0 && c >= 0; i--) {
-                    if (i < cap) path[i] = c;
-                    c = st_parent(__ldcg(B.state + c));
-                }
-            }
-        }
-        s_len = len;
+// Parent walk t -> s into buf[0..bcap), t first; returns the length (0 when
+// unreachable, -1 when the path is longer than buf).  One thread.
+__device__ inline int32_t walk_path(const SlotBufs &B, int32_t s, int32_t t, int32_t *buf, int32_t bcap) {
+    uint64_t st = __ldcg(B.state + t);
+    if (st_g(st) >= INF_G) return 0;
+    int32_t len = 0;
+    for (int32_t c = t; c >= 0;) {
+        if (len == bcap) return -1;
+        buf[len++] = c;
+        if (c == s) break;
+        c = st_parent(st);
+        if (c >= 0) st = __ldcg(B.state + c);
     }
-    __syncthreads();
-    const int32_t len = s_len;
-    if (len <= bcap)
-        for (int32_t i = threadIdx.x; i < len; i += blockDim.x)
-            if (len - 1 - i < cap) path[len - 1 - i] = buf[i];
+    return len;
+}
+
+// Path of a finished search into path[0..cap) in s..t order, by one CTA;
+// returns the length.  len: what walk_path left in buf (bcap ids in shared
+// memory), copied out by all threads (reversing it in place took as long again
+// as the walk); -1: too long for buf, one thread walks it twice.
+__device__ inline int32_t write_path_cta(const SlotBufs &B, int32_t s, int32_t t, int32_t *path, int32_t cap,
+                                         int32_t n, int *status, const int32_t *buf, int32_t len) {
+    __shared__ int32_t s_len;
+    if (len < 0) {
+        if (threadIdx.x == 0) {
+            int32_t l = 0;
+            for (int32_t c = t; c >= 0 && l <= n; c = c == s ? -1 : st_parent(__ldcg(B.state + c))) l++;
+            if (l > cap) atomicOr(status, ST_PATH_TRUNC);
+            int32_t c = t;
+            for (int32_t i = l - 1; i >= 0 && c >= 0; i--) {
+                if (i < cap) path[i] = c;
+                c = st_parent(__ldcg(B.state + c));
+            }
+            s_len = l;
+        }
+        __syncthreads();
+        return s_len;
+    }
+    if (len > cap && threadIdx.x == 0) atomicOr(status, ST_PATH_TRUNC);
+    for (int32_t i = threadIdx.x; i < len; i += blockDim.x)
+        if (len - 1 - i < cap) path[len - 1 - i] = buf[i];
     __syncthreads();
     return len;
 }

@@ -150,10 +150,12 @@ __global__ void k_reset_touched(SlotArrays sa) {
 // What a single-query kernel returns, in host memory mapped into the device:
 // the host reads it after one synchronisation, with no copies of its own.
 constexpr int SOLVE_PATH = 4096;  // path ids returned with it
+constexpr int SINGLE_PATH_BUF = MAX_WARPS * (int)(sizeof(WarpRows) / sizeof(int32_t));  // path ids the warp rows hold
 struct SolveOut {
     int32_t cost, len, status, iters;
     long long expanded, scanned, relaxed, far_scanned, touched;
     uint32_t hcap;  // BFS: hop cap of unreached nodes
+    int32_t kept;   // k_solve_single: a CTA has left its share of the labels (the host zeroes it)
     int32_t path[SOLVE_PATH];
 };
 
@@ -181,12 +183,12 @@ __global__ void __launch_bounds__(512) k_bfs_single(DevGraph G, SlotArrays sa, u
 }
 
 // The end of a single query, by its first CTA: path (to the device array and,
-// as far as it fits, to the host's), result and counters.  len >= 0: the
-// caller has written the path; else it is walked here.
+// as far as it fits, to the host's), result and counters.  WALKED: buf and
+// len come from walk_path; else the caller has written the path's len nodes.
+template <bool WALKED>
 __device__ void solve_report(const DevGraph &G, const SlotBufs &B, const SearchParams &P, const SearchResult &r,
-                             SolveOut *out, int32_t *path, int32_t path_cap, int32_t len, int32_t *buf, int32_t bcap) {
-    const bool ok = !(*(volatile int *)&B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT | ST_BUDGET));
-    if (len < 0) len = ok ? write_path_cta(B, P.s, P.t, path, path_cap, G.n, &B.ctl->status, buf, bcap) : 0;
+                             SolveOut *out, int32_t *path, int32_t path_cap, const int32_t *buf, int32_t len) {
+    if (WALKED) len = write_path_cta(B, P.s, P.t, path, path_cap, G.n, &B.ctl->status, buf, len);
     for (int32_t i = threadIdx.x; i < min(len, SOLVE_PATH); i += blockDim.x) out->path[i] = __ldcg(path + i);
     if (threadIdx.x == 0) {
         out->cost = r.cost >= INF_G ? DDP_INF : (int32_t)r.cost;
@@ -213,12 +215,24 @@ __global__ void __launch_bounds__(512, 1)
     SlotBufs B = slot_of(sa, 0);
     GridGroup grp{{&B.ctl->bar_count, &B.ctl->bar_gen}, &B.ctl->status};
     const SearchResult r = run_search(grp, G, B, H, P, wrows);
-    if (grp.first_cta())
-        solve_report(G, B, P, r, out, path, path_cap, -1, reinterpret_cast<int32_t *>(wrows),
-                     (int32_t)(sizeof(wrows) / sizeof(int32_t)));
-    grp.sync();  // the path is read: the labels may go
+    int32_t *buf = reinterpret_cast<int32_t *>(wrows);
+    if (grp.rank() == 0)
+        B.ctl->path_len = *(volatile int *)&B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT)
+                              ? 0
+                              : walk_path(B, P.s, P.t, buf, SINGLE_PATH_BUF);
+    grp.sync();  // a path that fits is in shared memory: the labels may go
+    // Not for a longer path, whose walk (a dependent load a node) must not keep
+    // the grid waiting, and not after a wait that ran out, when the log of
+    // touched nodes may still be growing: k_reset_touched, then (ddp_solve).
+    const int32_t len = *(volatile int *)&B.ctl->path_len;
+    const bool clear = len >= 0 && !(*(volatile int *)&B.ctl->status & ST_TIMEOUT);
     const int cnt = *(volatile int *)&B.ctl->touched;
-    for (int i = grp.rank(); i < cnt; i += grp.size()) B.state[B.touched[i]] = ~0ull;
+    if (grp.first_cta()) solve_report<true>(G, B, P, r, out, path, path_cap, buf, len);
+    if (clear) {
+        for (int i = grp.rank(); i < cnt; i += grp.size()) B.state[B.touched[i]] = ~0ull;
+    } else if (threadIdx.x == 0) {
+        out->kept = 1;
+    }
 }
 
 // Single query on one CTA by the bidirectional search (HK as in k_batch).
@@ -262,7 +276,7 @@ __global__ void __launch_bounds__(1024, 1)
         walk(R);
     }
     __syncthreads();
-    solve_report(G, B, P, r, out, path, path_cap, s_len, buf, 2 * PATH_BUF);
+    solve_report<false>(G, B, P, r, out, path, path_cap, nullptr, s_len);
     if constexpr (pair16_hk(HK)) {
         ulonglong4_32a ones;
         ones.x = ones.y = ones.z = ones.w = ~0ull;
@@ -878,8 +892,14 @@ __global__ void __launch_bounds__(512, 2)
     __shared__ CtaQ sq;
     SlotBufs B = slot_of(sa, 0);
     const SearchResult r = run_search_cta<Heur, true>(G, B, H, P, wrows, &sq);  // one query: latency first
-    solve_report(G, B, P, r, out, path, path_cap, -1, reinterpret_cast<int32_t *>(wrows),
-                 (int32_t)(sizeof(wrows) / sizeof(int32_t)));
+    __shared__ int32_t s_len;
+    int32_t *buf = reinterpret_cast<int32_t *>(wrows);
+    if (threadIdx.x == 0)
+        s_len = B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT)
+                    ? 0
+                    : walk_path(B, P.s, P.t, buf, SINGLE_PATH_BUF);
+    __syncthreads();
+    solve_report<true>(G, B, P, r, out, path, path_cap, buf, s_len);
     __syncthreads();
     if (B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT))
         for (int64_t i = threadIdx.x; i < B.cap_q; i += blockDim.x) B.q0[i].x = RING_EMPTY;
@@ -1544,6 +1564,7 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
         Workspace *w = g->ws;
         DDP_CUDA(workspace_begin(w, st));
         w->dirty = true;
+        w->h_res->kept = 0;
         cudaError_t e;
         const bool one_cta = (o.flags & DDP_OPT_ONE_CTA) != 0;
         if (one_cta && w->ring_dirty) {
@@ -1601,7 +1622,16 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
         if (e != cudaSuccess) return cuda_fail(e, "k_solve_single launch");
         if (!one_cta) w->ring_dirty = true;  // the phase-synchronous engine leaves entries in q0
         DDP_CUDA(cudaStreamSynchronize(st));
-        if (w->h_res->status & ST_TIMEOUT) return fail(DDP_ERR_TIMEOUT, "search barrier timed out");
+        if (w->h_res->status & ST_TIMEOUT) {
+            // CTAs went on apart: nothing that they left is used again
+            workspace_release(g);
+            return fail(DDP_ERR_TIMEOUT, "search barrier timed out");
+        }
+        if (!one_cta && w->h_res->kept) {
+            k_reset_touched<<<dim3(256, 1), 256, 0, st>>>(w->sa);
+            DDP_CUDA(cudaGetLastError());
+            DDP_CUDA(cudaStreamSynchronize(st));
+        }
         if (w->h_res->status & ST_OVERFLOW) {
             if (o.queue_cap > 0) return fail(DDP_ERR_QUEUE_OVERFLOW, "search queue overflow");
             cap *= 2;  // automatic capacity: grow and retry
