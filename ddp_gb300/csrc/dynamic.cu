@@ -1018,6 +1018,7 @@ int dyn_upload(ddp_graph *g, bool sync) {
     m->dirty_rarc.clear();
     m->dirty_row.clear();
     m->dirty_rrow.clear();
+    if (rc) m->full = true;  // a list did not arrive: the next upload sends everything
     // the device graph is current when this returns (other streams read it),
     // unless the caller synchronises the graph's stream itself
     if (!rc && sync) DDP_CUDA(cudaStreamSynchronize(g->stream));

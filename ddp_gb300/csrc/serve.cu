@@ -172,6 +172,7 @@ int svc_run(ddp_server *s, const SvcSub *subs, int nsub, int wait_buf = -1) {
         j->nsub = nsub;
         j->wait_buf = wait_buf;
         for (int i = 0; i < nsub; i++) j->sub[i] = subs[i];
+        __atomic_store_n(&j->claim, id, __ATOMIC_RELEASE);
         __atomic_store_n(&j->seq, id, __ATOMIC_RELEASE);
         const int64_t t0 = now_ns();
         for (int polls = 0;; polls++) {
@@ -184,7 +185,11 @@ int svc_run(ddp_server *s, const SvcSub *subs, int nsub, int wait_buf = -1) {
                 break;
             }
             const int64_t waited = now_ns() - t0;
-            if (waited > 30000000000LL)
+            int mine = id;
+            // given up: the job is taken back, unless the CTA has just claimed
+            // it (then it is done in a moment)
+            if (waited > SVC_WAIT_NS &&
+                __atomic_compare_exchange_n(&j->claim, &mine, 0, false, __ATOMIC_ACQ_REL, __ATOMIC_ACQUIRE))
                 return fail(DDP_ERR_TIMEOUT, "service CTA did not run the graph maintenance job");
             // a job of an ordinary batch takes some 10 us; the shortest sleep
             // takes 60
@@ -194,7 +199,7 @@ int svc_run(ddp_server *s, const SvcSub *subs, int nsub, int wait_buf = -1) {
         // one slot, no service CTA: its search may be on the buffer
         const int64_t t0 = now_ns();
         while (__atomic_load_n(&s->h_inflight[wait_buf], __ATOMIC_ACQUIRE) != 0 && kernel_running(s)) {
-            if (now_ns() - t0 > 30000000000LL) return fail(DDP_ERR_TIMEOUT, "graph version buffer stayed busy");
+            if (now_ns() - t0 > SVC_WAIT_NS) return fail(DDP_ERR_TIMEOUT, "graph version buffer stayed busy");
             std::this_thread::sleep_for(std::chrono::microseconds(20));
         }
     }

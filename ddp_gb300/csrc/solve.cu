@@ -763,7 +763,6 @@ __device__ void service_loop(const BatchArgs &A) {
             for (;;) {
                 const int seq = A.svc->seq;
                 if (seq != A.svc->done) {
-                    A.svc->taken = seq;
                     __threadfence_system();
                     const int ns = min(max(A.svc->nsub, 0), SVC_MAX_SUB);
                     for (int i = 0; i < ns; i++) {
@@ -775,19 +774,27 @@ __device__ void service_loop(const BatchArgs &A) {
                         sub[i].p2 = x.p2;
                         sub[i].p3 = x.p3;
                     }
-                    job[0] = 1;
-                    job[1] = ns;
-                    job[2] = seq;
                     // a version buffer is rewritten once no search runs on it
                     const int wb = A.svc->wait_buf;
-                    if (wb >= 0) {
-                        __threadfence_system();
+                    __threadfence_system();
+                    bool mine = A.svc->claim == seq, idle = true;
+                    if (mine && wb >= 0) {
                         uint32_t polls = 0;
-                        while (*(volatile int *)(A.inflight + wb) != 0 && ++polls < (1u << 25)) __nanosleep(500);
-                        if (polls >= (1u << 25)) job[0] = 0;  // leave: the host gives up first
+                        while (!(idle = *(volatile int *)(A.inflight + wb) == 0) && ++polls < SVC_POLLS) {
+                            __nanosleep(500);
+                            if ((polls & 31) == 0 && !(mine = A.svc->claim == seq)) break;
+                        }
                         __threadfence_system();
                     }
-                    break;
+                    if (mine && idle && atomicCAS_system(const_cast<int *>(&A.svc->claim), seq, 0) == seq) {
+                        job[0] = 1;
+                        job[1] = ns;
+                        job[2] = seq;
+                        break;
+                    }
+                    // taken back by the host: not looked at again; else the
+                    // buffer is still busy: the same job, from the start
+                    if (A.svc->claim != seq) A.svc->done = seq;
                 }
                 if (*(volatile int *)A.closing || *A.pause) break;
                 __nanosleep(300);

@@ -40,13 +40,27 @@ struct SvcSub {
     unsigned long long p0, p1, p2, p3;
 };
 constexpr int SVC_MAX_SUB = 8;
-// The host fills nsub, sub[] and wait_buf and publishes seq; the service CTA marks
-// taken = seq, runs the subs in order, and marks done = seq.
+// The host fills nsub, sub[], wait_buf and claim (= the job's number) and
+// publishes seq.  The service CTA waits for the buffer, claims the job (claim:
+// its number -> 0), runs the subs in order and marks done = seq.  A host that
+// gives up waiting takes the job back by the same step, so that a job it has
+// reported as failed never runs on lists that are written again.
 struct SvcJob {
-    int seq, taken, done, nsub;
+    int seq, claim, done, nsub;
     int wait_buf, pad;  // version buffer that no search may run on first (-1: none)
     SvcSub sub[SVC_MAX_SUB];
 };
+// Polls of a busy buffer after which the service CTA looks at its launch
+// again (closing, pause) before it waits on, and how long the host waits for
+// a job.  (A build with small numbers lets a test see both run out.)
+#ifndef DDP_SVC_POLLS
+#define DDP_SVC_POLLS (1u << 21)
+#endif
+#ifndef DDP_SVC_WAIT_NS
+#define DDP_SVC_WAIT_NS 30000000000LL
+#endif
+constexpr uint32_t SVC_POLLS = DDP_SVC_POLLS;
+constexpr long long SVC_WAIT_NS = DDP_SVC_WAIT_NS;
 
 struct BatchArgs {
     const int32_t *S, *T;

@@ -31,7 +31,7 @@ def short_waits(gpu, oracle, tmp_path_factory):
     root = tmp_path_factory.mktemp("short")
     for f in ("ddp_gb300", "include", "oracle"):
         shutil.copytree(os.path.join(ROOT, f), root / f, ignore=shutil.ignore_patterns("_build", "*.so", "__pycache__"))
-    env = dict(os.environ, DDP_NVCC_EXTRA="-DDDP_SPIN_LIMIT=256u")
+    env = dict(os.environ, DDP_NVCC_EXTRA="-DDDP_SPIN_LIMIT=256u -DDDP_SVC_POLLS=64u -DDDP_SVC_WAIT_NS=2000000LL")
     env.pop("PYTHONPATH", None)
     subprocess.run([sys.executable, "-m", "ddp_gb300.build"], cwd=root, env=env, check=True)
 
@@ -64,4 +64,51 @@ for s, t in zip(S.tolist(), T.tolist()):
         ok, why = O.check_path(m.off, m.col, m.w, r.path, s, t, want)
         assert ok, why
 dg.close()
+""")
+
+
+def test_updates_given_up_on_leave_the_server_exact(short_waits):
+    """Searches hold a version buffer for longer than an update waits: the
+    update fails, its maintenance job is taken back (the next one writes its
+    lists over), the service CTA stays, and later updates go through."""
+    short_waits("""
+import time
+g = d.gen_geometric(300_000, 6, 1 << 20, 1000, 17, 4)
+dg = d.DeviceGraph.from_csr(g)
+srv = d.Server(dg, d.H_BIDIR, max_requests=64, versions=2, grid=2)
+rng = np.random.default_rng(3)
+# long queries: from one corner region to the opposite one
+key = g.xy.sum(axis=1)
+order = np.argsort(key)
+S, T = order[rng.integers(0, 3000, 10)], order[-1 - rng.integers(0, 3000, 10)]
+src = np.repeat(np.arange(g.n, dtype=np.int32), np.diff(g.off))
+w, versions, failed = g.w.copy(), [g.w.copy()], 0
+first = srv.submit(S.astype(np.int32), T.astype(np.int32))
+for k in range(24):
+    j = rng.choice(g.e, 20000 if k % 2 else 200, replace=False)
+    w[j] = w[j] + rng.integers(1, 2000, len(j)).astype(np.uint32)
+    try:
+        srv.update(np.full(len(j), 2, np.int32), src[j], g.col[j], w[j])
+        versions.append(w.copy())
+    except d.DdpError as e:
+        assert e.code == 6, e
+        failed += 1
+ids, costs, _, ver = srv.drain()
+assert failed > 0, "no update ran into the wait"
+assert srv.stats()["version"] == len(versions) - 1
+for k in range(len(ids)):
+    i = int(ids[k]) - first
+    gv = d.CSR(g.n, g.off, g.col, versions[int(ver[k])])
+    assert costs[k] == cost(gv, int(S[i]), int(T[i])), (i, int(ver[k]))
+# nothing runs: an update and its answers
+j = rng.choice(g.e, 5000, replace=False)
+w[j] = w[j] + 7
+srv.update(np.full(len(j), 2, np.int32), src[j], g.col[j], w[j])
+srv.submit(S[:3].astype(np.int32), T[:3].astype(np.int32))
+ids, costs, _, _ = srv.drain()
+gv = d.CSR(g.n, g.off, g.col, w)
+for k in range(len(ids)):
+    i = int(ids[k]) - first - 10
+    assert costs[k] == cost(gv, int(S[i]), int(T[i]))
+srv.close()
 """)
