@@ -482,7 +482,8 @@ struct DynCtl {
     int relaxed;
     int reseeded;
     int stage, nf, odd;  // CTA 0's hand-back (RepairAt; odd: its buffers are swapped)
-    int pad[4];
+    int again;           // it is to go on alone
+    int pad[3];
 };
 
 __device__ __forceinline__ SlotBufs slot_of_dyn(const SlotArrays &sa) {
@@ -511,8 +512,9 @@ __device__ __forceinline__ CtaGroup dyn_group(CtaGroup *, const SlotBufs &B) { r
 // nodes: on a grid each level costs a barrier on top of its chain of memory
 // trips, so CTA 0 takes the whole repair alone (block barriers, counters in
 // shared memory, the frontier with its row bounds in shared memory too) and
-// the grid waits once.  It hands over what outgrows it: a level of more than
-// DYN_LOCAL_BAIL nodes, or more than DYN_LOCAL_SEED nodes to re-seed.  A
+// the grid waits once (once more for every DYN_LOCAL_LEVELS levels).  It hands
+// over what outgrows it: a level of more than DYN_LOCAL_BAIL nodes, or more
+// than DYN_LOCAL_SEED nodes to re-seed.  A
 // team of up to eight lanes (as many as spread the level over the
 // threads) walks one row, DYN_ARCS arcs a lane, so that a level is
 // one chain of arc -> node word -> atomic, where a thread walking a row of
@@ -525,14 +527,22 @@ __device__ __forceinline__ CtaGroup dyn_group(CtaGroup *, const SlotBufs &B) { r
 constexpr int DYN_LOCAL_UPD = 4096;   // updates CTA 0 takes alone
 constexpr int DYN_LOCAL_BAIL = 2048;
 constexpr int DYN_LOCAL_SEED = 1024;
+// Levels that CTA 0 walks before it lets the grid pass its barrier, whose wait
+// is bounded (seconds): a chain cut near its source is a level a node.
+#ifndef DDP_DYN_LEVELS
+#define DDP_DYN_LEVELS 4096
+#endif
+constexpr int DYN_LOCAL_LEVELS = DDP_DYN_LEVELS;
 constexpr int DYN_TEAM_SHIFT = 3;
 constexpr int DYN_ARCS = 2;
 enum { REP_HOPS, REP_HOPS_WALK, REP_TREE, REP_TREE_WALK, REP_SEED, REP_DONE };
 
-// The next step, and the frontier of a walk: nf nodes in fb.
+// The next step, and the frontier of a walk: nf nodes in fb.  again: CTA 0
+// stopped after DYN_LOCAL_LEVELS levels, not because the step is too wide.
 struct RepairAt {
     int stage, nf;
     int32_t *fa, *fb;
+    bool again;
 };
 
 // Runs the repair from `at` on.  SOLO: on one CTA that returns early (at
@@ -549,10 +559,12 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
     int *inv_n = SOLO ? cnt + 3 : &dc->inv_n;
     int *far_add = SOLO ? cnt + 4 : &dc->far_add;
     if (SOLO) {
-        if (threadIdx.x < 5) cnt[threadIdx.x] = 0;
+        // (dc->inv_n: nodes that an earlier turn invalidated)
+        if (threadIdx.x < 5) cnt[threadIdx.x] = threadIdx.x == 3 ? *(volatile int *)&dc->inv_n : 0;
         __syncthreads();
     }
-    int it = 0;
+    at.again = false;
+    int it = 0, levels = 0;
     // a level pushes into the counter after its own; the one that no thread
     // reads any more is cleared for the level after
     int *next = SOLO ? cnt + 1 : dc->cnt + 1;
@@ -580,7 +592,20 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
     };
     // walks levels until none is left; false: the level is too wide for SOLO
     auto walk = [&](const int32_t *rbeg, const int32_t *rend, auto expand) -> bool {
+        if (SOLO && it == 0) {
+            // another turn: the frontier with its row bounds
+            for (int i = threadIdx.x; i < min(at.nf, LOCAL_CAP); i += size) {
+                const int x = __ldcg(at.fb + i);
+                lists[i] = make_uint4((uint32_t)x, (uint32_t)row_begin(rbeg, rend, x), (uint32_t)row_end(rbeg, rend, x),
+                                      0u);
+            }
+            __syncthreads();
+        }
         while (at.nf > 0) {
+            if (SOLO && ++levels > DYN_LOCAL_LEVELS && at.nf <= DYN_LOCAL_BAIL) {
+                at.again = true;
+                return false;
+            }
             // a push past the buffer raised an overflow: its count is not a frontier
             if (SOLO ? at.nf > DYN_LOCAL_BAIL
                      : (*(volatile int *)&B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT)) != 0)
@@ -801,28 +826,34 @@ __global__ void __launch_bounds__(512, 1)
         RepairAt at{A.heur == 1 ? REP_HOPS : REP_TREE, 0, reinterpret_cast<int32_t *>(B.q0),
                     reinterpret_cast<int32_t *>(B.q1)};
         if constexpr (Grp::multi) {
-            if (nupd <= DYN_LOCAL_UPD) {
+            bool again = nupd <= DYN_LOCAL_UPD;
+            while (again) {
                 if (grp.first_cta()) {
                     __shared__ int cnt[5];
                     dyn_repair<true>(CtaGroup{&B.ctl->status}, G, B, hops, A, dc, nupd, at,
                                      reinterpret_cast<uint4 *>(wrows), cnt);
+                    __syncthreads();
                     if (threadIdx.x == 0) {
                         dc->inv_n = cnt[3];
                         dc->stage = at.stage;
                         dc->nf = at.nf;
                         dc->odd = at.fa != reinterpret_cast<int32_t *>(B.q0);
+                        dc->again = at.again;
                     }
                 }
                 grp.sync();  // CTA 0's changes and hand-back are visible to every CTA
+                // a wait that ran out: CTA 0 may still be at it
+                if (*(volatile int *)&B.ctl->status & ST_TIMEOUT) {
+                    if (rank == 0) A.out[2] = ST_TIMEOUT;
+                    return;
+                }
                 at.stage = *(volatile int *)&dc->stage;
                 at.nf = *(volatile int *)&dc->nf;
-                if (*(volatile int *)&dc->odd) {
-                    at.fa = reinterpret_cast<int32_t *>(B.q1);
-                    at.fb = reinterpret_cast<int32_t *>(B.q0);
-                } else {
-                    at.fa = reinterpret_cast<int32_t *>(B.q0);
-                    at.fb = reinterpret_cast<int32_t *>(B.q1);
-                }
+                again = *(volatile int *)&dc->again != 0;
+                const bool odd = *(volatile int *)&dc->odd != 0;
+                at.fa = reinterpret_cast<int32_t *>(odd ? B.q1 : B.q0);
+                at.fb = reinterpret_cast<int32_t *>(odd ? B.q0 : B.q1);
+                if (again) grp.sync();  // every CTA has read the words
             }
         }
         if (at.stage != REP_DONE) {

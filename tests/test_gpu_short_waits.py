@@ -31,7 +31,8 @@ def short_waits(gpu, oracle, tmp_path_factory):
     root = tmp_path_factory.mktemp("short")
     for f in ("ddp_gb300", "include", "oracle"):
         shutil.copytree(os.path.join(ROOT, f), root / f, ignore=shutil.ignore_patterns("_build", "*.so", "__pycache__"))
-    env = dict(os.environ, DDP_NVCC_EXTRA="-DDDP_SPIN_LIMIT=256u -DDDP_SVC_POLLS=64u -DDDP_SVC_WAIT_NS=2000000LL")
+    env = dict(os.environ, DDP_NVCC_EXTRA="-DDDP_SPIN_LIMIT=512u -DDDP_DYN_LEVELS=16 "
+                                                 "-DDDP_SVC_POLLS=64u -DDDP_SVC_WAIT_NS=2000000LL")
     env.pop("PYTHONPATH", None)
     subprocess.run([sys.executable, "-m", "ddp_gb300.build"], cwd=root, env=env, check=True)
 
@@ -47,7 +48,7 @@ def test_a_query_after_a_timed_out_one_is_exact(short_waits):
     """The grid waits for the phases that CTA 0 runs alone (milliseconds on
     a maze) and gives up; later queries read the same node labels."""
     short_waits("""
-m = d.gen_maze(300, 300, 0.25, 5)
+m = d.gen_maze(500, 500, 0.25, 5)
 dg = d.DeviceGraph.from_csr(m)
 rng = np.random.default_rng(1)
 S, T = rng.integers(0, m.n, 8), rng.integers(0, m.n, 8)
@@ -111,4 +112,38 @@ for k in range(len(ids)):
     i = int(ids[k]) - first - 10
     assert costs[k] == cost(gv, int(S[i]), int(T[i]))
 srv.close()
+""")
+
+
+def test_repairs_of_many_levels_hand_back(short_waits):
+    """Chains of 3,000 nodes: an insert lowers hop bounds along one, a delete
+    cuts the other near its source.  CTA 0 walks a level a node; the grid
+    waits for a few levels at a time.  (K = 100 keeps the searches on the
+    grid, whose waits are short.)"""
+    short_waits("""
+N = 3000
+# s = 0, t = 1; forward chain 2 .. N+1 from s; chain N+2 .. 2N+1 into t by way of two nodes
+s, t, f0, r0, a, b = 0, 1, 2, N + 2, 2 * N + 2, 2 * N + 3
+src = [s, s] + list(range(f0, f0 + N - 1)) + [r0, a, b] + list(range(r0 + 1, r0 + N)) + [f0 + N - 1]
+dst = [t, f0] + list(range(f0 + 1, f0 + N)) + [a, b, t] + list(range(r0, r0 + N - 1)) + [t]
+w = [2 * N + 50] + [1] * (len(src) - 1)
+n = 2 * N + 4
+src, dst, w = (np.array(x) for x in (src, dst, w))
+o = np.argsort(src, kind="stable")
+off = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+g = d.CSR(n, off, dst[o].astype(np.int32), w[o].astype(np.uint32))
+for hk in (d.H_BFS_HOPS, d.H_ZERO):
+    dg = d.DeviceGraph.from_csr(g)
+    dyn = d.DynamicSearch(dg, s, t, hk, K=100)
+    assert dyn.cost == N + 1
+    # hops of the second chain fall by two, node after node; nothing else changes
+    assert dyn.update([1], [r0], [t], [1]) == N + 1
+    assert dyn.update([1], [s], [r0 + N - 1], [2 * N]) == N + 1
+    # cut at the second node: 2,999 nodes lose their label, level by level
+    assert dyn.update([0], [f0], [f0 + 1], [0]) == 2 * N + 50
+    # and come back through an arc to the third
+    got = dyn.update([1], [s], [f0 + 2], [4])
+    assert got == 4 + N - 2, got
+    dyn.close()
+    dg.close()
 """)
