@@ -914,6 +914,9 @@ struct ddp_dyn {
     int64_t stats[10] = {0};
     int grid = 0;      // CTAs of the initial search
     int upd_grid = 0;  // CTAs of an update batch (1: the one-CTA kernel)
+    // a batch failed half way (a full queue, a wait that ran out): the labels
+    // do not fit the graph, the next batch searches anew
+    bool anew = false;
 };
 
 namespace ddp {
@@ -1212,6 +1215,7 @@ static int dyn_launch(ddp_dyn *d, int initial, int nupd, const int *dres = nullp
     d->t_wait_us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - tw).count();
     if (apply_status) *apply_status = out[DYN_OUT_APPLY + 1];
     if (dres && out[DYN_OUT_APPLY + 1]) return DDP_OK;  // nothing ran: the caller applies the batch on the host
+    d->anew = (out[2] & (ST_TIMEOUT | ST_OVERFLOW)) != 0;
     if (out[2] & ST_TIMEOUT) return fail(DDP_ERR_TIMEOUT, "dynamic search: barrier wait timed out");
     if (out[2] & ST_OVERFLOW) return fail(DDP_ERR_QUEUE_OVERFLOW, "dynamic search: queue overflow");
     d->cost = out[0];
@@ -1220,10 +1224,24 @@ static int dyn_launch(ddp_dyn *d, int initial, int nupd, const int *dres = nullp
     return DDP_OK;
 }
 
-}  // namespace ddp
-
-
-namespace ddp {
+// The search from the source on the graph as it is now: exact hops of a
+// reverse BFS, unreached labels, the first launch.
+static int dyn_start(ddp_dyn *d) {
+    ddp_graph *g = d->g;
+    const size_t n = (size_t)g->n;
+    DDP_CUDA(cudaMemsetAsync(d->sa.state, 0xFF, sizeof(unsigned long long) * n, g->stream));
+    DDP_CUDA(cudaMemsetAsync(d->sa.ctl, 0, sizeof(SearchCtl), g->stream));
+    if (d->hkind == DDP_H_BFS_HOPS) {
+        ddp_heuristic *h = nullptr;
+        const int rc = heuristic_build_locked(g, d->t, DDP_H_BFS_HOPS, nullptr, nullptr, &h);
+        if (rc) return rc;
+        const cudaError_t e = cudaMemcpyAsync(d->d_hops, heuristic_hops_ptr(h), sizeof(uint32_t) * n,
+                                              cudaMemcpyDeviceToDevice, g->stream);
+        ddp_heuristic_free(h);
+        if (e != cudaSuccess) return cuda_fail(e, "hops copy");
+    }
+    return dyn_launch(d, 1, 0);
+}
 
 // Switches g to the dynamic layout (rows with slack and explicit ends) and
 // builds its host mirror, once.
@@ -1409,7 +1427,6 @@ int ddp_dyn_create(ddp_graph *g, int32_t source, int32_t target, int32_t hkind, 
     d->cold_cap = capf;
     if (e1 == cudaSuccess) e1 = cudaMalloc(&d->d_cold, sizeof(uint2) * (size_t)capf);
     if (e1 != cudaSuccess) return bail(cuda_fail(e1, "cudaMalloc(dynamic state)"));
-    DDP_CUDA(cudaMemsetAsync(d->sa.ctl, 0, sizeof(SearchCtl), g->stream));
     int per_sm = 0, sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dyn<GridGroup>, 512, 0);
@@ -1425,18 +1442,7 @@ int ddp_dyn_create(ddp_graph *g, int32_t source, int32_t target, int32_t hkind, 
     // alone either way; the grid is there for the wide ones (the first split
     // of the open list alone took one CTA 7.1 ms on 1M nodes).
     d->upd_grid = d->o.group > 0 ? std::min(coresident, d->o.group) : d->grid;
-    if (hkind == DDP_H_BFS_HOPS) {
-        // exact reverse BFS from the target into the dynamic hop array
-        ddp_heuristic *h = nullptr;
-        g->mu.unlock();
-        rc = ddp_heuristic_build(g, target, DDP_H_BFS_HOPS, nullptr, nullptr, &h);
-        g->mu.lock();
-        if (rc) return bail(rc);
-        cudaError_t ce = cudaMemcpy(d->d_hops, heuristic_hops_ptr(h), sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice);
-        ddp_heuristic_free(h);
-        if (ce != cudaSuccess) return bail(cuda_fail(ce, "hops copy"));
-    }
-    rc = dyn_launch(d, 1, 0);
+    rc = dyn_start(d);
     if (rc) return bail(rc);
     *out = d;
     return DDP_OK;
@@ -1455,6 +1461,13 @@ int ddp_dyn_update(ddp_dyn *d, int32_t nupd, const int32_t *flag, const int32_t 
         d->d_upd = nullptr;
         DDP_CUDA(cudaMalloc(&d->d_upd, sizeof(int4) * std::max(nupd, 1)));
         d->upd_cap = nupd;
+    }
+    if (d->anew) {
+        int rc = dyn_graph_apply(g, nupd, flag, u, v, w, ups, true);
+        if (!rc) rc = dyn_start(d);
+        if (rc) return rc;
+        if (out_cost) *out_cost = d->cost;
+        return DDP_OK;
     }
     // on the device when the batch fits one CTA: k_apply, then k_dyn on the
     // same stream (one upload, one synchronisation)
@@ -1484,7 +1497,10 @@ int ddp_dyn_update(ddp_dyn *d, int32_t nupd, const int32_t *flag, const int32_t 
     // no synchronisation after the graph scatters: k_dyn runs on the same
     // stream, and dyn_launch synchronises it before returning
     rc = dyn_graph_apply(g, nupd, flag, u, v, w, ups, false);
-    if (rc) return rc;
+    if (rc) {
+        d->anew = true;  // part of the batch may be in the graph
+        return rc;
+    }
     const auto t1 = std::chrono::steady_clock::now();
     const int32_t k = (int32_t)ups.size();
     if (k > d->upd_cap) {

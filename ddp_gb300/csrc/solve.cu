@@ -1222,14 +1222,10 @@ static bool solve_bidir_first(const ddp_graph *g, int kind, const ddp_opts &o) {
 uint32_t *heuristic_hops_ptr(const ddp_heuristic *h) { return h ? h->d_hops : nullptr; }
 }  // namespace ddp
 
-extern "C" {
-
-int ddp_heuristic_build(ddp_graph *g, int32_t target, int32_t kind, const int32_t *user_h,
-                        int32_t *out_h, ddp_heuristic **out) {
-    if (!g || !out) return fail(DDP_ERR_INVALID, "null argument");
-    *out = nullptr;
-    if (target < 0 || target >= g->n) return fail(DDP_ERR_INVALID, "target out of range");
-    std::lock_guard<std::mutex> lk(g->mu);
+namespace ddp {
+// ddp_heuristic_build with the arguments checked and the graph's lock held.
+int heuristic_build_locked(ddp_graph *g, int32_t target, int32_t kind, const int32_t *user_h, int32_t *out_h,
+                           ddp_heuristic **out) {
     ddp_heuristic *h = new ddp_heuristic();
     h->g = g;
     graph_ref(g);
@@ -1328,8 +1324,16 @@ int ddp_heuristic_build(ddp_graph *g, int32_t target, int32_t kind, const int32_
     *out = h;
     return DDP_OK;
 }
+}  // namespace ddp
 
-}  // extern "C"
+extern "C" int ddp_heuristic_build(ddp_graph *g, int32_t target, int32_t kind, const int32_t *user_h, int32_t *out_h,
+                                   ddp_heuristic **out) {
+    if (!g || !out) return fail(DDP_ERR_INVALID, "null argument");
+    *out = nullptr;
+    if (target < 0 || target >= g->n) return fail(DDP_ERR_INVALID, "target out of range");
+    std::lock_guard<std::mutex> lk(g->mu);
+    return heuristic_build_locked(g, target, kind, user_h, out_h, out);
+}
 
 namespace ddp {
 // d(src, v) for every v (reverse: d(v, src)) into the device array dist.

@@ -141,6 +141,8 @@ int slots_alloc(SlotArrays &sa, int32_t n, int nslots, int64_t cap_q, int64_t ca
                 cudaStream_t st, int hbits = 0);
 void slots_free(SlotArrays &sa);
 uint32_t *heuristic_hops_ptr(const ddp_heuristic *h);
+int heuristic_build_locked(ddp_graph *g, int32_t target, int32_t kind, const int32_t *user_h, int32_t *out_h,
+                           ddp_heuristic **out);
 cudaError_t launch_slots(int hk, int grid, int block, bool coop, DevGraph G, SlotArrays sa, BatchArgs A,
                          cudaStream_t st);
 int slots_per_sm(int hk, int block, bool grouped);

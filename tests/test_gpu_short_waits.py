@@ -147,3 +147,36 @@ for hk in (d.H_BFS_HOPS, d.H_ZERO):
     dyn.close()
     dg.close()
 """)
+
+
+def test_a_failed_update_does_not_spoil_later_ones(short_waits):
+    """A chain that CTA 0 follows for milliseconds: the update that opens it
+    fails.  Later updates never answer from the labels it left."""
+    short_waits("""
+N = 6000
+s, t, f0 = 0, 1, 2
+src = [s, s] + list(range(f0, f0 + N))
+dst = [t, f0] + list(range(f0 + 1, f0 + N)) + [t]
+w = [5] + [1] * (len(src) - 1)
+n = N + 4
+off = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+g = d.CSR(n, off, np.array(dst, np.int32), np.array(w, np.uint32))
+for hk in (d.H_ZERO, d.H_BFS_HOPS):
+    dg = d.DeviceGraph.from_csr(g)
+    dyn = d.DynamicSearch(dg, s, t, hk, delta=1)
+    assert dyn.cost == 5
+    try:
+        dyn.update([0], [s], [t], [0])
+        raise SystemExit("the wait did not run out")
+    except d.DdpError as e:
+        assert e.code == 6, e
+    try:
+        assert dyn.update([1], [n - 1], [n - 2], [1]) == N + 1  # far from every path
+    except d.DdpError as e:
+        assert e.code == 6, e
+    assert dyn.update([1], [s], [t], [7]) == 7
+    assert dyn.update([1], [f0], [t], [3]) == 4
+    assert dyn.path().tolist() == [s, f0, t]
+    dyn.close()
+    dg.close()
+""")
