@@ -317,11 +317,26 @@ __device__ inline int32_t write_path_bidir(const DevGraph &G, const Rec &R, uint
         if (lane == 0) atomicOr(status, ST_TIMEOUT);  // no meeting arc: report the query failed
         return 0;
     }
-    // x..s by forward parents (lane 0) and y..t by reverse successors (lane 1)
+    // Arcs of weight 0: the halves may share nodes (of a cycle of weight 0
+    // through the meeting arc), each with both labels adding up to the cost.
+    // The path leaves the forward half at the one nearest to s: no node before
+    // it has such labels, so none is on its reverse half.
+    int32_t jx = x, jy = y;  // where the halves join: jx -> jy
+    if (G.wmin == 0) {
+        int32_t len = 0, up;
+        for (int32_t c = x; c >= 0 && len <= G.n; c = c == s ? -1 : up, len++) {
+            const uint32_t gf = lab(c, 0, &up);
+            if ((uint64_t)gf + lab(c, 1, &lk) == cost) {
+                jx = c;
+                jy = c == t ? -1 : lk;
+            }
+        }
+    }
+    // jx..s by forward parents (lane 0) and jy..t by reverse successors (lane 1)
     int32_t len = 0;
     if (lane < 2) {
         const int32_t end = lane ? t : s;
-        for (int32_t c = lane ? y : x; c >= 0 && len <= G.n;) {
+        for (int32_t c = lane ? jy : jx; c >= 0 && len <= G.n;) {
             if (len < PATH_BUF) buf[lane * PATH_BUF + len] = c;
             len++;
             if (c == end) break;
@@ -340,7 +355,7 @@ __device__ inline int32_t write_path_bidir(const DevGraph &G, const Rec &R, uint
     } else if (lane < 2) {
         // longer than the buffer: a second walk writes it
         int32_t i = lane ? lf : lf - 1;
-        for (int32_t c = lane ? y : x; c >= 0 && i >= 0 && i < lf + lr; i += lane ? 1 : -1) {
+        for (int32_t c = lane ? jy : jx; c >= 0 && i >= 0 && i < lf + lr; i += lane ? 1 : -1) {
             if (i < cap) path[i] = c;
             lab(c, (uint32_t)lane, &lk);
             c = lk;

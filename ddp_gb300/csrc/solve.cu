@@ -189,6 +189,7 @@ template <bool WALKED>
 __device__ void solve_report(const DevGraph &G, const SlotBufs &B, const SearchParams &P, const SearchResult &r,
                              SolveOut *out, int32_t *path, int32_t path_cap, const int32_t *buf, int32_t len) {
     if (WALKED) len = write_path_cta(B, P.s, P.t, path, path_cap, G.n, &B.ctl->status, buf, len);
+    len = min(len, path_cap);  // what path holds (a longer one set ST_PATH_TRUNC)
     for (int32_t i = threadIdx.x; i < min(len, SOLVE_PATH); i += blockDim.x) out->path[i] = __ldcg(path + i);
     if (threadIdx.x == 0) {
         out->cost = r.cost >= INF_G ? DDP_INF : (int32_t)r.cost;
@@ -1565,7 +1566,7 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
             cudaError_t e = cudaLaunchKernel(fn, dim3(1), dim3(1024), args, 0, st);
             if (e != cudaSuccess) return cuda_fail(e, "k_solve_bidir launch");
             DDP_CUDA(cudaStreamSynchronize(st));
-            if (!(w->h_res->status & (ST_OVERFLOW | ST_TIMEOUT | ST_BUDGET))) return result(w);
+            if (!(w->h_res->status & (ST_OVERFLOW | ST_TIMEOUT | ST_BUDGET | ST_PATH_TRUNC))) return result(w);
             // a long search: the whole GPU takes it
         }
     }
