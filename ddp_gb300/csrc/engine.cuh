@@ -505,6 +505,7 @@ struct SearchParams {
     // Euclidean: 1.11 against 1.30 ms).
     uint32_t delta_loose = 0;
     int64_t budget = 0;  // bidirectional search: entries it may expand (0: any number)
+    bool skewed = false;  // ... and the graph has hubs (skewed_rows)
 };
 
 struct SearchResult {

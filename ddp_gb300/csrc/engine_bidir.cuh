@@ -97,9 +97,26 @@ constexpr int WAVE_FILL = 32;
 // bucket per wave, and when its ball grows at last all of it counts as
 // opened (4M nodes: 472k expansions and 33 ms for one such query, 15k and
 // 1.3 ms with 2).  Frontiers on graphs with coordinates grow slowly and
-// profit from more overlap (maze, 2 -> 25.9 ms, 8 -> 19.4, 16 -> 19.1).
+// profit from more overlap (maze, 2 -> 25.9 ms, 8 -> 19.4, 16 -> 19.1).  On
+// graphs with hubs (skewed_rows) none are opened ahead: once a hub is reached,
+// its children up to the last bucket opened are expanded in one wave, and the
+// other hubs with them (the digraph above, 2,000 pairs: up to 206,000 expansions
+// for a query, 37 ms; 3,800 and 2.5 ms with none).
 constexpr uint32_t WAVE_AHEAD = 2, WAVE_AHEAD_XY = 16;
 constexpr int WAVE_FILTER = 1024;  // words of a direction's settled filter (32,768 bits)
+// Long rows: a wave's teams are a few lanes, chosen for the number of its
+// entries.  A row that would take its team more than LONG_STEPS steps goes to
+// the next wave in segments instead, which are entries like others there, so
+// that no wave waits for a hub.  With the rule on opening ahead below, a digraph
+// of 200,000 nodes with degrees by a power law (rows up to 19,000 arcs): 300
+// pairs 44.1 -> 1.08 ms, 2,000 81.4 -> 2.5, 500 requests served 53 -> 1.2.  On
+// graphs without long rows it costs 1 % (4,096 pairs on 4M nodes 3.43 -> 3.47 ms);
+// walking such rows in a pass of their own behind the wave cost 8-20 %, its code
+// taking registers and instruction fetches from the wave loop.
+constexpr int LONG_STEPS = 16;
+constexpr int LONG_SEG = 256;   // arcs of a segment (more for rows of more than LONG_SEGS segments)
+constexpr int LONG_SEGS = 1024;
+constexpr uint32_t SEG_BIT = 0x40000000u;  // in an entry's node: a segment (graphs of at most 2^30 nodes)
 
 // What a wave expands, decided between two waves by the CTA's first warp.
 struct WavePlan {
@@ -538,18 +555,32 @@ __device__ __forceinline__ uint64_t bi_key_bound(uint32_t mu) {
 
 // What an open entry holds: {node | dir << 31, key} and, with lazy labels, the
 // parent, with potentials, the label g that the key was made from.
-template <bool WIDE>
+// Segment k of a long row: the entry with SEG_BIT, and k in the place of what
+// it can do without: the parent with lazy labels (installed by now), the key
+// in the short form (the label is read from the record).
+template <bool LAZY, bool POT>
 struct WaveEntry {
     using T = uint4;
     __device__ static T make(uint32_t vd, uint32_t key, uint32_t x) { return make_uint4(vd, key, x, 0u); }
     __device__ static uint32_t extra(const T &e) { return e.z; }
+    __device__ static T segment(const T &e, uint32_t k) {
+        return LAZY ? make_uint4(e.x | SEG_BIT, e.y, k, 0u) : make_uint4(e.x | SEG_BIT, e.y, e.z, k);
+    }
+    __device__ static uint32_t segment(const T &e) { return LAZY ? e.z : e.w; }
 };
 template <>
-struct WaveEntry<false> {
+struct WaveEntry<false, false> {
     using T = uint2;
     __device__ static T make(uint32_t vd, uint32_t key, uint32_t) { return make_uint2(vd, key); }
     __device__ static uint32_t extra(const T &e) { return e.y; }  // no potentials: the key is g
+    __device__ static T segment(const T &e, uint32_t k) { return make_uint2(e.x | SEG_BIT, k); }
+    __device__ static uint32_t segment(const T &e) { return e.y; }
 };
+
+// Arcs of one segment of a row of len arcs.
+__device__ __forceinline__ int long_seg(int len) {
+    return len <= LONG_SEG * LONG_SEGS ? LONG_SEG : (len + LONG_SEGS - 1) / LONG_SEGS;
+}
 
 // ep: the slot's epoch for this query (never 0; units of other epochs read
 // as unreached).
@@ -557,7 +588,7 @@ template <bool LAZY, class Pot, class Rec>
 __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const SlotBufs &B, const SearchParams &P, uint32_t ep,
                                       WaveQ *q, const Pot &pot, const Rec &R) {
     static_assert(!(LAZY && Pot::on), "lazy labels are keyed by g");
-    using WE = WaveEntry<LAZY || Pot::on>;
+    using WE = WaveEntry<LAZY, Pot::on>;
     using E = typename WE::T;
     SearchCtl *ctl = B.ctl;
     const int lane = lane_id();
@@ -565,7 +596,8 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
     // (two 32-byte records per lane would not fit the registers)
     constexpr int AU = LAZY ? 4 : Pot::on || !Rec::logs ? 1 : 2;
     // (eager labels without potentials: coordinates, or a flooding search)
-    const uint32_t ahead = G.xy || (!LAZY && !Pot::on) ? WAVE_AHEAD_XY : WAVE_AHEAD;
+    const uint32_t seg_bit = G.n <= (int)SEG_BIT ? SEG_BIT : 0u, node_mask = NODE_MASK & ~seg_bit;
+    const uint32_t ahead = P.skewed ? 0u : G.xy || (!LAZY && !Pot::on) ? WAVE_AHEAD_XY : WAVE_AHEAD;
     // the slot's far memory: 2 x 32 lists (at most a quarter), two halves of a
     // pile, two spill areas for waves that outgrow shared memory (a sixteenth
     // each)
@@ -734,18 +766,37 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
         }
         push((uint32_t)v | (dir << 31), nk, ng);
     };
+    // whether a team of 2^tsh lanes leaves a row of len arcs to the next wave
+    auto too_long = [&](int len, int tsh) -> bool {
+        return len > max(2 * LONG_SEG, LONG_STEPS * AU << tsh) && seg_bit;
+    };
+    // lane sub of tw: its share of the segments of entry en (key, dir), a row of len arcs
+    auto to_segments = [&](const E en, uint32_t key, uint32_t dir, int len, int sub, int tw) {
+        const int seg = long_seg(len);
+        for (int k = sub; k * (int64_t)seg < len; k += tw)
+            if (!to_near(WE::segment(en, (uint32_t)k), key, dir, wv + 1)) atomicOr(&q->status, ST_OVERFLOW);
+    };
     // expands one entry with a team of 2^tsh lanes
     auto expand = [&](const E en, const int tsh) {
         const int tw = 1 << tsh, sub = lane & (tw - 1);
         const uint32_t vd = en.x, key = en.y;
         const uint32_t dir = vd >> 31;
-        const int u = (int)(vd & NODE_MASK);
+        const int u = (int)(vd & node_mask);
+        const bool segment = (vd & seg_bit) != 0;
         const uint32_t lbo = dir ? lb0 : lb1;
         // row bounds load beside the record
-        const int r0 = dir ? row_begin(G.roff, G.roend, u) : row_begin(G.off, G.oend, u);
-        const int r1 = dir ? row_end(G.roff, G.roend, u) : row_end(G.off, G.oend, u);
+        int r0 = dir ? row_begin(G.roff, G.roend, u) : row_begin(G.off, G.oend, u);
+        int r1 = dir ? row_end(G.roff, G.roend, u) : row_end(G.off, G.oend, u);
         const uint2 *arcs = dir ? G.rarc : G.arc;
         uint2 a[AU];
+        // (here, after the record's load: looking at the bounds any earlier
+        // would wait for them first)
+        auto cut = [&] {
+            if (!segment) return;
+            const int seg = long_seg(r1 - r0);
+            r0 += (int)WE::segment(en) * seg;
+            r1 = min(r1, r0 + seg);
+        };
         auto load_arcs = [&](int j) {
 #pragma unroll
             for (int k = 0; k < AU; k++)
@@ -758,7 +809,9 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
             gu = key;
             typename Rec::U *w = nullptr;
             typename Rec::U c{};
-            if (sub == 0 && key < key_limit(mu_now(), lbo)) {
+            if (segment) {
+                ok = true;  // installed when the row was set aside
+            } else if (sub == 0 && key < key_limit(mu_now(), lbo)) {
                 typename Rec::U *rv = R.claim(u, ep);
                 if (rv) {
                     w = rv + dir;
@@ -767,6 +820,7 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
                     atomicOr(&q->status, ST_OVERFLOW);  // the slot's table is full
                 }
             }
+            cut();
             load_arcs(r0 + sub);  // beside the label's compare-and-swap
             if (w) {
                 const typename Rec::U nv = Rec::make(ep, gu, WE::extra(en), dir ? 0u : R.keyw(u));
@@ -793,11 +847,16 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
             gu = WE::extra(en);
             const typename Rec::U *ru = R.find(u, ep);
             const uint32_t gl = Rec::g(Rec::ld(ru + dir), ep);
+            cut();
             load_arcs(r0 + sub);
             // current, and a path through it may still be shorter
             ok = gl == gu && key < key_limit(mu_now(), lbo);
         }
         if (!ok) return;
+        if (too_long(r1 - r0, tsh) && !segment) {
+            to_segments(en, key, dir, r1 - r0, sub, tw);
+            return;
+        }
         if (sub == 0) {
             n_exp++;
             n_scan += (unsigned long long)(r1 - r0);
@@ -882,8 +941,9 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
     // maze 18.6 -> 19.9 ms): their stages are short or rare.
     auto expand_warp = [&](const bool have, const E en, const int tsh) {
         const int tw = 1 << tsh, sub = lane & (tw - 1);
-        const uint32_t dir = en.x >> 31, gu = WE::extra(en);
-        const int u = (int)(en.x & NODE_MASK);
+        const uint32_t dir = en.x >> 31;
+        const int u = (int)(en.x & node_mask);
+        const bool segment = (en.x & seg_bit) != 0;
         const uint32_t lbo = dir ? lb0 : lb1;
         const uint2 *arcs = dir ? G.rarc : G.arc;
         int r0 = 0, r1 = 0;
@@ -893,7 +953,13 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
             r0 = dir ? row_begin(G.roff, G.roend, u) : row_begin(G.off, G.oend, u);
             r1 = dir ? row_end(G.roff, G.roend, u) : row_end(G.off, G.oend, u);
             gl = Rec::g(Rec::ld(R.find(u, ep) + dir), ep);
+            if (segment) {
+                const int seg = long_seg(r1 - r0);
+                r0 += (int)WE::segment(en) * seg;
+                r1 = min(r1, r0 + seg);
+            }
         }
+        const uint32_t gu = segment ? gl : WE::extra(en);  // a segment goes by the label as it is now
         uint2 a[AU];
         auto load_arcs = [&](int j) {
 #pragma unroll
@@ -903,7 +969,11 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
         };
         load_arcs(r0 + sub);
         // current, and a path through it may still be shorter
-        const bool ok = have && gl == gu && en.y < key_limit(mu_now(), lbo);
+        bool ok = have && gl == gu && gu < key_limit(mu_now(), lbo);
+        if (ok && too_long(r1 - r0, tsh) && !segment) {
+            to_segments(en, gu, dir, r1 - r0, sub, tw);
+            ok = false;
+        }
         if (ok && sub == 0) {
             n_exp++;
             n_scan += (unsigned long long)(r1 - r0);

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "graph.cuh"
+#include "rules.h"
 
 namespace ddp {
 
@@ -107,6 +108,12 @@ static int upload_csr(ddp_graph *g, const int32_t *off, const int32_t *col, cons
     }
     for (int32_t v = 0; v < n; v++) roff[(size_t)v + 1] += roff[(size_t)v];
     const int64_t live = roff[(size_t)n];
+    int64_t in_long = 0;
+    for (int32_t v = 0; v < n; v++) {
+        in_long += long_row_arcs(off[v + 1] - off[v]);
+        in_long += long_row_arcs(roff[(size_t)v + 1] - roff[(size_t)v]);
+    }
+    g->skewed = skewed_rows(in_long, e + live);
     std::vector<uint2> rarc((size_t)(live > 0 ? live : 1));
     std::vector<int32_t> fill(roff.begin(), roff.end() - 1);
     for (int32_t u = 0; u < n; u++)

@@ -28,4 +28,10 @@ DDP_RULE int local_handback(int m, int list_cap, int64_t cap_q) {
 // than 32 threads there would be none.
 DDP_RULE int block_threads(int want, int top) { return want >= top ? top : (want + 31) & ~31; }
 
+// Whether a graph's degrees are skewed: rows of more than 256 arcs hold a
+// sixteenth of its arcs or more (of 2e, forward and reverse).  The bidirectional
+// search opens no buckets ahead there (WAVE_AHEAD).
+DDP_RULE int64_t long_row_arcs(int64_t len) { return len > 256 ? len : 0; }
+DDP_RULE bool skewed_rows(int64_t in_long, int64_t arcs) { return in_long > 0 && in_long >= arcs / 16; }
+
 }  // namespace ddp

@@ -524,6 +524,7 @@ __device__ __forceinline__ void batch_loop(const Grp &grp, const DevGraph &G0, c
             continue;
         }
         SearchParams P{s, t, A.delta, A.K, 0, 0};
+        P.skewed = A.skewed;
         SearchResult r;
         if (HK == 1) {
             const uint32_t tag = *(volatile uint32_t *)&ctl->tag;
@@ -1071,6 +1072,7 @@ void bidir_args(const ddp_graph *g, int32_t delta, BatchArgs *A) {
     // the second start).  Too low a budget starts long random searches again
     // (8 sqrt(n): 4.7 ms for the 4M-node batch that takes 3.7).
     A->lazy_budget = 4096 + (int64_t)(24.0 * std::sqrt((double)g->n));
+    A->skewed = g->skewed;
     A->eager_delta = delta > 0 ? (uint32_t)delta : auto_delta(g);
 }
 
@@ -1561,6 +1563,7 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
             SearchParams Pb = P;
             Pb.delta = auto_delta_bidir(g);
             Pb.budget = SOLVE_BIDIR_BUDGET;
+            Pb.skewed = g->skewed;
             void *args[] = {&G, &w->pa, &Pb, &w->d_res, &w->d_path, &g->n};
             const void *fn = pair16_hk(w->pa_hk) ? (const void *)k_solve_bidir<9> : (const void *)k_solve_bidir<5>;
             cudaError_t e = cudaLaunchKernel(fn, dim3(1), dim3(1024), args, 0, st);
@@ -1835,7 +1838,7 @@ static bool same_args(const BatchArgs &x, const BatchArgs &y) {
            x.paths == y.paths && x.path_cap == y.path_cap && x.qstatus == y.qstatus && x.stats == y.stats &&
            x.tstart == y.tstart && x.tend == y.tend && x.work == y.work && x.status == y.status && x.order == y.order &&
            x.delta == y.delta && x.K == y.K && x.bfs_budget == y.bfs_budget && x.lazy_budget == y.lazy_budget &&
-           x.eager_delta == y.eager_delta && x.group == y.group &&
+           x.eager_delta == y.eager_delta && x.skewed == y.skewed && x.group == y.group &&
            x.sync_engine == y.sync_engine;
 }
 

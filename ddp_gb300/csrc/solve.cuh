@@ -76,6 +76,7 @@ struct BatchArgs {
     int64_t bfs_budget;  // capped heuristic BFS (0 = run to completion)
     int64_t lazy_budget;   // entries a search may expand before it starts again with eager labels
     uint32_t eager_delta;  // bucket width of that second start
+    bool skewed;           // the graph has hubs (skewed_rows)
     int group;           // CTAs per query slot
     int sync_engine;     // 1: phase-synchronous engine even for one-CTA slots
     // serving mode (continuous batching): requests are published in host

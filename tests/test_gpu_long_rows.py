@@ -1,0 +1,72 @@
+"""Hubs in the bidirectional searches: rows around the lengths at which a
+team hands a row on in segments (512 arcs; segments of 256, longer ones past
+1,024 of them), forward and reverse, on every record layout, in batches, single
+queries and served requests.  Costs against the oracle, every path valid."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _hub_graph(d, L, wmax, seed):
+    """A hub with L arcs out (node 0), one with L arcs in (node 1), L nodes
+    between them, and two random arcs a node."""
+    rng = np.random.default_rng(seed)
+    n = L + 40
+    mid = np.arange(2, 2 + L)
+    src = np.concatenate([np.zeros(L, np.int64), mid, rng.integers(0, n, 2 * n)])
+    dst = np.concatenate([mid, np.ones(L, np.int64), rng.integers(0, n, 2 * n)])
+    keep = src != dst
+    src, dst = src[keep], dst[keep]
+    o = np.argsort(src, kind="stable")
+    off = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+    return d.CSR(n, off, dst[o].astype(np.int32), rng.integers(1, wmax + 1, len(src)).astype(np.uint32))
+
+
+@pytest.mark.parametrize("wmax", [4, 1000])
+@pytest.mark.parametrize("L", [255, 511, 512, 513, 1025, 5000, 262143, 262145])
+def test_rows_in_segments(gpu, oracle, L, wmax):
+    d, O = gpu, oracle
+    g = _hub_graph(d, L, wmax, L + wmax)
+    rng = np.random.default_rng(L)
+    q = 64 if L < 100000 else 16
+    S, T = (rng.integers(0, g.n, q).astype(np.int32) for _ in range(2))
+    # from and to the hubs, and to the nodes at the ends of segments
+    S[:6], T[:6] = [0, 0, 0, 5, 2 + L - 1, 0], [1, 2 + L - 1, 2 + min(L - 1, 256), 1, 1, 3]
+    gs = g.with_sentinel()
+    want, _, _, done = O.astar_many(gs.n, gs.off[:-1], gs.col, gs.w, S, T, hkind=0, mode=O.HEAP_POSMAP, threads=4,
+                                    budget_s=1e9)
+    assert done == q
+
+    def check(p, i):
+        if want[i] != d.INF:
+            ok, why = O.check_path(g.off, g.col, g.w, p, int(S[i]), int(T[i]), int(want[i]))
+            assert ok, (i, why)
+
+    for coords in (False, True):
+        dg = d.DeviceGraph.from_csr(g)
+        if coords:
+            dg.set_coords(rng.integers(0, 1000, (g.n, 2)).astype(np.int32))
+            dg.set_euclid(0)  # potentials of 0: consistent whatever the coordinates
+        dg.build_landmarks(8, seed=1, bits=8)
+        kinds = [(d.H_BIDIR, {}), (d.H_BIDIR, {"block": 32}), (d.H_LANDMARK, {})]
+        kinds += [(d.H_BIDIR_EUCLID, {})] if coords else [(d.H_BIDIR, {"flags": d.OPT_HASH})]
+        for kind, kw in kinds:
+            eng = d.BatchEngine(dg, kind, **kw)
+            cost, _ = eng.solve(S, T)
+            assert np.array_equal(cost, want), (coords, kind, kw)
+            for i in range(0, q, 5):
+                check(eng.path(i), i)
+            eng.close()
+        for i in range(8):
+            r = dg.solve(int(S[i]), int(T[i]))
+            assert r.cost == want[i]
+            check(r.path, i)
+        dg.close()
+    dg = d.DeviceGraph.from_csr(g)
+    srv = d.Server(dg, d.H_BIDIR, max_requests=256)
+    first = srv.submit(S, T)
+    ids, cost, _, _ = srv.drain()
+    assert np.array_equal(cost, want[ids - first])
+    srv.close()
+    dg.close()

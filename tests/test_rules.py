@@ -13,6 +13,8 @@ SHIM = """
 extern "C" {
 int local_handback(int m, int list_cap, int64_t cap_q) { return ddp::local_handback(m, list_cap, cap_q); }
 int block_threads(int want, int top) { return ddp::block_threads(want, top); }
+int64_t long_row_arcs(int64_t len) { return ddp::long_row_arcs(len); }
+int skewed_rows(int64_t in_long, int64_t arcs) { return ddp::skewed_rows(in_long, arcs); }
 }
 """
 
@@ -41,3 +43,12 @@ def test_blocks_are_whole_warps(rules, top):
     for want in (1, 16, 31, 32, 33, 48, 100, 511, 512, 513, 1023, 1025, (1 << 31) - 1):
         got = rules.block_threads(want, top)
         assert got % 32 == 0 and got >= min(want, top) and got <= min(want + 31, top)
+
+
+@pytest.mark.parametrize("e", [1, 15, 16, 1000, 5_000_000_000])
+def test_graphs_with_hubs(rules, e):
+    long_arcs, skew = rules.long_row_arcs, rules.skewed_rows
+    long_arcs.restype = C.c_int64
+    assert [long_arcs(C.c_int64(x)) for x in (0, 256, 257, 1 << 40)] == [0, 0, 257, 1 << 40]
+    f = lambda k: bool(skew(C.c_int64(k), C.c_int64(e)))  # noqa: E731
+    assert not f(0) and f(e) and f(max(e // 16, 1)) and (e // 16 < 2 or not f(e // 16 - 1))
