@@ -914,8 +914,8 @@ struct ddp_dyn {
     int64_t stats[10] = {0};
     int grid = 0;      // CTAs of the initial search
     int upd_grid = 0;  // CTAs of an update batch (1: the one-CTA kernel)
-    // a batch failed half way (a full queue, a wait that ran out): the labels
-    // do not fit the graph, the next batch searches anew
+    // a batch failed half way (a wait that ran out, no memory for longer
+    // queues): the labels do not fit the graph, the next batch searches anew
     bool anew = false;
 };
 
@@ -1243,6 +1243,35 @@ static int dyn_start(ddp_dyn *d) {
     return dyn_launch(d, 1, 0);
 }
 
+// dyn_start with the queues grown until they hold the search: a hub reached
+// again and again under smaller labels, or rows of hundreds of arcs, push more
+// entries between two compactions than twice the nodes.
+static int dyn_start_growing(ddp_dyn *d) {
+    for (int attempt = 0;; attempt++) {
+        const int rc = dyn_start(d);
+        if (rc != DDP_ERR_QUEUE_OVERFLOW || attempt == 5) return rc;
+        SlotArrays sa;
+        uint2 *cold = nullptr;
+        const int64_t cap_q = 2 * d->sa.cap_q, cap_f = 2 * d->sa.cap_f;
+        int rc2 = slots_alloc(sa, d->g->n, 1, cap_q, cap_f, 0, d->g->stream);
+        if (!rc2) {
+            const cudaError_t e = cudaMalloc(&cold, sizeof(uint2) * (size_t)cap_f);
+            if (e != cudaSuccess) rc2 = cuda_fail(e, "cudaMalloc(dynamic state)");
+        }
+        if (rc2) {  // no memory for more: the search stays as it is
+            slots_free(sa);
+            d->anew = true;
+            return rc2;
+        }
+        slots_free(d->sa);
+        cudaFree(d->d_cold);
+        d->sa = sa;
+        d->d_cold = cold;
+        d->cold_cap = cap_f;
+        trace("dyn: queues grown to %lld near, %lld far entries", (long long)cap_q, (long long)cap_f);
+    }
+}
+
 // Switches g to the dynamic layout (rows with slack and explicit ends) and
 // builds its host mirror, once.
 int dyn_graph_prepare(ddp_graph *g) {
@@ -1442,7 +1471,7 @@ int ddp_dyn_create(ddp_graph *g, int32_t source, int32_t target, int32_t hkind, 
     // alone either way; the grid is there for the wide ones (the first split
     // of the open list alone took one CTA 7.1 ms on 1M nodes).
     d->upd_grid = d->o.group > 0 ? std::min(coresident, d->o.group) : d->grid;
-    rc = dyn_start(d);
+    rc = dyn_start_growing(d);
     if (rc) return bail(rc);
     *out = d;
     return DDP_OK;
@@ -1464,7 +1493,7 @@ int ddp_dyn_update(ddp_dyn *d, int32_t nupd, const int32_t *flag, const int32_t 
     }
     if (d->anew) {
         int rc = dyn_graph_apply(g, nupd, flag, u, v, w, ups, true);
-        if (!rc) rc = dyn_start(d);
+        if (!rc) rc = dyn_start_growing(d);
         if (rc) return rc;
         if (out_cost) *out_cost = d->cost;
         return DDP_OK;
@@ -1475,6 +1504,7 @@ int ddp_dyn_update(ddp_dyn *d, int32_t nupd, const int32_t *flag, const int32_t 
     if (rc == DDP_OK) {
         int st = 0;
         rc = dyn_launch(d, 0, 0, d->d_out + DYN_OUT_APPLY, &st);
+        if (rc == DDP_ERR_QUEUE_OVERFLOW) rc = dyn_start_growing(d);  // the batch is in the graph
         if (rc) return rc;
         if (!st) {
             if (trace_on()) {
@@ -1511,6 +1541,7 @@ int ddp_dyn_update(ddp_dyn *d, int32_t nupd, const int32_t *flag, const int32_t 
     }
     if (k) DDP_CUDA(cudaMemcpyAsync(d->d_upd, ups.data(), sizeof(int4) * k, cudaMemcpyHostToDevice, g->stream));
     rc = dyn_launch(d, 0, k);
+    if (rc == DDP_ERR_QUEUE_OVERFLOW) rc = dyn_start_growing(d);
     if (rc) return rc;
     if (trace_on()) {
         const auto t2 = std::chrono::steady_clock::now();

@@ -99,3 +99,37 @@ def test_dynamic_paths_around_the_host_buffer(gpu, length):
     assert dyn.update(*_batch([(2, 0, 1, 7)])) == (2 * (length - 1) + 5 if length > 1 else 0)
     assert np.array_equal(dyn.path(), np.arange(length))
     dyn.close()
+
+
+def test_queues_grow_with_the_search(gpu, oracle):
+    """Rows of hundreds of arcs push more entries than the queues are made
+    for (twice the nodes): they grow, and every cost is exact."""
+    d = gpu
+    rng = np.random.default_rng(4)
+    n, deg = 3000, 400
+    off = np.arange(0, n * deg + 1, deg).astype(np.int32)
+    col = rng.integers(0, n, n * deg).astype(np.int32)
+    w = rng.integers(1, 1001, n * deg).astype(np.uint32)
+    g = d.CSR(n, off, col, w)
+    for hk in (d.H_BFS_HOPS, d.H_ZERO):
+        dg = d.DeviceGraph.from_csr(g)
+        dyn = d.DynamicSearch(dg, 5, 77, hk)
+        o, c, ww = off[:-1].copy(), col.copy(), w.copy()
+
+        def want():
+            f, x, _, _, _ = oracle.astar(n, o, c, ww, np.zeros(n, np.int32), 5, 77, mode=oracle.HEAP_POSMAP)
+            return x if f else d.INF
+        assert dyn.cost == want()
+        for k in range(4):
+            p = dyn.path()
+            # the path's arcs go, 300 others change
+            j = rng.choice(n * deg, 300, replace=False)
+            u = np.concatenate([p[:-1], j // deg]).astype(np.int32)
+            v = np.concatenate([p[1:], col[j]]).astype(np.int32)
+            f = np.concatenate([np.zeros(len(p) - 1, np.int32), np.full(300, 2, np.int32)])
+            x = rng.integers(1, 1001, len(u)).astype(np.uint32)
+            got = dyn.update(f, u, v, x)
+            o, c, ww, _ = oracle.apply_batch(n, o, c, ww, f, u, v, x)
+            assert got == want(), (hk, k)
+        dyn.close()
+        dg.close()
