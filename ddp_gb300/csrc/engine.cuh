@@ -504,6 +504,7 @@ struct SearchParams {
     // 1M points 16.5 -> 11.6 ms.  Tight bounds keep the quarter (200k points,
     // Euclidean: 1.11 against 1.30 ms).
     uint32_t delta_loose = 0;
+    bool long_rows = true;  // A* searches on a grid: there may be rows of more than LOCAL_ROW arcs
     int64_t budget = 0;  // bidirectional search: entries it may expand (0: any number)
     bool skewed = false;  // ... and the graph has hubs (skewed_rows)
 };
@@ -534,6 +535,18 @@ constexpr int LOCAL_IN = 256, LOCAL_OUT = 512;
 constexpr int LOCAL_FAR = 4096;
 constexpr int LOCAL_FILL = 32, LOCAL_AHEAD = 16;
 constexpr int LOCAL_WAVES = 4096;
+// Where rows may be long (SearchParams::long_rows), arcs decide too.  A row of
+// more than LOCAL_LONG arcs goes to the next phase in segments, one a team (the
+// entry's row end carries SEG_END).  A phase whose arcs (in rows of more than
+// LOCAL_ROW) outnumber LOCAL_ARCS is the grid's, unless most are in one row: a
+// grid phase gives that to one warp, 64 arcs a step, CTA 0 walks it with all its
+// threads.  After LOCAL_WORK arcs the grid may pass its barrier, whose wait is
+// bounded.  400,000 nodes with 20 hubs of 100,000 arcs, a caller's bound: 28 ms
+// with every phase on the grid, 33 with eight lanes a row whatever its length, 17
+// so; 200,000 nodes with degrees by a power law: 5.0, 5.3, 4.2 ms.  The code costs
+// the 511 x 511 maze 1 % (1,445 -> 1,464 us), 250,000 nodes nothing.
+constexpr int LOCAL_ROW = 32, LOCAL_ARCS = 8192, LOCAL_LONG = 256;
+constexpr unsigned int LOCAL_WORK = 1u << 24, SEG_END = 0x80000000u;
 
 // entries that the warp rows (16 per CTA in every search kernel) hold as two
 // lists of uint4
@@ -556,6 +569,15 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
     __shared__ int cnt[3];  // entries per wave, rotating
     __shared__ int c_far, c_touch, c_alt;
     __shared__ unsigned int tg, far_min;  // far_min: no far entry has a smaller f
+    __shared__ unsigned int arcs[3], longest[3];  // of a wave's rows of more than LOCAL_ROW arcs
+    const bool rows = P.long_rows;
+    // a row of len arcs joins wave w (rows of more than 2^21 count as that: no sum overflows)
+    auto count_row = [&](int w, int len) {
+        if (len <= LOCAL_ROW) return;
+        atomicAdd(&arcs[w], (unsigned int)min(len, 1 << 21));
+        atomicMax(&longest[w], (unsigned int)min(len, 1 << 21));
+    };
+    auto wide = [&](int w) { return rows && arcs[w] > LOCAL_ARCS + 8 * longest[w]; };
     // lanes per entry: four for rows of four arcs or fewer on average
     const int lanes = G.e <= 4 * (int64_t)G.n ? 4 : 8;
     const int sub = threadIdx.x & (lanes - 1);
@@ -564,22 +586,26 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
     if (threadIdx.x == 0) {
         cnt[0] = nnear;
         cnt[1] = cnt[2] = 0;
+        for (int w = 0; w < 3; w++) arcs[w] = longest[w] = 0;
         c_far = c_touch = 0;
         far_min = 0;
         tg = P.t >= 0 ? st_g(__ldcg(B.state + P.t)) : 0xFFFFFFFFu;
     }
+    if (rows) __syncthreads();
     for (int i = threadIdx.x; i < nnear; i += blockDim.x) {
         const uint2 en = __ldcg(qcur + i);
-        buf[i] = make_uint4(en.x, en.y, (uint32_t)row_begin(G.off, G.oend, (int)en.x),
-                            (uint32_t)row_end(G.off, G.oend, (int)en.x));
+        const int rb = row_begin(G.off, G.oend, (int)en.x), re = row_end(G.off, G.oend, (int)en.x);
+        buf[i] = make_uint4(en.x, en.y, (uint32_t)rb, (uint32_t)re);
+        if (rows) count_row(0, re - rb);
     }
     __syncthreads();
     int m = nnear, wv = 0, ahead = 0, flip = 0, done = 0;
     bool recheck = KEEP;
     if (!KEEP) cold_x = 0xFFFFFFFFu;
     unsigned long long n_far = 0;
+    unsigned int work = 0;  // arcs in long rows so far
     uint4 *cur = buf, *nxt = buf + cap;
-    for (;;) {
+    while (wv || !wide(0)) {  // (a wide list goes back at once)
         if (m < (KEEP ? 1 : LOCAL_FILL)) {
             // the list is empty or narrow: the far pile's turn
             const int64_t nf = nfar0 + c_far;
@@ -607,8 +633,9 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                     if (e.z < T && (!KEEP || e.z < ft)) {
                         const int p = atomicAdd(&cnt[wv % 3], 1);
                         if (p < cap) {
-                            cur[p] = make_uint4(e.x, e.y, (uint32_t)row_begin(G.off, G.oend, (int)e.x),
-                                                (uint32_t)row_end(G.off, G.oend, (int)e.x));
+                            const int rb = row_begin(G.off, G.oend, (int)e.x), re = row_end(G.off, G.oend, (int)e.x);
+                            cur[p] = make_uint4(e.x, e.y, (uint32_t)rb, (uint32_t)re);
+                            if (rows) count_row(wv % 3, re - rb);
                             return;
                         }
                     }
@@ -658,12 +685,16 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                 if (threadIdx.x == 0) c_far = 0;
                 __syncthreads();
                 if (m == 0) continue;  // far_min is known now: the next split moves something
+                if (wide(wv % 3)) break;
             } else if (m == 0) {
                 break;  // a large pile, or the cold tier's turn: the grid splits it
             }
         }
         int *push = &cnt[(wv + 1) % 3];
-        if (threadIdx.x == 0) cnt[(wv + 2) % 3] = 0;
+        if (threadIdx.x == 0) {
+            cnt[(wv + 2) % 3] = 0;
+            if (rows) arcs[(wv + 2) % 3] = longest[(wv + 2) % 3] = 0;
+        }
         const uint64_t ft64 = (uint64_t)(*(volatile unsigned int *)&tg) + ht;
         const uint32_t ft = ft64 >= 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)ft64;
         auto to_far = [&](uint32_t v, uint32_t g, uint32_t f) {
@@ -677,7 +708,7 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
             const int u = (int)en.x;
             const uint32_t gu = en.y;
             int j = (int)en.z + sub;
-            const int r1 = (int)en.w;
+            const int r1 = (int)(en.w & ~SEG_END);
             // the first arcs load beside the label that decides about them
             uint2 a = j < r1 ? (G.oend ? __ldcg(G.arc + j) : __ldg(G.arc + j)) : make_uint2(0xFFFFFFFFu, 0u);
             const uint64_t su = __ldcg(B.state + u);
@@ -686,6 +717,19 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
             if ((uint64_t)gu + hu >= ft) {
                 // keep mode: stays open beyond f(t)
                 if (KEEP && sub == 0) to_far((uint32_t)u, gu, sat_add(gu, hu));
+                continue;
+            }
+            if ((int)en.w - (int)en.z > LOCAL_LONG && rows) {
+                // (a segment's end is negative here)
+                const int len = (int)en.w - (int)en.z, seg = max(LOCAL_LONG, (len + teams - 1) / teams);
+                for (int k = sub; k * seg < len; k += lanes) {
+                    const int b = (int)en.z + k * seg, p = atomicAdd(push, 1);
+                    count_row((wv + 1) % 3, min(seg, r1 - b));
+                    if (p < cap) nxt[p] = make_uint4(en.x, gu, (uint32_t)b, (uint32_t)min(b + seg, r1) | SEG_END);
+                    else if (p < B.cap_q) qcur[p] = make_uint2(en.x, gu);  // (the grid walks the whole row)
+                    else atomicOr(&ctl->status, ST_OVERFLOW);
+                }
+                if (sub == 0) atomicMax(&longest[(wv + 1) % 3], (unsigned int)min(len, 1 << 21));
                 continue;
             }
             if (sub == 0) {
@@ -729,6 +773,7 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                         const uint64_t fv = (uint64_t)ng + hv;
                         if (fv < T) {
                             n_rel++;
+                            if (rows) count_row((wv + 1) % 3, re - rb);
                             const int p = atomicAdd(push, 1);
                             if (p < cap) nxt[p] = make_uint4((uint32_t)v, ng, (uint32_t)rb, (uint32_t)re);
                             else if (p < B.cap_q) qcur[p] = make_uint2((uint32_t)v, ng);  // past shared memory
@@ -756,13 +801,23 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
         cur = nxt;
         nxt = t;
         if (m > LOCAL_OUT || wv >= LOCAL_WAVES || nfar0 + c_far > B.cap_f / 2) break;
+        if (rows) {
+            work += arcs[wv % 3];
+            if (wide(wv % 3) || work > LOCAL_WORK) break;
+        }
         __syncthreads();  // every thread has read the counters
     }
     __syncthreads();
     // the entries left go back to the near list (those past the shared list
     // are there already)
     const int back = local_handback(m, cap, B.cap_q);
-    for (int i = threadIdx.x; i < back; i += blockDim.x) qcur[i] = make_uint2(cur[i].x, cur[i].y);
+    for (int i = threadIdx.x; i < back; i += blockDim.x) {
+        const uint4 en = cur[i];
+        // of a row in segments (all of them are here) the first goes back as
+        // the node, the others with a label that no node has
+        const bool dead = (en.w & SEG_END) && (int)en.z != row_begin(G.off, G.oend, (int)en.x);
+        qcur[i] = make_uint2(en.x, dead ? INF_G : en.y);
+    }
     if (threadIdx.x == 0) {
         if (m > B.cap_q) atomicOr(&ctl->status, ST_OVERFLOW);
         ctl->loc_near = m;

@@ -3,6 +3,7 @@
 // Replaces LIB/include/graph.h:93-118 (Graph<T>::read_graph), graph.cuh:62-72
 // (GPU_Graph<T>::__gpu_alloc) and DA_star/genOpCSR.cpp:31-53 (reverse CSR,
 // built here in memory instead of written to graph_op.txt).
+#include <algorithm>
 #include <chrono>
 #include <cstdarg>
 #include <cstdio>
@@ -110,8 +111,9 @@ static int upload_csr(ddp_graph *g, const int32_t *off, const int32_t *col, cons
     const int64_t live = roff[(size_t)n];
     int64_t in_long = 0;
     for (int32_t v = 0; v < n; v++) {
-        in_long += long_row_arcs(off[v + 1] - off[v]);
-        in_long += long_row_arcs(roff[(size_t)v + 1] - roff[(size_t)v]);
+        const int32_t f = off[v + 1] - off[v], r = roff[(size_t)v + 1] - roff[(size_t)v];
+        in_long += long_row_arcs(f) + long_row_arcs(r);
+        g->max_row = std::max(g->max_row, std::max(f, r));
     }
     g->skewed = skewed_rows(in_long, e + live);
     std::vector<uint2> rarc((size_t)(live > 0 ? live : 1));

@@ -35,6 +35,7 @@ struct ddp_graph {
     int64_t e_rev = 0;  // arcs in the reverse CSR
     uint32_t wmin = 0, wmax = 0;
     uint32_t rho_fp = 0;  // Euclidean heuristic scale (16.16)
+    int32_t max_row = 0;  // longest row, forward or reverse, as the graph was made
     bool skewed = false;  // hubs hold many of the arcs (rules.h), as the graph was made
     int32_t *d_off = nullptr;
     uint2 *d_arc = nullptr;

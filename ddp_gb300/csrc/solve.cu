@@ -1528,6 +1528,7 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
     DevGraph G = graph_view(g);
     SearchParams P{source, target, delta, o.K, 0, 0};
     if (o.delta <= 0) P.delta_loose = loose_delta(g);
+    P.long_rows = g->dyn || g->max_row > LOCAL_ROW;
     const int kind = h ? h->kind : DDP_H_ZERO;
     // reads what a kernel left in w->h_res; path ids past the host's part come from the device
     auto result = [&](Workspace *w) -> int {

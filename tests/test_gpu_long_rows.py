@@ -70,3 +70,58 @@ def test_rows_in_segments(gpu, oracle, L, wmax):
     assert np.array_equal(cost, want[ids - first])
     srv.close()
     dg.close()
+
+
+@pytest.mark.parametrize("hubs,L", [(1, 256), (1, 257), (1, 16384), (1, 16385), (1, 70000), (3, 5000), (9, 20000),
+                                    (40, 300), (200, 60), (33, 257)])
+def test_rows_in_narrow_phases(gpu, oracle, hubs, L):
+    """Hubs met by the whole-grid search while one CTA runs its phases:
+    rows in segments (one a team: 64 or 128), lists that the segments make too
+    long, phases too wide in arcs; then the same graph under update batches."""
+    d, O = gpu, oracle
+    rng = np.random.default_rng(hubs * 1000 + L)
+    mid, tail = 3000, 60
+    n = 1 + hubs + mid + tail
+    h, m0, t0 = 1, 1 + hubs, 1 + hubs + mid
+    src = np.concatenate([np.zeros(hubs), np.repeat(h + np.arange(hubs), L), m0 + np.arange(mid),
+                          t0 + np.arange(tail - 1)]).astype(np.int64)
+    dst = np.concatenate([h + np.arange(hubs), m0 + rng.integers(0, mid, hubs * L), t0 + rng.integers(0, 20, mid),
+                          t0 + 1 + np.arange(tail - 1)]).astype(np.int64)
+    o = np.argsort(src, kind="stable")
+    off = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+    g = d.CSR(n, off, dst[o].astype(np.int32), rng.integers(1, 60, len(src)).astype(np.uint32))
+    gs, s = g.with_sentinel(), 0
+
+    def want(t, off=gs.off[:-1], col=gs.col, w=gs.w):
+        f, c, _, _, _ = O.astar(len(off), off, col, w, np.zeros(len(off), np.int32), s, t, mode=O.HEAP_POSMAP)
+        return c if f else d.INF
+
+    dg = d.DeviceGraph.from_csr(g)
+    for t in (n - 1, t0 + 7, m0 + 5, h + hubs - 1):
+        hz = d.Heuristic(dg, t, d.H_USER, user_h=np.zeros(n, np.int32))
+        c = want(t)
+        for kw in ({}, {"K": 600}, {"grid": 3, "delta": 1}, {"delta": 100000}):
+            r = dg.solve(s, t, hz, **kw)
+            assert r.cost == c, (t, kw)
+            if c != d.INF:
+                ok, why = O.check_path(g.off, g.col, g.w, r.path, s, t, c)
+                assert ok, (t, kw, why)
+        hz.close()
+    dg.close()
+    for hk in (d.H_ZERO, d.H_BFS_HOPS):
+        dg = d.DeviceGraph.from_csr(g)
+        dyn = d.DynamicSearch(dg, s, n - 1, hk)
+        off, col, w = gs.off[:-1].copy(), gs.col.copy(), gs.w.copy()
+        assert dyn.cost == want(n - 1)
+        for k in range(3):
+            # the best path's arcs go, some come at new weights
+            p = dyn.path()
+            u = np.concatenate([p[:1], rng.integers(h, h + hubs, 30)]).astype(np.int32)
+            v = np.concatenate([p[1:2], m0 + rng.integers(0, mid, 30)]).astype(np.int32)
+            f = np.concatenate([[2], np.ones(30)]).astype(np.int32)
+            x = rng.integers(1, 90, 31).astype(np.uint32)
+            got = dyn.update(f, u, v, x)
+            off, col, w, _ = O.apply_batch(len(off), off, col, w, f, u, v, x)
+            assert got == want(n - 1, off, col, w), (hk, k)
+        dyn.close()
+        dg.close()
