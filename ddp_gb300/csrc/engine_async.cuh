@@ -29,9 +29,12 @@ constexpr uint32_t RING_EMPTY = 0xFFFFFFFFu;
 
 // Fewest ring entries a warp claims at once (at most 32): it claims
 // ceil(available / warps), so a small bucket is spread over the CTA's warps.
-// Landmark batch (500 queries, 400,000 nodes): always 32 -> 9.63 ms, at
-// least 4 -> 9.21 ms, at least 1 no better.
-constexpr int ASYNC_CLAIM_MIN = 4;
+// With coordinate bounds, 64 queries (least claim 4, 16, 32): 200,000 points
+// 6.3, 6.5, 6.7 ms; 150 x 150 maze 5.2, 5.2, 5.7; 700 x 700 maze 32.3, 29.7, 29.0.
+// With bounds from a table it is always 32: one query on the points under hops
+// 6.6 ms at 4, 6.1 at 16, 5.5.
+template <class H>
+constexpr int async_claim_min() { return heur_cheap<H>::value ? 16 : 32; }
 
 struct CtaQ {
     int head, tail;      // ring positions of the current bucket
@@ -127,7 +130,7 @@ __device__ SearchResult run_search_cta(const DevGraph &G, const SlotBufs &B, con
                         for (uint32_t spins = 0;; spins++) {
                             const int h = *(volatile int *)&sq->head, t = *(volatile int *)&sq->tail;
                             if (h < t) {
-                                const int k = min(t - h, min(32, max(ASYNC_CLAIM_MIN, (t - h + nw - 1) / nw)));
+                                const int k = min(t - h, min(32, max(async_claim_min<Heur>(), (t - h + nw - 1) / nw)));
                                 if (atomicCAS(&sq->head, h, h + k) == h) {
                                     n = k;
                                     h0 = h;
