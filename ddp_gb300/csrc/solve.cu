@@ -824,22 +824,25 @@ __device__ void service_loop(const BatchArgs &A) {
 // with both engines, 1,706 once the group engine also ran narrow phases).
 template <int HK, bool SERVE>
 __global__ void __launch_bounds__(bidir_hk(HK) ? 1024 : 512, bidir_hk(HK) ? 1 : 2)
-    k_batch(const __grid_constant__ DevGraph G, SlotArrays sa, BatchArgs A) {
+    k_batch(const __grid_constant__ DevGraph G, SlotArrays sa, SlotArrays more, BatchArgs A) {
     if constexpr (SERVE) {
         if (A.svc && (int)blockIdx.x == A.serve_slots) {
             service_loop(A);
             return;
         }
     }
-    SlotBufs B = slot_of(sa, blockIdx.x);
+    // slots that a large batch added come after the first ones
+    const int slot = (int)blockIdx.x;
+    SlotBufs B = slot < sa.nslots ? slot_of(sa, slot) : slot_of(more, slot - sa.nslots);
+    uint32_t *epoch = slot < sa.nslots ? sa.epoch + slot : more.epoch + (slot - sa.nslots);
     CtaGroup grp{&B.ctl->status};
     if constexpr (bidir_hk(HK)) {
         __shared__ WaveQ bq;
-        batch_loop<HK, true, SERVE>(grp, G, B, A, sa.epoch + blockIdx.x, nullptr, nullptr, &bq);
+        batch_loop<HK, true, SERVE>(grp, G, B, A, epoch, nullptr, nullptr, &bq);
     } else {
         __shared__ WarpRows wrows[MAX_WARPS];
         __shared__ CtaQ sq;
-        batch_loop<HK, true, SERVE>(grp, G, B, A, sa.epoch + blockIdx.x, wrows, &sq, nullptr);
+        batch_loop<HK, true, SERVE>(grp, G, B, A, epoch, wrows, &sq, nullptr);
     }
 }
 
@@ -881,7 +884,7 @@ __global__ void __launch_bounds__(256) k_order(const int32_t *S, const int32_t *
 // Slots of A.group CTAs each (cooperative launch), and one-CTA slots on the
 // phase-synchronous engine (DDP_OPT_SYNC).
 template <int HK>
-__global__ void __launch_bounds__(512, 2) k_batch_group(DevGraph G, SlotArrays sa, BatchArgs A) {
+__global__ void __launch_bounds__(512, 2) k_batch_group(DevGraph G, SlotArrays sa, SlotArrays, BatchArgs A) {
     __shared__ WarpRows wrows[MAX_WARPS];
     if (A.svc && (int)blockIdx.x == A.serve_slots) {
         service_loop(A);
@@ -1036,7 +1039,8 @@ cudaError_t svc_run_direct(const SvcSub *subs, int nsub, cudaStream_t st) {
 
 cudaError_t launch_slots(int hk, int grid, int block, bool coop, DevGraph G, SlotArrays sa, BatchArgs A,
                          cudaStream_t st) {
-    void *args[] = {&G, &sa, &A};
+    SlotArrays more;
+    void *args[] = {&G, &sa, &more, &A};
     const void *fn = batch_kernel_hk(hk, A.group > 1 || A.sync_engine, true);
     if (coop) return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(block), args, 0, st);
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, st);
@@ -1692,8 +1696,13 @@ struct ddp_batch {
     int hkind = DDP_H_ZERO;
     ddp_opts o{};
     cudaStream_t stream = nullptr;
-    int block = 512;
+    int block = 512;       // threads per CTA of the last launch (of the next, where told or not bidirectional)
     SlotArrays sa;
+    // Bidirectional launches choose their own threads per query: two slots an SM
+    // to begin with, up to max_slots once a batch wants them (batch_extend).
+    SlotArrays more;
+    int max_slots = 0;
+    size_t slot_size = 0;  // bytes of one
     // device buffers sized for the largest batch seen
     int32_t cap_q_n = 0;
     int32_t *d_S = nullptr, *d_T = nullptr, *d_cost = nullptr, *d_plen = nullptr, *d_paths = nullptr;
@@ -1757,18 +1766,44 @@ static bool batch_ranked(const ddp_batch *b, const DevGraph &G, int32_t n) {
     return bidir_hk(b->hk) && G.xy && n <= ORDER_MAX;
 }
 
-// CTAs of a launch of n queries and the threads of one.  A ranked batch holds
+// CTAs that a launch of n queries wants, and the threads of one.  A ranked batch holds
 // on to wide CTAs longer, since its second round is its short queries: 300
 // pairs on 1M points take 23.5 ms on 1,024 threads, 38.9 ms on 512 (50k
 // points: 1.92, 2.59), 600 pairs on 50k points 3.63 and 2.65 ms.
-static int batch_grid(const ddp_batch *b, const DevGraph &G, int32_t n, int *block) {
+static int batch_shape(const ddp_batch *b, const DevGraph &G, int32_t n, int *block) {
     *block = b->block;
-    const int grid = b->sa.nslots * b->group;
-    if (!bidir_hk(b->hk) || b->o.block > 0) return grid;
+    if (!bidir_hk(b->hk) || b->o.block > 0) return INT32_MAX;
     const int sms = device_sms();
     const int wide = batch_ranked(b, G, n) ? 5 * sms / 2 : sms + sms / 2;
     *block = n <= wide ? 1024 : n <= 6 * sms ? 512 : 256;
-    return std::min({grid, 1024 / *block * sms, std::max(n, 1)});
+    return std::min(1024 / *block * sms, std::max(n, 1));
+}
+
+static int batch_grid(const ddp_batch *b, const DevGraph &G, int32_t n, int *block) {
+    return std::min(batch_shape(b, G, n, block), (b->sa.nslots + b->more.nslots) * b->group);
+}
+
+// More slots for a batch that wants them, once, within half of the memory that
+// is free or the engine's.  (Four an SM from the start took 148 GB at 4M nodes
+// for batches of any size, now 78 GB up to 912 queries; the engine is made in 7.5
+// ms instead of 13.6 and the first larger batch takes 10.1 instead of 3.7.)
+// Without the memory the batch runs on the slots there are.
+static void batch_extend(ddp_batch *b, const DevGraph &G, int32_t n) {
+    int block = 0;
+    if (b->max_slots <= b->sa.nslots || batch_shape(b, G, n, &block) <= b->sa.nslots) return;
+    size_t freeb = 0, totalb = 0;
+    cudaMemGetInfo(&freeb, &totalb);
+    const size_t own = b->slot_size * (size_t)b->sa.nslots, half = (freeb + own) / 2;
+    const int add = (int)std::min<size_t>((size_t)(b->max_slots - b->sa.nslots),
+                                          half > own ? (half - own) / b->slot_size : 0);
+    b->max_slots = 0;  // asked once
+    if (add < 1) return;
+    if (slots_alloc(b->more, b->sa.n, add, b->sa.cap_q, b->sa.cap_f, hk_slot_kind(b->hk), b->stream, b->sa.hbits)) {
+        (void)cudaGetLastError();
+        slots_free(b->more);
+        return;
+    }
+    b->gkey_valid = false;  // a captured launch has the old slots
 }
 
 // Kernel arguments of one batch launch.  Returns false when the landmark
@@ -1808,16 +1843,19 @@ static cudaError_t batch_launch_args(ddp_batch *b, DevGraph G, BatchArgs A) {
     if (e != cudaSuccess) return e;
     // fresh control blocks (barrier counters included) for every launch
     e = cudaMemsetAsync(b->sa.ctl, 0, sizeof(SearchCtl) * (size_t)b->sa.nslots, b->stream);
+    if (e == cudaSuccess && b->more.nslots)
+        e = cudaMemsetAsync(b->more.ctl, 0, sizeof(SearchCtl) * (size_t)b->more.nslots, b->stream);
     if (e != cudaSuccess) return e;
     int block = 0;
     const int grid = batch_grid(b, G, A.nq, &block);
+    b->block = block;
     if (A.order) {
         k_order<<<(A.nq + 255) / 256, 256, 0, b->stream>>>(A.S, A.T, G.xy, G.n, A.nq, A.order);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    SlotArrays sa = b->sa;
-    void *args[] = {&G, &sa, &A};
+    SlotArrays sa = b->sa, more = b->more;
+    void *args[] = {&G, &sa, &more, &A};
     const void *fn = batch_kernel_hk(b->hk, A.group > 1 || A.sync_engine, false);
     if (b->group > 1)
         return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(block), args, 0, b->stream);
@@ -1878,13 +1916,17 @@ int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batc
     // slots: occupancy-limited, then memory-limited (half of free memory)
     int per_sm = 0;
     b->group = bidir ? 1 : std::max(1, b->o.group);  // bidirectional slots are one CTA
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, batch_kernel_hk(b->hk, b->group > 1 || (b->o.flags & DDP_OPT_SYNC), false),
-        bidir && b->o.block <= 0 ? 256 : b->block, 0);
+    const void *kernel = batch_kernel_hk(b->hk, b->group > 1 || (b->o.flags & DDP_OPT_SYNC), false);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, b->block, 0);
     const int coresident = std::max(1, per_sm) * sm_count();
     if (b->group > coresident) b->group = coresident;
     int nslots = coresident / b->group;
     if (b->o.grid > 0) nslots = std::min(b->o.grid, b->group > 1 ? nslots : b->o.grid);
+    else if (bidir && b->o.block <= 0) {
+        int most = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, kernel, 256, 0);
+        b->max_slots = most * sm_count();
+    }
     const int64_t cap = b->o.queue_cap > 0      ? b->o.queue_cap
                         : bidir               ? std::min<int64_t>((int64_t)g->n + 4096, 1 << 18)
                                                 : (int64_t)g->n + 4096;
@@ -1897,6 +1939,7 @@ int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batc
     const int skind = hk_slot_kind(b->hk);
     const int hb = (skind & SLOT_HASH) ? hash_bits(g->n) : 0;
     const size_t per = slot_bytes(g->n, cap, cap_f, skind, hb);
+    b->slot_size = per;
     const size_t budget = freeb / 2;
     if ((size_t)nslots * per > budget) nslots = (int)std::max<size_t>(1, budget / per);
     int rc = slots_alloc(b->sa, g->n, nslots, cap, cap_f, skind, b->stream, hb);
@@ -1926,6 +1969,7 @@ int ddp_batch_solve_device(ddp_batch *b, int32_t n, const int32_t *d_sources,
     int32_t *plen = d_path_len ? d_path_len : b->d_plen;
     DevGraph G;
     BatchArgs A;
+    batch_extend(b, graph_view(b->g), n);
     if (!batch_args(b, n, d_sources, d_targets, d_cost, plen, &G, &A))
         return fail(DDP_ERR_INVALID, "landmark table is stale (graph updated since ddp_landmarks_build)");
     b->overflow_paths.clear();
@@ -1988,6 +2032,7 @@ int ddp_batch_solve(ddp_batch *b, int32_t n, const int32_t *sources, const int32
                                  cudaMemcpyHostToDevice, b->stream));
         DevGraph G;
         BatchArgs A;
+        batch_extend(b, graph_view(b->g), n);
         if (!batch_args(b, n, b->d_S, b->d_T, b->d_cost, b->d_plen, &G, &A))
             return fail(DDP_ERR_INVALID, "landmark table is stale (graph updated since ddp_landmarks_build)");
         cudaError_t e = batch_launch_args(b, G, A);
@@ -2094,8 +2139,8 @@ int ddp_batch_stats(ddp_batch *b, int64_t *stats, int64_t *t_start_ns, int64_t *
 
 int ddp_batch_info(const ddp_batch *b, int32_t *slots, int64_t *queue_cap, int32_t *block) {
     if (!b) return fail(DDP_ERR_INVALID, "null batch");
-    if (slots) *slots = b->sa.nslots;
-    if (queue_cap) *queue_cap = b->sa.cap_q;
+    if (slots) *slots = b->sa.nslots + b->more.nslots;
+    if (queue_cap) *queue_cap = bidir_hk(b->hk) ? b->sa.cap_f : b->sa.cap_q;
     if (block) *block = b->block;
     return DDP_OK;
 }
@@ -2116,6 +2161,7 @@ int ddp_batch_free(ddp_batch *b) {
     if (!b) return DDP_OK;
     if (b->gexec) cudaGraphExecDestroy(b->gexec);
     slots_free(b->sa);
+    slots_free(b->more);
     cudaFree(b->d_S);
     cudaFree(b->d_T);
     cudaFree(b->d_cost);

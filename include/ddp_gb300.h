@@ -214,8 +214,11 @@ int ddp_batch_path(ddp_batch *b, int32_t i, int32_t *buf, int32_t cap, int32_t *
 /* Per-query device counters of the last solve: stats[DDP_STATS*i + k] as
  * in ddp_query_stats; start/end (optional) = device timestamps in ns. */
 int ddp_batch_stats(ddp_batch *b, int64_t *stats, int64_t *t_start_ns, int64_t *t_end_ns);
-/* Engine shape: concurrent query slots, queue capacity per slot, threads
- * per CTA. */
+/* Engine shape: concurrent query slots (bidirectional engines that choose
+ * their own shape add slots when a batch first wants more than two an SM),
+ * entries of a slot's queues (bidirectional: 8-byte units of either half of
+ * its far memory, at least 2^18 whatever opts.queue_cap says), threads per CTA
+ * of the last launch. */
 int ddp_batch_info(const ddp_batch *b, int32_t *slots, int64_t *queue_cap, int32_t *block);
 /* CTAs per query slot of the batch engine. */
 int ddp_batch_group(const ddp_batch *b, int32_t *group);

@@ -187,3 +187,55 @@ def test_device_batch_overflow_reports_minus_one(gpu, oracle):
         assert np.array_equal(got[~over], want[~over])
     be.close()
     dg.close()
+
+
+@pytest.mark.parametrize("coords", [False, True])
+def test_slots_added_by_a_large_batch(gpu, oracle, coords):
+    """A bidirectional engine begins with two slots an SM; the first larger
+    batch adds more, on host and device pointers, with a replayed graph before
+    and after it, and answers stay those of the small batches."""
+    torch = pytest.importorskip("torch")
+    d = gpu
+    g = d.gen_random_chain(3000, 5, 1, 100, 19)
+    dg = d.DeviceGraph.from_csr(g)
+    rng = np.random.default_rng(6)
+    if coords:
+        dg.set_coords(rng.integers(0, 300, (g.n, 2)).astype(np.int32))
+    S, T = (rng.integers(0, g.n, 3000).astype(np.int32) for _ in range(2))
+    gs = g.with_sentinel()
+    want, _, _, done = oracle.astar_many(gs.n, gs.off[:-1], gs.col, gs.w, S, T, hkind=0, mode=oracle.HEAP_POSMAP,
+                                         threads=4, budget_s=1e9)
+    assert done == len(S)
+    dS, dT = torch.from_numpy(S).cuda(), torch.from_numpy(T).cuda()
+    dc = torch.empty(len(S), dtype=torch.int32, device="cuda")
+
+    def on_device(eng, q):
+        dc.fill_(-7)
+        torch.cuda.synchronize()
+        eng.solve_device(q, dS.data_ptr(), dT.data_ptr(), dc.data_ptr())
+        eng.sync()
+        assert np.array_equal(dc.cpu().numpy()[:q], want[:q])
+
+    for first in ("host", "device"):
+        eng = d.BatchEngine(dg, d.H_BIDIR)
+        few = eng.info()["slots"]
+        for q in (1, 300, 300):
+            on_device(eng, q)
+            assert np.array_equal(eng.solve(S[:q], T[:q])[0], want[:q])
+        assert eng.info()["slots"] == few
+        if first == "host":
+            assert np.array_equal(eng.solve(S, T)[0], want)
+        on_device(eng, 3000)
+        assert eng.info()["slots"] > few
+        for q in (300, 3000, 1200):
+            on_device(eng, q)
+            assert np.array_equal(eng.solve(S[:q], T[:q])[0], want[:q])
+            i = q - 1
+            if want[i] != d.INF:
+                ok, why = oracle.check_path(g.off, g.col, g.w, eng.path(i), int(S[i]), int(T[i]), int(want[i]))
+                assert ok, why
+        eng.close()
+    eng = d.BatchEngine(dg, d.H_BIDIR, grid=40)  # as many as asked for
+    assert np.array_equal(eng.solve(S, T)[0], want) and eng.info()["slots"] == 40
+    eng.close()
+    dg.close()
