@@ -841,16 +841,24 @@ __global__ void __launch_bounds__(512, 1)
                         dc->again = at.again;
                     }
                 }
-                grp.sync();  // CTA 0's changes and hand-back are visible to every CTA
+                // CTA 0's changes and hand-back are visible to every CTA now
+                __shared__ int back[5];  // read once: the CTA's threads agree
+                grp.sync_fetch([&] {
+                    back[0] = *(volatile int *)&B.ctl->status;
+                    back[1] = *(volatile int *)&dc->stage;
+                    back[2] = *(volatile int *)&dc->nf;
+                    back[3] = *(volatile int *)&dc->again;
+                    back[4] = *(volatile int *)&dc->odd;
+                });
                 // a wait that ran out: CTA 0 may still be at it
-                if (*(volatile int *)&B.ctl->status & ST_TIMEOUT) {
+                if (back[0] & ST_TIMEOUT) {
                     if (rank == 0) A.out[2] = ST_TIMEOUT;
                     return;
                 }
-                at.stage = *(volatile int *)&dc->stage;
-                at.nf = *(volatile int *)&dc->nf;
-                again = *(volatile int *)&dc->again != 0;
-                const bool odd = *(volatile int *)&dc->odd != 0;
+                at.stage = back[1];
+                at.nf = back[2];
+                again = back[3] != 0;
+                const bool odd = back[4] != 0;
                 at.fa = reinterpret_cast<int32_t *>(odd ? B.q1 : B.q0);
                 at.fb = reinterpret_cast<int32_t *>(odd ? B.q0 : B.q1);
                 if (again) grp.sync();  // every CTA has read the words
