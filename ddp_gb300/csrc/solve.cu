@@ -147,6 +147,14 @@ __global__ void k_reset_touched(SlotArrays sa) {
         B.state[B.touched[i]] = ~0ull;
 }
 
+// Labels of all slots, if a wait ran out in the launch before (its status).
+__global__ void k_slots_heal(SlotArrays sa, const int *status) {
+    if (!(*status & ST_TIMEOUT)) return;
+    const size_t words = (size_t)sa.sstride * sa.nslots;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (size_t)gridDim.x * blockDim.x)
+        sa.state[i] = ~0ull;
+}
+
 // What a single-query kernel returns, in host memory mapped into the device:
 // the host reads it after one synchronisation, with no copies of its own.
 constexpr int SOLVE_PATH = 4096;  // path ids returned with it
@@ -366,6 +374,20 @@ __device__ __forceinline__ void batch_loop(const Grp &grp, const DevGraph &G0, c
         int32_t s, t;
         unsigned long long g[GW];
     } sh;
+    // Slots of several CTAs: whether a wait ran out (the CTA's threads agree).
+    // The CTAs have then gone on apart: the slot takes no more queries, and the
+    // next launch clears its labels (k_slots_heal).
+    auto apart = [&]() -> bool {
+        if constexpr (!Grp::multi) return false;
+        __shared__ int s_apart;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s_apart = *(volatile int *)&ctl->status & ST_TIMEOUT;
+            if (s_apart) atomicOr(A.status, ST_TIMEOUT);
+        }
+        __syncthreads();
+        return s_apart != 0;
+    };
     long long t0 = 0;
     int vbuf = -1;  // versioned serving: graph buffer the current search holds
     for (;;) {
@@ -599,6 +621,14 @@ __device__ __forceinline__ void batch_loop(const Grp &grp, const DevGraph &G0, c
             for (int64_t i = grp.rank(); i < B.cap_q; i += grp.size()) B.q0[i].x = RING_EMPTY;
             grp.sync();
         }
+        if (apart()) {
+            if (grp.rank() == 0) {
+                A.cost[q] = -1;
+                if (A.plen) A.plen[q] = 0;
+                if (A.qstatus) A.qstatus[q] = ST_TIMEOUT;
+            }
+            break;
+        }
         int32_t blen = 0;  // path length (bidirectional kinds; the first warp)
         if constexpr (bidir_hk(HK)) {
             if (grp.rank() < 32 && A.paths && !(*(volatile int *)&ctl->status & (ST_OVERFLOW | ST_TIMEOUT))) {
@@ -654,6 +684,7 @@ __device__ __forceinline__ void batch_loop(const Grp &grp, const DevGraph &G0, c
             atomicOr(A.status, ctl->status);
         }
         grp.sync();
+        if (apart()) break;
         const int cnt = *(volatile int *)&ctl->touched;
         if (pair16_hk(HK)) {
             // every word of a finished slot returns to all-ones, so the whole
@@ -668,6 +699,7 @@ __device__ __forceinline__ void batch_loop(const Grp &grp, const DevGraph &G0, c
             for (int i = grp.rank(); i < cnt; i += grp.size()) B.state[B.touched[i]] = ~0ull;
         }
         grp.sync();
+        if (apart()) break;
         if (grp.rank() == 0) {
             if (A.tstart) A.tstart[q] = t0;
             if (A.tend) A.tend[q] = global_ns();
@@ -1839,7 +1871,15 @@ static bool batch_args(ddp_batch *b, int32_t n, const int32_t *dS, const int32_t
 }
 
 static cudaError_t batch_launch_args(ddp_batch *b, DevGraph G, BatchArgs A) {
-    cudaError_t e = cudaMemsetAsync(b->d_work, 0, sizeof(int) * 2, b->stream);
+    cudaError_t e = cudaSuccess;
+    if (b->group > 1) {
+        // slots whose CTAs may go apart: labels of the last launch, and costs
+        // of queries that no slot is left to take (-1: the host runs them)
+        k_slots_heal<<<4 * device_sms(), 256, 0, b->stream>>>(b->sa, b->d_status);
+        e = cudaMemsetAsync(A.cost, 0xFF, sizeof(int32_t) * (size_t)A.nq, b->stream);
+        if (e != cudaSuccess) return e;
+    }
+    e = cudaMemsetAsync(b->d_work, 0, sizeof(int) * 2, b->stream);
     if (e != cudaSuccess) return e;
     // fresh control blocks (barrier counters included) for every launch
     e = cudaMemsetAsync(b->sa.ctl, 0, sizeof(SearchCtl) * (size_t)b->sa.nslots, b->stream);
@@ -1947,6 +1987,8 @@ int ddp_batch_create(ddp_graph *g, int32_t hkind, const ddp_opts *opts, ddp_batc
         cudaError_t e1 = cudaMalloc(&b->d_work, sizeof(int) * 2);
         if (e1 != cudaSuccess) rc = cuda_fail(e1, "cudaMalloc(work)");
         else b->d_status = b->d_work + 1;
+        if (rc == DDP_OK && cudaMemsetAsync(b->d_work, 0, sizeof(int) * 2, b->stream) != cudaSuccess)
+            rc = cuda_fail(cudaGetLastError(), "cudaMemsetAsync(work)");
     }
     if (rc) {
         ddp_batch_free(b);

@@ -180,3 +180,34 @@ for hk in (d.H_ZERO, d.H_BFS_HOPS):
     dyn.close()
     dg.close()
 """)
+
+
+def test_batches_after_a_timed_out_one_are_exact(short_waits):
+    """Slots of several CTAs whose waits run out: their queries are run again
+    alone, or fail, and later batches of the engine are exact or fail too, never
+    wrong by the labels that were left."""
+    short_waits("""
+m = d.gen_maze(500, 500, 0.25, 5)
+dg = d.DeviceGraph.from_csr(m)
+rng = np.random.default_rng(2)
+near = lambda q: (lambda a: (a, np.minimum(a + rng.integers(0, 4, q), m.n - 1)))(rng.integers(0, m.n, q))
+eng = d.BatchEngine(dg, d.H_MANHATTAN, group=4, grid=6)
+timed_out = 0
+for rep in range(6):
+    # long queries first: CTA 0 of a slot runs their phases, the others wait
+    if rep % 2 == 0:
+        S, T = rng.integers(0, m.n // 20, 12), rng.integers(m.n - m.n // 20, m.n, 12)
+    else:
+        S, T = near(40)
+    S, T = S.astype(np.int32), T.astype(np.int32)
+    want = [cost(m, int(s), int(t)) for s, t in zip(S, T)]
+    try:
+        got = eng.solve(S, T)[0].tolist()
+        assert got == want, (rep, got, want)
+    except d.DdpError as e:
+        assert e.code == 6, e
+        timed_out += 1
+assert timed_out > 0, "no wait ran out"
+eng.close()
+dg.close()
+""")
