@@ -519,11 +519,12 @@ __device__ __forceinline__ CtaGroup dyn_group(CtaGroup *, const SlotBufs &B) { r
 // threads) walks one row, DYN_ARCS arcs a lane, so that a level is
 // one chain of arc -> node word -> atomic, where a thread walking a row of
 // ten arcs alone ran two such chains and read the row bounds first.
-// 1M nodes, 1000-update batches (median of 100 updates in the call): 334 us
-// with these steps and the resumed search's splits on 76 CTAs (hops 28 us,
-// invalidation 70, re-seeding and relaxing 17, search 100), 154 us here.  1024 x
-// 1024 maze, batches of 2,238 changes with 17k nodes invalidated over hundreds
-// of levels: 5.0 -> 3.1 ms (6.9 with every level on the grid).
+// 1M nodes, 1000-update batches: less than half the time of these steps and the
+// resumed search's splits on 76 CTAs.  DYN_LOCAL_BAIL and _SEED (512 and 256, 2,048
+// and 1,024, 8,192 and 4,096): 1024 x 1024 maze, 2,238 arcs out or back in, 21k
+// nodes invalidated over hundreds of levels, 5.7, 4.9, 5.1 ms; 300,000 random nodes,
+// 4,000 arcs, 3.3k invalidated, 0.49, 0.53, 0.54; 300,000 points, 500 arcs, 46k
+// invalidated, 4.4 at all three.
 constexpr int DYN_LOCAL_UPD = 4096;   // updates CTA 0 takes alone
 constexpr int DYN_LOCAL_BAIL = 2048;
 constexpr int DYN_LOCAL_SEED = 1024;

@@ -621,8 +621,8 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
     // ceil(b 2^32 / rec_dk): two multiplications by 2^64 / rec_dk come out at
     // most a few below it.  With a 64-bit division here, four in each plan,
     // the CTA waited about a microsecond longer for every wave: 16 maze pairs
-    // 26.2 -> 22.3 ms, 200 pairs on 1M points 23.2 -> 22.0, 4,096 on 4M nodes
-    // 3.69 -> 3.59, 500 landmark queries 1.47 -> 1.37.
+    // 18 % longer, 200 pairs on 1M points 5, 4,096 on 4M nodes 3, 500 landmark
+    // queries 7.
     if (threadIdx.x == 0) q->edge_mul = ~0ull / rec_dk;
     auto edge = [&](uint32_t b) -> uint32_t {
         const unsigned long long M = q->edge_mul;

@@ -1245,13 +1245,18 @@ struct ddp_query {
 
 namespace ddp {
 // Entries a single query may expand bidirectionally on one CTA before the
-// whole GPU takes it.
+// whole GPU takes it.  Searches that end within it gain most, those that do not
+// lose the attempt (8,192, 32,768, 131,072, no coordinates): 200,000 points 4.9,
+// 5.3, 6.5 ms; 20,000 points 0.86, 1.20, 0.99; 300 x 300 grid 1.46, 1.60, 1.44; 1M
+// random nodes 0.11 at all three.
 constexpr int64_t SOLVE_BIDIR_BUDGET = 32768;
 
 // Whether a single query tries the bidirectional search first: no bound, or
 // a hop bound where the weights differ enough that it says little (with unit
 // weights hops are the distance itself and A* walks straight to the target),
-// and no option that asks for the A* engine's launch.
+// and no option that asks for the A* engine's launch.  300,000 random nodes,
+// weights 1..4: 100 us by A*, 54 so; 10..40: 100 and 74; 10..30, which the rule
+// leaves to A*: 91 and 83; 50..100: 72 and 78.
 static bool solve_bidir_first(const ddp_graph *g, int kind, const ddp_opts &o) {
     if (o.flags || o.grid || o.block || o.delta || o.queue_cap || o.group) return false;
     if (kind == DDP_H_ZERO) return true;
@@ -1799,7 +1804,9 @@ static bool batch_ranked(const ddp_batch *b, const DevGraph &G, int32_t n) {
 }
 
 // CTAs that a launch of n queries wants, and the threads of one.  A ranked batch holds
-// on to wide CTAs longer, since its second round is its short queries: 300
+// on to wide CTAs longer, since its second round is its short queries (others:
+// 1M random nodes on 1,024, 512, 256 threads, 100 queries 225, 301, 436 us; 350: 424,
+// 386, 472; 600: 575, 512, 591; 912: 823, 637, 632; 1,100: 933, 709, 684): 300
 // pairs on 1M points take 23.5 ms on 1,024 threads, 38.9 ms on 512 (50k
 // points: 1.92, 2.59), 600 pairs on 50k points 3.63 and 2.65 ms.
 static int batch_shape(const ddp_batch *b, const DevGraph &G, int32_t n, int *block) {

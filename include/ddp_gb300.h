@@ -92,13 +92,19 @@ typedef struct ddp_batch ddp_batch;         /* multi-query engine (slots)       
 
 /* Search options (all fields 0 = automatic). */
 typedef struct ddp_opts {
-    int32_t K;         /* nodes expanded per iteration (the reference's K queues);
-                          0 = the whole current bucket                          */
+    int32_t K;         /* nodes expanded per iteration of the A* engine (the
+                          reference's K queues); 0 = the whole current bucket.
+                          Bidirectional searches expand waves of their own size
+                          whatever K says: bidirectional kinds, one-CTA batch
+                          slots of no bound, hop and landmark bounds, and single
+                          queries of no bound or hop bounds without flags, grid,
+                          block, delta, queue_cap and group                      */
     int32_t delta;     /* bucket width on f; 0 = chosen from the arc weights    */
     int32_t block;     /* threads per CTA (bidirectional batches: 0 = chosen by
                           the batch's size)                                       */
     int32_t grid;      /* CTAs (single query) or concurrent slots (batch)        */
-    int64_t queue_cap; /* entries per search queue                               */
+    int64_t queue_cap; /* entries per search queue (far memory of bidirectional
+                          slots: at least 2^18 units, ddp_batch_info)            */
     void *stream;      /* cudaStream_t; NULL = the handle's own stream           */
     int32_t group;     /* batch: CTAs working on one query (1 = one CTA)          */
     int32_t flags;     /* DDP_OPT_* bits                                          */
