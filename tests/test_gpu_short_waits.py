@@ -76,18 +76,21 @@ def test_updates_given_up_on_leave_the_server_exact(short_waits):
 import time
 g = d.gen_geometric(300_000, 6, 1 << 20, 1000, 17, 4)
 dg = d.DeviceGraph.from_csr(g)
-srv = d.Server(dg, d.H_BIDIR, max_requests=64, versions=2, grid=2)
+srv = d.Server(dg, d.H_BIDIR, max_requests=128, versions=2, grid=2)
 rng = np.random.default_rng(3)
 # long queries: from one corner region to the opposite one
 key = g.xy.sum(axis=1)
 order = np.argsort(key)
-S, T = order[rng.integers(0, 3000, 10)], order[-1 - rng.integers(0, 3000, 10)]
+q = 60
+S, T = order[rng.integers(0, 3000, q)], order[-1 - rng.integers(0, 3000, q)]
 src = np.repeat(np.arange(g.n, dtype=np.int32), np.diff(g.off))
-w, versions, failed = g.w.copy(), [g.w.copy()], 0
-first = srv.submit(S.astype(np.int32), T.astype(np.int32))
-for k in range(24):
+w, versions, failed, batches = g.w.copy(), [g.w.copy()], 0, []
+for k in range(24):  # made before the requests, which then outlast them
     j = rng.choice(g.e, 20000 if k % 2 else 200, replace=False)
-    w[j] = w[j] + rng.integers(1, 2000, len(j)).astype(np.uint32)
+    batches.append((j, rng.integers(1, 2000, len(j)).astype(np.uint32)))
+first = srv.submit(S.astype(np.int32), T.astype(np.int32))
+for j, more in batches:
+    w[j] = w[j] + more
     try:
         srv.update(np.full(len(j), 2, np.int32), src[j], g.col[j], w[j])
         versions.append(w.copy())
@@ -96,8 +99,8 @@ for k in range(24):
         failed += 1
 ids, costs, _, ver = srv.drain()
 assert failed > 0, "no update ran into the wait"
-assert srv.stats()["version"] == len(versions) - 1
-for k in range(len(ids)):
+assert srv.stats()["version"] == len(versions) - 1 and len(ids) == q
+for k in range(0, q, 3):
     i = int(ids[k]) - first
     gv = d.CSR(g.n, g.off, g.col, versions[int(ver[k])])
     assert costs[k] == cost(gv, int(S[i]), int(T[i])), (i, int(ver[k]))
@@ -109,7 +112,7 @@ srv.submit(S[:3].astype(np.int32), T[:3].astype(np.int32))
 ids, costs, _, _ = srv.drain()
 gv = d.CSR(g.n, g.off, g.col, w)
 for k in range(len(ids)):
-    i = int(ids[k]) - first - 10
+    i = int(ids[k]) - first - q
     assert costs[k] == cost(gv, int(S[i]), int(T[i]))
 srv.close()
 """)
