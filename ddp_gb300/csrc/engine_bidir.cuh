@@ -466,14 +466,17 @@ struct PotALT {
     static __device__ __forceinline__ uint32_t lo16(uint32_t x) { return __byte_perm(x, 0u, 0x4140); }  // bytes 0, 1
     static __device__ __forceinline__ uint32_t hi16(uint32_t x) { return __byte_perm(x, 0u, 0x4342); }  // bytes 2, 3
     // Fills words (two per four landmarks: forward, then backward half):
-    // {t, 256 - s} forward, {256 - t, s} backward.  All threads of a CTA.
-    static __device__ void query_row(const HeurALT &alt, int32_t s, uint4 *words) {
+    // {t, 256 - s} forward, {256 - t, s} backward.  All threads of a CTA; sets
+    // *cut when a landmark proves that s cannot reach t (it reaches s and not
+    // t, or t reaches it and s does not).
+    static __device__ void query_row(const HeurALT &alt, int32_t s, uint4 *words, int *cut) {
         const int n4 = alt.L / 4;  // 4-byte words per half row
         const uint32_t *rt = reinterpret_cast<const uint32_t *>(alt.tab) + (size_t)alt.t * (2 * n4);
         const uint32_t *rs = reinterpret_cast<const uint32_t *>(alt.tab) + (size_t)s * (2 * n4);
         for (int i = threadIdx.x; i < 2 * n4; i += blockDim.x) {
             const uint32_t t = __ldg(rt + i), x = __ldg(rs + i);
             const uint32_t neg = i < n4 ? x : t, pos = i < n4 ? t : x;
+            if (__vcmpeq4(pos, 0xFFFFFFFFu) & ~__vcmpeq4(neg, 0xFFFFFFFFu)) *cut = 1;
             words[i] = make_uint4(lo16(pos), hi16(pos), C256 - lo16(neg), C256 - hi16(neg));
         }
     }

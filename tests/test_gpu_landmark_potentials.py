@@ -51,3 +51,42 @@ def test_costs_for_every_row_width(gpu, oracle, bits, counts, kind):
                     assert ok, why
             be.close()
     dg.close()
+
+
+@pytest.mark.parametrize("count,bits", [(8, 8), (24, 8), (16, 16)])
+@pytest.mark.parametrize("ways", [0, 1])
+def test_pairs_without_a_path(gpu, oracle, count, bits, ways):
+    """Two halves with no arcs between them, or arcs one way only: a landmark
+    on the right side proves that there is no path and nothing is expanded;
+    every cost equals the oracle's, reachable pairs and equal ends among them."""
+    d = gpu
+    a = d.gen_random_chain(1500, 4, 1, 100, 5)
+    n, rng = 2 * a.n, np.random.default_rng(count + ways)
+    src = np.repeat(np.arange(a.n), np.diff(a.off))
+    s2, d2 = np.concatenate([src, src + a.n]), np.concatenate([a.col, a.col + a.n])
+    if ways:
+        s2, d2 = np.concatenate([s2, rng.integers(0, a.n, 50)]), np.concatenate([d2, rng.integers(a.n, n, 50)])
+    o = np.argsort(s2, kind="stable")
+    off = np.concatenate([[0], np.cumsum(np.bincount(s2, minlength=n))]).astype(np.int32)
+    g = d.CSR(n, off, d2[o].astype(np.int32), rng.integers(1, 101, len(s2)).astype(np.uint32))
+    S, T = (rng.integers(0, n, 200).astype(np.int32) for _ in range(2))
+    T[:5] = S[:5]
+    gs = g.with_sentinel()
+    want, _, _, done = oracle.astar_many(gs.n, gs.off[:-1], gs.col, gs.w, S, T, hkind=0, mode=oracle.HEAP_POSMAP,
+                                         threads=4, budget_s=1e9)
+    assert done == len(S)
+    dg = d.DeviceGraph.from_csr(g)
+    dg.build_landmarks(count, seed=2, bits=bits)
+    eng = d.BatchEngine(dg, d.H_LANDMARK)
+    for _ in range(2):
+        cost, plen = eng.solve(S, T)
+        assert np.array_equal(cost, want)
+        none = cost == d.INF
+        assert none.any() and not none.all() and (plen[none] == 0).all()
+        assert (eng.stats()[0][none, 0] == 0).mean() > 0.9  # expanded: nothing
+    for i in range(0, 200, 7):
+        if cost[i] != d.INF:
+            ok, why = oracle.check_path(g.off, g.col, g.w, eng.path(i), int(S[i]), int(T[i]), int(cost[i]))
+            assert ok, why
+    eng.close()
+    dg.close()
