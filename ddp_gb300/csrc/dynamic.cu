@@ -565,6 +565,8 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
         __syncthreads();
     }
     at.again = false;
+    __shared__ int words[2];
+    bool failed = false;
     int it = 0, levels = 0;
     // a level pushes into the counter after its own; the one that no thread
     // reads any more is cleared for the level after
@@ -577,10 +579,15 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
             at.nf = *(volatile int *)&cnt[it % 3];
             next = cnt + (it + 1) % 3;
         } else {
-            grp.sync();
+            // read once: the CTA's threads agree on whether to go on
+            grp.sync_fetch([&] {
+                words[0] = *(volatile int *)&dc->cnt[(it + 1) & 3];
+                words[1] = *(volatile int *)&B.ctl->status;
+            });
             if (rank == 0) dc->cnt[(it + 3) & 3] = 0;
             it++;
-            at.nf = *(volatile int *)&dc->cnt[it & 3];
+            at.nf = words[0];
+            failed = (words[1] & (ST_OVERFLOW | ST_TIMEOUT)) != 0;
             next = dc->cnt + ((it + 1) & 3);
         }
     };
@@ -608,9 +615,7 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
                 return false;
             }
             // a push past the buffer raised an overflow: its count is not a frontier
-            if (SOLO ? at.nf > DYN_LOCAL_BAIL
-                     : (*(volatile int *)&B.ctl->status & (ST_OVERFLOW | ST_TIMEOUT)) != 0)
-                return !SOLO;
+            if (SOLO ? at.nf > DYN_LOCAL_BAIL : failed) return !SOLO;
             int32_t *t = at.fa;
             at.fa = at.fb;
             at.fb = t;
