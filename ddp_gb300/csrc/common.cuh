@@ -73,13 +73,15 @@ struct DevGraph {
     // Landmark distances (ALT heuristic), null when not built: row v holds
     // lm_L values q(L_i, v) then lm_L values q(v, L_i), lm_bits (16 or 8)
     // each, with q = floor(d / lm_scale) and the all-ones entry
-    // (LM_UNREACHED16 / LM_UNREACHED8) when there is no path.  Each half row
+    // (LM_UNREACHED16 / LM_UNREACHED8) when there is no path, or only one
+    // longer than that entry times lm_scale (at most INF_G).  Each half row
     // is a whole number of 8-byte words: lm_L is a multiple of 4 (16-bit)
     // or of 8 (8-bit).
     const uint2 *lm;
     int32_t lm_L;
     int32_t lm_scale;
     int32_t lm_bits;
+    int32_t lm_cut;  // the marker means unreachable (not merely a distance past INF_G)
 };
 constexpr int32_t LM_UNREACHED = 0x7FFFFFFF;  // exhaustive-search distances
 constexpr uint32_t LM_UNREACHED16 = 0xFFFFu;  // 16-bit table entries

@@ -191,12 +191,17 @@ struct HeurALT {
     int32_t L;         // landmarks, a multiple of 4 (16-bit) or 8 (8-bit)
     int32_t s;         // DevGraph::lm_scale
     int32_t t;
-    int32_t bits;      // DevGraph::lm_bits: 16 or 8
+    int32_t mode;      // DevGraph::lm_bits (16 or 8) + 256 lm_cut
+    __device__ __forceinline__ bool bytes() const { return (mode & 255) == 8; }
+    __device__ __forceinline__ bool cut() const { return mode >= 256; }
     // One packed word of B-bit entries, a from the row that must be larger:
-    // the lanes' a - b, saturated at 0 and zeroed where either side is the
-    // unreachable marker, fold into the lane-wise maximum m; lanes where a
+    // the lanes' a - b, saturated at 0, fold into the lane-wise maximum m (the
+    // marker counts as an entry: as b it leaves nothing, as a it stands for a
+    // distance of at least that many scales, so the bound stays one, and stays
+    // consistent, where a distance was too long for the table); lanes where a
     // is the marker and b is not (the landmark relates v and t one way
-    // only, so v cannot reach t) fold into the cut mask cm.  Since s >= 1,
+    // only, so v cannot reach t if every finite distance is in the table:
+    // cut) fold into the cut mask cm.  Since s >= 1,
     // the maximum over terms of s (a - b) - (s - 1), floored at 0, is
     // s max(a - b) - (s - 1) when that maximum is positive, else 0.
     template <int B>
@@ -204,11 +209,11 @@ struct HeurALT {
         if (B == 8) {
             const uint32_t ea = __vcmpeq4(a, 0xFFFFFFFFu), eb = __vcmpeq4(b, 0xFFFFFFFFu);
             cm |= ea & ~eb;
-            m = __vmaxu4(m, __vsubus4(a, b) & ~(ea | eb));
+            m = __vmaxu4(m, __vsubus4(a, b));
         } else {
             const uint32_t ea = __vcmpeq2(a, 0xFFFFFFFFu), eb = __vcmpeq2(b, 0xFFFFFFFFu);
             cm |= ea & ~eb;
-            m = __vmaxu2(m, __vsubus2(a, b) & ~(ea | eb));
+            m = __vmaxu2(m, __vsubus2(a, b));
         }
     }
     template <int B>
@@ -246,17 +251,17 @@ struct HeurALT {
                 terms<B>(bv, bt, m, cm);
             }
         }
-        return cm ? INF_G : top<B>(m);
+        return cm && cut() ? INF_G : top<B>(m);
     }
     // the bound of the lane-wise maximum m
     template <int B>
     __device__ __forceinline__ uint32_t top(uint32_t m) const {
         const uint32_t mx = B == 8 ? max(max(m & 0xFFu, (m >> 8) & 0xFFu), max((m >> 16) & 0xFFu, m >> 24))
                                    : max(m & 0xFFFFu, m >> 16);
-        // mx s <= q s <= the largest table distance, below INF_G
+        // mx s is at most the marker times s, at most INF_G
         return mx ? mx * (uint32_t)s - (uint32_t)(s - 1) : 0u;
     }
-    __device__ uint32_t operator()(int32_t v) const { return bits == 8 ? eval<8>(v) : eval<16>(v); }
+    __device__ uint32_t operator()(int32_t v) const { return bytes() ? eval<8>(v) : eval<16>(v); }
 };
 
 // floor(sqrt(x)) for x < 2^62, exact: a float estimate, then integer fix-up

@@ -141,6 +141,7 @@ struct WaveQ {
     unsigned int pile_min[2];        // their smallest key
     int status;
     int touched;
+    int no_path;  // table potentials: t is known to be out of s's reach, the search starts empty
     long long spent;                 // entries expanded or dropped
     unsigned long long edge_mul;     // 2^64 / (2^32 / bucket width)
     uint32_t settled[2][WAVE_FILTER];  // lazy labels: filter over settled nodes
@@ -445,15 +446,14 @@ struct PotManhattan {
 // table entries floor(d / sc) each bound lies at most 2 (sc - 1) below the
 // exact landmark bound, which is consistent, and never above it: a key
 // exceeds its consistent one by at most the error of the bound it subtracts.
-// A bound of INF_G says that the pair is not connected.
 //
 // What an evaluation costs is its instructions.  With 8-bit entries the bytes
 // of a row are spread into 16-bit halves and each difference is one
 // add-and-maximum per pair (256 + a - b, floored at 256); the rows of t and s
 // are prepared in shared memory in the form that the sums want (query_row).
-// The unreachable marker 255 needs no test: as the subtracted entry it gives
+// The unreachable marker (255, 65535) needs no test: as the subtracted entry it gives
 // a negative difference, and as the one subtracted from it says that there is
-// no path, for which every bound holds.  The per-byte compare, subtract and
+// no path, for which every bound holds, or one of at least 255 scales.  The per-byte compare, subtract and
 // maximum intrinsics, which the hardware does not have, took 2,000
 // instructions per evaluation of 64 landmarks instead of 300.
 struct PotALT {
@@ -476,7 +476,7 @@ struct PotALT {
         for (int i = threadIdx.x; i < 2 * n4; i += blockDim.x) {
             const uint32_t t = __ldg(rt + i), x = __ldg(rs + i);
             const uint32_t neg = i < n4 ? x : t, pos = i < n4 ? t : x;
-            if (__vcmpeq4(pos, 0xFFFFFFFFu) & ~__vcmpeq4(neg, 0xFFFFFFFFu)) *cut = 1;
+            if (alt.cut() && (__vcmpeq4(pos, 0xFFFFFFFFu) & ~__vcmpeq4(neg, 0xFFFFFFFFu))) *cut = 1;
             words[i] = make_uint4(lo16(pos), hi16(pos), C256 - lo16(neg), C256 - hi16(neg));
         }
     }
@@ -524,18 +524,22 @@ struct PotALT {
         const int W = alt.L / 4;  // 8-byte words per half row
         const uint2 *rv = alt.tab + (size_t)v * (2 * W);
         const uint2 *rt = alt.tab + (size_t)alt.t * (2 * W), *rs = alt.tab + (size_t)s * (2 * W);
-        uint32_t mt = 0, ct = 0, ms = 0, cs = 0;
+        uint32_t mt = 0, ms = 0;
+        auto fold = [](uint2 a, uint2 b, uint32_t &m) {
+            m = __vmaxu2(m, __vsubus2(a.x, b.x));
+            m = __vmaxu2(m, __vsubus2(a.y, b.y));
+        };
 #pragma unroll 2
         for (int i = 0; i < W; i++) {
             const uint2 f = __ldg(rv + i), b = __ldg(rv + W + i);
-            alt.terms<16>(__ldg(rt + i), f, mt, ct);
-            alt.terms<16>(b, __ldg(rt + W + i), mt, ct);
-            alt.terms<16>(f, __ldg(rs + i), ms, cs);
-            alt.terms<16>(__ldg(rs + W + i), b, ms, cs);
+            fold(__ldg(rt + i), f, mt);
+            fold(b, __ldg(rt + W + i), mt);
+            fold(f, __ldg(rs + i), ms);
+            fold(__ldg(rs + W + i), b, ms);
         }
-        return make_uint2(ct ? INF_G : alt.top<16>(mt), cs ? INF_G : alt.top<16>(ms));
+        return make_uint2(alt.top<16>(mt), alt.top<16>(ms));
     }
-    __device__ uint2 at(int v) const { return alt.bits == 8 ? eval8(v) : eval16(v); }
+    __device__ uint2 at(int v) const { return alt.bytes() ? eval8(v) : eval16(v); }
 };
 
 // Bucket key of label g in direction dir, with pot = {pt(v), ps(v)}.
@@ -673,7 +677,7 @@ __device__ __forceinline__ SearchResult run_bidir_cta(const DevGraph &G, const S
             q->plan.lo[1] = bucket(kt);
             q->plan.c[0] = q->plan.lo[0] - 1;  // nothing opened yet
             q->plan.c[1] = q->plan.lo[1] - 1;
-            if (room >= 1) {
+            if (room >= 1 && !(Pot::table && q->no_path)) {
                 // lazy: no parent; else the label
                 const uint32_t x = LAZY ? NONE : 0u;
                 const int l0 = (int)(q->plan.lo[0] % WAVE_LISTS), l1 = (int)(q->plan.lo[1] % WAVE_LISTS);

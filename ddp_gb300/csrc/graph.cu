@@ -75,6 +75,7 @@ DevGraph graph_view(const ddp_graph *g) {
     d.lm_L = lm_ok ? g->lm_L : 0;
     d.lm_scale = lm_ok ? g->lm_scale : 1;
     d.lm_bits = lm_ok ? g->lm_bits : 16;
+    d.lm_cut = lm_ok && g->lm_cut;
     return d;
 }
 

@@ -66,6 +66,7 @@ struct ddp_graph {
     int32_t lm_L = 0;
     int32_t lm_scale = 1;
     int32_t lm_bits = 16;
+    bool lm_cut = false;  // DevGraph::lm_cut
     int64_t lm_stamp = -1;
     std::vector<int32_t> lm_ids;
     // arrays of n words that freed heuristics left for the next ones (two at most)

@@ -323,7 +323,7 @@ template <class E>
 __global__ void k_pack_landmarks(const int32_t *tab32, E *tab, int64_t count, int32_t scale) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
         const int32_t d = tab32[i];
-        tab[i] = d == LM_UNREACHED ? (E)~(E)0 : (E)(d / scale);
+        tab[i] = d == LM_UNREACHED || d / scale >= (E)~(E)0 ? (E)~(E)0 : (E)(d / scale);
     }
 }
 
@@ -331,7 +331,7 @@ __global__ void k_pack_landmarks(const int32_t *tab32, E *tab, int64_t count, in
 __global__ void k_alt_values(DevGraph G, int32_t t, int32_t *out) {
     const int32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= G.n) return;
-    const uint32_t h = HeurALT{G.lm, G.lm_L, G.lm_scale, t, G.lm_bits}(v);
+    const uint32_t h = HeurALT{G.lm, G.lm_L, G.lm_scale, t, G.lm_bits + 256 * G.lm_cut}(v);
     out[v] = h >= INF_G ? -1 : (int32_t)h;
 }
 
@@ -349,15 +349,6 @@ __device__ SearchResult slot_search(const Grp &grp, const DevGraph &G, const Slo
     // the heuristic is cheap enough that one atomic per arc wins
     if constexpr (ASYNC) return run_search_cta<Heur, heur_cheap<Heur>::value>(G, B, H, P, wrows, sq);
     else return run_search(grp, G, B, H, P, wrows);
-}
-
-// The counters and the meeting word of a search that found no path unsearched.
-__device__ __forceinline__ void bidir_no_path(SearchCtl *ctl, WaveQ *q) {
-    ctl->iters = 0;
-    ctl->expanded = ctl->scanned = ctl->relaxed = 0;
-    ctl->far_scanned = 0;
-    ctl->touched = 0;
-    q->mu = ~0ull;
 }
 
 // The plain bidirectional search with labels installed at once (not inlined:
@@ -568,7 +559,7 @@ __device__ __forceinline__ void batch_loop(const Grp &grp, const DevGraph &G0, c
             int2 tp = reinterpret_cast<const int2 *>(G.xy)[t];
             r = slot_search<ASYNC>(grp, G, B, HeurEuclid{G.xy, tp.x, tp.y, G.rho_fp}, P, wrows, sq);
         } else if (HK == 4) {
-            r = slot_search<ASYNC>(grp, G, B, HeurALT{G.lm, G.lm_L, G.lm_scale, t, G.lm_bits}, P, wrows, sq);
+            r = slot_search<ASYNC>(grp, G, B, HeurALT{G.lm, G.lm_L, G.lm_scale, t, G.lm_bits + 256 * G.lm_cut}, P, wrows, sq);
         } else if (bidir_hk(HK)) {
             // bidirectional: one-CTA slots only (the host never launches
             // these kinds with wider slots)
@@ -603,24 +594,16 @@ __device__ __forceinline__ void batch_loop(const Grp &grp, const DevGraph &G0, c
                     r = run_bidir_cta<true>(G, B, P, ep, bq, PotNone{}, R);
                 } else if constexpr (HK == 10) {
                     __shared__ uint4 words[2 * 32];  // up to 128 landmarks of 8 bits
-                    __shared__ int cut;
-                    const HeurALT alt{G.lm, G.lm_L, G.lm_scale, t, G.lm_bits};
-                    if (threadIdx.x == 0) cut = alt.bits == 16 && alt(s) >= INF_G;
+                    const HeurALT alt{G.lm, G.lm_L, G.lm_scale, t, G.lm_bits + 256 * G.lm_cut};
+                    // no path: the two searches would take all they reach (64
+                    // pairs between the halves of 200,000 nodes 32.9 ms, 6.9 by
+                    // A* under the same bound, which cut so too)
+                    if (threadIdx.x == 0) bq->no_path = !alt.bytes() && alt(s) >= INF_G;
                     grp.sync();
-                    if (alt.bits == 8) PotALT::query_row(alt, s, words, &cut);
+                    if (alt.bytes()) PotALT::query_row(alt, s, words, &bq->no_path);
                     grp.sync();
-                    if (cut) {
-                        // no path: the two searches would take all they reach
-                        // (64 pairs between the halves of 200,000 nodes 32.9 ms,
-                        // 6.9 by A* under the same bound, which cut so too)
-                        if (threadIdx.x == 0) bidir_no_path(ctl, bq);
-                        grp.sync();
-                        r.cost = 0xFFFFFFFFu;
-                        r.iters = 0;
-                    } else {
-                        r = run_bidir_cta<false>(G, B, P, ep, bq, PotALT{alt, s, words, words + alt.L / 4},
-                                                 RecDense{{}, B.state});
-                    }
+                    r = run_bidir_cta<false>(G, B, P, ep, bq, PotALT{alt, s, words, words + alt.L / 4},
+                                             RecDense{{}, B.state});
                 } else if constexpr (HK == 9) {
                     r = run_bidir_cta<false>(G, B, P, ep, bq, PotNone{}, RecPair16{B.state});
                 } else {
@@ -1536,7 +1519,10 @@ int ddp_landmarks_build_bits(ddp_graph *g, int32_t count, int32_t bits, uint64_t
     // entries q = floor(d / scale) with every finite q below the all-ones
     // unreachable marker: the smallest scale with maxd / scale <= marker - 1
     const int32_t top = bits == 16 ? 65534 : 254;
-    const int32_t scale = std::max(1, (int32_t)(((int64_t)maxd + top - 1) / top));
+    // (the marker times the scale stays within INF_G: longer distances than that
+    // get the marker too)
+    const int32_t scale = std::min((int32_t)(INF_G / (uint32_t)(top + 1)),
+                                   std::max(1, (int32_t)(((int64_t)maxd + top - 1) / top)));
     void *packed = nullptr;
     e = cudaMalloc(&packed, (size_t)(bits / 8) * (size_t)n * width);
     if (e != cudaSuccess) return done(cuda_fail(e, "cudaMalloc(landmarks)"));
@@ -1554,6 +1540,8 @@ int ddp_landmarks_build_bits(ddp_graph *g, int32_t count, int32_t bits, uint64_t
     g->d_lm = reinterpret_cast<uint2 *>(packed);
     g->lm_scale = scale;
     g->lm_bits = bits;
+    // the marker proves that there is no path unless a distance was too long
+    g->lm_cut = (int64_t)maxd + g->wmax < (int64_t)INF_G && maxd / scale <= top;
     g->lm_L = count;
     g->lm_stamp = g->update_count;
     g->lm_ids = ids;
@@ -1656,7 +1644,7 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
             HeurManhattan Hm{g->d_xy, h ? h->tx : 0, h ? h->ty : 0, g->wmin};
             HeurEuclid He{g->d_xy, h ? h->tx : 0, h ? h->ty : 0, g->rho_fp};
             HeurArray Ha{h ? reinterpret_cast<const int32_t *>(h->d_h) : nullptr};
-            HeurALT Hl{G.lm, G.lm_L, G.lm_scale, target, G.lm_bits};
+            HeurALT Hl{G.lm, G.lm_L, G.lm_scale, target, G.lm_bits + 256 * G.lm_cut};
             HeurZero Hz{};
             const void *fn;
             if (kind == DDP_H_BFS_HOPS || kind == DDP_H_BFS_CAPPED) { fn = (const void *)k_solve_cta<HeurHops>; hp = &Hh; }
@@ -1688,7 +1676,7 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
             void *args[] = {&G, &w->sa, &H, &P, &w->d_res, &w->d_path, &g->n};
             e = coop_launch(k_solve_single<HeurArray>, grid, block, args, st);
         } else if (kind == DDP_H_LANDMARK) {
-            HeurALT H{G.lm, G.lm_L, G.lm_scale, target, G.lm_bits};
+            HeurALT H{G.lm, G.lm_L, G.lm_scale, target, G.lm_bits + 256 * G.lm_cut};
             int grid = coop_grid(k_solve_single<HeurALT>, block, o.grid);
             void *args[] = {&G, &w->sa, &H, &P, &w->d_res, &w->d_path, &g->n};
             e = coop_launch(k_solve_single<HeurALT>, grid, block, args, st);
@@ -1938,7 +1926,7 @@ static bool same_view(const DevGraph &x, const DevGraph &y) {
            x.rarc == y.rarc && x.xy == y.xy && x.wmin == y.wmin && x.rho_fp == y.rho_fp && x.doff == y.doff &&
            x.darc == y.darc && x.droff == y.droff && x.drarc == y.drarc && x.oend == y.oend &&
            x.roend == y.roend && x.lm == y.lm && x.lm_L == y.lm_L && x.lm_scale == y.lm_scale &&
-           x.lm_bits == y.lm_bits;
+           x.lm_bits == y.lm_bits && x.lm_cut == y.lm_cut;
 }
 
 static bool same_args(const BatchArgs &x, const BatchArgs &y) {

@@ -90,3 +90,36 @@ def test_pairs_without_a_path(gpu, oracle, count, bits, ways):
             assert ok, why
     eng.close()
     dg.close()
+
+
+@pytest.mark.parametrize("bits,count", [(8, 8), (16, 8)])
+@pytest.mark.parametrize("wmax", [900_000, 2_500_000, 150_000_000])
+def test_distances_past_the_tables(gpu, oracle, bits, count, wmax):
+    """A long chain with shortcuts and heavy arcs: landmark distances reach
+    and pass the largest cost (2^31), so that a table's unreachable marker no
+    longer proves that there is no path."""
+    d = gpu
+    rng = np.random.default_rng(wmax)
+    n = 3000
+    s, t = np.arange(n - 1), np.arange(1, n)
+    e = rng.integers(0, n, 300)
+    s, t = np.concatenate([s, e]), np.concatenate([t, np.minimum(e + rng.integers(1, 50, 300), n - 1)])
+    o = np.argsort(s, kind="stable")
+    off = np.concatenate([[0], np.cumsum(np.bincount(s, minlength=n))]).astype(np.int32)
+    g = d.CSR(n, off, t[o].astype(np.int32), rng.integers(1, wmax + 1, len(s)).astype(np.uint32))
+    S = rng.integers(0, n, 200).astype(np.int32)
+    T = np.minimum(S + rng.integers(0, 60 if wmax > 10_000_000 else 3000, 200), n - 1).astype(np.int32)
+    want = _want(oracle, g, S, T)
+    assert (want != INF).any()
+    dg = d.DeviceGraph.from_csr(g)
+    dg.build_landmarks(count, seed=3, bits=bits)
+    for kw in ({}, {"group": 2}, {"flags": d.OPT_SYNC}):
+        be = d.BatchEngine(dg, d.H_LANDMARK, **kw)
+        cost, _ = be.solve(S, T)
+        assert np.array_equal(cost, want), (kw, np.flatnonzero(cost != want)[:5])
+        be.close()
+    for i in range(0, 200, 20):
+        h = dg.heuristic(int(T[i]), d.H_LANDMARK)
+        assert dg.solve(int(S[i]), int(T[i]), h).cost == want[i]
+        h.close()
+    dg.close()
