@@ -2174,6 +2174,9 @@ int ddp_batch_path(ddp_batch *b, int32_t i, int32_t *buf, int32_t cap, int32_t *
         *len = (int32_t)q->path.size();
         if (buf && cap > 0)
             std::memcpy(buf, q->path.data(), sizeof(int32_t) * std::min<size_t>(cap, q->path.size()));
+        // a caller asks for the length, then for the nodes: of one path (another
+        // run may find another of equal cost)
+        b->overflow_paths[i] = std::move(q->path);
         ddp_query_free(q);
         return DDP_OK;
     }

@@ -81,3 +81,28 @@ def test_single_query_paths_are_simple(gpu, oracle, n, weights):
                     else:
                         _check(O, g, r.path, s, t, c)
             dg.close()
+
+
+def test_long_paths_read_back_whole(gpu, oracle):
+    """Paths longer than a slot keeps (1,024 nodes) are found again when they
+    are asked for; length and nodes are of one path, although ties leave many."""
+    d, O = gpu, oracle
+    rng = np.random.default_rng(9)
+    n = 7000
+    src = np.repeat(np.arange(n), 8)
+    col = np.clip(src + rng.integers(-5, 6, 8 * n), 0, n - 1)
+    off = np.arange(0, 8 * n + 1, 8).astype(np.int32)
+    g = d.CSR(n, off, col.astype(np.int32), rng.integers(1, 4, 8 * n).astype(np.uint32))
+    S, T = np.arange(0, 40, 2).astype(np.int32), np.arange(n - 40, n, 2).astype(np.int32)
+    want = _wants(O, g, S, T)
+    dg = d.DeviceGraph.from_csr(g)
+    for kind, kw in ((d.H_BIDIR, {}), (d.H_BFS_HOPS, {}), (d.H_ZERO, {"flags": d.OPT_SYNC})):
+        eng = d.BatchEngine(dg, kind, **kw)
+        cost, plen = eng.solve(S, T)
+        assert np.array_equal(cost, want) and plen.min() > 1024
+        for i in range(len(S)):
+            p = eng.path(i)
+            _check(O, g, p, int(S[i]), int(T[i]), int(cost[i]))
+            assert np.array_equal(p, eng.path(i))
+        eng.close()
+    dg.close()
