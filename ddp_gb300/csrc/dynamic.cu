@@ -22,7 +22,9 @@
 //   device, one cooperative kernel (CTA 0 alone while a step is narrow):
 //     A. heuristic repair: an inserted arc can shorten hop distances to the
 //        target; hops are lowered by decrease propagation over the reverse
-//        graph, so h stays admissible and consistent;
+//        graph, so h stays admissible and consistent.  Nodes that could not
+//        reach the target before were never labelled: they join the nodes to
+//        re-seed;
 //     B. invalidation: a deleted (or heavier) arc that is the parent arc of
 //        its head invalidates the head's subtree of the shortest-path tree
 //        (found by walking child arcs whose head names the node as parent);
@@ -483,7 +485,8 @@ struct DynCtl {
     int reseeded;
     int stage, nf, odd;  // CTA 0's hand-back (RepairAt; odd: its buffers are swapped)
     int again;           // it is to go on alone
-    int pad[3];
+    int opened;          // nodes of step A among those to re-seed
+    int pad[2];
 };
 
 __device__ __forceinline__ SlotBufs slot_of_dyn(const SlotArrays &sa) {
@@ -560,8 +563,11 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
     int *inv_n = SOLO ? cnt + 3 : &dc->inv_n;
     int *far_add = SOLO ? cnt + 4 : &dc->far_add;
     if (SOLO) {
-        // (dc->inv_n: nodes that an earlier turn invalidated)
-        if (threadIdx.x < 5) cnt[threadIdx.x] = threadIdx.x == 3 ? *(volatile int *)&dc->inv_n : 0;
+        // (what earlier turns invalidated and opened)
+        if (threadIdx.x < 5)
+            cnt[threadIdx.x] = threadIdx.x == 3   ? *(volatile int *)&dc->inv_n
+                               : threadIdx.x == 4 ? *(volatile int *)&dc->far_add
+                                                  : 0;
         __syncthreads();
     }
     at.again = false;
@@ -642,6 +648,28 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
         return true;
     };
 
+    // an open entry for node x at label g
+    auto to_far = [&](int x, uint32_t g) {
+        const int s = atomicAdd(far_add, 1);
+        if (far_base + s < B.cap_f) far_buf[far_base + s] = make_uint4((uint32_t)x, g, 0u, 0u);
+        else atomicOr(&B.ctl->status, ST_OVERFLOW);
+    };
+    // Node p's hops were lowered from old.  If it had none, or a bound past the
+    // largest cost, the searches have passed it over until now: without a label it
+    // is re-seeded (each node once, and never one that B invalidates), with one
+    // (the source, heads of inserted arcs) it is opened again.
+    auto lowered = [&](int p, uint32_t old, int rb, int re) {
+        push(p, rb, re);
+        atomicAdd(&dc->hops_lowered, 1);
+        if (old != HOPS_INF && (unsigned long long)old * G.wmin < INF_G) return;
+        const uint32_t g = st_g(__ldcg(B.state + p));
+        if (g < INF_G) {
+            to_far(p, g);
+        } else {
+            A.inv[atomicAdd(inv_n, 1)] = p;
+            atomicAdd(&dc->opened, 1);
+        }
+    };
     // ---- A. heuristic repair: lower hops over inserted arcs ---------------
     if (at.stage == REP_HOPS) {
         for (int i = rank; i < nupd; i += size) {
@@ -650,10 +678,8 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
             const uint32_t hv = __ldcg(hops + up.z);
             const int rb = row_begin(G.roff, G.roend, up.y), re = row_end(G.roff, G.roend, up.y);
             if (hv == HOPS_INF) continue;
-            if (hv + 1 < atomicMin(hops + up.y, hv + 1)) {
-                push(up.y, rb, re);
-                atomicAdd(&dc->hops_lowered, 1);
-            }
+            const uint32_t old = atomicMin(hops + up.y, hv + 1);
+            if (hv + 1 < old) lowered(up.y, old, rb, re);
         }
         level_end();
         at.stage = REP_HOPS_WALK;
@@ -686,9 +712,11 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
 #pragma unroll
                 for (int k = 0; k < DYN_ARCS; k++) {
                     if (hu + 1 >= old[k]) continue;
-                    if (!SOLO && hu + 1 >= atomicMin(hops + p[k], hu + 1)) continue;
-                    push(p[k], rb[k], re[k]);
-                    atomicAdd(&dc->hops_lowered, 1);
+                    if (!SOLO) {
+                        old[k] = atomicMin(hops + p[k], hu + 1);
+                        if (hu + 1 >= old[k]) continue;
+                    }
+                    lowered(p[k], old[k], rb[k], re[k]);
                 }
             }
         };
@@ -775,9 +803,7 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
         if (bv.x >= INF_G) continue;
         const int x = A.inv[i];
         B.state[x] = st_make(bv.x, (int32_t)bv.y);
-        const int s = atomicAdd(far_add, 1);
-        if (far_base + s < B.cap_f) far_buf[far_base + s] = make_uint4((uint32_t)x, bv.x, 0u, 0u);
-        else atomicOr(&B.ctl->status, ST_OVERFLOW);
+        to_far(x, bv.x);
         atomicAdd(&dc->reseeded, 1);
     }
     grp.sync();
@@ -794,9 +820,7 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
         while (ng < st_g(cur)) {
             const uint64_t got = atomicCAS(B.state + up.z, cur, st_make(ng, up.y));
             if (got == cur) {
-                const int s = atomicAdd(far_add, 1);
-                if (far_base + s < B.cap_f) far_buf[far_base + s] = make_uint4((uint32_t)up.z, ng, 0u, 0u);
-                else atomicOr(&B.ctl->status, ST_OVERFLOW);
+                to_far(up.z, ng);
                 atomicAdd(&dc->relaxed, 1);
                 break;
             }
@@ -841,6 +865,7 @@ __global__ void __launch_bounds__(512, 1)
                     __syncthreads();
                     if (threadIdx.x == 0) {
                         dc->inv_n = cnt[3];
+                        dc->far_add = cnt[4];
                         dc->stage = at.stage;
                         dc->nf = at.nf;
                         dc->odd = at.fa != reinterpret_cast<int32_t *>(B.q0);
@@ -888,7 +913,7 @@ __global__ void __launch_bounds__(512, 1)
         A.out[1] = plen;
         A.out[2] = B.ctl->status;
         A.out[3] = r.iters;
-        A.out[4] = *(volatile int *)&dc->inv_n;
+        A.out[4] = *(volatile int *)&dc->inv_n - *(volatile int *)&dc->opened;
         A.out[5] = *(volatile int *)&dc->reseeded;
         A.out[6] = *(volatile int *)&dc->relaxed;
         A.out[7] = *(volatile int *)&dc->hops_lowered;
@@ -1505,6 +1530,10 @@ int ddp_dyn_update(ddp_dyn *d, int32_t nupd, const int32_t *flag, const int32_t 
         DDP_CUDA(cudaMalloc(&d->d_upd, sizeof(int4) * std::max(nupd, 1)));
         d->upd_cap = nupd;
     }
+    // a smaller least weight lowers every bound at once, also bounds past the
+    // largest cost, whose nodes the searches have passed over
+    if (d->hkind == DDP_H_BFS_HOPS && (uint64_t)g->n * g->wmin >= INF_G)
+        for (int32_t i = 0; i < nupd && !d->anew; i++) d->anew = flag[i] != 0 && w[i] < g->wmin;
     if (d->anew) {
         int rc = dyn_graph_apply(g, nupd, flag, u, v, w, ups, true);
         if (!rc) rc = dyn_start_growing(d);

@@ -133,3 +133,74 @@ def test_queues_grow_with_the_search(gpu, oracle):
             assert got == want(), (hk, k)
         dyn.close()
         dg.close()
+
+
+@pytest.mark.parametrize("kw", [{}, {"group": 1}, {"grid": 5}, {"K": 100}])
+@pytest.mark.parametrize("extra", [0, 6000])
+def test_targets_that_come_within_reach(gpu, oracle, kw, extra):
+    """The target cannot be reached, or only from part of the graph, when the
+    search is made; inserts open ways over nodes that had no hop bound, in one
+    batch or several, some through nodes labelled before they reached it.
+    extra: further inserts, so that the batch takes the host's path."""
+    d = gpu
+    rng = np.random.default_rng(3 + extra)
+    part = d.gen_random_chain(800, 2, 1, 30, 8)
+    k, n = 4, 4 * part.n
+    src = np.repeat(np.arange(part.n), np.diff(part.off))
+    src, dst = (np.concatenate([x + i * part.n for i in range(k)]) for x in (src, part.col))
+    off = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+    g = d.CSR(n, off, dst.astype(np.int32), rng.integers(1, 31, len(src)).astype(np.uint32))
+    s, t = 5, n - 9
+    for hk in (d.H_BFS_HOPS, d.H_ZERO):
+        dg = d.DeviceGraph.from_csr(g)
+        dyn = d.DynamicSearch(dg, s, t, hk, **kw)
+        o, c, w = g.with_sentinel().off[:-1].copy(), g.col.copy(), g.w.copy()
+        assert dyn.cost == d.INF
+
+        def step(f, u, v, ww):
+            nonlocal o, c, w
+            more = rng.integers(0, part.n, (2, extra))  # inside the first part
+            f, u = np.concatenate([f, np.ones(extra)]), np.concatenate([u, more[0]])
+            v, ww = np.concatenate([v, more[1]]), np.concatenate([ww, np.full(extra, 1000)])
+            f, u, v, ww = f.astype(np.int32), u.astype(np.int32), v.astype(np.int32), ww.astype(np.uint32)
+            got = dyn.update(f, u, v, ww)
+            o, c, w, _ = oracle.apply_batch(len(o), o, c, w, f, u, v, ww)
+            f_, want, _, _, _ = oracle.astar(len(o), o, c, w, np.zeros(len(o), np.int32), s, t,
+                                             mode=oracle.HEAP_POSMAP)
+            assert got == (want if f_ else d.INF), (hk, got, want)
+
+        at = lambda i: int(rng.integers(0, part.n)) + i * part.n  # noqa: E731
+        step([1], [at(0)], [at(1)], [3])           # heads labelled, still no way
+        step([1, 1], [at(2), at(1)], [at(3), at(1)], [5, 2])
+        step([1], [at(1)], [at(2)], [4])           # now there is one
+        step([0, 1, 1], [at(0), at(0), at(1)], [at(0), at(3), at(3)], [0, 40, 9])
+        for _ in range(3):
+            j = rng.choice(np.flatnonzero(c >= 0), 60, replace=False)
+            src_now = np.repeat(np.arange(len(o)), np.diff(np.append(o, len(c))))
+            step(rng.choice([0, 2], 60), src_now[j], c[j], rng.integers(1, 31, 60))
+            step(np.ones(8), rng.integers(0, n, 8), rng.integers(0, n, 8), rng.integers(1, 60, 8))
+        dyn.close()
+        dg.close()
+
+
+def test_bounds_past_the_largest_cost(gpu, oracle):
+    """Hops times the least weight beyond 2^31: such nodes count as out of
+    reach until inserts shorten their hops or a light arc lowers the bounds."""
+    d = gpu
+    n = 3000
+    off = np.concatenate([np.arange(n), [n - 1]]).astype(np.int32)
+    g = d.CSR(n, off, np.arange(1, n, dtype=np.int32), np.full(n - 1, 2_000_000, np.uint32))
+    for light in (2_000_000, 7):
+        dg = d.DeviceGraph.from_csr(g)
+        dyn = d.DynamicSearch(dg, 0, n - 1, d.H_BFS_HOPS)
+        assert dyn.cost == d.INF
+        o, c, w = g.with_sentinel().off[:-1].copy(), g.col.copy(), g.w.copy()
+        for u, v, x in ((900, 2100, light), (10, 880, light), (2300, 2990, light), (0, 5, light)):
+            f, u, v, x = (np.array([a]) for a in (1, u, v, x))
+            got = dyn.update(f, u, v, x)
+            o, c, w, _ = oracle.apply_batch(len(o), o, c, w, f, u, v, x)
+            f_, want, _, _, _ = oracle.astar(len(o), o, c, w, np.zeros(len(o), np.int32), 0, n - 1,
+                                             mode=oracle.HEAP_POSMAP)
+            assert got == (want if f_ else d.INF), (light, u, got, want)
+        dyn.close()
+        dg.close()
