@@ -1286,9 +1286,9 @@ static int dyn_start(ddp_dyn *d) {
 // again and again under smaller labels, or rows of hundreds of arcs, push more
 // entries between two compactions than twice the nodes.
 static int dyn_start_growing(ddp_dyn *d) {
-    for (int attempt = 0;; attempt++) {
+    for (;;) {
         const int rc = dyn_start(d);
-        if (rc != DDP_ERR_QUEUE_OVERFLOW || attempt == 5) return rc;
+        if (rc != DDP_ERR_QUEUE_OVERFLOW || !queue_cap_ok(d->g, 2 * d->sa.cap_q)) return rc;
         SlotArrays sa;
         uint2 *cold = nullptr;
         const int64_t cap_q = 2 * d->sa.cap_q, cap_f = 2 * d->sa.cap_f;

@@ -1124,6 +1124,10 @@ uint32_t auto_delta(const ddp_graph *g) {
     return d < 1 ? 1 : d;
 }
 
+bool queue_cap_ok(const ddp_graph *g, int64_t cap) {
+    return cap <= 8 * ((int64_t)g->n + 1024) || cap <= 4 * (g->e + (int64_t)g->n);
+}
+
 uint32_t loose_delta(const ddp_graph *g) { return std::max(auto_delta(g), g->wmin / 2 + g->wmax / 2); }
 
 }  // namespace ddp
@@ -1397,7 +1401,7 @@ static int sssp_into(ddp_graph *g, int32_t src, bool reverse, int32_t *dist) {
     }
     SearchParams P{src, -1, auto_delta(g), 0, 0, 0};
     int64_t cap = (int64_t)g->n + 1024;
-    for (int attempt = 0; attempt < 4; attempt++) {
+    while (queue_cap_ok(g, cap)) {
         int rc = workspace_ensure(g, cap);
         if (rc) return rc;
         Workspace *w = g->ws;
@@ -1625,7 +1629,7 @@ int ddp_solve(ddp_graph *g, const ddp_heuristic *h, int32_t source, int32_t targ
             // a long search: the whole GPU takes it
         }
     }
-    for (int attempt = 0; attempt < 4; attempt++) {
+    while (o.queue_cap > 0 || queue_cap_ok(g, cap)) {
         int rc = workspace_ensure(g, cap);
         if (rc) return rc;
         Workspace *w = g->ws;

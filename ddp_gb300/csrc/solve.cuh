@@ -154,5 +154,11 @@ uint32_t auto_delta_bidir(const ddp_graph *g);
 // Fills the bucket widths and the budget of a bidirectional launch.
 void bidir_args(const ddp_graph *g, int32_t delta, BatchArgs *A);
 int64_t bfs_budget(int32_t n);
+// Whether queues of cap entries are worth a try: they begin at about the number
+// of nodes and are doubled when one overflows.  A phase pushes an entry for
+// each arc that improves its head at most, so that hubs whose rows name the
+// nodes many times over want far more entries than nodes, but never many more
+// than arcs.
+bool queue_cap_ok(const ddp_graph *g, int64_t cap);
 
 }  // namespace ddp

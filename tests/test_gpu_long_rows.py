@@ -125,3 +125,36 @@ def test_rows_in_narrow_phases(gpu, oracle, hubs, L):
             assert got == want(n - 1, off, col, w), (hk, k)
         dyn.close()
         dg.close()
+
+
+def test_queues_grow_with_the_arcs(gpu, oracle):
+    """Hubs whose rows name every node many times: a phase pushes more entries
+    than eight times the nodes."""
+    d, O = gpu, oracle
+    rng = np.random.default_rng(12)
+    n, k, L = 1500, 6, 60000
+    h = np.arange(k)
+    src = np.concatenate([np.repeat(h, L), rng.integers(0, n, 4 * n), rng.integers(0, n, k * L // 4)])
+    dst = np.concatenate([rng.integers(0, n, k * L), rng.integers(0, n, 4 * n), np.repeat(h, L // 4)])
+    o = np.argsort(src, kind="stable")
+    off = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+    g = d.CSR(n, off, dst[o].astype(np.int32), rng.integers(1, 1000001, len(src)).astype(np.uint32))
+    S, T = (rng.integers(0, n, 24).astype(np.int32) for _ in range(2))
+    gs = g.with_sentinel()
+    want, _, _, done = O.astar_many(gs.n, gs.off[:-1], gs.col, gs.w, S, T, hkind=0, mode=O.HEAP_POSMAP, threads=4,
+                                    budget_s=1e9)
+    assert done == len(S)
+    dg = d.DeviceGraph.from_csr(g)
+    dg.build_landmarks(16, seed=3, bits=8)
+    eng = d.BatchEngine(dg, d.H_LANDMARK)
+    assert np.array_equal(eng.solve(S, T)[0], want)
+    eng.close()
+    for i in range(24):
+        for kw in ({"grid": 7}, {"K": 700}, {"delta": 50}, {"delta": 1000000}):
+            assert dg.solve(int(S[i]), int(T[i]), **kw).cost == want[i], kw
+    dg.close()
+    dg = d.DeviceGraph.from_csr(g)
+    dyn = d.DynamicSearch(dg, int(S[0]), int(T[0]), d.H_BFS_HOPS)
+    assert dyn.cost == want[0]
+    dyn.close()
+    dg.close()
