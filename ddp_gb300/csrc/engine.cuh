@@ -1072,13 +1072,17 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
                         if (go[r]) {
                             uint64_t cur = sv[r];
                             uint64_t got = prev[r];
-                            // retry only when another relaxation got in between
-                            while (got != cur) {
+                            bool won = got == cur;
+                            // retry only when another relaxation got in between;
+                            // one that is no longer better pushes nothing: entries
+                            // pushed twice are expanded by two warps at once and
+                            // would double again at every node they reach
+                            while (!won && ng[r] < st_g(got)) {
                                 cur = got;
-                                if (ng[r] >= st_g(cur)) break;
                                 got = atomicCAS(B.state + v[r], cur, st_make(ng[r], wr.u[o[r]]));
+                                won = got == cur;
                             }
-                            if (got == cur) {
+                            if (won) {
                                 first = !P.no_touch_log && st_g(cur) >= INF_G;
                                 const uint64_t fv = (uint64_t)ng[r] + hv[r];
                                 if (fv < T) to_near = true;
