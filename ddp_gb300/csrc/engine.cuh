@@ -736,11 +736,14 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                     else if (p < B.cap_q) qcur[p] = make_uint2(en.x, gu);  // (the grid walks the whole row)
                     else atomicOr(&ctl->status, ST_OVERFLOW);
                 }
-                if (sub == 0) atomicMax(&longest[(wv + 1) % 3], (unsigned int)min(len, 1 << 21));
+                if (sub == 0) {
+                    n_exp++;
+                    atomicMax(&longest[(wv + 1) % 3], (unsigned int)min(len, 1 << 21));
+                }
                 continue;
             }
             if (sub == 0) {
-                n_exp++;
+                n_exp += (int)en.w >= 0;  // (a row in segments was counted when it was cut)
                 n_scan += (unsigned long long)(r1 - (int)en.z);
             }
             for (;;) {
