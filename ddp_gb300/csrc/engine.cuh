@@ -505,9 +505,9 @@ struct SearchParams {
     // delta).  Under so weak a bound, less than an arc, the search is little
     // but rounds over buckets, and wider ones save more rounds than they
     // repeat expansions: hop bounds and none at half the weight range instead
-    // of a quarter, 250k nodes of 10 arcs 367 -> 315 us, of 4 arcs 333 -> 282,
-    // 1M points 16.5 -> 11.6 ms.  Tight bounds keep the quarter (200k points,
-    // Euclidean: 1.11 against 1.30 ms).
+    // of a quarter, 250k nodes of 10 arcs 353 -> 331 us, of 4 arcs 400 -> 312,
+    // 1M points 9.8 -> 7.2 ms.  Tight bounds keep the quarter (200k points,
+    // Euclidean: 1.01 against 1.06 ms).
     uint32_t delta_loose = 0;
     bool long_rows = true;  // A* searches on a grid: there may be rows of more than LOCAL_ROW arcs
     int64_t budget = 0;  // bidirectional search: entries it may expand (0: any number)
@@ -527,7 +527,7 @@ struct SearchResult {
 // relaxation that pushed it), eight lanes walk one row, and a phase ends with
 // a block barrier.  It hands the list back when it outgrows LOCAL_OUT entries
 // or after LOCAL_WAVES phases (the other CTAs wait in a bounded barrier).
-// While the far pile is small (LOCAL_FAR) it splits it too, and while the
+// While the far pile is small (LOCAL_FAR, LOCAL_FAR_KEEP) it splits it too, and while the
 // list is narrow (LOCAL_FILL) it takes the next bucket in early, so that the
 // floods of successive buckets overlap instead of running one after the other
 // (at most LOCAL_AHEAD buckets before the list empties; not in keep mode,
@@ -535,11 +535,15 @@ struct SearchResult {
 // A phase of a 511 x 511 maze query (20-70 entries) takes about 2.5 us so, on
 // the grid it took 23, and overlapping buckets halve their number (16, 32 or 64
 // entries alike; wider buckets instead expand nodes again and again).
-// LOCAL_FAR 1,024, 4,096, 16,384: another maze 5.37, 4.92, 4.92 ms, updates of 1M
-// nodes 202, 199, 211 us, 250,000 random nodes alike, but 200,000 points under
-// Euclidean bounds 4.9, 7.1, 7.4 ms.
+// LOCAL_FAR: one CTA takes about 20 us over a pile of 4,096 entries, a grid
+// split 4.  Single queries, 4,096, 2,048, 1,024 and 512 entries: 1M points
+// without bounds 26.8, 18.1, 14.8, 14.8 ms, 200,000 points under hop bounds
+// 3.04, 3.04, 2.63, 2.42, a 2,047 x 2,047 maze without bounds 8.8, 8.8, 6.9,
+// 7.1, a 700 x 700 one 2.04, 2.04, 2.04, 2.21, 511 x 511 and 250,000 random
+// nodes alike.  Keep mode rarely splits and then needs the far pile's minimum
+// at once: updates of 1M nodes at 1,024, 4,096, 16,384 entries 202, 199, 211 us.
 constexpr int LOCAL_IN = 256, LOCAL_OUT = 512;
-constexpr int LOCAL_FAR = 4096;
+constexpr int LOCAL_FAR = 1024, LOCAL_FAR_KEEP = 4096;
 constexpr int LOCAL_FILL = 32, LOCAL_AHEAD = 16;
 constexpr int LOCAL_WAVES = 4096;
 // Where rows may be long (SearchParams::long_rows), arcs decide too.  A row of
@@ -626,7 +630,7 @@ __device__ void local_phases(const DevGraph &G, const SlotBufs &B, const Heur &H
                     done = 1;  // no open node with f < f(t)
                     break;
                 }
-            } else if (nf > 0 && nf <= LOCAL_FAR && (m == 0 || ahead < LOCAL_AHEAD) &&
+            } else if (nf > 0 && nf <= (KEEP ? LOCAL_FAR_KEEP : LOCAL_FAR) && (m == 0 || ahead < LOCAL_AHEAD) &&
                        min(ft, sat_add(max(fm, T), P.delta)) <= cold_x) {
                 T = sat_add(max(fm, T), P.delta);  // above the smallest f: something moves
                 ahead++;
@@ -922,12 +926,12 @@ __device__ SearchResult run_search(const Grp &grp, const DevGraph &G, const Slot
     bool cold_take = false, cold_pass = false;
     if (resume && P.cold) {
         cold_take = ncold > 0 && ncold + nfar > B.cap_f / 2;
-        if (!cold_take && nfar > LOCAL_FAR) {
+        if (!cold_take && nfar > LOCAL_FAR_KEEP) {
             if (ncold == 0) cold_x = P.cold_x;
             cold_pass = cold_x != 0xFFFFFFFFu;
         }
     }
-    if (resume && !cold_take && !cold_pass && local_ok && nfar <= LOCAL_FAR) splitting = false;
+    if (resume && !cold_take && !cold_pass && local_ok && nfar <= LOCAL_FAR_KEEP) splitting = false;
     uint2 *cold_stage = reinterpret_cast<uint2 *>(wr.snr);
 
     for (;;) {
