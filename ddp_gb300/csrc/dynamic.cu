@@ -655,9 +655,9 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
         else atomicOr(&B.ctl->status, ST_OVERFLOW);
     };
     // Node p's hops were lowered from old.  If it had none, or a bound past the
-    // largest cost, the searches have passed it over until now: without a label it
-    // is re-seeded (each node once, and never one that B invalidates), with one
-    // (the source, heads of inserted arcs) it is opened again.
+    // largest cost, the searches have passed it over until now: it has no label and
+    // is re-seeded (each node once, and never one that B invalidates), or it is the
+    // source, which is opened again.
     auto lowered = [&](int p, uint32_t old, int rb, int re) {
         push(p, rb, re);
         atomicAdd(&dc->hops_lowered, 1);
@@ -816,6 +816,12 @@ __device__ void dyn_repair(const Grp &grp, const DevGraph &G, const SlotBufs &B,
         if (gu >= INF_G) continue;
         const uint64_t ng64 = (uint64_t)gu + (uint32_t)up.w;
         if (ng64 >= INF_G) continue;
+        // The searches pass over a node without hops, so a label that it got here
+        // would miss every better one: it is re-seeded when it comes within reach.
+        if (A.heur == 1) {
+            const uint32_t hv = __ldcg(hops + up.z);
+            if (hv == HOPS_INF || (unsigned long long)hv * G.wmin >= INF_G) continue;
+        }
         const uint32_t ng = (uint32_t)ng64;
         while (ng < st_g(cur)) {
             const uint64_t got = atomicCAS(B.state + up.z, cur, st_make(ng, up.y));

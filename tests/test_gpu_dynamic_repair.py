@@ -140,7 +140,7 @@ def test_queues_grow_with_the_search(gpu, oracle):
 def test_targets_that_come_within_reach(gpu, oracle, kw, extra):
     """The target cannot be reached, or only from part of the graph, when the
     search is made; inserts open ways over nodes that had no hop bound, in one
-    batch or several, some through nodes labelled before they reached it.
+    batch or several, some through heads of earlier inserts.
     extra: further inserts, so that the batch takes the host's path."""
     d = gpu
     rng = np.random.default_rng(3 + extra)
@@ -170,7 +170,7 @@ def test_targets_that_come_within_reach(gpu, oracle, kw, extra):
             assert got == (want if f_ else d.INF), (hk, got, want)
 
         at = lambda i: int(rng.integers(0, part.n)) + i * part.n  # noqa: E731
-        step([1], [at(0)], [at(1)], [3])           # heads labelled, still no way
+        step([1], [at(0)], [at(1)], [3])           # heads in reach of s, still no way
         step([1, 1], [at(2), at(1)], [at(3), at(1)], [5, 2])
         step([1], [at(1)], [at(2)], [4])           # now there is one
         step([0, 1, 1], [at(0), at(0), at(1)], [at(0), at(3), at(3)], [0, 40, 9])
@@ -204,3 +204,28 @@ def test_bounds_past_the_largest_cost(gpu, oracle):
             assert got == (want if f_ else d.INF), (light, u, got, want)
         dyn.close()
         dg.close()
+
+
+@pytest.mark.parametrize("kw", [{}, {"group": 1}, {"grid": 5}])
+def test_inserts_into_nodes_out_of_reach(gpu, oracle, kw):
+    """An arc into a node that cannot reach the target, then a shorter way to
+    that arc's tail, then an arc from the node to the target."""
+    d = gpu
+    # 0 -> 1 (100), 1 -> 2 (200); the target is 2, node 3 has no arc out, 4 .. 9 a chain after it
+    off = np.array([0, 1, 2, 2, 3, 4, 5, 6, 7, 8, 8], np.int32)
+    g = d.CSR(10, off, np.array([1, 2, 4, 5, 6, 7, 8, 9], np.int32), np.array([100, 200, 1, 1, 1, 1, 1, 1], np.uint32))
+    for hk in (d.H_BFS_HOPS, d.H_ZERO):
+        for steps in ([(1, 1, 3, 1), (2, 0, 1, 10), (1, 3, 2, 5)],
+                      [(1, 1, 3, 1), (1, 0, 3, 90), (2, 0, 1, 10), (1, 9, 2, 5)],
+                      [(1, 0, 3, 150), (2, 0, 3, 120), (1, 1, 3, 1), (2, 0, 1, 10), (1, 6, 2, 5), (0, 1, 3, 0)],
+                      [(1, 1, 3, 1), (0, 1, 3, 0), (1, 1, 3, 4), (2, 0, 1, 10), (1, 3, 2, 5)]):
+            dg = d.DeviceGraph.from_csr(g)
+            dyn = d.DynamicSearch(dg, 0, 2, hk, **kw)
+            o, c, w = g.with_sentinel().off[:-1].copy(), g.col.copy(), g.w.copy()
+            for i, st in enumerate(steps):
+                f, u, v, x = _batch([st])
+                got = dyn.update(f, u, v, x)
+                o, c, w, _ = oracle.apply_batch(len(o), o, c, w, f, u, v, x)
+                assert got == _scratch(oracle, o, c, w, 0, 2), (hk, steps, i)
+            dyn.close()
+            dg.close()
